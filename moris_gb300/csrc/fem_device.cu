@@ -1236,6 +1236,7 @@ fem_gpu_status assemble_set(fem_gpu_ctx* c, int set, const double* u, double* va
     SetData& s = c->sets[set];
     if (cluster_set(c, set))
         return cluster_launch_set(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0);
+    if (lattice_set(c, set)) return lattice_assemble(c, set, u, vals, rhs, true, true);
     if (s.kind == 0)
         return launch_bulk(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0, nullptr, nullptr);
     return launch_side(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0);
@@ -1316,6 +1317,7 @@ HostPipe* host_pipe(fem_gpu_ctx* c) {
 
 void device_release(fem_gpu_ctx* c) {
     host_pipe_release(c);
+    lattice_release(c);
     cluster_release(c);
     sensitivity_release(c);
     for (auto& s : c->sets) {
@@ -1528,6 +1530,7 @@ fem_gpu_status device_finalize(fem_gpu_ctx* c) {
             s.sidx.clear();
         }
     }
+    if ((st = lattice_finalize(c)) != FEM_GPU_OK) return st;
     e = cudaStreamSynchronize(sm);
     if (e != cudaSuccess) return cuda_fail(c, e, "finalize sync");
     c->dev_final = true;
@@ -1667,23 +1670,33 @@ fem_gpu_status fem_gpu_assemble(fem_gpu_ctx* c, const double* u, double* vals, d
         if ((st = stage_out_alloc(c, r, nad * sizeof(double), host, sr)) != FEM_GPU_OK) return st;
     }
     cudaStream_t sm = stream_of(c);
-    if (!acc) {
+    HostPipe* hp = (host && v) ? host_pipe(c) : nullptr;
+    // a lattice set stores every CSR value and residual: assembled first, it
+    // needs no zero fill, and the other sets add to it (the chunks of a host
+    // assembly are element ranges, which the lattice kernels do not have)
+    int lead = -1;
+    for (int k = 0; k < (int)c->sets.size() && lead < 0 && !hp; ++k)
+        if (lattice_set(c, k)) lead = k;
+    if (!acc && lead < 0) {
         if (sv.dev) cudaMemsetAsync(sv.dev, 0, c->nnz * sizeof(double), sm);
         if (sr.dev) cudaMemsetAsync(sr.dev, 0, nad * sizeof(double), sm);
     }
     cudaMemsetAsync(c->d_status.p, 0, sizeof(int), sm);
+    if (lead >= 0)
+        st = lattice_assemble(c, lead, (const double*)su.dev, (double*)sv.dev, (double*)sr.dev, acc, acc);
     auto run = [&](int k, int64_t first, int64_t count) {
         SetData& s = c->sets[k];
         if (cluster_set(c, k))
             return cluster_launch_set(c, k, MODE_ASSEMBLE, first, count, (const double*)su.dev, (double*)sv.dev,
                                       (double*)sr.dev, nullptr, nullptr, 0);
+        if (lead >= 0 && lattice_set(c, k))
+            return lattice_assemble(c, k, (const double*)su.dev, (double*)sv.dev, (double*)sr.dev, true, true);
         if (s.kind == 0)
             return launch_bulk(c, k, MODE_ASSEMBLE, first, count, (const double*)su.dev, (double*)sv.dev,
                                (double*)sr.dev, nullptr, nullptr, 0, nullptr, nullptr);
         return launch_side(c, k, MODE_ASSEMBLE, first, count, (const double*)su.dev, (double*)sv.dev, (double*)sr.dev,
                            nullptr, nullptr, 0);
     };
-    HostPipe* hp = (host && v) ? host_pipe(c) : nullptr;
     if (hp) {
         const int64_t nu = c->num_used;
         int64_t done_rank = 0;
@@ -1709,7 +1722,8 @@ fem_gpu_status fem_gpu_assemble(fem_gpu_ctx* c, const double* u, double* vals, d
         if (e == cudaSuccess) e = cudaStreamWaitEvent(sm, hp->done.back(), 0);
         if (e != cudaSuccess) st = cuda_fail(c, e, "assemble copy back");
     } else {
-        for (int k = 0; k < (int)c->sets.size() && st == FEM_GPU_OK; ++k) st = run(k, 0, c->sets[k].neq);
+        for (int k = 0; k < (int)c->sets.size() && st == FEM_GPU_OK; ++k)
+            if (k != lead) st = run(k, 0, c->sets[k].neq);
         if (st == FEM_GPU_OK && host) {
             cudaError_t e = cudaSuccess;
             if (v) e = cudaMemcpyAsync(v, sv.dev, c->nnz * sizeof(double), cudaMemcpyDeviceToHost, sm);
@@ -1927,13 +1941,22 @@ fem_gpu_status fem_gpu_apply(fem_gpu_ctx* c, const double* x, double* y, uint32_
     if ((st = stage_in(c, x, nad * sizeof(double), host, sx)) != FEM_GPU_OK) return st;
     if ((st = stage_out_alloc(c, y, nad * sizeof(double), host, sy)) != FEM_GPU_OK) return st;
     cudaStream_t sm = stream_of(c);
-    if (!(flags & FEM_GPU_ACCUMULATE)) cudaMemsetAsync(sy.dev, 0, nad * sizeof(double), sm);
+    int lead = -1;  // a lattice set stores every entry of y: no zero fill
+    for (int k = 0; k < (int)c->sets.size() && lead < 0; ++k)
+        if (lattice_set(c, k)) lead = k;
+    const bool acc = flags & FEM_GPU_ACCUMULATE;
+    if (!acc && lead < 0) cudaMemsetAsync(sy.dev, 0, nad * sizeof(double), sm);
+    if (lead >= 0) st = lattice_assemble(c, lead, (const double*)sx.dev, nullptr, (double*)sy.dev, false, acc);
     for (int k = 0; k < (int)c->sets.size() && st == FEM_GPU_OK; ++k) {
         SetData& s = c->sets[k];
-        if (s.neq == 0) continue;
+        if (s.neq == 0 || k == lead) continue;
         if (s.kind != 0) {
             st = fail(c, FEM_GPU_UNSUPPORTED, "matrix-free apply covers bulk sets only");
             break;
+        }
+        if (lattice_set(c, k)) {
+            st = lattice_assemble(c, k, (const double*)sx.dev, nullptr, (double*)sy.dev, false, true);
+            continue;
         }
         st = launch_bulk(c, k, MODE_APPLY, 0, s.neq, nullptr, nullptr, nullptr, nullptr, nullptr, 0,
                          (const double*)sx.dev, (double*)sy.dev);
@@ -2030,6 +2053,7 @@ fem_gpu_status fem_gpu_set_variant(fem_gpu_ctx* c, int32_t set, int32_t variant)
     if (!c || set < 0 || set >= (int32_t)c->sets.size() || variant < 0 || variant >= NUM_VARIANTS)
         return FEM_GPU_BAD_ARG;
     c->sets[set].variant = variant;
+    c->sets[set].pinned = true;
     return FEM_GPU_OK;
 }
 

@@ -89,6 +89,9 @@ struct SetData {
     int ngp = 0;            // Gauss points of the set's rule
     int nbsel = 0;          // padded basis width of the kernel instance
     int variant = 0;        // bulk kernel variant (set by fem_gpu_autotune)
+    bool pinned = false;    // variant chosen by fem_gpu_set_variant: that kernel assembles the set
+    bool lattice = false;   // the set covers a tensor lattice (fem_lattice.cu)
+    DeviceBuf d_latE, d_latrho;  // lattice sets: modulus in cell order (if the set's order differs), nodal densities
     double tuned_ms = 0.0;  // time of the chosen variant on the tuning run
 };
 
@@ -130,6 +133,7 @@ struct fem_gpu_ctx {
     bool stream_set = false;           // caller chose a stream (NULL = legacy default stream)
     fem::DeviceBuf d_rowptr, d_ulen, d_tables, d_scratch, d_status;
     void* batch = nullptr;             // batched-launch state (fem_cluster.cu)
+    void* lattice = nullptr;           // tensor-lattice data (fem_lattice.cu)
     void* host_pipe = nullptr;         // chunked assembly with overlapped copy-back (fem_device.cu)
     // IG vertex table (shape sensitivities)
     std::vector<int32_t> vkind, vpar;  // [nv], [nv][8]
@@ -171,6 +175,12 @@ double ip_cell_measure(const fem_gpu_ctx* c, int64_t cell);
 fem_gpu_status interface_volumes(fem_gpu_ctx* c);
 // one set's assembly through its kernel (fem_device.cu); vals / rhs may be NULL
 fem_gpu_status assemble_set(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs);
+// tensor lattices of brick cells (fem_lattice.cu)
+fem_gpu_status lattice_finalize(fem_gpu_ctx* c);
+void lattice_release(fem_gpu_ctx* c);
+inline bool lattice_set(const fem_gpu_ctx* c, int set) { return c->sets[set].lattice && !c->sets[set].pinned; }
+fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs, bool acc_v,
+                                bool acc_r);
 // device address of fem_gpu_pcg_noalloc's fixed array on the current device,
 // resolved once per device (fem_solver.cu); loads that file's module
 fem_gpu_status noalloc_prepare(fem_gpu_ctx* c);

@@ -1,0 +1,947 @@
+// fem_lattice.cu -- assembly on uniform tensor lattices of brick cells.
+//
+// A level-0 HMR mesh is a tensor lattice: nodes, cells and B-splines numbered
+// i-fastest, the extraction row of a node the same for every node (one basis
+// for linear splines, the eight bases around it with weight 1/8 for quadratic
+// ones).  Then sum_e T_e^T K_e T_e = T^T (sum_e K_e) T with T the node-to-basis
+// matrix of the whole mesh, and both factors are stencils:
+//
+//   lattice_const / lattice_density   the 27-point block stencil of sum_e K_e,
+//       one thread per node: every 3 x 3 block is a sum over the elements that
+//       share the node pair, gathered in a fixed order (no atomics, no zero
+//       fill, one store per value), and the nodal residual K u on the way;
+//   lattice_project   T^T S T for quadratic splines, axis by axis: 3 -> 5 taps
+//       per axis with 5 additions (the weights are powers of two, folded into
+//       the modulus), written row by row into the CSR.
+//
+// The element loop (fem_bulk_cta.cuh) spends 6,561 atomic updates on each
+// quadratic element and is bound by shared-memory latency and the L2's atomic
+// rate; here a CSR value costs about 2.5 FP64 additions and one store.  The
+// FP64 pipe (2 lanes per SM and clock on GB300) binds: 2,340 additions per
+// basis for the projection, 750 operations per node for the stencil.
+//
+// Measured on GB300 against the element loop (whole calls, residual included):
+// 64^3 quadratic 7.75 -> 2.23 ms, 15 x 13 x 11 quadratic 120 -> 86 us, 96^3
+// density set with linear splines 13.4 -> 3.56 ms, matrix-free product of 48 x
+// 47 x 45 quadratic cells 969 -> 206 us.  The stencil and projection kernels
+// keep the FP64 pipe 72-77 % busy, lattice_density 55 % (register-bound
+// occupancy).  Smaller models gain less but none was slower, so there is no
+// size limit.
+//
+// A model takes this path when lattice_finalize finds all of the above to hold
+// exactly (coordinates, numbering, weights, and a CSR whose rows are the full
+// boxes of neighbours); any other model keeps the element loop.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <string>
+#include <vector>
+
+#include "fem_bits.cuh"
+#include "fem_internal.hpp"
+
+namespace fem {
+namespace {
+
+// a stencil CTA: 32 consecutive nodes, one warp per z offset
+constexpr int kStencilNodes = 32, kStencilThreads = 3 * kStencilNodes;
+// bases of a projection tile
+constexpr int kPX = 5, kPY = 3;
+
+enum { OUT_NONE = 0, OUT_STENCIL = 1, OUT_CSR = 2 };
+
+struct LatArgs {
+    int ne[3], nn[3];
+    int64_t pitch;         // x pitch of the stencil array
+    const double* E;       // modulus per cell
+    const double* jac;     // half edge lengths [ne0], [ne1], [ne2], then their reciprocals
+    const double* rho;     // nodal densities (density sets)
+    double* Q;             // density sets: element sums [kQN][ne2 + 2][ne1 + 2][ne0 + 2], zero around the lattice
+    const double* u;       // nodal displacements [3][nodes] (nullable: zero)
+    double* r;             // nodal residual [3][nodes] (nullable)
+    double* S;             // [27][9][nn2][nn1][pitch]
+    double* vals;          // CSR values (linear splines: node = basis)
+    const int32_t* rowptr;
+    int acc_v, acc_r;      // add to vals / r instead of storing
+    int* status;
+    double coef[27][9];    // constant E: see lattice_const
+    double xq[3], wq[27];  // density: 1-D points, weights (x fastest) times mu
+    double beta, ld, lo;   // density exponent, (lam + mu) / mu, lam / mu
+};
+
+// One warp's share of a node's row: the blocks of neighbour offsets
+// (dx, dy, DZ), consumed as they are formed.
+template <int OUT, int DZ>
+struct NodeOut {
+    const LatArgs& p;
+    int x, y, z;
+    int64_t node, nodes;
+    int32_t row[3];
+    int cx, cy, cz, lx, ly, lz;  // CSR box of the node's row
+    double r[3] = {0.0, 0.0, 0.0};
+    bool live, bad = false;
+
+    __device__ NodeOut(const LatArgs& a, int64_t n) : p(a), node(n) {
+        nodes = (int64_t)p.nn[0] * p.nn[1] * p.nn[2];
+        live = node < nodes;
+        const unsigned i = live ? (unsigned)node : 0u, yz = i / (unsigned)p.nn[0];
+        x = (int)(i - yz * (unsigned)p.nn[0]);
+        z = (int)(yz / (unsigned)p.nn[1]);
+        y = (int)(yz - (unsigned)z * (unsigned)p.nn[1]);
+        if constexpr (OUT == OUT_CSR) {
+            lx = x > 0 ? -1 : 0;
+            ly = y > 0 ? -1 : 0;
+            lz = z > 0 ? -1 : 0;
+            cx = (x + 1 < p.nn[0] ? 2 : 1) - lx;
+            cy = (y + 1 < p.nn[1] ? 2 : 1) - ly;
+            cz = (z + 1 < p.nn[2] ? 2 : 1) - lz;
+            for (int f = 0; f < 3; ++f) row[f] = live ? __ldg(p.rowptr + f * nodes + node) : 0;
+        }
+    }
+    __device__ __forceinline__ void block(int dx, int dy, const double K[9]) {
+        const bool in = live && x + dx >= 0 && x + dx < p.nn[0] && y + dy >= 0 && y + dy < p.nn[1] && z + DZ >= 0 &&
+                        z + DZ < p.nn[2];
+        if (p.u && in) {
+            const int64_t j = node + dx + (int64_t)p.nn[0] * (dy + (int64_t)p.nn[1] * DZ);
+#pragma unroll
+            for (int g = 0; g < 3; ++g) {
+                const double ug = __ldg(p.u + g * nodes + j);
+#pragma unroll
+                for (int f = 0; f < 3; ++f) r[f] = fma(K[f * 3 + g], ug, r[f]);
+            }
+        }
+        if constexpr (OUT != OUT_NONE) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) bad |= !fem_finite(K[k]);
+        }
+        if constexpr (OUT == OUT_STENCIL) {
+            // blocks that leave the lattice are sums over no element: zeros the projection reads
+            const int k = (dx + 1) + 3 * (dy + 1) + 9 * (DZ + 1);
+            const int64_t plane = (int64_t)p.nn[2] * p.nn[1] * p.pitch;
+            double* s = p.S + (int64_t)k * 9 * plane + ((int64_t)z * p.nn[1] + y) * p.pitch + x;
+            if (live) {
+#pragma unroll
+                for (int c = 0; c < 9; ++c) s[c * plane] = K[c];
+            }
+        } else if (OUT == OUT_CSR && in) {
+            const int at = ((DZ - lz) * cy + (dy - ly)) * cx + (dx - lx), ul = cx * cy * cz;
+#pragma unroll
+            for (int f = 0; f < 3; ++f)
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    double* v = p.vals + row[f] + g * ul + at;
+                    *v = p.acc_v ? *v + K[f * 3 + g] : K[f * 3 + g];
+                }
+        }
+    }
+    __device__ void finish(double red[3][kStencilNodes][3]) {
+        if (bad && live) atomicOr(p.status, 1);
+        for (int f = 0; f < 3; ++f) red[DZ + 1][threadIdx.x % kStencilNodes][f] = r[f];
+    }
+};
+
+// the three warps' shares of the nodal residual, in the order of the z offsets
+__device__ __forceinline__ void store_residual(const LatArgs& p, int64_t node, const double red[3][kStencilNodes][3]) {
+    const int64_t nodes = (int64_t)p.nn[0] * p.nn[1] * p.nn[2];
+    if (!p.r || node >= nodes || threadIdx.x >= kStencilNodes) return;
+    for (int f = 0; f < 3; ++f) {
+        const double v = (red[0][threadIdx.x][f] + red[1][threadIdx.x][f]) + red[2][threadIdx.x][f];
+        double* q = p.r + f * nodes + node;
+        *q = p.acc_r ? *q + v : v;
+    }
+}
+
+// Constant modulus per element.  With detJ = J0 J1 J2 an element's block is
+//   K[(f,a),(f,b)] = sum_k w_k c_fk(a,b),  w_k = E detJ / J_k^2
+//   K[(f,a),(g,b)] = v_h H_fg(a,b),        v_h = E J_h (h the third axis)
+// and c, H factor into 1-D mass, stiffness and gradient matrices whose entries
+// depend on the node offset only, up to a sign along gradient axes: for offset
+// 0 the lower element counts + and the upper one -.  So a block needs the box
+// sums of six element weights (summed along mass and stiffness axes,
+// differenced along the two gradient axes) times the coefficients p.coef[k] =
+// {c_00..c_02 as G_kk, H_fg}: 500 FP64 operations per node against 960 for the
+// product of every shared element.
+// A thread forms the nine blocks of one z offset, so that 96 threads work on
+// 32 nodes: a small lattice still fills the SMs, and consecutive lanes are
+// consecutive nodes whatever the edge lengths (no partial tiles).
+template <int OUT, int DZ>
+__device__ __forceinline__ void const_blocks(const LatArgs& p, int64_t node, double red[3][kStencilNodes][3]) {
+    NodeOut<OUT, DZ> out(p, node);
+    // columns after the z axis: weights 0-2 and the xy pair (v_2) sum, the xz
+    // (v_1) and yz (v_0) pairs difference
+    double c[6][2][2];
+    const double* ij = p.jac + p.ne[0] + p.ne[1] + p.ne[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            double w[2][6];
+            const int ex = out.x - 1 + i, ey = out.y - 1 + j;
+            const int qx = min(max(ex, 0), p.ne[0] - 1), qy = p.ne[0] + min(max(ey, 0), p.ne[1] - 1);
+            const double j0 = __ldg(p.jac + qx), i0 = __ldg(ij + qx), j1 = __ldg(p.jac + qy), i1 = __ldg(ij + qy);
+#pragma unroll
+            for (int k = DZ > 0 ? 1 : 0; k <= (DZ < 0 ? 0 : 1); ++k) {
+                const int ez = out.z - 1 + k, qz = p.ne[0] + p.ne[1] + min(max(ez, 0), p.ne[2] - 1);
+                const double j2 = __ldg(p.jac + qz), i2 = __ldg(ij + qz);
+                const bool in =
+                    out.live && ex >= 0 && ex < p.ne[0] && ey >= 0 && ey < p.ne[1] && ez >= 0 && ez < p.ne[2];
+                const double E = in ? __ldg(p.E + ((int64_t)ez * p.ne[1] + ey) * p.ne[0] + ex) : 0.0;
+                w[k][3] = E * j0;
+                w[k][4] = E * j1;
+                w[k][5] = E * j2;
+                w[k][0] = w[k][4] * j2 * i0;
+                w[k][1] = w[k][3] * j2 * i1;
+                w[k][2] = w[k][3] * j1 * i2;
+            }
+#pragma unroll
+            for (int m = 0; m < 6; ++m)
+                c[m][j][i] = DZ < 0             ? w[0][m]
+                             : DZ > 0           ? w[1][m]
+                             : m == 3 || m == 4 ? w[0][m] - w[1][m]
+                                                : w[0][m] + w[1][m];
+        }
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy) {
+        double d[6][2];
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                d[m][i] = dy < 0             ? c[m][0][i]
+                          : dy > 0           ? c[m][1][i]
+                          : m == 3 || m == 5 ? c[m][0][i] - c[m][1][i]
+                                             : c[m][0][i] + c[m][1][i];
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
+            double s[6];
+#pragma unroll
+            for (int m = 0; m < 6; ++m)
+                s[m] = dx < 0 ? d[m][0] : dx > 0 ? d[m][1] : m == 4 || m == 5 ? d[m][0] - d[m][1] : d[m][0] + d[m][1];
+            const double* q = p.coef[(dx + 1) + 3 * (dy + 1) + 9 * (DZ + 1)];
+            const double a0 = s[0] * q[0], a1 = s[1] * q[1], a2 = s[2] * q[2], tr = a0 + a1 + a2;
+            const double K[9] = {fma(p.ld, a0, tr), s[5] * q[3],       s[4] * q[4],
+                                 s[5] * q[5],       fma(p.ld, a1, tr), s[3] * q[6],
+                                 s[4] * q[7],       s[3] * q[8],       fma(p.ld, a2, tr)};
+            out.block(dx, dy, K);
+        }
+    }
+    out.finish(red);
+}
+
+template <int OUT>
+__global__ void __launch_bounds__(kStencilThreads) lattice_const(LatArgs p) {
+    __shared__ double red[3][kStencilNodes][3];
+    const int64_t node = (int64_t)blockIdx.x * kStencilNodes + threadIdx.x % kStencilNodes;
+    const int w = threadIdx.x / kStencilNodes;
+    if (w == 0) const_blocks<OUT, -1>(p, node, red);
+    else if (w == 1) const_blocks<OUT, 0>(p, node, red);
+    else const_blocks<OUT, 1>(p, node, red);
+    __syncthreads();
+    store_residual(p, node, red);
+}
+
+// 1-D factors of the density path.  Along an axis a pair of nodes (offset d)
+// meets the lower element (side 0, d <= 0) and the upper one (side 1, d >= 0);
+// type 0: N' N' (one quadrature sum), 1: N N (three sums, of (1+x)^2, (1-x)^2
+// and 1-x^2), 2: N' N (row differentiated) and 3: N N' (two sums, of 1+x and
+// 1-x); each element contributes one of the sums with a sign.
+__device__ constexpr int ax_n(int d) { return d == 0 ? 2 : 1; }
+__device__ constexpr int ax_side(int d, int i) { return d == 0 ? i : d < 0 ? 0 : 1; }
+__device__ constexpr int ax_var(int type, int d, int i) {
+    return type == 0   ? 0
+           : type == 1 ? (d == 0 ? i : 2)
+           : type == 2 ? (d == 0 ? i : d < 0 ? 1 : 0)
+                       : (d == 0 ? i : d < 0 ? 0 : 1);
+}
+__device__ constexpr bool ax_neg(int type, int d, int i) {
+    return type == 0   ? d != 0
+           : type == 1 ? false
+           : type == 2 ? (d == 0 ? i == 1 : d > 0)
+                       : (d == 0 ? i == 1 : d < 0);
+}
+__device__ constexpr int ax_vars(int type) { return type == 0 ? 1 : type == 1 ? 3 : 2; }
+
+// sums of an element: {xx, yy, zz, xy, xz, yz} at these offsets, the variants
+// of the axes in x, y, z order (z fastest)
+constexpr int kXX = 0, kYY = 9, kZZ = 18, kXY = 27, kXZ = 39, kYZ = 51, kQN = 63;
+
+// block entry of a node from the sums of its elements; q: the sums of the
+// lower element along every axis, qs / ey / ez: strides of a sum, an element
+// row and an element layer
+template <int TX, int TY, int TZ, int DZ>
+__device__ __forceinline__ double gather(const double* __restrict__ q, int64_t qs, int64_t ey, int64_t ez, int off,
+                                         int dx, int dy) {
+    double s = 0.0;
+    bool first = true;
+#pragma unroll
+    for (int k = 0; k < ax_n(DZ); ++k)
+#pragma unroll
+        for (int j = 0; j < ax_n(dy); ++j)
+#pragma unroll
+            for (int i = 0; i < ax_n(dx); ++i) {
+                const int at = off + (ax_var(TX, dx, i) * ax_vars(TY) + ax_var(TY, dy, j)) * ax_vars(TZ) +
+                               ax_var(TZ, DZ, k);
+                const double v = __ldg(q + at * qs + ax_side(DZ, k) * ez + ax_side(dy, j) * ey + ax_side(dx, i));
+                const bool neg = ax_neg(TX, dx, i) ^ ax_neg(TY, dy, j) ^ ax_neg(TZ, DZ, k);
+                s = first ? (neg ? -v : v) : neg ? s - v : s + v;
+                first = false;
+            }
+    return s;
+}
+
+// Density sets: E(x_q) = E rho(x_q)^beta at N^3 tensor Gauss points.  A brick's
+// gradients factor per axis, so its 300 Gram entries are signed copies of 63
+// sums over the points (1-D factors above), formed axis by axis: 300 FMAs
+// instead of 300 N^3.  One thread per element writes them (504 bytes, read back
+// from L2 and L1 by the eight nodes around it); staging them per node tile in
+// shared memory instead recomputed 1.76 elements per node and left a quarter of
+// the lanes on partial tiles.
+template <int N>
+__global__ void __launch_bounds__(128) lattice_moments(LatArgs p) {
+    const unsigned cells = (unsigned)p.ne[0] * p.ne[1] * p.ne[2];
+    const int64_t qy = p.ne[0] + 2, qz = qy * (p.ne[1] + 2), qs = qz * (p.ne[2] + 2);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < cells; t += gridDim.x * blockDim.x) {
+        const int ex = (int)(t % p.ne[0]), yz = (int)(t / p.ne[0]), ey = yz % p.ne[1], ez = yz / p.ne[1];
+        double* q = p.Q + (ez + 1) * qz + (ey + 1) * qy + ex + 1;
+        const double E = p.E[((int64_t)ez * p.ne[1] + ey) * p.ne[0] + ex];
+        double W[N][N][N];  // [z][y][x]
+        {
+            // densities at the points, interpolated axis by axis
+            const int64_t n0 = ((int64_t)ez * p.nn[1] + ey) * p.nn[0] + ex;
+            double c[2][2][N];
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const double* r = p.rho + n0 + (int64_t)p.nn[0] * (j + (int64_t)p.nn[1] * k);
+                    const double m = 0.5 * (r[0] + r[1]), d = 0.5 * (r[1] - r[0]);
+#pragma unroll
+                    for (int i = 0; i < N; ++i) c[k][j][i] = fma(p.xq[i], d, m);
+                }
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    double l[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+                        l[k] = fma(p.xq[j], 0.5 * (c[k][1][i] - c[k][0][i]), 0.5 * (c[k][0][i] + c[k][1][i]));
+                    const double m = 0.5 * (l[0] + l[1]), d = 0.5 * (l[1] - l[0]);
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                        const double r = fma(p.xq[k], d, m);
+                        W[k][j][i] = p.wq[(k * N + j) * N + i] * E * (p.beta == 3.0 ? r * r * r : pow(r, p.beta));
+                    }
+                }
+        }
+        // 1-D coefficients: [axis][variant][point], with the axis' Jacobian factor
+        // (1/J for N' N', J for N N, 1 for N' N)
+        const double J[3] = {__ldg(p.jac + ex), __ldg(p.jac + p.ne[0] + ey), __ldg(p.jac + p.ne[0] + p.ne[1] + ez)};
+        double iJ[3], M[3][3][N], G[2][N];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            iJ[a] = 1.0 / J[a];
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const double x = p.xq[i];
+                M[a][0][i] = J[a] * ((1.0 + x) * (1.0 + x));
+                M[a][1][i] = J[a] * ((1.0 - x) * (1.0 - x));
+                M[a][2][i] = J[a] * ((1.0 + x) * (1.0 - x));
+                G[0][i] = 1.0 + x;
+                G[1][i] = 1.0 - x;
+            }
+        }
+        auto dot = [](const double* v, const double* w) {
+            double s = v[0] * w[0];
+#pragma unroll
+            for (int i = 1; i < N; ++i) s = fma(v[i], w[i], s);
+            return s;
+        };
+        auto sum = [](const double* v, double f) {
+            double s = v[0];
+#pragma unroll
+            for (int i = 1; i < N; ++i) s += v[i];
+            return s * f;
+        };
+        // x variants: 0 = N' N', 1-3 = N N, 4-5 = N' N
+#pragma unroll
+        for (int vx = 0; vx < 6; ++vx) {
+            double X[N][N];  // [z][y]
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+#pragma unroll
+                for (int j = 0; j < N; ++j)
+                    X[k][j] = vx == 0  ? sum(W[k][j], iJ[0])
+                              : vx < 4 ? dot(W[k][j], M[0][vx - 1])
+                                       : dot(W[k][j], G[vx - 4]);
+            double Y[N];
+            if (vx > 0 && vx < 4) {  // yy: y differentiated
+#pragma unroll
+                for (int k = 0; k < N; ++k) Y[k] = sum(X[k], iJ[1]);
+#pragma unroll
+                for (int vz = 0; vz < 3; ++vz) q[(kYY + (vx - 1) * 3 + vz) * qs] = dot(Y, M[2][vz]);
+            }
+#pragma unroll
+            for (int vy = 0; vy < 3; ++vy) {
+#pragma unroll
+                for (int k = 0; k < N; ++k) Y[k] = dot(X[k], M[1][vy]);
+                if (vx == 0) {
+#pragma unroll
+                    for (int vz = 0; vz < 3; ++vz) q[(kXX + vy * 3 + vz) * qs] = dot(Y, M[2][vz]);
+                } else if (vx < 4) {
+                    q[(kZZ + (vx - 1) * 3 + vy) * qs] = sum(Y, iJ[2]);
+                } else {
+#pragma unroll
+                    for (int vz = 0; vz < 2; ++vz) q[(kXZ + ((vx - 4) * 3 + vy) * 2 + vz) * qs] = dot(Y, G[vz]);
+                }
+            }
+            if (vx > 0) {
+#pragma unroll
+                for (int vy = 0; vy < 2; ++vy) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) Y[k] = dot(X[k], G[vy]);
+                    if (vx < 4) {
+#pragma unroll
+                        for (int vz = 0; vz < 2; ++vz) q[(kYZ + ((vx - 1) * 2 + vy) * 2 + vz) * qs] = dot(Y, G[vz]);
+                    } else {
+#pragma unroll
+                        for (int vz = 0; vz < 3; ++vz) q[(kXY + ((vx - 4) * 2 + vy) * 3 + vz) * qs] = dot(Y, M[2][vz]);
+                    }
+                }
+            }
+        }
+    }
+}
+
+template <int OUT, int DZ>
+__device__ __forceinline__ void density_blocks(const LatArgs& p, int64_t node, double red[3][kStencilNodes][3]) {
+    NodeOut<OUT, DZ> out(p, node);
+    const int64_t ey = p.ne[0] + 2, ez = ey * (p.ne[1] + 2), qs = ez * (p.ne[2] + 2);
+    const double* q = p.Q + out.z * ez + out.y * ey + out.x;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
+            const double a0 = gather<0, 1, 1, DZ>(q, qs, ey, ez, kXX, dx, dy),
+                         a1 = gather<1, 0, 1, DZ>(q, qs, ey, ez, kYY, dx, dy),
+                         a2 = gather<1, 1, 0, DZ>(q, qs, ey, ez, kZZ, dx, dy), tr = a0 + a1 + a2;
+            const double xy = gather<2, 3, 1, DZ>(q, qs, ey, ez, kXY, dx, dy),
+                         yx = gather<3, 2, 1, DZ>(q, qs, ey, ez, kXY, dx, dy),
+                         xz = gather<2, 1, 3, DZ>(q, qs, ey, ez, kXZ, dx, dy),
+                         zx = gather<3, 1, 2, DZ>(q, qs, ey, ez, kXZ, dx, dy),
+                         yz = gather<1, 2, 3, DZ>(q, qs, ey, ez, kYZ, dx, dy),
+                         zy = gather<1, 3, 2, DZ>(q, qs, ey, ez, kYZ, dx, dy);
+            // K_fg = lam A_fg + mu A_gf (+ mu tr A), mu inside the weights
+            const double K[9] = {fma(p.ld, a0, tr), fma(p.lo, xy, yx), fma(p.lo, xz, zx),
+                                 fma(p.lo, yx, xy), fma(p.ld, a1, tr), fma(p.lo, yz, zy),
+                                 fma(p.lo, zx, xz), fma(p.lo, zy, yz), fma(p.ld, a2, tr)};
+            out.block(dx, dy, K);
+        }
+    out.finish(red);
+}
+
+template <int OUT>
+__global__ void __launch_bounds__(kStencilThreads, 4) lattice_density(LatArgs p) {
+    __shared__ double red[3][kStencilNodes][3];
+    const int64_t node = (int64_t)blockIdx.x * kStencilNodes + threadIdx.x % kStencilNodes;
+    const int w = threadIdx.x / kStencilNodes;
+    if (w == 0) density_blocks<OUT, -1>(p, node, red);
+    else if (w == 1) density_blocks<OUT, 0>(p, node, red);
+    else density_blocks<OUT, 1>(p, node, red);
+    __syncthreads();
+    store_residual(p, node, red);
+}
+
+// A = T^T S T for quadratic splines (basis b covers the nodes b-1 and b along
+// every axis; the weights are inside S).  Along one axis, with the row sums
+// r(-2) = s_-(-1), r(-1) = s_-(0) + s(-1), r(0) = s_-(1) + s(0), r(1) = s(1) of
+// the stencils s_- and s of nodes b-1 and b, the basis stencil is A(D) =
+// r(D-1) + r(D): 5 additions for 5 taps, 2,340 per basis with the tile's halo.
+// A CTA takes 5 x 3 bases and one row component and marches along z, one node
+// plane per step: x stage from global memory (every stencil value is read once
+// per tile), y stage, then the z stage on registers: thread (g, Dy, Dx) keeps
+// the three z taps of the previous plane for five of the columns and writes the
+// five z offsets of every row straight into the CSR, 25 consecutive values per
+// (row, g, Dz).  48 KB and 80 registers, three CTAs per SM (two with 118
+// registers and no spill: 2 % slower at 64^3), 225 of 256 threads in the y and z
+// stages.  A first version that looped over Dz with all nine components and
+// staged the values for the copy took 3.3 ms at 64^3 (FP64 pipe 49 % busy, 47
+// instructions per FP64 one, most of them index arithmetic).
+struct ProjArgs {
+    int nn[3], nb[3];
+    int tx, ty, chunks;
+    int64_t pitch;
+    const double* S;
+    double* vals;
+    const int32_t* rowptr;
+    int acc;
+    int* status;
+};
+constexpr int kProjThreads = 256, kProjCtas = 3;
+constexpr int kXLen = (kPY + 1) * kPX * 135, kXYLen = kPY * kPX * 225;
+constexpr size_t kProjSmem = (size_t)(kXLen + kXYLen) * sizeof(double);
+
+__global__ void __launch_bounds__(kProjThreads, kProjCtas) lattice_project(ProjArgs p) {
+    extern __shared__ double sm[];
+    double* X = sm;            // [iy][ix][Dx][ky][kz][g]
+    double* XY = sm + kXLen;   // [iy][ix][kz][g][Dy][Dx]
+    const int tid = threadIdx.x;
+    const int f = blockIdx.x % 3, tile = blockIdx.x / 3, bx = tile % p.tx, by = tile / p.tx;
+    // tiles and z ranges of nearly equal size
+    const int x0 = (int)((int64_t)p.nb[0] * bx / p.tx), wx = (int)((int64_t)p.nb[0] * (bx + 1) / p.tx) - x0;
+    const int y0 = (int)((int64_t)p.nb[1] * by / p.ty), wy = (int)((int64_t)p.nb[1] * (by + 1) / p.ty) - y0;
+    const int z0 = (int)((int64_t)p.nb[2] * blockIdx.y / p.chunks);
+    const int z1 = (int)((int64_t)p.nb[2] * (blockIdx.y + 1) / p.chunks);
+    const int64_t plane = (int64_t)p.nn[2] * p.nn[1] * p.pitch, layer = (int64_t)p.nn[1] * p.pitch;
+    const int64_t nb01 = (int64_t)p.nb[0] * p.nb[1], nu = nb01 * p.nb[2];
+    // x stage: line (ky, kz, g) of node row iy
+    const int xl = tid % 27, xiy = tid / 27, xg = xl % 3, xkz = xl / 3 % 3, xky = xl / 9, xrow = y0 - 1 + xiy;
+    const bool xlive = xiy <= wy && xrow >= 0 && xrow < p.nn[1];
+    const double* xs = p.S + (int64_t)((xkz * 3 + xky) * 27 + f * 3 + xg) * plane +
+                       (int64_t)(xlive ? xrow : 0) * p.pitch + x0 - 1;
+    unsigned xin = 0;  // nodes x0 - 1 + i of the row that exist
+    for (int i = 0; i <= wx; ++i)
+        if (xlive && x0 - 1 + i >= 0 && x0 - 1 + i < p.nn[0]) xin |= 1u << i;
+    // y stage: line (Dx, kz, g) of base column ix
+    const int yix = tid / 45, yl = tid % 45, yd = yl / 9, yk = yl % 9;
+    // z stage: (g, Dy, Dx), columns zc, zc + 3, ...
+    const int zl = tid % 75, zc = tid / 75, zg = zl / 25, zdy = zl % 25 / 5 - 2, zdx = zl % 5 - 2;
+    double m[5][3];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) m[k][0] = m[k][1] = m[k][2] = 0.0;
+    // per column its index and the in-plane box of its row: lengths cx, cy and
+    // the column's own place ox, oy (cx = 0: no such column).  In shared memory:
+    // as registers they and their products, hoisted out of the z loop, spill
+    __shared__ int cidx[kPX * kPY], cbox[kPX * kPY];
+    if (tid < kPX * kPY) {
+        const int ix = tid % kPX, iy = tid / kPX, gx = x0 + ix, gy = y0 + iy;
+        const int ox = min(gx, 2), oy = min(gy, 2);
+        const int cx = ix < wx && iy < wy ? min(gx + 2, p.nb[0] - 1) - (gx - ox) + 1 : 0;
+        const int cy = min(gy + 2, p.nb[1] - 1) - (gy - oy) + 1;
+        cidx[tid] = gy * p.nb[0] + gx;
+        cbox[tid] = cx | cy << 8 | ox << 16 | oy << 24;
+    }
+    __syncthreads();
+    bool bad = false;
+    for (int z = z0 - 1; z < z1; ++z) {  // node plane z; basis layer z from z0 on
+        const bool have = z >= 0 && z < p.nn[2];
+        if (have) {
+            if (xiy <= wy) {
+                double v[kPX + 1][3];
+                const double* s0 = xs + z * layer;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+#pragma unroll
+                    for (int i = 0; i <= kPX; ++i) v[i][k] = xin >> i & 1 ? __ldg(s0 + i) : 0.0;
+                    s0 += 9 * plane;
+                }
+                double* o = X + xiy * kPX * 135 + xl;
+#pragma unroll
+                for (int i = 0; i < kPX; ++i)
+                    if (i < wx) {
+                        const double ra = v[i][1] + v[i + 1][0], rb = v[i][2] + v[i + 1][1];
+                        o[i * 135] = v[i][0];
+                        o[i * 135 + 27] = v[i][0] + ra;
+                        o[i * 135 + 54] = ra + rb;
+                        o[i * 135 + 81] = rb + v[i + 1][2];
+                        o[i * 135 + 108] = v[i + 1][2];
+                    }
+            }
+            __syncthreads();
+            if (yix < wx) {
+                const double* q = X + yix * 135 + yd * 27 + yk;
+                double m0 = q[0], m1 = q[9], m2 = q[18];
+                double* o = XY + yix * 225 + yk * 25 + yd;
+                for (int i = 0; i < wy; ++i) {
+                    q += kPX * 135;
+                    const double s0 = q[0], s1 = q[9], s2 = q[18];
+                    const double ra = m1 + s0, rb = m2 + s1;
+                    o[0] = m0;
+                    o[5] = m0 + ra;
+                    o[10] = ra + rb;
+                    o[15] = rb + s2;
+                    o[20] = s2;
+                    o += kPX * 225;
+                    m0 = s0;
+                    m1 = s1;
+                    m2 = s2;
+                }
+            }
+            __syncthreads();
+        }
+        if (zc < 3) {
+            const int lz = max(z - 2, 0), cz = min(z + 2, p.nb[2] - 1) - lz + 1;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const int c = zc + 3 * k, box = cbox[c];
+                const double* q = XY + c * 225 + zl;
+                const double s[3] = {have ? q[0] : 0.0, have ? q[75] : 0.0, have ? q[150] : 0.0};
+                const int cx = box & 255, cy = box >> 8 & 255, ax = (box >> 16 & 255) + zdx, ay = (box >> 24) + zdy;
+                if (z >= z0 && ax >= 0 && ax < cx && ay >= 0 && ay < cy) {
+                    const double ra = m[k][1] + s[0], rb = m[k][2] + s[1];
+                    const double v[5] = {m[k][0], m[k][0] + ra, ra + rb, rb + s[2], s[2]};
+                    const int cxy = cx * cy;
+                    double* w = p.vals + __ldg(p.rowptr + f * nu + z * nb01 + cidx[c]) + ay * cx + ax +
+                                (zg * cz - lz + z - 2) * cxy;
+#pragma unroll
+                    for (int D = -2; D <= 2; ++D) {
+                        if (z + D >= 0 && z + D < p.nb[2]) {
+                            bad |= !fem_finite(v[D + 2]);
+                            *w = p.acc ? *w + v[D + 2] : v[D + 2];
+                        }
+                        w += cxy;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) m[k][i] = s[i];
+            }
+        }
+    }
+    if (bad) atomicOr(p.status, 1);
+}
+
+// nodal values of a quadratic spline field: un[g][node] = 1/8 of the sum of its eight bases
+__global__ void lattice_nodal(int n0, int n1, int n2, const double* __restrict__ u, double* __restrict__ un) {
+    const int64_t nodes = (int64_t)n0 * n1 * n2, nu = (int64_t)(n0 + 1) * (n1 + 1) * (n2 + 1);
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nodes;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const int g = (int)(t / nodes);
+        const int64_t i = t - g * nodes;
+        const int x = (int)(i % n0), y = (int)(i / n0 % n1), z = (int)(i / ((int64_t)n0 * n1));
+        const double* b = u + g * nu + ((int64_t)z * (n1 + 1) + y) * (n0 + 1) + x;
+        const int64_t sy = n0 + 1, sz = sy * (n1 + 1);
+        const double lo = (b[0] + b[1]) + (b[sy] + b[sy + 1]);
+        const double up = (b[sz] + b[sz + 1]) + (b[sz + sy] + b[sz + sy + 1]);
+        un[t] = 0.125 * (lo + up);
+    }
+}
+
+// r[f][basis] (+)= scale * the sum of rn over the basis' eight nodes
+__global__ void lattice_restrict(int n0, int n1, int n2, const double* __restrict__ rn, double scale, int acc,
+                                 double* __restrict__ r) {
+    const int b0 = n0 + 1, b1 = n1 + 1, b2 = n2 + 1;
+    const int64_t nodes = (int64_t)n0 * n1 * n2, nu = (int64_t)b0 * b1 * b2;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nu; t += (int64_t)gridDim.x * blockDim.x) {
+        const int f = (int)(t / nu);
+        const int64_t i = t - f * nu;
+        const int x = (int)(i % b0), y = (int)(i / b0 % b1), z = (int)(i / ((int64_t)b0 * b1));
+        double s = 0.0;
+        for (int k = max(z - 1, 0); k <= min(z, n2 - 1); ++k)
+            for (int j = max(y - 1, 0); j <= min(y, n1 - 1); ++j)
+                for (int l = max(x - 1, 0); l <= min(x, n0 - 1); ++l)
+                    s += rn[f * nodes + ((int64_t)k * n1 + j) * n0 + l];
+        r[t] = acc ? fma(scale, s, r[t]) : scale * s;
+    }
+}
+
+struct Lattice {
+    int p = 0;
+    int ne[3], nn[3], nb[3];
+    int64_t pitch = 0;
+    DeviceBuf jac;     // half edge lengths and their reciprocals
+    DeviceBuf S, vec;  // quadratic splines: stencil, nodal vectors
+    DeviceBuf Q;       // density sets: element sums
+};
+
+void dfree(DeviceBuf& b) {
+    if (b.p) cudaFree(b.p);
+    b.p = nullptr;
+    b.bytes = 0;
+}
+
+template <class T>
+cudaError_t upload(DeviceBuf& b, const std::vector<T>& v, cudaStream_t st) {
+    dfree(b);
+    b.bytes = std::max<size_t>(v.size() * sizeof(T), 16);
+    cudaError_t e = cudaMalloc(&b.p, b.bytes);
+    if (e == cudaSuccess && !v.empty())
+        e = cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
+    return e;
+}
+
+// the lattice of a mesh, or nothing where any of its properties does not hold exactly
+bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
+    if (c->dim != 3 || c->shape != FEM_GPU_SHAPE_RECTANGULAR || c->num_used != c->num_bases) return false;
+    const double* X = c->coords.data();
+    const int64_t N = c->num_nodes;
+    int64_t n0 = 1, n1 = 1;
+    while (n0 < N && X[n0 * 3 + 1] == X[1] && X[n0 * 3 + 2] == X[2]) ++n0;
+    while (n1 * n0 < N && X[n1 * n0 * 3 + 2] == X[2]) ++n1;
+    if (N % (n0 * n1)) return false;
+    const int64_t n2 = N / (n0 * n1), nn[3] = {n0, n1, n2};
+    const int64_t step[3] = {1, n0, n0 * n1};
+    const int64_t width = c->t_off[1];
+    if (width != 1 && width != 8) return false;
+    L.p = width == 1 ? 1 : 2;
+    int64_t cells = 1, bases = 1;
+    for (int d = 0; d < 3; ++d) {
+        if (nn[d] < 2 || nn[d] > 1 << 20) return false;
+        L.nn[d] = (int)nn[d];
+        L.ne[d] = (int)nn[d] - 1;
+        L.nb[d] = L.ne[d] + L.p;
+        cells *= L.ne[d];
+        bases *= L.nb[d];
+        for (int e = 0; e < L.ne[d]; ++e) {
+            jac.push_back(0.5 * (X[(e + 1) * step[d] * 3 + d] - X[e * step[d] * 3 + d]));
+            if (!(jac.back() > 0.0)) return false;
+        }
+    }
+    if (c->num_cells != cells || c->num_bases != bases) return false;
+    const double w = L.p == 1 ? 1.0 : 0.125;
+    for (int64_t n = 0, k = 0; n < N; ++n) {
+        const int64_t i[3] = {n % n0, n / n0 % n1, n / (n0 * n1)};
+        for (int d = 0; d < 3; ++d)
+            if (X[n * 3 + d] != X[i[d] * step[d] * 3 + d]) return false;
+        if (c->t_off[n + 1] - c->t_off[n] != width) return false;
+        for (int q = 0; q < width; ++q, ++k) {
+            const int64_t b = ((i[2] + (q >> 2)) * L.nb[1] + i[1] + (q >> 1 & 1)) * L.nb[0] + i[0] + (q & 1);
+            if (c->t_bases[k] != b || c->t_w[k] != w) return false;
+        }
+    }
+    static const int corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
+                                     {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
+    for (int64_t e = 0; e < cells; ++e) {
+        const int64_t i = e % L.ne[0], j = e / L.ne[0] % L.ne[1], k = e / ((int64_t)L.ne[0] * L.ne[1]);
+        for (int a = 0; a < 8; ++a)
+            if (c->cells[e * 8 + a] != ((k + corner[a][2]) * n1 + j + corner[a][1]) * n0 + i + corner[a][0])
+                return false;
+    }
+    // CSR rows: the full box of bases within p along every axis (the bulk set
+    // puts the box into every row, so equal lengths are equal rows)
+    for (int64_t b = 0; b < bases; ++b) {
+        const int64_t i[3] = {b % L.nb[0], b / L.nb[0] % L.nb[1], b / ((int64_t)L.nb[0] * L.nb[1])};
+        int64_t len = 1;
+        for (int d = 0; d < 3; ++d)
+            len *= std::min<int64_t>(i[d] + L.p, L.nb[d] - 1) - std::max<int64_t>(i[d] - L.p, 0) + 1;
+        if (c->ulen[b] != len) return false;
+    }
+    L.pitch = (L.nn[0] + 3) / 4 * 4;
+    for (size_t k = 0, n = jac.size(); k < n; ++k) jac.push_back(1.0 / jac[k]);
+    return true;
+}
+
+}  // namespace
+
+void lattice_release(fem_gpu_ctx* c);
+
+// Finds out whether the model is a lattice and which of its bulk sets cover
+// every cell exactly once; those are assembled here (SetData::lattice).
+fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
+    Lattice L;
+    std::vector<double> jac;
+    cudaStream_t st = (cudaStream_t)c->stream;
+    bool any = false;
+    for (const SetData& s : c->sets) any |= s.kind == 0 && s.ig_off.empty() && s.neq == c->num_cells;
+    if (!any || !find_lattice(c, L, jac)) return FEM_GPU_OK;
+    cudaError_t e = cudaSuccess;
+    any = false;
+    for (SetData& s : c->sets) {
+        if (s.kind != 0 || !s.ig_off.empty() || s.neq != c->num_cells) continue;
+        const int rule = s.bulk.integration_rule;
+        if (rule != FEM_GPU_RULE_HEX_2x2x2 && rule != FEM_GPU_RULE_HEX_3x3x3) continue;
+        std::vector<char> seen(c->num_cells, 0);
+        bool once = true, ordered = true;
+        for (int64_t i = 0; i < s.neq; ++i) {
+            once &= !seen[s.ip_cell[i]];
+            seen[s.ip_cell[i]] = 1;
+            ordered &= s.ip_cell[i] == i;
+        }
+        if (!once) continue;
+        if (!ordered && e == cudaSuccess) {
+            std::vector<double> E(s.neq);
+            for (int64_t i = 0; i < s.neq; ++i) E[s.ip_cell[i]] = s.E[i];
+            e = upload(s.d_latE, E, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        }
+        if (!s.node_rho.empty() && e == cudaSuccess) e = upload(s.d_latrho, s.node_rho, st);
+        s.lattice = any = true;
+    }
+    if (!any) return FEM_GPU_OK;
+    auto* K = new Lattice(L);
+    c->lattice = K;
+    if (e == cudaSuccess) e = upload(K->jac, jac, st);
+    // workspaces (quadratic splines: 243 doubles and six nodal values per node,
+    // 0.22 of the CSR values; density sets: 63 doubles per cell, 0.26 of them for
+    // linear splines); a device that cannot hold them keeps the element loop
+    bool rho = false;
+    for (const SetData& s : c->sets) rho |= s.lattice && !s.node_rho.empty();
+    const size_t want[3] = {K->p == 2 ? (size_t)243 * L.nn[2] * L.nn[1] * L.pitch : 0,
+                            K->p == 2 ? (size_t)6 * c->num_nodes : 0,
+                            rho ? (size_t)kQN * (L.ne[0] + 2) * (L.ne[1] + 2) * (L.ne[2] + 2) : 0};
+    DeviceBuf* const buf[3] = {&K->S, &K->vec, &K->Q};
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
+        if (!want[k]) continue;
+        buf[k]->bytes = want[k] * sizeof(double);
+        if (cudaMalloc(&buf[k]->p, buf[k]->bytes) != cudaSuccess) {
+            cudaGetLastError();
+            buf[k]->p = nullptr;
+            cudaStreamSynchronize(st);
+            lattice_release(c);
+            return FEM_GPU_OK;
+        }
+    }
+    if (rho && e == cudaSuccess) e = cudaMemsetAsync(K->Q.p, 0, K->Q.bytes, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    return e == cudaSuccess ? FEM_GPU_OK
+                            : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice data: ") + cudaGetErrorString(e));
+}
+
+void lattice_release(fem_gpu_ctx* c) {
+    for (SetData& s : c->sets) {
+        dfree(s.d_latE);
+        dfree(s.d_latrho);
+        s.lattice = false;
+    }
+    Lattice* L = (Lattice*)c->lattice;
+    if (!L) return;
+    dfree(L->jac);
+    dfree(L->S);
+    dfree(L->vec);
+    dfree(L->Q);
+    delete L;
+    c->lattice = nullptr;
+}
+
+// One lattice set: CSR values (nullable) and residual (nullable) of the adof
+// vector u (nullable), stored, or added with acc_v / acc_r.
+fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs, bool acc_v,
+                                bool acc_r) {
+    Lattice& L = *(Lattice*)c->lattice;
+    const SetData& s = c->sets[set];
+    cudaStream_t st = (cudaStream_t)c->stream;
+    const int64_t nodes = (int64_t)L.nn[0] * L.nn[1] * L.nn[2];
+    const bool quad = L.p == 2;
+    cudaError_t e = cudaSuccess;
+    LatArgs a{};
+    for (int d = 0; d < 3; ++d) {
+        a.ne[d] = L.ne[d];
+        a.nn[d] = L.nn[d];
+    }
+    a.pitch = L.pitch;
+    a.E = (const double*)(s.d_latE.p ? s.d_latE.p : s.d_E.p);
+    a.jac = (const double*)L.jac.p;
+    a.rho = s.node_rho.empty() ? nullptr : (const double*)s.d_latrho.p;
+    a.rowptr = (const int32_t*)c->d_rowptr.p;
+    a.status = (int*)c->d_status.p;
+    a.vals = vals;
+    a.S = (double*)L.S.p;
+    a.Q = (double*)L.Q.p;
+    double* un = (double*)L.vec.p;
+    double* rn = un + 3 * nodes;
+    const bool want_u = u && rhs;
+    a.u = want_u ? (quad ? un : u) : nullptr;
+    a.r = rhs ? (quad ? rn : rhs) : nullptr;
+    a.acc_v = acc_v;
+    a.acc_r = quad ? 0 : acc_r;
+    // material and rule: T^T S T with T = P / 8 is P^T (S / 64) P (exact powers of two)
+    const double nu = s.bulk.poisson_ratio, scale = quad ? 1.0 / 64.0 : 1.0;
+    const double lam = nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), mu = 1.0 / (2.0 * (1.0 + nu));
+    a.ld = (lam + mu) / mu;
+    a.lo = lam / mu;
+    a.beta = s.bulk.density_exponent;
+    const Rule r = gauss_rule(s.bulk.integration_rule);
+    const int N = r.n == 8 ? 2 : 3;
+    for (int i = 0; i < N; ++i) a.xq[i] = N == 2 ? (i ? -r.pts[0] : r.pts[0]) : (i - 1) * -r.pts[0];
+    // the rule's points to tensor order, weights with the material factor and the 1/64 of the shape functions
+    for (int q = 0; q < r.n; ++q) {
+        int at = 0, mul = 1;
+        for (int d = 0; d < 3; ++d, mul *= N) {
+            const double x = r.pts[q * 3 + d];
+            at += mul * (N == 2 ? x > 0.0 : x < 0.0 ? 0 : x > 0.0 ? 2 : 1);
+        }
+        a.wq[at] = r.w[q] * mu * scale / 64.0;
+    }
+    if (!a.rho) {
+        // coefficients of every offset: the reference sums for the element and
+        // nodes that lattice_const counts with a plus sign
+        for (int k = 0; k < 27; ++k) {
+            const int d[3] = {k % 3 - 1, k / 3 % 3 - 1, k / 9 - 1};
+            double sa[3], sb[3];  // corner signs of the row node and its neighbour in that element
+            for (int i = 0; i < 3; ++i) {
+                sa[i] = d[i] > 0 ? -1.0 : 1.0;
+                sb[i] = d[i] < 0 ? -1.0 : 1.0;
+            }
+            double G[3][3] = {};
+            for (int q = 0; q < N * N * N; ++q) {
+                const double x[3] = {a.xq[q % N], a.xq[q / N % N], a.xq[q / (N * N)]};
+                double ga[3], gb[3];
+                for (int i = 0; i < 3; ++i) {
+                    ga[i] = sa[i];
+                    gb[i] = sb[i];
+                    for (int o = 0; o < 3; ++o)
+                        if (o != i) {
+                            ga[i] *= 1.0 + sa[o] * x[o];
+                            gb[i] *= 1.0 + sb[o] * x[o];
+                        }
+                }
+                for (int i = 0; i < 3; ++i)
+                    for (int j = 0; j < 3; ++j) G[i][j] += a.wq[q] * ga[i] * gb[j];
+            }
+            double* o = a.coef[k];
+            for (int i = 0; i < 3; ++i) o[i] = G[i][i];
+            int m = 3;
+            static const int fg[6][2] = {{0, 1}, {0, 2}, {1, 0}, {1, 2}, {2, 0}, {2, 1}};
+            for (const auto& q : fg) o[m++] = a.lo * G[q[0]][q[1]] + G[q[1]][q[0]];
+        }
+    }
+    const unsigned grid3 = (unsigned)sm_count() * 16;
+    if (quad && want_u) {
+        lattice_nodal<<<(unsigned)std::min<int64_t>((3 * nodes + 255) / 256, grid3), 256, 0, st>>>(
+            L.nn[0], L.nn[1], L.nn[2], u, un);
+        c->launches++;
+    }
+    const unsigned ctas = (unsigned)((nodes + kStencilNodes - 1) / kStencilNodes);
+    const int out = !vals ? OUT_NONE : quad ? OUT_STENCIL : OUT_CSR;
+    using Fn = void (*)(LatArgs);
+    const Fn fn[2][3] = {{lattice_const<0>, lattice_const<1>, lattice_const<2>},
+                         {lattice_density<0>, lattice_density<1>, lattice_density<2>}};
+    if (a.rho) {
+        const unsigned g = (unsigned)std::min<int64_t>((c->num_cells + 127) / 128, (int64_t)sm_count() * 64);
+        if (N == 2) lattice_moments<2><<<g, 128, 0, st>>>(a);
+        else lattice_moments<3><<<g, 128, 0, st>>>(a);
+        c->launches++;
+    }
+    fn[a.rho != nullptr][out]<<<ctas, kStencilThreads, 0, st>>>(a);
+    c->launches++;
+    if (quad && vals && e == cudaSuccess) {
+        ProjArgs q{};
+        for (int d = 0; d < 3; ++d) {
+            q.nn[d] = L.nn[d];
+            q.nb[d] = L.nb[d];
+        }
+        q.tx = (L.nb[0] + kPX - 1) / kPX;
+        q.ty = (L.nb[1] + kPY - 1) / kPY;
+        q.pitch = L.pitch;
+        q.S = a.S;
+        q.vals = vals;
+        q.rowptr = a.rowptr;
+        q.acc = acc_v;
+        q.status = a.status;
+        // z ranges: every range repeats one node plane, and the CTAs should fill
+        // whole waves; the count with the fewest plane steps in sequence
+        const int64_t tiles = (int64_t)q.tx * q.ty * 3, slots = (int64_t)sm_count() * kProjCtas;
+        int64_t best = INT64_MAX;
+        for (int n = 1; n <= q.nb[2]; ++n) {
+            const int64_t steps = (tiles * n + slots - 1) / slots * ((q.nb[2] + n - 1) / n + 1);
+            if (steps < best) {
+                best = steps;
+                q.chunks = n;
+            }
+        }
+        e = cudaFuncSetAttribute(lattice_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmem);
+        if (e == cudaSuccess)
+            lattice_project<<<dim3((unsigned)tiles, (unsigned)q.chunks), kProjThreads, kProjSmem, st>>>(q);
+        c->launches++;
+    }
+    if (quad && rhs && e == cudaSuccess) {
+        lattice_restrict<<<(unsigned)std::min<int64_t>((3 * (c->num_used) + 255) / 256, grid3), 256, 0, st>>>(
+            L.nn[0], L.nn[1], L.nn[2], rn, 8.0, acc_r, rhs);
+        c->launches++;
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return e == cudaSuccess ? FEM_GPU_OK
+                            : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice launch: ") + cudaGetErrorString(e));
+}
+
+}  // namespace fem
