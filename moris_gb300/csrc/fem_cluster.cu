@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "fem_bits.cuh"
+#include "fem_brick.cuh"
 #include "fem_internal.hpp"
 #include "fem_shape.hpp"
 
@@ -1048,6 +1049,8 @@ struct Batch {
     cudaGraphExec_t exec = nullptr;
     const void *gu = nullptr, *gv = nullptr, *gr = nullptr;
     int nside = 0;
+    int nbrick = 0;  // sets with equation objects for the brick kernels
+    bool gzero = false;
 };
 
 void dfree(DeviceBuf& b) {
@@ -1127,9 +1130,10 @@ int64_t points_of(const SetData& s, int64_t e) {
     return (s.ig_off[e + 1] - s.ig_off[e]) * s.ngp;
 }
 
-void add_items(const SetData& s, int set, int64_t first, int64_t count, int split, std::vector<Item>& items,
-               std::vector<double>& cost) {
+void add_items(const SetData& s, int set, int64_t first, int64_t count, int split, bool skip_fast,
+               std::vector<Item>& items, std::vector<double>& cost) {
     for (int64_t e = first; e < first + count; ++e) {
+        if (skip_fast && !s.fast.empty() && s.fast[e]) continue;
         const int64_t np = points_of(s, e);
         if (s.kind == 2 || split <= 0 || np <= split) {
             items.push_back({set, 0, (int32_t)np, 0, e});
@@ -1200,14 +1204,21 @@ fem_gpu_status build_batch(fem_gpu_ctx* c, Batch* b) {
     std::vector<Item> items, warp_items;
     std::vector<double> cost;
     int nb = 0;
-    b->nside = 0;
+    b->nside = b->nbrick = 0;
     for (size_t k = 0; k < c->sets.size(); ++k) {
-        const SetData& s = c->sets[k];
+        SetData& s = c->sets[k];
         if (s.neq == 0) continue;
         if (s.kind == 1) {
             b->nside++;
             continue;
         }
+        if (s.lattice && s.fast.empty()) {
+            // cells of a plain lattice are classified when a batch first needs them
+            brick_classify(c, s);
+            const fem_gpu_status r = brick_upload(c, s);
+            if (r != FEM_GPU_OK) return r;
+        }
+        if (!s.fast.empty()) b->nbrick++;
         const int w = s.kind == 2 ? s.maxnb : s.nbsel;
         if (nb && w != nb) return fail(c, FEM_GPU_UNSUPPORTED, "batched launch needs one basis width for all sets");
         nb = w;
@@ -1215,10 +1226,11 @@ fem_gpu_status build_batch(fem_gpu_ctx* c, Batch* b) {
         if (!devs[k].gp) return fail(c, FEM_GPU_NOT_FINALIZED, "set rule tables");
         if (s.kind == 0 && !devs[k].cut && devs[k].rect && devs[k].g0) {
             // uncut rectangular cells: the warp phase, in mesh order
-            for (int64_t e = 0; e < s.neq; ++e) warp_items.push_back({(int32_t)k, 0, s.ngp, 0, e});
+            for (int64_t e = 0; e < s.neq; ++e)
+                if (s.fast.empty() || !s.fast[e]) warp_items.push_back({(int32_t)k, 0, s.ngp, 0, e});
             continue;
         }
-        add_items(s, (int)k, 0, s.neq, b->split, items, cost);
+        add_items(s, (int)k, 0, s.neq, b->split, true, items, cost);
     }
     if (!nb && items.empty() && warp_items.empty()) nb = 8;  // every volume set empty: the launch finds no items
     if (nb != 8 && nb != 27) return fail(c, FEM_GPU_UNSUPPORTED, "batched launch: basis width must be 8 or 27");
@@ -1249,20 +1261,25 @@ fem_gpu_status enqueue_batch(fem_gpu_ctx* c, Batch* b, const double* u, double* 
         if (vals) cudaMemsetAsync(vals, 0, c->nnz * sizeof(double), st);
         if (rhs) cudaMemsetAsync(rhs, 0, nad * sizeof(double), st);
     }
-    cudaMemsetAsync(b->counter.p, 0, 2 * sizeof(unsigned long long), st);
-    Kernel k;
-    if (!pick_kernel(b->nb, b->warps, k)) return fail(c, FEM_GPU_UNSUPPORTED, "no cluster kernel instance");
-    ClusterArgs a = base_args(c);
-    a.sets = (const SetDev*)b->sets.p;
-    a.items = (const Item*)b->items.p;
-    a.nitems = b->nitems;
-    a.nwarp_items = b->nwarp;
-    a.counter = (unsigned long long*)b->counter.p;
-    a.u = u;
-    a.vals = vals;
-    a.rhs = rhs;
-    a.mode = CM_ASSEMBLE;
-    fem_gpu_status r = launch(c, k, a, st);
+    fem_gpu_status r = FEM_GPU_OK;
+    if (b->nitems + b->nwarp > 0) {
+        cudaMemsetAsync(b->counter.p, 0, 2 * sizeof(unsigned long long), st);
+        Kernel k;
+        if (!pick_kernel(b->nb, b->warps, k)) return fail(c, FEM_GPU_UNSUPPORTED, "no cluster kernel instance");
+        ClusterArgs a = base_args(c);
+        a.sets = (const SetDev*)b->sets.p;
+        a.items = (const Item*)b->items.p;
+        a.nitems = b->nitems;
+        a.nwarp_items = b->nwarp;
+        a.counter = (unsigned long long*)b->counter.p;
+        a.u = u;
+        a.vals = vals;
+        a.rhs = rhs;
+        a.mode = CM_ASSEMBLE;
+        r = launch(c, k, a, st);
+    }
+    for (size_t s = 0; s < c->sets.size() && r == FEM_GPU_OK; ++s)
+        r = brick_launch(c, c->sets[s], 0, c->sets[s].neq, u, vals, rhs, st);
     for (size_t s = 0; s < c->sets.size() && r == FEM_GPU_OK; ++s)
         if (c->sets[s].kind == 1 && c->sets[s].neq > 0) r = side(c, (int)s, u, vals, rhs, st);
     return r;
@@ -1291,6 +1308,7 @@ fem_gpu_status cluster_finalize(fem_gpu_ctx* c, int set) {
     s.ngp = r.n;
     // repack to the kernel width W (the host arrays are already in that layout
     // when the set's basis width is W)
+    brick_classify(c, s);
     const bool same = W == s.maxnb;
     std::vector<int32_t> bases(same ? 0 : (size_t)s.neq * sides * W, -1);
     std::vector<double> T(same ? 0 : (size_t)s.neq * sides * 8 * W, 0.0);
@@ -1339,7 +1357,7 @@ fem_gpu_status cluster_finalize(fem_gpu_ctx* c, int set) {
     s.T.shrink_to_fit();
     s.sidx.clear();
     s.sidx.shrink_to_fit();
-    return FEM_GPU_OK;
+    return brick_upload(c, s);
 }
 
 void cluster_release(fem_gpu_ctx* c) {
@@ -1353,6 +1371,7 @@ void cluster_release(fem_gpu_ctx* c) {
         dfree(s.d_fcxf);
         dfree(s.d_EF);
         dfree(s.d_vol);
+        brick_release(s);
     }
     if (c->batch) {
         Batch* b = (Batch*)c->batch;
@@ -1372,11 +1391,16 @@ fem_gpu_status cluster_launch_set(fem_gpu_ctx* c, int set, int mode, int64_t fir
     if (count <= 0) return FEM_GPU_OK;
     const SetData& s = c->sets[set];
     cudaStream_t st = (cudaStream_t)c->stream;
+    // element outputs come from the general kernel
+    if (mode != 1) {
+        const fem_gpu_status r = brick_launch(c, s, first, count, u, vals, rhs, st);
+        if (r != FEM_GPU_OK || brick_count(s, first, count) == count) return r;
+    }
     SetDev d;
     if (!set_dev(c, s, d)) return fail(c, FEM_GPU_UNSUPPORTED, "set not supported by the cluster kernel");
     std::vector<Item> items;
     std::vector<double> cost;
-    add_items(s, 0, first, count, mode == 1 ? 0 : 64, items, cost);
+    add_items(s, 0, first, count, mode == 1 ? 0 : 64, mode != 1, items, cost);
     Kernel k;
     if (!pick_kernel(s.nbsel, 4, k)) return fail(c, FEM_GPU_UNSUPPORTED, "no cluster kernel instance");
     void* dsets = nullptr;
@@ -1446,7 +1470,7 @@ fem_gpu_status fem_gpu_assemble_batched(fem_gpu_ctx* c, const double* u, double*
     fem_gpu_status st;
     if (!b->built && (st = build_batch(c, b)) != FEM_GPU_OK) return st;
     const bool zero = !(flags & FEM_GPU_ACCUMULATE);
-    if (b->exec && (b->gu != u || b->gv != v || b->gr != r)) drop_graph(b);
+    if (b->exec && (b->gu != u || b->gv != v || b->gr != r || b->gzero != zero)) drop_graph(b);
     if (!b->exec) {
         if (!b->cap) {
             cudaError_t e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
@@ -1473,10 +1497,11 @@ fem_gpu_status fem_gpu_assemble_batched(fem_gpu_ctx* c, const double* u, double*
         b->gu = u;
         b->gv = v;
         b->gr = r;
+        b->gzero = zero;
     }
     cudaError_t e = cudaGraphLaunch(b->exec, (cudaStream_t)c->stream);
     if (e != cudaSuccess) return cfail(c, e, "graph launch");
-    c->launches += 1 + b->nside;
+    c->launches += (b->nitems + b->nwarp > 0) + b->nbrick + b->nside;
     if (flags & FEM_GPU_ASYNC) return FEM_GPU_OK;
     return fem_gpu_check_status(c);
 }

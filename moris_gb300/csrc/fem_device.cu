@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "fem_bits.cuh"
+#include "fem_brick.cuh"
 #include "fem_internal.hpp"
 #include "fem_shape.hpp"
 
@@ -1232,11 +1233,20 @@ int sm_count() {
 }
 
 
+// a range of uncut cells that is all bricks with linear splines: the warp kernel
+// of fem_brick.cu (quadratic cells assemble faster in bulk_cta_kernel)
+static bool brick_range(const fem_gpu_ctx* c, int set, int64_t first, int64_t count) {
+    const SetData& s = c->sets[set];
+    return s.kind == 0 && s.ig_off.empty() && !s.pinned && s.maxnb == 8 && count > 0 &&
+           brick_count(s, first, count) == count;
+}
+
 fem_gpu_status assemble_set(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs) {
     SetData& s = c->sets[set];
     if (cluster_set(c, set))
         return cluster_launch_set(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0);
     if (lattice_set(c, set)) return lattice_assemble(c, set, u, vals, rhs, true, true);
+    if (brick_range(c, set, 0, s.neq)) return brick_launch(c, s, 0, s.neq, u, vals, rhs, c->stream);
     if (s.kind == 0)
         return launch_bulk(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0, nullptr, nullptr);
     return launch_side(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0);
@@ -1531,6 +1541,12 @@ fem_gpu_status device_finalize(fem_gpu_ctx* c) {
         }
     }
     if ((st = lattice_finalize(c)) != FEM_GPU_OK) return st;
+    for (size_t k = 0; k < c->sets.size(); ++k) {
+        SetData& s = c->sets[k];
+        if (s.kind != 0 || !s.ig_off.empty() || s.lattice) continue;
+        brick_classify(c, s);
+        if ((st = brick_upload(c, s)) != FEM_GPU_OK) return st;
+    }
     e = cudaStreamSynchronize(sm);
     if (e != cudaSuccess) return cuda_fail(c, e, "finalize sync");
     c->dev_final = true;
@@ -1691,6 +1707,8 @@ fem_gpu_status fem_gpu_assemble(fem_gpu_ctx* c, const double* u, double* vals, d
                                       (double*)sr.dev, nullptr, nullptr, 0);
         if (lead >= 0 && lattice_set(c, k))
             return lattice_assemble(c, k, (const double*)su.dev, (double*)sv.dev, (double*)sr.dev, true, true);
+        if (brick_range(c, k, first, count))
+            return brick_launch(c, s, first, count, (const double*)su.dev, (double*)sv.dev, (double*)sr.dev, c->stream);
         if (s.kind == 0)
             return launch_bulk(c, k, MODE_ASSEMBLE, first, count, (const double*)su.dev, (double*)sv.dev,
                                (double*)sr.dev, nullptr, nullptr, 0, nullptr, nullptr);
