@@ -81,9 +81,8 @@ struct SetData {
     DeviceBuf d_igoff, d_igx, d_igxi;            // cut clusters: integration cells
     DeviceBuf d_adjul;      // cut clusters: pdof values of u and lambda per cluster, cluster of each cell (sensitivities)
     DeviceBuf d_items;      // interface clusters: volume items (e * 2 + side, cell) of the sensitivities
-    DeviceBuf d_tperm;      // cut clusters: integration cells grouped by their number of moving vertices
-    int64_t tperm_off[5] = {0, 0, 0, 0, 0};  // group of cells with m moving vertices: [off[m-1], off[m]), m = 1..4
-    int64_t nitems = 0;
+    DeviceBuf d_moving;     // cut clusters: integration cells with a moving vertex (sensitivities)
+    int64_t nitems = 0, nmoving = 0;
     DeviceBuf d_fcoff, d_fcx, d_fcxl, d_fcxf;    // double-sided: facets
     DeviceBuf d_EF, d_vol;
     int ngp = 0;            // Gauss points of the set's rule
@@ -148,6 +147,7 @@ struct fem_gpu_ctx {
     fem::DeviceBuf d_vval;             // vertex values (phi at background parents)
     bool ls_phi = false;               // d_vval holds the current table's values
     fem::DeviceBuf d_lscols, d_lst;    // level-set field: coefficient ids and weights [nodes][width]
+    fem::DeviceBuf d_lsw;              // node weights of the chain to the coefficients
     int64_t ls_nbn = 0, ls_ncoef = 0;  // field sizes (0 nodes: none)
     int32_t ls_width = 0;
     int64_t ls_checked_nbn = -1;       // vertex parents checked against this many background nodes

@@ -10,10 +10,11 @@
 // FEM/INT/src/IWG/cl_FEM_IWG.cpp:2997-3154, plus the cluster-measure terms
 // :3827-3924) and contracts with the adjoint in Interpolation_Element::
 // compute_dQIdp_explicit_implicit (FEM/INT/src/ELEM/cl_FEM_Interpolation_
-// Element.cpp:820-948).  Here the derivative is exact: every integration
-// cell (TET4) and interface facet (TRI3) is evaluated once in forward-mode
-// dual arithmetic with one derivative slot per vertex, and the contraction
-// with u and lambda happens inside the kernel:
+// Element.cpp:820-948).  Here the derivative is exact and taken in reverse:
+// per integration cell (TET4) and interface facet (TRI3) the integrand and its
+// spatial gradient at every point, from which the derivative by each vertex is
+// a sum over the points; the contraction with u and lambda happens inside the
+// kernel:
 //
 //   tet     F = sum_q w detJ (1/2 sigma(u):eps(u) - sigma(u):eps(lambda))
 //   facet   -lambda^T R_interface = -( w_L A + w_F B + gamma C ),
@@ -34,72 +35,6 @@
 
 namespace fem {
 namespace {
-
-template <int M>
-struct Dual {
-    double v;
-    double d[M];
-    __device__ Dual() {}
-    __device__ explicit Dual(double x) : v(x) {
-        for (int i = 0; i < M; ++i) d[i] = 0.0;
-    }
-};
-template <int M>
-__device__ __forceinline__ Dual<M> operator+(const Dual<M>& a, const Dual<M>& b) {
-    Dual<M> r;
-    r.v = a.v + b.v;
-    for (int i = 0; i < M; ++i) r.d[i] = a.d[i] + b.d[i];
-    return r;
-}
-template <int M>
-__device__ __forceinline__ Dual<M> operator-(const Dual<M>& a, const Dual<M>& b) {
-    Dual<M> r;
-    r.v = a.v - b.v;
-    for (int i = 0; i < M; ++i) r.d[i] = a.d[i] - b.d[i];
-    return r;
-}
-template <int M>
-__device__ __forceinline__ Dual<M> operator*(const Dual<M>& a, const Dual<M>& b) {
-    Dual<M> r;
-    r.v = a.v * b.v;
-    for (int i = 0; i < M; ++i) r.d[i] = fma(a.d[i], b.v, a.v * b.d[i]);
-    return r;
-}
-template <int M>
-__device__ __forceinline__ Dual<M> operator*(double s, const Dual<M>& a) {
-    Dual<M> r;
-    r.v = s * a.v;
-    for (int i = 0; i < M; ++i) r.d[i] = s * a.d[i];
-    return r;
-}
-template <int M>
-__device__ __forceinline__ Dual<M> operator+(double s, const Dual<M>& a) {
-    Dual<M> r = a;
-    r.v += s;
-    return r;
-}
-template <int M>
-__device__ __forceinline__ Dual<M> dsqrt(const Dual<M>& a) {
-    Dual<M> r;
-    r.v = sqrt(a.v);
-    const double h = a.v > 0.0 ? 0.5 / r.v : 0.0;
-    for (int i = 0; i < M; ++i) r.d[i] = h * a.d[i];
-    return r;
-}
-template <int M>
-__device__ __forceinline__ Dual<M> dinv(const Dual<M>& a) {
-    Dual<M> r;
-    r.v = 1.0 / a.v;
-    const double h = -r.v * r.v;
-    for (int i = 0; i < M; ++i) r.d[i] = h * a.d[i];
-    return r;
-}
-// a += s * b (s constant)
-template <int M>
-__device__ __forceinline__ void axpy(double s, const Dual<M>& b, Dual<M>& a) {
-    a.v = fma(s, b.v, a.v);
-    for (int i = 0; i < M; ++i) a.d[i] = fma(s, b.d[i], a.d[i]);
-}
 
 // A trilinear field of a rectangular HEX8 cell (nodal values f_a, shape
 // functions N_a = (1 + s_x xi)(1 + s_y eta)(1 + s_z zeta) / 8) written as a
@@ -131,40 +66,51 @@ __device__ double monomial_coefficient(const double* f, const double* X, int r) 
     return c / den;
 }
 
-// a0 + a1 p + a2 q + a3 r (constant coefficients)
-template <int M>
-__device__ __forceinline__ Dual<M> lin3(double a0, double a1, const Dual<M>& p, double a2, const Dual<M>& q, double a3,
-                                        const Dual<M>& r) {
-    Dual<M> o;
-    o.v = fma(a3, r.v, fma(a2, q.v, fma(a1, p.v, a0)));
-    for (int i = 0; i < M; ++i) o.d[i] = fma(a3, r.d[i], fma(a2, q.d[i], a1 * p.d[i]));
-    return o;
+// One component of such a field at the offsets x (pr = xy, yz, xz): gradient
+// g[d] and mixed second derivatives h = (xy, yz, xz); the pure ones vanish.
+__device__ __forceinline__ void mono_grad(const double* __restrict__ c, const double x[3], const double pr[3],
+                                          double g[3], double h[3]) {
+    const double c1 = c[1], c2 = c[2], c3 = c[3], c4 = c[4], c5 = c[5], c6 = c[6], c7 = c[7];
+    g[0] = fma(c7, pr[1], fma(c6, x[2], fma(c4, x[1], c1)));
+    g[1] = fma(c7, pr[2], fma(c5, x[2], fma(c4, x[0], c2)));
+    g[2] = fma(c7, pr[0], fma(c5, x[1], fma(c6, x[0], c3)));
+    h[0] = fma(c7, x[2], c4);
+    h[1] = fma(c7, x[0], c5);
+    h[2] = fma(c7, x[1], c6);
+}
+// its value, given g[0]: k0 + k2 y + k3 z + k5 yz + x df/dx
+__device__ __forceinline__ double mono_value(const double* __restrict__ c, const double x[3], const double pr[3],
+                                             double g0) {
+    return fma(x[0], g0, fma(c[5], pr[1], fma(c[3], x[2], fma(c[2], x[1], c[0]))));
 }
 
-// gradient grad[comp][d] (and with VAL the value) of a field in monomial form
-// k[comp * 8 + m] at the offsets x[3]; pr = {xy, yz, xz}
-template <int M, bool VAL>
-__device__ __forceinline__ void mono_field(const double* __restrict__ k, const Dual<M> x[3], const Dual<M> pr[3],
-                                           Dual<M> val[3], Dual<M> grad[3][3]) {
-    for (int fl = 0; fl < 3; ++fl) {
-        const double* c = k + fl * 8;
-        grad[fl][0] = lin3(c[1], c[4], x[1], c[6], x[2], c[7], pr[1]);
-        grad[fl][1] = lin3(c[2], c[4], x[0], c[5], x[2], c[7], pr[2]);
-        grad[fl][2] = lin3(c[3], c[6], x[0], c[5], x[1], c[7], pr[0]);
-        // k0 + k2 y + k3 z + k5 yz + x df/dx
-        if (VAL) val[fl] = lin3(c[0], c[2], x[1], c[3], x[2], c[5], pr[1]) + x[0] * grad[fl][0];
+// sigma = lam tr(G) I + mu (G + G^T) of a displacement gradient G[f][i] = du_f/dx_i,
+// as xx, yy, zz, xy, yz, xz
+__device__ __forceinline__ void stress(const double G[3][3], double lam, double mu, double S[6]) {
+    const double tr = lam * (G[0][0] + G[1][1] + G[2][2]), m2 = 2.0 * mu;
+    for (int i = 0; i < 3; ++i) S[i] = fma(m2, G[i][i], tr);
+    S[3] = mu * (G[0][1] + G[1][0]);
+    S[4] = mu * (G[1][2] + G[2][1]);
+    S[5] = mu * (G[0][2] + G[2][0]);
+}
+__device__ constexpr int sym(int i, int j) { return i == j ? i : i + j == 1 ? 3 : i + j == 3 ? 4 : 5; }
+
+// o[d] += sum_fj W_fj dG_fj/dx_d with a symmetric W and dG_fj/dx_d = h_f(j, d) (0 for j = d)
+__device__ __forceinline__ void push_gradient(const double W[6], const double H[3][3], double o[3]) {
+    for (int f = 0; f < 3; ++f) {
+        const double w0 = W[sym(f, 0)], w1 = W[sym(f, 1)], w2 = W[sym(f, 2)];
+        o[0] = fma(w1, H[f][0], fma(w2, H[f][2], o[0]));
+        o[1] = fma(w0, H[f][0], fma(w2, H[f][1], o[1]));
+        o[2] = fma(w0, H[f][2], fma(w1, H[f][1], o[2]));
     }
 }
-
-// sigma = lam tr(G) I + mu (G + G^T) of a displacement gradient G[f][i] = du_f/dx_i
-template <int M>
-__device__ void stress(const Dual<M> G[3][3], double lam, double mu, Dual<M> S[3][3]) {
-    const Dual<M> tr = G[0][0] + G[1][1] + G[2][2];
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) {
-            S[i][j] = mu * (G[i][j] + G[j][i]);
-            if (i == j) axpy(lam, tr, S[i][j]);
-        }
+__device__ __forceinline__ void cross(const double a[3], const double b[3], double c[3]) {
+    c[0] = a[1] * b[2] - a[2] * b[1];
+    c[1] = a[2] * b[0] - a[0] * b[2];
+    c[2] = a[0] * b[1] - a[1] * b[0];
+}
+__device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
+    return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0]));
 }
 
 struct AdjArgs {
@@ -209,44 +155,50 @@ __device__ void pdof_values(const double* T, const int32_t* bases, int nb, int W
     }
 }
 
-// vertex position as a dual in slot `slot` (intersection vertices move with t)
-template <int M>
-__device__ void vertex_dual(const AdjArgs& A, int32_t v, int slot, Dual<M> x[3], bool& moving) {
-    moving = A.vkind[v] == 3;
+// position of a vertex, and (moving vertices: intersections) dx/dt; returns whether it moves
+__device__ __forceinline__ bool vertex(const AdjArgs& A, int32_t v, double x[3], double dx[3]) {
+    const bool moving = A.vkind[v] == 3;
+    const int32_t p0 = moving ? A.vpar[(int64_t)v * 8] : v, p1 = moving ? A.vpar[(int64_t)v * 8 + 1] : v;
     for (int d = 0; d < 3; ++d) {
-        x[d] = Dual<M>(A.vx[(int64_t)v * 3 + d]);
-        if (moving) {
-            const int32_t p0 = A.vpar[(int64_t)v * 8], p1 = A.vpar[(int64_t)v * 8 + 1];
-            const double dx = A.vx[(int64_t)p1 * 3 + d] - A.vx[(int64_t)p0 * 3 + d];
-            // slot chosen at run time: a select per slot keeps the dual in registers
-#pragma unroll
-            for (int i = 0; i < M; ++i) x[d].d[i] = i == slot ? dx : x[d].d[i];
-        }
+        x[d] = A.vx[(int64_t)v * 3 + d];
+        dx[d] = A.vx[(int64_t)p1 * 3 + d] - A.vx[(int64_t)p0 * 3 + d];
     }
+    return moving;
 }
 
-template <int M>
-__device__ Dual<M> tet_volume(const Dual<M> X[4][3]) {
-    Dual<M> a[3], b[3], c[3];
+// signed volume of a TET4 (vertices X, edges from vertex 2) and its gradient by every vertex
+__device__ __forceinline__ double tet_volume(const double X[4][3], double dV[4][3]) {
+    double a[3], b[3], c[3];
     for (int d = 0; d < 3; ++d) {
         a[d] = X[0][d] - X[2][d];
         b[d] = X[1][d] - X[2][d];
         c[d] = X[3][d] - X[2][d];
     }
-    const Dual<M> det = a[0] * (b[1] * c[2] - c[1] * b[2]) - a[1] * (b[0] * c[2] - b[2] * c[0]) +
-                        a[2] * (b[0] * c[1] - b[1] * c[0]);
-    return (1.0 / 6.0) * det;
+    cross(b, c, dV[0]);
+    cross(c, a, dV[1]);
+    cross(a, b, dV[3]);
+    const double v = dot3(a, dV[0]);
+    for (int d = 0; d < 3; ++d) {
+        for (int k : {0, 1, 3}) dV[k][d] *= 1.0 / 6.0;
+        dV[2][d] = -(dV[0][d] + dV[1][d] + dV[3][d]);
+    }
+    return v * (1.0 / 6.0);
 }
 
-// Cut clusters: F = sum_q w detJ (1/2 sigma(u):eps(u) - sigma(u):eps(lambda))
-// over every integration cell in forward-mode dual arithmetic with one slot
-// per tet vertex, dF/dt added to G of the moving vertices.  One thread per
-// integration cell of the whole set: the cells of a cluster (1 to about 100)
-// rarely fill whole warps, and on this GPU
-// an FP64 warp instruction costs the pipe the same however few of its lanes
-// are active.  The cluster's pdof values u and lambda are gathered once per
-// cluster first (adjoint_cluster_values), which also writes every cell's
-// cluster index.
+// Cut clusters: F = detJ Phi, Phi = sum_q w phi(x_q), phi = 1/2 sigma(u):eps(u) -
+// sigma(u):eps(lambda), over every integration cell.  Then
+//   dF/dX_k = Phi ddetJ/dX_k + detJ sum_q w N_k(q) grad phi(x_q),
+// added along dx/dt to G of the moving vertices.  The gradient of phi costs 60
+// FMAs on top of the 110 of phi, whatever the number of moving vertices, where
+// dual numbers multiplied the whole integrand by 1 + that number.  One thread
+// per integration cell with a moving vertex (listed in `cells`): the cells of a
+// cluster (1 to about 100) rarely fill whole warps, and on this GPU an FP64 warp
+// instruction costs the pipe the same however few of its lanes are active.  (A
+// lane per point, summed by shuffles, was slower: the FP64 pipe binds, not the
+// number of warps.)  The cluster's field polynomials are formed once per cluster
+// first (adjoint_cluster_values), which also writes every cell's cluster index.
+// Measured, 156 k moving cells (44^3): 700 -> 260 us with six CTAs per SM (168
+// registers; at 246 registers and four CTAs 274 us).
 __global__ void adjoint_cluster_values(AdjArgs A, CutSetDev S, double* UL /*[neq][48]*/, int32_t* cell_cluster) {
     const int64_t e = blockIdx.x;
     if (e >= S.neq) return;
@@ -260,62 +212,60 @@ __global__ void adjoint_cluster_values(AdjArgs A, CutSetDev S, double* UL /*[neq
         UL[e * 48 + r] = monomial_coefficient(nod + (r / 24) * 24, S.xe + e * 24, r % 24);
 }
 
-// Cells with exactly M moving vertices (listed in `cells`): the moving
-// vertices take derivative slots 0..M-1 in vertex order; cells without a
-// moving vertex contribute nothing and are not listed.
-template <int M>
-__global__ void adjoint_tets_flat(AdjArgs A, CutSetDev S, const double* __restrict__ UL,
-                                  const int32_t* __restrict__ cell_cluster, const int32_t* __restrict__ cells,
-                                  int64_t ncells) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ncells;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t g = cells[i];
-        const int64_t e = cell_cluster[g];
-        const double* X = S.xe + e * 24;
-        const double* U = UL + e * 48;
-        const double* L = U + 24;
-        const double xc[3] = {0.5 * (X[18] + X[0]), 0.5 * (X[19] + X[1]), 0.5 * (X[20] + X[2])};
-        const double lam = S.E[e] * S.lam_c, mu = S.E[e] * S.mu_c;
-        Dual<M> Xv[4][3], xo[4][3];  // vertices, their offsets from the cell centre
-        bool mv[4];
-        int32_t vids[4];
-        int slot[4], next = 0;
-        for (int k = 0; k < 4; ++k) {
-            vids[k] = S.vid[g * 4 + k];
-            slot[k] = A.vkind[vids[k]] == 3 ? next++ : -1;
-            vertex_dual<M>(A, vids[k], slot[k], Xv[k], mv[k]);
-            for (int d = 0; d < 3; ++d) xo[k][d] = (-xc[d]) + Xv[k][d];
-        }
-        const Dual<M> detJ = tet_volume<M>(Xv);
-        Dual<M> F(0.0);
-        for (int q = 0; q < S.ngp; ++q) {
-            const double z0 = S.gp[q * 3], z1 = S.gp[q * 3 + 1], z2 = S.gp[q * 3 + 2];
-            const double Nt[4] = {z0, z1, 1.0 - z0 - z1 - z2, z2};
-            Dual<M> xq[3];
-            for (int d = 0; d < 3; ++d) {
-                xq[d] = Dual<M>(0.0);
-                for (int k = 0; k < 4; ++k) axpy(Nt[k], xo[k][d], xq[d]);
-            }
-            const Dual<M> pr[3] = {xq[0] * xq[1], xq[1] * xq[2], xq[0] * xq[2]};
-            Dual<M> Gu[3][3], Gl[3][3], Su[3][3];
-            mono_field<M, false>(U, xq, pr, nullptr, Gu);
-            mono_field<M, false>(L, xq, pr, nullptr, Gl);
-            stress<M>(Gu, lam, mu, Su);
-            Dual<M> phi(0.0);
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j) phi = phi + Su[i][j] * (0.5 * Gu[i][j] + (-1.0) * Gl[i][j]);
-            // skipped points (detJ < -1e-6) contribute nothing (cl_FEM_Element_Bulk.cpp:164)
-            if (detJ.v < -1.0e-6) continue;
-            axpy(S.gw[q], detJ * phi, F);
-        }
-        for (int k = 0; k < 4; ++k)
-            if (mv[k]) {
-                double dk = 0.0;
-#pragma unroll
-                for (int i2 = 0; i2 < M; ++i2) dk = i2 == slot[k] ? F.d[i2] : dk;
-                atomicAdd(A.G + vids[k], dk);
-            }
+__global__ void __launch_bounds__(64, 6) adjoint_tets(AdjArgs A, CutSetDev S, const double* __restrict__ UL,
+                                                   const int32_t* __restrict__ cell_cluster,
+                                                   const int32_t* __restrict__ cells, int64_t ncells) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ncells) return;
+    const int64_t g = cells[i], e = cell_cluster[g];
+    const double* X = S.xe + e * 24;
+    const double* U = UL + e * 48;
+    const double lam = S.E[e] * S.lam_c, mu = S.E[e] * S.mu_c;
+    double Xv[4][3], R[4][3] = {};  // vertex offsets from the cell centre
+    for (int d = 0; d < 3; ++d) {
+        const double xc = 0.5 * (X[18 + d] + X[d]);
+        for (int k = 0; k < 4; ++k) Xv[k][d] = A.vx[(int64_t)S.vid[g * 4 + k] * 3 + d] - xc;
     }
+    double Phi = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < S.ngp; ++q) {
+        asm volatile("" : "+l"(U));  // keeps the 48 coefficients out of registers
+        const double* L = U + 24;
+        const double z0 = S.gp[q * 3], z1 = S.gp[q * 3 + 1], z2 = S.gp[q * 3 + 2], w = S.gw[q];
+        const double N[4] = {z0, z1, 1.0 - z0 - z1 - z2, z2};
+        double x[3];
+        for (int d = 0; d < 3; ++d)
+            x[d] = fma(N[3], Xv[3][d], fma(N[2], Xv[2][d], fma(N[1], Xv[1][d], N[0] * Xv[0][d])));
+        const double pr[3] = {x[0] * x[1], x[1] * x[2], x[0] * x[2]};
+        double Gu[3][3], Hu[3][3], Gl[3][3], Hl[3][3], Su[6], Sl[6];
+        for (int f = 0; f < 3; ++f) {
+            mono_grad(U + f * 8, x, pr, Gu[f], Hu[f]);
+            mono_grad(L + f * 8, x, pr, Gl[f], Hl[f]);
+        }
+        stress(Gu, lam, mu, Su);
+        stress(Gl, lam, mu, Sl);
+        double phi = 0.0, gr[3] = {0.0, 0.0, 0.0};
+        for (int f = 0; f < 3; ++f)
+            for (int j = 0; j < 3; ++j) phi = fma(Su[sym(f, j)], fma(0.5, Gu[f][j], -Gl[f][j]), phi);
+        Phi = fma(w, phi, Phi);
+        // dphi = (sigma(u) - sigma(lambda)) : dGu - sigma(u) : dGl
+        for (int m = 0; m < 6; ++m) {
+            Sl[m] = w * (Su[m] - Sl[m]);
+            Su[m] *= -w;
+        }
+        push_gradient(Sl, Hu, gr);
+        push_gradient(Su, Hl, gr);
+        for (int k = 0; k < 4; ++k)
+            for (int d = 0; d < 3; ++d) R[k][d] = fma(N[k], gr[d], R[k][d]);
+    }
+    double dx[4][3], dV[4][3];
+    bool mv[4];
+    for (int k = 0; k < 4; ++k) mv[k] = vertex(A, S.vid[g * 4 + k], Xv[k], dx[k]);
+    const double detJ = tet_volume(Xv, dV);
+    // skipped points (detJ < -1e-6) contribute nothing (cl_FEM_Element_Bulk.cpp:164)
+    if (detJ < -1.0e-6) return;
+    for (int k = 0; k < 4; ++k)
+        if (mv[k]) atomicAdd(A.G + S.vid[g * 4 + k], fma(Phi, dot3(dV[k], dx[k]), detJ * dot3(R[k], dx[k])));
 }
 
 struct IfSetDev {
@@ -338,23 +288,63 @@ struct IfSetDev {
     const int32_t* link;   // [neq][4]: leader (set, eq), follower (set, eq) among the cut sets
 };
 
-// The interface sum, flattened like the cut cells (a cluster has a few
-// facets).  The facet integrals are formed once, in dual arithmetic:
-//   iface_cluster_values   per cluster: pdof values of u and lambda of both
-//                          sides, each facet's cluster index;
-//   iface_facets           one thread per facet: the values A, B, C, |G| into
-//                          the cluster sums, the derivatives kept per facet;
-//   iface_apply            one thread per facet: dF/dt with the now known
-//                          cluster sums (w_L, w_F, gamma);
+// The interface sum, flattened like the cut cells (a cluster has a few facets).
+// With the facet's vector area cr / 2 = (x0 - x2) x (x1 - x2) / 2, the mean
+// stress s(.) = w_L sigma_L + w_F sigma_F and the jumps [.], the facet's share of
+// w_L A + w_F B + gamma C is
+//   1/2 sum_q w ( cr . (beta s(lambda) [u] - s(u) [lambda]) + gamma |cr| [lambda].[u] ),
+// with no unit normal in it.  The weights depend on the cluster volumes only and
+// gamma on the volumes and the cluster's area, so with the area summed first the
+// derivative is one reverse sweep.  Jumps and stresses are linear in the fields,
+// so each cluster combines the sides' polynomials beforehand, about the leader's
+// centre: the jump u_L - u_F, the mean w_L E_L u_L + w_F E_F u_F (its unit-modulus
+// stress is s) and the difference E_L u_L - E_F u_F (for A - B), of u and lambda.
+//   iface_cluster_values   per cluster: the six polynomials, area, weights and
+//                          gamma, each facet's cluster index;
+//   iface_facets           one thread per facet: A - B and C into the cluster
+//                          sums, per vertex the derivative at fixed gamma and
+//                          that of the area;
+//   iface_apply            one thread per facet: dF/dt with the cluster's C;
 //   iface_volumes          one thread per (cluster, side, cell of the linked
 //                          cut cluster): dF/dV through w_L, w_F and gamma.
-constexpr int kIfParts = 12;  // dA, dB, dC, d|G| for the three vertices
+// Measured for 43 k facets of 7 points (44^3): iface_facets 1,167 -> 300 us.
+// The whole call with the chain to the coefficients takes 774 us (2,620 before).
+constexpr int kIfParts = 6;     // per vertex: derivative at fixed gamma, of the area
+constexpr int kIfFields = 144;  // [jump, mean, difference][u, lambda][3][8]
+constexpr int kIfSums = 8;      // A - B, C, |G|, gamma, w_L, w_F, 1 / (V_L/E_L + V_F/E_F)
 
-__global__ void iface_cluster_values(AdjArgs A, IfSetDev S, double* UL /*[neq][96]*/, int32_t* facet_cluster) {
+// k about another origin: p(x + d)
+__device__ void shift_polynomial(double* k, const double d[3]) {
+    const double xy = d[0] * d[1], yz = d[1] * d[2], xz = d[0] * d[2], k7 = k[7];
+    k[0] += k[1] * d[0] + k[2] * d[1] + k[3] * d[2] + k[4] * xy + k[5] * yz + k[6] * xz + k7 * xy * d[2];
+    k[1] += k[4] * d[1] + k[6] * d[2] + k7 * yz;
+    k[2] += k[4] * d[0] + k[5] * d[2] + k7 * xz;
+    k[3] += k[6] * d[0] + k[5] * d[1] + k7 * xy;
+    k[4] += k7 * d[2];
+    k[5] += k7 * d[0];
+    k[6] += k7 * d[1];
+}
+
+__global__ void iface_cluster_values(AdjArgs A, IfSetDev S, double* fields /*[neq][kIfFields]*/,
+                                     int32_t* facet_cluster, double* sums /*[neq][kIfSums]*/) {
     const int64_t e = blockIdx.x;
     if (e >= S.neq) return;
-    __shared__ double nod[96];
-    for (int64_t f = S.fc_off[e] + threadIdx.x; f < S.fc_off[e + 1]; f += blockDim.x) facet_cluster[f] = (int32_t)e;
+    __shared__ double nod[96], pol[96], part[2], wt[2];
+    double wsum = 0.0, area = 0.0;
+    for (int q = 0; q < S.ngp; ++q) wsum += S.gw[q];
+    for (int64_t f = S.fc_off[e] + threadIdx.x; f < S.fc_off[e + 1]; f += blockDim.x) {
+        facet_cluster[f] = (int32_t)e;
+        double a[3], b[3], c[3];
+        for (int d = 0; d < 3; ++d) {
+            const double o = A.vx[(int64_t)S.vid[f * 3 + 2] * 3 + d];
+            a[d] = A.vx[(int64_t)S.vid[f * 3] * 3 + d] - o;
+            b[d] = A.vx[(int64_t)S.vid[f * 3 + 1] * 3 + d] - o;
+        }
+        cross(a, b, c);
+        area = fma(0.5 * wsum, sqrt(dot3(c, c)), area);
+    }
+    for (int o = 16; o > 0; o >>= 1) area += __shfl_xor_sync(0xffffffffu, area, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = area;
     for (int s = 0; s < 2; ++s) {
         const int nb = S.nb[2 * e + s];
         pdof_values(S.T + (e * 2 + s) * 8 * S.W, S.bases + (e * 2 + s) * S.W, nb, S.W, A.u, A.nu, nod + 24 * s,
@@ -363,158 +353,198 @@ __global__ void iface_cluster_values(AdjArgs A, IfSetDev S, double* UL /*[neq][9
                     nod + 48 + 24 * s, threadIdx.x, blockDim.x);
     }
     __syncthreads();
+    const double* X = S.xe + e * 48;
     // [u side 0, u side 1, lambda side 0, lambda side 1], each on its side's cell
     for (int r = threadIdx.x; r < 96; r += blockDim.x)
-        UL[e * 96 + r] = monomial_coefficient(nod + (r / 24) * 24, S.xe + e * 48 + 24 * ((r / 24) & 1), r % 24);
-}
-
-__global__ void iface_facets(AdjArgs A, IfSetDev S, const double* __restrict__ UL,
-                             const int32_t* __restrict__ facet_cluster, int64_t nfacets, double* sums /*[neq][4]*/,
-                             double* parts /*[nf][kIfParts]*/) {
-    for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < nfacets;
-         f += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = facet_cluster[f];
-        const double* X = S.xe + e * 48;
-        const double* U = UL + e * 96;
-        const double* L = U + 48;
-        const double Es[2] = {S.E[e], S.EF[e]};
-        const double beta = S.beta_sym ? -1.0 : 1.0;
-        double* P = parts + f * kIfParts;
-        Dual<3> Xv[3][3];
-        bool mv[3];
-        for (int k = 0; k < 3; ++k) vertex_dual<3>(A, S.vid[f * 3 + k], k, Xv[k], mv[k]);
-        // facet detJ |(x0-x2) x (x1-x2)| / 2 and the unit normal
-        Dual<3> a[3], b[3], cr[3];
-        for (int d = 0; d < 3; ++d) {
-            a[d] = Xv[0][d] - Xv[2][d];
-            b[d] = Xv[1][d] - Xv[2][d];
-        }
-        cr[0] = a[1] * b[2] - a[2] * b[1];
-        cr[1] = a[2] * b[0] - a[0] * b[2];
-        cr[2] = a[0] * b[1] - a[1] * b[0];
-        const Dual<3> nn = dsqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
-        if (!(nn.v > 0.0)) {
-            for (int k = 0; k < kIfParts; ++k) P[k] = 0.0;
-            continue;
-        }
-        const Dual<3> inv = dinv(nn);
-        const Dual<3> n[3] = {cr[0] * inv, cr[1] * inv, cr[2] * inv};
-        const Dual<3> detJ = 0.5 * nn;
-        double xc[2][3];  // the sides' cell centres
-        for (int s = 0; s < 2; ++s)
-            for (int d = 0; d < 3; ++d) xc[s][d] = 0.5 * (X[24 * s + 18 + d] + X[24 * s + d]);
-        Dual<3> fa(0.0), fb(0.0), fc(0.0), fr(0.0);
-        for (int q = 0; q < S.ngp; ++q) {
-            const double z0 = S.gp[q * 2], z1 = S.gp[q * 2 + 1];
-            const double Nf[3] = {z0, z1, 1.0 - z0 - z1};
-            // per side: values and tractions t_s(.) = sigma_s(.) n, each
-            // gradient turned into its traction at once
-            Dual<3> uv[2][3], lv[2][3], tu[2][3], tl[2][3], xp[3];
-            for (int d = 0; d < 3; ++d) {
-                xp[d] = Dual<3>(0.0);
-                for (int k = 0; k < 3; ++k) axpy(Nf[k], Xv[k][d], xp[d]);
-            }
-            for (int s = 0; s < 2; ++s) {
-                Dual<3> xq[3];
-                for (int d = 0; d < 3; ++d) xq[d] = (-xc[s][d]) + xp[d];
-                const Dual<3> pr[3] = {xq[0] * xq[1], xq[1] * xq[2], xq[0] * xq[2]};
-                for (int fld = 0; fld < 2; ++fld) {
-                    Dual<3> Gf[3][3], Sf[3][3];
-                    mono_field<3, true>((fld ? L : U) + 24 * s, xq, pr, fld ? lv[s] : uv[s], Gf);
-                    stress<3>(Gf, Es[s] * S.lam_c, Es[s] * S.mu_c, Sf);
-                    Dual<3>* t = fld ? tl[s] : tu[s];
-                    for (int i2 = 0; i2 < 3; ++i2) t[i2] = Sf[i2][0] * n[0] + Sf[i2][1] * n[1] + Sf[i2][2] * n[2];
-                }
-            }
-            Dual<3> qa(0.0), qb(0.0), qc(0.0);
-            for (int i = 0; i < 3; ++i) {
-                const Dual<3> ju = uv[0][i] - uv[1][i], jl = lv[0][i] - lv[1][i];
-                qa = qa + beta * (tl[0][i] * ju) - jl * tu[0][i];
-                qb = qb + beta * (tl[1][i] * ju) - jl * tu[1][i];
-                qc = qc + jl * ju;
-            }
-            const Dual<3> ws = S.gw[q] * detJ;
-            fa = fa + ws * qa;
-            fb = fb + ws * qb;
-            fc = fc + ws * qc;
-            fr = fr + ws;
-        }
-        atomicAdd(sums + e * 4 + 0, fa.v);
-        atomicAdd(sums + e * 4 + 1, fb.v);
-        atomicAdd(sums + e * 4 + 2, fc.v);
-        atomicAdd(sums + e * 4 + 3, fr.v);
-        for (int k = 0; k < 3; ++k) {
-            // a vertex that does not move has no derivative slot
-            P[k] = mv[k] ? fa.d[k] : 0.0;
-            P[3 + k] = mv[k] ? fb.d[k] : 0.0;
-            P[6 + k] = mv[k] ? fc.d[k] : 0.0;
-            P[9 + k] = mv[k] ? fr.d[k] : 0.0;
-        }
+        pol[r] = monomial_coefficient(nod + (r / 24) * 24, X + 24 * ((r / 24) & 1), r % 24);
+    if (threadIdx.x == 0) {
+        const double vl = S.vol[2 * e] / S.E[e], vf = S.vol[2 * e + 1] / S.EF[e], inv = 1.0 / (vl + vf);
+        double* q = sums + e * kIfSums;
+        q[0] = q[1] = 0.0;
+        q[2] = part[0] + part[1];
+        q[3] = 2.0 * S.alpha * q[2] * inv;
+        q[4] = vl * inv;
+        q[5] = vf * inv;
+        q[6] = inv;
+        wt[0] = q[4] * S.E[e];
+        wt[1] = q[5] * S.EF[e];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        // the follower's polynomials about the leader's centre
+        const int fl = threadIdx.x / 3;
+        double d[3];
+        for (int i = 0; i < 3; ++i) d[i] = 0.5 * (X[18 + i] + X[i]) - 0.5 * (X[42 + i] + X[24 + i]);
+        if (d[0] != 0.0 || d[1] != 0.0 || d[2] != 0.0) shift_polynomial(pol + fl * 48 + 24 + threadIdx.x % 3 * 8, d);
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < kIfFields; r += blockDim.x) {
+        const int kind = r / 48, at = (r / 24 & 1) * 48 + r % 24;
+        const double p0 = pol[at], p1 = pol[at + 24];
+        fields[e * kIfFields + r] = kind == 0   ? p0 - p1
+                                    : kind == 1 ? fma(wt[0], p0, wt[1] * p1)
+                                                : S.E[e] * p0 - S.EF[e] * p1;
     }
 }
 
-// the cluster's Nitsche weights and gamma from its sums and volumes
-__device__ __forceinline__ void iface_weights(const IfSetDev& S, int64_t e, double& wl, double& wf, double& Ssum) {
-    const double vl = S.vol[2 * e] / S.E[e], vf = S.vol[2 * e + 1] / S.EF[e];
-    Ssum = vl + vf;
-    wl = vl / Ssum;
-    wf = vf / Ssum;
+__global__ void __launch_bounds__(64, 6) iface_facets(AdjArgs A, IfSetDev S, const double* __restrict__ fields,
+                                                   const int32_t* __restrict__ facet_cluster, int64_t nfacets,
+                                                   double* sums, double* parts /*[nf][kIfParts]*/) {
+    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= nfacets) return;
+    const int64_t e = facet_cluster[f];
+    const double* X = S.xe + e * 48;
+    const double* P = fields + e * kIfFields;
+    const double beta = S.beta_sym ? -1.0 : 1.0, gamma = sums[e * kIfSums + 3];
+    double Xv[3][3], a[3], b[3], cr[3];
+    for (int k = 0; k < 3; ++k)
+        for (int d = 0; d < 3; ++d) Xv[k][d] = A.vx[(int64_t)S.vid[f * 3 + k] * 3 + d] - 0.5 * (X[18 + d] + X[d]);
+    for (int d = 0; d < 3; ++d) {
+        a[d] = Xv[0][d] - Xv[2][d];
+        b[d] = Xv[1][d] - Xv[2][d];
+    }
+    cross(a, b, cr);
+    const double nn = sqrt(dot3(cr, cr));
+    double* out = parts + f * kIfParts;
+    if (!(nn > 0.0)) {
+        for (int k = 0; k < kIfParts; ++k) out[k] = 0.0;
+        return;
+    }
+    const double gn = gamma * nn;
+    double V[3] = {0.0, 0.0, 0.0}, cs = 0.0, ab = 0.0, wsum = 0.0;  // sums of v, [lambda].[u], A - B, w
+    double R[3][3] = {};
+#pragma unroll 1
+    for (int q = 0; q < S.ngp; ++q) {
+        // the coefficients stay in L1: hoisted out of the loop, all 144 spill
+        asm volatile("" : "+l"(P));
+        const double z0 = S.gp[q * 2], z1 = S.gp[q * 2 + 1], w = S.gw[q];
+        const double N[3] = {z0, z1, 1.0 - z0 - z1};
+        double x[3], gr[3] = {0.0, 0.0, 0.0}, jv[2][3], dj[2][3][3], t[2][3], v[3] = {0.0, 0.0, 0.0};
+        for (int d = 0; d < 3; ++d) x[d] = fma(N[2], Xv[2][d], fma(N[1], Xv[1][d], N[0] * Xv[0][d]));
+        const double pr[3] = {x[0] * x[1], x[1] * x[2], x[0] * x[2]};
+#pragma unroll
+        for (int fl = 0; fl < 2; ++fl)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                double h[3];
+                mono_grad(P + fl * 24 + i * 8, x, pr, dj[fl][i], h);
+                jv[fl][i] = mono_value(P + fl * 24 + i * 8, x, pr, dj[fl][i][0]);
+            }
+        // v = beta s(lambda) [u] - s(u) [lambda], t = s(.) cr, and the gradient of
+        // cr . v through the stresses: (sigma(G) cr) . j = G : W with
+        // W = lam (cr . j) I + mu (cr j^T + j cr^T)
+        double da = 0.0;
+#pragma unroll
+        for (int fl = 0; fl < 2; ++fl) {
+            const double sg = fl ? beta : -1.0;
+            const double* j = jv[1 - fl];
+            double G[3][3], H[3][3], Sg[6], W[6];
+            for (int i = 0; i < 3; ++i) mono_grad(P + 48 + fl * 24 + i * 8, x, pr, G[i], H[i]);
+            stress(G, S.lam_c, S.mu_c, Sg);
+            const double tr = S.lam_c * sg * dot3(cr, j), m = S.mu_c * sg;
+            const double mj[3] = {m * j[0], m * j[1], m * j[2]};
+            for (int k = 0; k < 3; ++k) {
+                W[k] = fma(2.0 * cr[k], mj[k], tr);
+                const double row[3] = {Sg[sym(k, 0)], Sg[sym(k, 1)], Sg[sym(k, 2)]};
+                t[fl][k] = dot3(row, cr);
+                v[k] = fma(sg, dot3(row, j), v[k]);
+            }
+            W[3] = fma(cr[0], mj[1], cr[1] * mj[0]);
+            W[4] = fma(cr[1], mj[2], cr[2] * mj[1]);
+            W[5] = fma(cr[0], mj[2], cr[2] * mj[0]);
+            push_gradient(W, H, gr);
+            // the share of A - B: the same product with the difference field
+            for (int i = 0; i < 3; ++i) {
+                mono_grad(P + 96 + fl * 24 + i * 8, x, pr, G[i], H[i]);
+                for (int k = 0; k < 3; ++k) da = fma(W[sym(i, k)], G[i][k], da);
+            }
+        }
+        ab = fma(w, da, ab);
+        cs = fma(w, dot3(jv[0], jv[1]), cs);
+        wsum += w;
+        for (int i = 0; i < 3; ++i) {
+            V[i] = fma(w, v[i], V[i]);
+            // the gradient through [u] and [lambda]
+            const double au = fma(gn, jv[1][i], beta * t[1][i]), al = fma(gn, jv[0][i], -t[0][i]);
+            for (int d = 0; d < 3; ++d) gr[d] = fma(au, dj[0][i][d], fma(al, dj[1][i][d], gr[d]));
+        }
+        for (int k = 0; k < 3; ++k) {
+            const double wn = 0.5 * w * N[k];
+            for (int d = 0; d < 3; ++d) R[k][d] = fma(wn, gr[d], R[k][d]);
+        }
+    }
+    atomicAdd(sums + e * kIfSums, 0.5 * ab);
+    atomicAdd(sums + e * kIfSums + 1, 0.5 * nn * cs);
+    // by the vector area: Y = (V + gamma cs cr / |cr|) / 2, the area's own cr / (2 |cr|)
+    double Y[3], Z[3], d0[3], d1[3], dx[3][3];
+    bool mv[3];
+    for (int k = 0; k < 3; ++k) mv[k] = vertex(A, S.vid[f * 3 + k], d0, dx[k]);
+    const double in = 1.0 / nn;
+    for (int i = 0; i < 3; ++i) {
+        Z[i] = 0.5 * wsum * cr[i] * in;
+        Y[i] = 0.5 * fma(gamma * cs, cr[i] * in, V[i]);
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+        const double* y = pass ? Z : Y;
+        cross(b, y, d0);
+        cross(y, a, d1);
+        for (int k = 0; k < 3; ++k) {
+            double s = 0.0;
+            for (int d = 0; d < 3; ++d) {
+                const double g = k == 0 ? d0[d] : k == 1 ? d1[d] : -(d0[d] + d1[d]);
+                s = fma(pass ? g : g + R[k][d], dx[k][d], s);
+            }
+            // a vertex that does not move has no derivative
+            out[pass * 3 + k] = mv[k] ? s : 0.0;
+        }
+    }
 }
 
 __global__ void iface_apply(AdjArgs A, IfSetDev S, const int32_t* __restrict__ facet_cluster, int64_t nfacets,
                             const double* __restrict__ sums, const double* __restrict__ parts) {
-    for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < nfacets;
-         f += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = facet_cluster[f];
-        double wl, wf, Ssum;
-        iface_weights(S, e, wl, wf, Ssum);
-        // F = -(wL A + wF B + gamma C), gamma = 2 alpha |G| / S
-        const double gamma = 2.0 * S.alpha * sums[e * 4 + 3] / Ssum;
-        const double dg_darea = 2.0 * S.alpha / Ssum;
-        const double* P = parts + f * kIfParts;
-        for (int k = 0; k < 3; ++k) {
-            const double g = -(wl * P[k] + wf * P[3 + k] + gamma * P[6 + k] + sums[e * 4 + 2] * dg_darea * P[9 + k]);
-            if (P[k] != 0.0 || P[3 + k] != 0.0 || P[6 + k] != 0.0 || P[9 + k] != 0.0)
-                atomicAdd(A.G + S.vid[f * 3 + k], g);
-        }
-    }
+    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= nfacets) return;
+    // F = -(wL A + wF B + gamma C), gamma = 2 alpha |G| / S
+    const double* q = sums + facet_cluster[f] * (int64_t)kIfSums;
+    const double cg = q[1] * 2.0 * S.alpha * q[6];
+    const double* P = parts + f * kIfParts;
+    for (int k = 0; k < 3; ++k)
+        if (P[k] != 0.0 || P[3 + k] != 0.0) atomicAdd(A.G + S.vid[f * 3 + k], -fma(cg, P[3 + k], P[k]));
 }
 
 // items: (interface cluster e, side) per cell of the linked cut cluster
 __global__ void iface_volumes(AdjArgs A, IfSetDev S, const CutSetDev* cuts, int64_t nitems,
                               const int64_t* __restrict__ item_e, const int64_t* __restrict__ item_cell,
                               const double* __restrict__ sums) {
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nitems;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t es = item_e[t], e = es >> 1;
-        const int side = (int)(es & 1);
-        const CutSetDev& C = cuts[S.link[e * 4 + side * 2]];
-        const int64_t g = item_cell[t];
-        double wl, wf, Ssum;
-        iface_weights(S, e, wl, wf, Ssum);
-        const double vl = S.vol[2 * e] / S.E[e], vf = S.vol[2 * e + 1] / S.EF[e];
-        const double gamma = 2.0 * S.alpha * sums[e * 4 + 3] / Ssum;
-        const double dwl = side == 0 ? vf / (Ssum * Ssum) : -vl / (Ssum * Ssum);
-        const double dg_dv = -gamma / Ssum;
-        const double Es = side == 0 ? S.E[e] : S.EF[e];
-        // dF/dvol = -((A - B) dwL/dv + C dgamma/dv) / E_side
-        const double coef = -((sums[e * 4 + 0] - sums[e * 4 + 1]) * dwl + sums[e * 4 + 2] * dg_dv) / Es;
-        Dual<4> Xv[4][3];
-        bool mv[4];
-        int32_t vids[4];
-        for (int k = 0; k < 4; ++k) {
-            vids[k] = C.vid[g * 4 + k];
-            vertex_dual<4>(A, vids[k], k, Xv[k], mv[k]);
-        }
-        const Dual<4> vol = tet_volume<4>(Xv);
-        for (int k = 0; k < 4; ++k)
-            if (mv[k]) atomicAdd(A.G + vids[k], coef * vol.d[k]);
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nitems) return;
+    const int64_t es = item_e[t], e = es >> 1;
+    const int side = (int)(es & 1);
+    const CutSetDev& C = cuts[S.link[e * 4 + side * 2]];
+    const int64_t g = item_cell[t];
+    double Xv[4][3], dx[4][3], dV[4][3];
+    bool mv[4], any = false;
+    int32_t vids[4];
+    for (int k = 0; k < 4; ++k) {
+        vids[k] = C.vid[g * 4 + k];
+        mv[k] = vertex(A, vids[k], Xv[k], dx[k]);
+        any |= mv[k];
     }
+    if (!any) return;
+    // dw_L/dV_L = w_F / S, dw_L/dV_F = -w_L / S, dgamma/dV = -gamma / S (per V / E)
+    const double* q = sums + e * kIfSums;
+    const double coef = -(q[0] * (side == 0 ? q[5] : -q[4]) - q[1] * q[3]) * q[6] / (side == 0 ? S.E[e] : S.EF[e]);
+    tet_volume(Xv, dV);
+    for (int k = 0; k < 4; ++k)
+        if (mv[k]) atomicAdd(A.G + vids[k], coef * dot3(dV[k], dx[k]));
 }
 
-// dqdp[j] += G[v] dt_v/dp_j through the parents' level set
-__global__ void dqdp_chain(int64_t nv, const int32_t* vkind, const int32_t* vpar, const double* vphi,
-                           const double* G, int width, const int32_t* cols, const double* tmat, double* dqdp) {
+// dQ/dp = sum_v G[v] dt_v/dp through the parents' level set, in two steps: the
+// weight of every background node (a vertex touches up to 16), then the nodes'
+// coefficients, one warp per node with a weight.  A vertex writing its
+// coefficients itself repeats the width (64 for cubic splines) for every node.
+__global__ void dqdp_nodes(int64_t nv, const int32_t* vkind, const int32_t* vpar, const double* vphi, const double* G,
+                           double* node_weight) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nv || vkind[v] != 3 || G[v] == 0.0) return;
     const int32_t p[2] = {vpar[v * 8], vpar[v * 8 + 1]};
@@ -527,13 +557,19 @@ __global__ void dqdp_chain(int64_t nv, const int32_t* vkind, const int32_t* vpar
         const int kind = vkind[q];
         const int cnt = kind == 0 ? 1 : kind == 1 ? 4 : 8;
         const double w = G[v] * dt[k] / (double)cnt;
-        for (int m = 0; m < cnt; ++m) {
-            const int64_t node = vpar[(int64_t)q * 8 + m];
-            for (int j = 0; j < width; ++j) {
-                const double tv = tmat[node * width + j];
-                if (tv != 0.0) atomicAdd(dqdp + cols[node * width + j], w * tv);
-            }
-        }
+        for (int m = 0; m < cnt; ++m) atomicAdd(node_weight + vpar[(int64_t)q * 8 + m], w);
+    }
+}
+__global__ void dqdp_coefficients(int64_t nbn, int width, const int32_t* __restrict__ cols,
+                                  const double* __restrict__ tmat, const double* __restrict__ node_weight,
+                                  double* dqdp) {
+    const int64_t n = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (n >= nbn) return;
+    const double w = node_weight[n];
+    if (w == 0.0) return;
+    for (int j = threadIdx.x & 31; j < width; j += 32) {
+        const double tv = tmat[n * width + j];
+        if (tv != 0.0) atomicAdd(dqdp + cols[n * width + j], w * tv);
     }
 }
 
@@ -600,6 +636,7 @@ void sensitivity_release(fem_gpu_ctx* c) {
     dfree(c->d_vval);
     dfree(c->d_lscols);
     dfree(c->d_lst);
+    dfree(c->d_lsw);
     c->ls_nbn = 0;
     c->ls_phi = false;
     for (auto& s : c->sets) {
@@ -607,9 +644,8 @@ void sensitivity_release(fem_gpu_ctx* c) {
         dfree(s.d_link);
         dfree(s.d_adjul);
         dfree(s.d_items);
-        dfree(s.d_tperm);
-        s.nitems = 0;
-        for (int64_t& o : s.tperm_off) o = 0;
+        dfree(s.d_moving);
+        s.nitems = s.nmoving = 0;
     }
     c->adj_topo = c->adj_coords = false;
 }
@@ -807,7 +843,8 @@ fem_gpu_status fem_gpu_drdp_adjoint(fem_gpu_ctx* c, const double* u, const doubl
         const int64_t ncells = s.ig_off.empty() ? 0 : s.ig_off.back();
         // per-cluster pdof values of u and lambda, then one thread per cell
         // [neq][48] doubles, then [ncells] cluster indices
-        const size_t need = (size_t)d.neq * 48 * sizeof(double) + (size_t)std::max<int64_t>(ncells, 1) * sizeof(int32_t);
+        const size_t need =
+            (size_t)d.neq * 48 * sizeof(double) + (size_t)std::max<int64_t>(ncells, 1) * sizeof(int32_t);
         if (!s.d_adjul.p || s.d_adjul.bytes < need) {
             dfree(s.d_adjul);
             if ((e = cudaMalloc(&s.d_adjul.p, need)) != cudaSuccess) return sfail(c, e, "adjoint cluster values");
@@ -816,38 +853,22 @@ fem_gpu_status fem_gpu_drdp_adjoint(fem_gpu_ctx* c, const double* u, const doubl
         double* UL = (double*)s.d_adjul.p;
         int32_t* cc = reinterpret_cast<int32_t*>(UL + (size_t)d.neq * 48);
         if (topo) {
-            // integration cells grouped by their number of moving (intersection)
-            // vertices, 1 to 4; cells without one are left out
-            std::vector<int32_t> cnt(ncells);
-            int64_t grp[5] = {0, 0, 0, 0, 0};
-            for (int64_t g = 0; g < ncells; ++g) {
-                int m = 0;
-                for (int k = 0; k < 4; ++k) m += c->vkind[s.vid[g * 4 + k]] == 3;
-                cnt[g] = m;
-                ++grp[m];
-            }
-            s.tperm_off[0] = 0;
-            for (int m = 1; m <= 4; ++m) s.tperm_off[m] = s.tperm_off[m - 1] + grp[m];
-            std::vector<int32_t> perm(std::max<int64_t>(s.tperm_off[4], 1));
-            int64_t pos[5] = {0, s.tperm_off[0], s.tperm_off[1], s.tperm_off[2], s.tperm_off[3]};
+            // integration cells with a moving (intersection) vertex
+            std::vector<int32_t> moving;
             for (int64_t g = 0; g < ncells; ++g)
-                if (cnt[g] > 0) perm[pos[cnt[g]]++] = (int32_t)g;
-            if ((e = upload(s.d_tperm, perm, st)) != cudaSuccess) return sfail(c, e, "moving-vertex groups");
+                for (int k = 0; k < 4; ++k)
+                    if (c->vkind[s.vid[g * 4 + k]] == 3) {
+                        moving.push_back((int32_t)g);
+                        break;
+                    }
+            s.nmoving = (int64_t)moving.size();
+            if ((e = upload(s.d_moving, moving, st)) != cudaSuccess) return sfail(c, e, "moving cells");
         }
         adjoint_cluster_values<<<(unsigned)std::max<int64_t>(d.neq, 1), 64, 0, st>>>(A, d, UL, cc);
         c->launches++;
-        const int32_t* perm = (const int32_t*)s.d_tperm.p;
-        for (int m = 1; m <= 4; ++m) {
-            const int64_t a0 = s.tperm_off[m - 1], n = s.tperm_off[m] - a0;
-            if (n <= 0) continue;
-            const unsigned grid =
-                (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, (int64_t)sm_count() * 16));
-            switch (m) {
-                case 1: adjoint_tets_flat<1><<<grid, 64, 0, st>>>(A, d, UL, cc, perm + a0, n); break;
-                case 2: adjoint_tets_flat<2><<<grid, 64, 0, st>>>(A, d, UL, cc, perm + a0, n); break;
-                case 3: adjoint_tets_flat<3><<<grid, 64, 0, st>>>(A, d, UL, cc, perm + a0, n); break;
-                default: adjoint_tets_flat<4><<<grid, 64, 0, st>>>(A, d, UL, cc, perm + a0, n); break;
-            }
+        if (s.nmoving > 0) {
+            adjoint_tets<<<(unsigned)((s.nmoving + 63) / 64), 64, 0, st>>>(A, d, UL, cc, (const int32_t*)s.d_moving.p,
+                                                                           s.nmoving);
             c->launches++;
         }
     }
@@ -911,13 +932,13 @@ fem_gpu_status fem_gpu_drdp_adjoint(fem_gpu_ctx* c, const double* u, const doubl
         d.ngp = s.ngp;
         d.vol = (const double*)s.d_vol.p;
         d.link = (const int32_t*)s.d_link.p;
-        // scratch: per cluster U, L (96) and sums (4); per facet the cluster
+        // scratch: per cluster the field polynomials and sums; per facet the cluster
         // index and the derivative parts; the volume items
         const int64_t nf = s.fc_off.empty() ? 0 : s.fc_off.back();
         const int64_t ni = s.nitems;
         const int64_t* item_e = (const int64_t*)s.d_items.p;
-        const size_t need = (size_t)s.neq * 100 * sizeof(double) + (size_t)std::max<int64_t>(nf, 1) * kIfParts * sizeof(double) +
-                            (size_t)std::max<int64_t>(nf, 1) * sizeof(int32_t);
+        const size_t need = (size_t)s.neq * (kIfFields + kIfSums) * sizeof(double) +
+                            (size_t)std::max<int64_t>(nf, 1) * (kIfParts * sizeof(double) + sizeof(int32_t));
         if (!s.d_adjul.p || s.d_adjul.bytes < need) {
             dfree(s.d_adjul);
             if ((e = cudaMalloc(&s.d_adjul.p, need)) != cudaSuccess) {
@@ -927,14 +948,11 @@ fem_gpu_status fem_gpu_drdp_adjoint(fem_gpu_ctx* c, const double* u, const doubl
             s.d_adjul.bytes = need;
         }
         double* UL = (double*)s.d_adjul.p;
-        double* sums = UL + (size_t)s.neq * 96;
-        double* parts = sums + (size_t)s.neq * 4;
+        double* sums = UL + (size_t)s.neq * kIfFields;
+        double* parts = sums + (size_t)s.neq * kIfSums;
         int32_t* fcl = reinterpret_cast<int32_t*>(parts + (size_t)std::max<int64_t>(nf, 1) * kIfParts);
-        cudaMemsetAsync(sums, 0, (size_t)s.neq * 4 * sizeof(double), st);
-        const auto grid_of = [](int64_t n) {
-            return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, (int64_t)sm_count() * 16));
-        };
-        iface_cluster_values<<<(unsigned)std::max<int64_t>(s.neq, 1), 64, 0, st>>>(A, d, UL, fcl);
+        const auto grid_of = [](int64_t n) { return (unsigned)std::max<int64_t>(1, (n + 63) / 64); };
+        iface_cluster_values<<<(unsigned)std::max<int64_t>(s.neq, 1), 64, 0, st>>>(A, d, UL, fcl, sums);
         iface_facets<<<grid_of(nf), 64, 0, st>>>(A, d, UL, fcl, nf, sums, parts);
         iface_apply<<<grid_of(nf), 64, 0, st>>>(A, d, fcl, nf, sums, parts);
         iface_volumes<<<grid_of(ni), 64, 0, st>>>(A, d, (const CutSetDev*)c->d_adjcuts.p, ni, item_e, item_e + ni,
@@ -969,6 +987,11 @@ fem_gpu_status fem_gpu_set_level_set_field(fem_gpu_ctx* c, int64_t nbn, int32_t 
         dfree(c->d_lst);
         if ((e = cudaMalloc(&c->d_lst.p, (size_t)n * sizeof(double))) == cudaSuccess)
             c->d_lst.bytes = (size_t)n * sizeof(double);
+    }
+    if (e == cudaSuccess && (!c->d_lsw.p || c->d_lsw.bytes < (size_t)nbn * sizeof(double))) {
+        dfree(c->d_lsw);
+        if ((e = cudaMalloc(&c->d_lsw.p, (size_t)nbn * sizeof(double))) == cudaSuccess)
+            c->d_lsw.bytes = (size_t)nbn * sizeof(double);
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(c->d_lscols.p, cols, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, st);
@@ -1008,13 +1031,16 @@ fem_gpu_status fem_gen_dqdp(fem_gpu_ctx* c, const double* G, int64_t nbn, int32_
     if (e == cudaSuccess && !c->adj_topo) e = refresh(c->d_vkind, c->vkind, st);
     if (e == cudaSuccess && !c->adj_topo) e = refresh(c->d_vpar, c->vpar, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(dqdp, 0, ncoef * sizeof(double), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_lsw.p, 0, nbn * sizeof(double), st);
     if (e == cudaSuccess) {
         c->ls_phi = true;
-        dqdp_chain<<<(unsigned)((nv + 255) / 256), 256, 0, st>>>(nv, (const int32_t*)c->d_vkind.p,
-                                                                 (const int32_t*)c->d_vpar.p, (const double*)c->d_vval.p,
-                                                                 G, width, (const int32_t*)c->d_lscols.p,
-                                                                 (const double*)c->d_lst.p, dqdp);
-        c->launches++;
+        double* nw = (double*)c->d_lsw.p;
+        dqdp_nodes<<<(unsigned)((nv + 127) / 128), 128, 0, st>>>(nv, (const int32_t*)c->d_vkind.p,
+                                                                 (const int32_t*)c->d_vpar.p,
+                                                                 (const double*)c->d_vval.p, G, nw);
+        dqdp_coefficients<<<(unsigned)((nbn + 7) / 8), 256, 0, st>>>(nbn, width, (const int32_t*)c->d_lscols.p,
+                                                                     (const double*)c->d_lst.p, nw, dqdp);
+        c->launches += 2;
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
