@@ -635,8 +635,123 @@ __global__ void lattice_restrict(int n0, int n1, int n2, const double* __restric
     }
 }
 
+// ---------------------------------------------------------------------------
+// Plane lattices (QUAD4, splines of order 1 to 3, constant modulus per element).
+// With the extraction of one axis a (p + 1) x 2 matrix, the element matrices
+// between splines are products of 1-D ones (mass M, stiffness D, gradient G), so
+//   A_xx(i, j) = sum_e E J_y / J_x D(i_x, j_x) M(i_y, j_y), ...
+// over the at most (p + 1)^2 elements that splines i and j share: summed along x,
+// then along y, four products per element and offset, no element matrix.  Lane =
+// basis, warp = y offset; a thread forms the 2 p + 1 blocks of its offsets and
+// their share of the residual.  The element loop spent a CTA on 8 x 8 to 32 x 32
+// matrices; measured (assembly with two side sets): 257 x 130, p = 2, 237 -> 107 us,
+// 24 x 17, p = 1, 61 -> 47 us.
+struct PlaneArgs {
+    int ne[2], nb[2];
+    const double* E;
+    const double* jac;  // half edge lengths [ne0], [ne1], then their reciprocals
+    const double* u;
+    double* vals;
+    double* rhs;
+    const int32_t* rowptr;
+    int acc_v, acc_r;
+    int* status;
+    double mu, ld, lo;                      // mu per unit modulus, (lam + mu) / mu, lam / mu
+    double M[4][4], D[4][4], G[4][4];       // 1-D matrices on the reference element
+};
+
+template <int P>
+__global__ void __launch_bounds__(32 * (2 * P + 1)) lattice_plane(PlaneArgs p) {
+    constexpr int ND = 2 * P + 1;
+    __shared__ double red[ND][32][2];
+    const int lane = threadIdx.x & 31, Dy = (int)(threadIdx.x >> 5) - P;
+    const int nu = p.nb[0] * p.nb[1], b = blockIdx.x * 32 + lane;
+    const bool live = b < nu;
+    const int bx = live ? b % p.nb[0] : 0, by = live ? b / p.nb[0] : 0;
+    const bool row = live && by + Dy >= 0 && by + Dy < p.nb[1];
+    const int nj = p.ne[0] + p.ne[1];
+    double S[ND][4];  // xx, yy, xy, yx of offset Dx
+#pragma unroll
+    for (int d = 0; d < ND; ++d) S[d][0] = S[d][1] = S[d][2] = S[d][3] = 0.0;
+#pragma unroll 1
+    for (int iy = max(0, -Dy); iy <= min(P, P - Dy); ++iy) {
+        const int ey = by - iy, jy = iy + Dy;
+        if (!(row && ey >= 0 && ey < p.ne[1])) continue;
+        const double Jy = __ldg(p.jac + p.ne[0] + ey), Iy = __ldg(p.jac + nj + p.ne[0] + ey);
+        double E[P + 1], wx[P + 1], wy[P + 1];
+#pragma unroll
+        for (int i = 0; i <= P; ++i) {
+            const int ex = bx - i;
+            const bool in = ex >= 0 && ex < p.ne[0];
+            E[i] = in ? __ldg(p.E + (int64_t)ey * p.ne[0] + ex) * p.mu : 0.0;
+            wx[i] = E[i] * Jy * (in ? __ldg(p.jac + nj + ex) : 0.0);
+            wy[i] = E[i] * Iy * (in ? __ldg(p.jac + ex) : 0.0);
+        }
+        const double My = p.M[iy][jy], Dyy = p.D[iy][jy], Gy = p.G[iy][jy], Hy = p.G[jy][iy];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+#pragma unroll
+            for (int i = 0; i <= P; ++i) {
+                const int j = i + d - P;
+                if (j < 0 || j > P) continue;
+                a0 = fma(wx[i], p.D[i][j], a0);
+                a1 = fma(wy[i], p.M[i][j], a1);
+                a2 = fma(E[i], p.G[i][j], a2);
+                a3 = fma(E[i], p.G[j][i], a3);
+            }
+            S[d][0] = fma(a0, My, S[d][0]);
+            S[d][1] = fma(a1, Dyy, S[d][1]);
+            S[d][2] = fma(a2, Hy, S[d][2]);
+            S[d][3] = fma(a3, Gy, S[d][3]);
+        }
+    }
+    double r[2] = {0.0, 0.0};
+    bool bad = false;
+    if (row) {
+        const int lx = max(bx - P, 0), cx = min(bx + P, p.nb[0] - 1) - lx + 1;
+        const int ly = max(by - P, 0), cy = min(by + P, p.nb[1] - 1) - ly + 1;
+        const int32_t r0 = p.vals ? __ldg(p.rowptr + b) : 0, r1 = p.vals ? __ldg(p.rowptr + nu + b) : 0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            const int x = bx + d - P;
+            if (x < 0 || x >= p.nb[0]) continue;
+            const double tr = S[d][0] + S[d][1];
+            const double K[4] = {fma(p.ld, S[d][0], tr), fma(p.lo, S[d][2], S[d][3]), fma(p.lo, S[d][3], S[d][2]),
+                                 fma(p.ld, S[d][1], tr)};
+            if (p.u) {
+                const int j = (by + Dy) * p.nb[0] + x;
+                const double u0 = __ldg(p.u + j), u1 = __ldg(p.u + nu + j);
+                r[0] = fma(K[0], u0, fma(K[1], u1, r[0]));
+                r[1] = fma(K[2], u0, fma(K[3], u1, r[1]));
+            }
+            if (p.vals) {
+                const int at = (by + Dy - ly) * cx + x - lx, ul = cx * cy;
+                double* v[4] = {p.vals + r0 + at, p.vals + r0 + ul + at, p.vals + r1 + at, p.vals + r1 + ul + at};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    bad |= !fem_finite(K[k]);
+                    *v[k] = p.acc_v ? *v[k] + K[k] : K[k];
+                }
+            }
+        }
+    }
+    if (bad) atomicOr(p.status, 1);
+    if (!p.rhs) return;
+    red[Dy + P][lane][0] = r[0];
+    red[Dy + P][lane][1] = r[1];
+    __syncthreads();
+    if (threadIdx.x < 64 && blockIdx.x * 32 + (threadIdx.x & 31) < nu) {
+        const int f = threadIdx.x >> 5;
+        double v = 0.0;
+        for (int k = 0; k < ND; ++k) v += red[k][lane][f];
+        double* q = p.rhs + f * nu + b;
+        *q = p.acc_r ? *q + v : v;
+    }
+}
+
 struct Lattice {
-    int p = 0;
+    int dim = 3, p = 0;
     int ne[3], nn[3], nb[3];
     int64_t pitch = 0;
     DeviceBuf jac;     // half edge lengths and their reciprocals
@@ -660,51 +775,75 @@ cudaError_t upload(DeviceBuf& b, const std::vector<T>& v, cudaStream_t st) {
     return e;
 }
 
-// the lattice of a mesh, or nothing where any of its properties does not hold exactly
+// weights of the splines at a node along one axis (splines i .. i + p - 1 of node i)
+const double* axis_weights(int p) {
+    static const double w[3][3] = {{1.0}, {0.5, 0.5}, {1.0 / 6.0, 4.0 / 6.0, 1.0 / 6.0}};
+    return w[p - 1];
+}
+
+// the lattice of a mesh, or nothing where any of its properties does not hold
+// exactly (the extraction weights of order 3, which are not dyadic, up to 1e-15)
 bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
-    if (c->dim != 3 || c->shape != FEM_GPU_SHAPE_RECTANGULAR || c->num_used != c->num_bases) return false;
+    const int D = c->dim;
+    if (c->shape != FEM_GPU_SHAPE_RECTANGULAR || c->num_used != c->num_bases) return false;
     const double* X = c->coords.data();
     const int64_t N = c->num_nodes;
-    int64_t n0 = 1, n1 = 1;
-    while (n0 < N && X[n0 * 3 + 1] == X[1] && X[n0 * 3 + 2] == X[2]) ++n0;
-    while (n1 * n0 < N && X[n1 * n0 * 3 + 2] == X[2]) ++n1;
-    if (N % (n0 * n1)) return false;
-    const int64_t n2 = N / (n0 * n1), nn[3] = {n0, n1, n2};
-    const int64_t step[3] = {1, n0, n0 * n1};
+    int64_t nn[3] = {1, 1, 1}, step[3] = {1, 1, 1};
+    // nodes with the coordinates of node 0 along all later axes
+    for (int d = 0; d + 1 < D; ++d) {
+        step[d + 1] = step[d];
+        const auto same = [&](int64_t n) {
+            for (int k = d + 1; k < D; ++k)
+                if (X[n * D + k] != X[k]) return false;
+            return true;
+        };
+        while (nn[d] * step[d] < N && same(nn[d] * step[d])) ++nn[d];
+        step[d + 1] = step[d] * nn[d];
+    }
+    if (N % step[D - 1]) return false;
+    nn[D - 1] = N / step[D - 1];
     const int64_t width = c->t_off[1];
-    if (width != 1 && width != 8) return false;
-    L.p = width == 1 ? 1 : 2;
+    L.dim = D;
+    L.p = 0;
+    for (int p = 1; p <= 4 - D + 1; ++p)
+        if (width == (D == 2 ? p * p : p * p * p)) L.p = p;
+    if (!L.p) return false;
     int64_t cells = 1, bases = 1;
     for (int d = 0; d < 3; ++d) {
-        if (nn[d] < 2 || nn[d] > 1 << 20) return false;
         L.nn[d] = (int)nn[d];
-        L.ne[d] = (int)nn[d] - 1;
-        L.nb[d] = L.ne[d] + L.p;
+        L.ne[d] = d < D ? (int)nn[d] - 1 : 1;
+        L.nb[d] = d < D ? L.ne[d] + L.p : 1;
+        if (d >= D) continue;
+        if (nn[d] < 2 || nn[d] > 1 << 20) return false;
         cells *= L.ne[d];
         bases *= L.nb[d];
         for (int e = 0; e < L.ne[d]; ++e) {
-            jac.push_back(0.5 * (X[(e + 1) * step[d] * 3 + d] - X[e * step[d] * 3 + d]));
+            jac.push_back(0.5 * (X[(e + 1) * step[d] * D + d] - X[e * step[d] * D + d]));
             if (!(jac.back() > 0.0)) return false;
         }
     }
     if (c->num_cells != cells || c->num_bases != bases) return false;
-    const double w = L.p == 1 ? 1.0 : 0.125;
+    const double* w1 = axis_weights(L.p);
+    const double tol = L.p == 3 ? 1e-15 : 0.0;
     for (int64_t n = 0, k = 0; n < N; ++n) {
-        const int64_t i[3] = {n % n0, n / n0 % n1, n / (n0 * n1)};
-        for (int d = 0; d < 3; ++d)
-            if (X[n * 3 + d] != X[i[d] * step[d] * 3 + d]) return false;
+        const int64_t i[3] = {n % nn[0], n / nn[0] % nn[1], n / (nn[0] * nn[1])};
+        for (int d = 0; d < D; ++d)
+            if (X[n * D + d] != X[i[d] * step[d] * D + d]) return false;
         if (c->t_off[n + 1] - c->t_off[n] != width) return false;
         for (int q = 0; q < width; ++q, ++k) {
-            const int64_t b = ((i[2] + (q >> 2)) * L.nb[1] + i[1] + (q >> 1 & 1)) * L.nb[0] + i[0] + (q & 1);
-            if (c->t_bases[k] != b || c->t_w[k] != w) return false;
+            const int a = q % L.p, b = q / L.p % L.p, z = q / (L.p * L.p);
+            const int64_t basis = ((i[2] + z) * L.nb[1] + i[1] + b) * L.nb[0] + i[0] + a;
+            const double w = w1[a] * w1[b] * (D == 3 ? w1[z] : 1.0);
+            if (c->t_bases[k] != basis || !(std::abs(c->t_w[k] - w) <= tol)) return false;
         }
     }
     static const int corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
                                      {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
+    const int npe = D == 2 ? 4 : 8;
     for (int64_t e = 0; e < cells; ++e) {
         const int64_t i = e % L.ne[0], j = e / L.ne[0] % L.ne[1], k = e / ((int64_t)L.ne[0] * L.ne[1]);
-        for (int a = 0; a < 8; ++a)
-            if (c->cells[e * 8 + a] != ((k + corner[a][2]) * n1 + j + corner[a][1]) * n0 + i + corner[a][0])
+        for (int a = 0; a < npe; ++a)
+            if (c->cells[e * npe + a] != ((k + corner[a][2]) * nn[1] + j + corner[a][1]) * nn[0] + i + corner[a][0])
                 return false;
     }
     // CSR rows: the full box of bases within p along every axis (the bulk set
@@ -712,7 +851,7 @@ bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
     for (int64_t b = 0; b < bases; ++b) {
         const int64_t i[3] = {b % L.nb[0], b / L.nb[0] % L.nb[1], b / ((int64_t)L.nb[0] * L.nb[1])};
         int64_t len = 1;
-        for (int d = 0; d < 3; ++d)
+        for (int d = 0; d < D; ++d)
             len *= std::min<int64_t>(i[d] + L.p, L.nb[d] - 1) - std::max<int64_t>(i[d] - L.p, 0) + 1;
         if (c->ulen[b] != len) return false;
     }
@@ -739,7 +878,9 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
     for (SetData& s : c->sets) {
         if (s.kind != 0 || !s.ig_off.empty() || s.neq != c->num_cells) continue;
         const int rule = s.bulk.integration_rule;
-        if (rule != FEM_GPU_RULE_HEX_2x2x2 && rule != FEM_GPU_RULE_HEX_3x3x3) continue;
+        if (c->dim == 3 ? rule != FEM_GPU_RULE_HEX_2x2x2 && rule != FEM_GPU_RULE_HEX_3x3x3
+                        : rule != FEM_GPU_RULE_QUAD_2x2 || !s.node_rho.empty())
+            continue;
         std::vector<char> seen(c->num_cells, 0);
         bool once = true, ordered = true;
         for (int64_t i = 0; i < s.neq; ++i) {
@@ -766,8 +907,9 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
     // linear splines); a device that cannot hold them keeps the element loop
     bool rho = false;
     for (const SetData& s : c->sets) rho |= s.lattice && !s.node_rho.empty();
-    const size_t want[3] = {K->p == 2 ? (size_t)243 * L.nn[2] * L.nn[1] * L.pitch : 0,
-                            K->p == 2 ? (size_t)6 * c->num_nodes : 0,
+    const bool quad = c->dim == 3 && K->p == 2;
+    const size_t want[3] = {quad ? (size_t)243 * L.nn[2] * L.nn[1] * L.pitch : 0,
+                            quad ? (size_t)6 * c->num_nodes : 0,
                             rho ? (size_t)kQN * (L.ne[0] + 2) * (L.ne[1] + 2) * (L.ne[2] + 2) : 0};
     DeviceBuf* const buf[3] = {&K->S, &K->vec, &K->Q};
     for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
@@ -803,12 +945,65 @@ void lattice_release(fem_gpu_ctx* c) {
     c->lattice = nullptr;
 }
 
+namespace {
+
+fem_gpu_status plane_assemble(fem_gpu_ctx* c, const Lattice& L, const SetData& s, const double* u, double* vals,
+                              double* rhs, bool acc_v, bool acc_r) {
+    PlaneArgs a{};
+    for (int d = 0; d < 2; ++d) {
+        a.ne[d] = L.ne[d];
+        a.nb[d] = L.nb[d];
+    }
+    a.E = (const double*)(s.d_latE.p ? s.d_latE.p : s.d_E.p);
+    a.jac = (const double*)L.jac.p;
+    a.u = rhs ? u : nullptr;
+    a.vals = vals;
+    a.rhs = rhs;
+    a.rowptr = (const int32_t*)c->d_rowptr.p;
+    a.acc_v = acc_v;
+    a.acc_r = acc_r;
+    a.status = (int*)c->d_status.p;
+    const double nu = s.bulk.poisson_ratio;
+    const double lam = s.bulk.model_type == FEM_GPU_MODEL_PLANE_STRESS ? nu / (1.0 - nu * nu)
+                                                                       : nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
+    a.mu = 1.0 / (2.0 * (1.0 + nu));
+    a.ld = (lam + a.mu) / a.mu;
+    a.lo = lam / a.mu;
+    // 1-D matrices from the rule's points along one axis (unit weights of the 2 x 2 rule)
+    const Rule r = gauss_rule(s.bulk.integration_rule);
+    double T[2][4] = {};  // extraction of the element's two nodes
+    for (int k = 0; k < L.p; ++k) T[0][k] = T[1][k + 1] = axis_weights(L.p)[k];
+    const double x = std::abs(r.pts[0]);
+    for (int i = 0; i <= L.p; ++i)
+        for (int j = 0; j <= L.p; ++j)
+            for (int n = 0; n < 2; ++n)
+                for (int m = 0; m < 2; ++m)
+                    for (const double q : {-x, x}) {
+                        const double sn = n ? 0.5 : -0.5, sm = m ? 0.5 : -0.5, w = T[n][i] * T[m][j];
+                        a.M[i][j] += w * (0.5 + sn * q) * (0.5 + sm * q);
+                        a.D[i][j] += w * sn * sm;
+                        a.G[i][j] += w * sn * (0.5 + sm * q);
+                    }
+    const unsigned g = (unsigned)((c->num_used + 31) / 32);
+    cudaStream_t st = (cudaStream_t)c->stream;
+    if (L.p == 1) lattice_plane<1><<<g, 96, 0, st>>>(a);
+    else if (L.p == 2) lattice_plane<2><<<g, 160, 0, st>>>(a);
+    else lattice_plane<3><<<g, 224, 0, st>>>(a);
+    c->launches++;
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? FEM_GPU_OK
+                            : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice launch: ") + cudaGetErrorString(e));
+}
+
+}  // namespace
+
 // One lattice set: CSR values (nullable) and residual (nullable) of the adof
 // vector u (nullable), stored, or added with acc_v / acc_r.
 fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs, bool acc_v,
                                 bool acc_r) {
     Lattice& L = *(Lattice*)c->lattice;
     const SetData& s = c->sets[set];
+    if (L.dim == 2) return plane_assemble(c, L, s, u, vals, rhs, acc_v, acc_r);
     cudaStream_t st = (cudaStream_t)c->stream;
     const int64_t nodes = (int64_t)L.nn[0] * L.nn[1] * L.nn[2];
     const bool quad = L.p == 2;

@@ -110,3 +110,51 @@ def test_non_finite_blocks_are_reported(torch):
             with pytest.raises(mg.FemGpuError) as e:
                 _assemble(torch, m, None)
             assert e.value.status == 3
+
+
+@pytest.mark.parametrize("p", [1, 2, 3])
+@pytest.mark.parametrize("ne", [(1, 1), (2, 3), (5, 1), (31, 2), (7, 33)], ids=lambda n: "x".join(map(str, n)))
+def test_plane_lattice_matches_oracle_and_element_loop(torch, ne, p):
+    prod, orc, _ = problem(2, ne, p, mg.SHAPE_RECTANGULAR, mg.RULE_QUAD_2x2, sides=True)
+    prod.finalize()
+    orc.finalize()
+    un = uniform01(37, prod.num_adofs) - 0.5
+    u = torch.tensor(un, device="cuda")
+    rp, _ = prod.graph()
+    vo, ro = orc.assemble(un)
+    vals, rhs = _assemble(torch, prod, u)
+    assert csr_row_rel_err(rp, vals.cpu().numpy(), vo) <= RTOL
+    assert rel_err(rhs.cpu().numpy(), ro) <= RTOL
+    assert rel_err(_assemble(torch, prod, u, mg.NO_JACOBIAN)[1].cpu().numpy(), ro) <= RTOL
+    v2, r2 = _assemble(torch, prod, u, mg.ACCUMULATE, vals.clone(), rhs.clone())
+    assert csr_row_rel_err(rp, v2.cpu().numpy(), 2 * vo) <= RTOL and rel_err(r2.cpu().numpy(), 2 * ro) <= RTOL
+    prod.set_variant(0, 2)
+    vg, rg = _assemble(torch, prod, u)
+    assert csr_row_rel_err(rp, vals.cpu().numpy(), vg.cpu().numpy()) <= RTOL
+    assert rel_err(rhs.cpu().numpy(), rg.cpu().numpy()) <= RTOL
+
+
+@pytest.mark.parametrize("p", [1, 2, 3])
+def test_plane_stress_graded_lattice(torch, p):
+    """Plane stress, graded cells, cells in another order, matrix-free product."""
+    mesh = mg.hmr_uniform_mesh(2, (9, 6), (1.0, 0.7), p)
+    x = mesh["coords"]
+    x[:, 1] = x[:, 1] ** 2 + 0.2 * x[:, 1]
+    nc = len(mesh["cells"])
+    order = np.random.default_rng(2).permutation(nc).astype(np.int32)
+    out = []
+    for pin in (False, True):
+        m = mg.FemModel(2, mesh, mg.SHAPE_RECTANGULAR)
+        m.add_bulk_set(order, uniform01(3, nc) + 0.1, 0.2, mg.RULE_QUAD_2x2, mg.MODEL_PLANE_STRESS)
+        m.finalize()
+        if pin:
+            m.set_variant(0, 2)
+        u = torch.tensor(uniform01(5, m.num_adofs) - 0.5, device="cuda")
+        vals, rhs = _assemble(torch, m, u)
+        y = torch.full_like(u, float("nan"))
+        m.apply(u, y)
+        torch.cuda.synchronize()
+        out.append([t.cpu().numpy() for t in (vals, rhs, y)])
+    rp, _ = m.graph()
+    assert csr_row_rel_err(rp, out[0][0], out[1][0]) <= RTOL
+    assert rel_err(out[0][1], out[1][1]) <= RTOL and rel_err(out[0][2], out[1][2]) <= RTOL
