@@ -1,5 +1,6 @@
 // fem_brick.cu -- XFEM clusters on axis-aligned brick cells: uncut cells, cut
-// clusters, Nitsche interfaces inside one cell and ghost faces.
+// clusters, Nitsche interfaces inside one cell, ghost faces and (linear splines)
+// boundary facets.
 //
 // The general cluster kernel (fem_cluster.cu) forms every element matrix from
 // per-point operators and projects it through column lists.  On bricks with
@@ -35,6 +36,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <thread>
 
@@ -44,7 +46,8 @@
 namespace fem {
 namespace {
 
-enum { KIND_UNCUT = 0, KIND_CUT = 1, KIND_GHOST = 2, KIND_INTERFACE = 3 };
+enum { KIND_UNCUT = 0, KIND_CUT = 1, KIND_GHOST = 2, KIND_INTERFACE = 3, KIND_SIDE = 4 };
+__host__ __device__ constexpr int sides_of(int kind) { return kind == KIND_GHOST || kind == KIND_INTERFACE ? 2 : 1; }
 
 struct BrickArgs {
     int64_t n;             // equation objects
@@ -58,8 +61,9 @@ struct BrickArgs {
     const uint16_t* sidx;  // [neq][sides W][sides W]
     const double* gp;      // integration cell / facet points
     const double* gw;
-    int ngp, normal_field;
+    int ngp, normal_field, neumann;
     double lam_c, mu_c, alpha, beta;
+    double value[3], thickness;  // boundary facets
     const double* tab;     // uncut: 63 reference sums; ghost: kGhostTab per face
     const int64_t* off;    // integration cells / facets of an object
     const double* x;       // their vertex coordinates
@@ -522,9 +526,72 @@ __device__ __forceinline__ void interface_block(const InterfaceCoef& c, const do
         }
 }
 
+// ---------------------------------------------------------------------------
+// boundary facet: the Nitsche terms of IWG_Isotropic_Struc_Linear_Dirichlet with
+// M = I (..._Dirichlet.cpp:52-240).  On a brick face n = +-e_k, and with
+// I_i(a, b) = integral N_a dN_b/dx_i, NN(a, b) = integral N_a N_b (w* includes the
+// thickness) the traction of column b has the entries
+//   T(k, k) = (lam + 2 mu) n I_k,  T(t, t) = mu n I_k,  T(k, t) = lam n I_t,
+//   T(t, k) = mu n I_t,
+// K = -T(a, b) + beta T(b, a)^T + gamma NN, gamma = alpha E / h, h = sqrt(4 A / pi).  A
+// constant displacement has no traction, so the residual is K (u - g); the
+// Neumann residual is -t integral N_a.
+// Bound by the atomics of the 24 x 24 blocks, a warp per facet: with the general
+// side kernel (a CTA per facet, operators per point) the two faces of 9,216 facets
+// of a 96^3 density model cost 231 us more: 3563 -> 3332 us for its assembly.
+struct SideCoef {
+    int k;
+    double kk, tt, lam[3], mu[3], nn;  // scales of I_k, I_k, I_t, I_t, NN
+};
+__device__ SideCoef side_coef(const BrickArgs& p, int64_t e, int ord, int lane) {
+    SideCoef c;
+    c.k = ord == 1 || ord == 3 ? 0 : ord == 0 || ord == 2 ? 1 : 2;
+    const bool up = ord == 1 || ord == 2 || ord == 5;
+    const double* X = p.xe + e * 24;
+    const double j = 0.5 * (X[18 + lane % 3] - X[lane % 3]), r = 1.0 / j;
+    const double area = shfl(j, c.k == 0 ? 1 : 0) * shfl(j, c.k == 2 ? 1 : 2);  // detJ of the face
+    const double E = p.E[e], w = area * p.thickness;
+    const double s = up ? w * E : -w * E;
+    const double rk = shfl(r, c.k);
+    c.kk = (p.lam_c + 2.0 * p.mu_c) * s * rk;
+    c.tt = p.mu_c * s * rk;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const double ri = s * shfl(r, i);
+        c.lam[i] = p.lam_c * ri;
+        c.mu[i] = p.mu_c * ri;
+    }
+    c.nn = p.neumann ? w : p.alpha * E * w / sqrt(16.0 * area / 3.14159265358979323846);
+    return c;
+}
+__device__ __forceinline__ void side_block(const SideCoef& c, const double* tab, double beta, int a, int b,
+                                           double K[9]) {
+    double ab[3], ba[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        ab[i] = __ldg(tab + i * 64 + b * 8 + a);
+        ba[i] = beta * __ldg(tab + i * 64 + a * 8 + b);
+    }
+    const double ik = c.k == 0 ? ab[0] : c.k == 1 ? ab[1] : ab[2], jk = c.k == 0 ? ba[0] : c.k == 1 ? ba[1] : ba[2];
+    const double nn = c.nn * __ldg(tab + 192 + b * 8 + a);
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            double v = 0.0;
+            if (f == g) v = fma(f == c.k ? c.kk : c.tt, jk - ik, nn);
+            else if (f == c.k) v = fma(c.mu[g], ba[g], -c.lam[g] * ab[g]);
+            else if (g == c.k) v = fma(c.lam[f], ba[f], -c.mu[f] * ab[f]);
+            K[f * 3 + g] = v;
+        }
+}
+
 template <int KIND>
 __host__ __device__ constexpr int warp_doubles() {
-    return KIND == KIND_UNCUT ? 64 : KIND == KIND_CUT ? 32 * kPt + 64 : KIND == KIND_GHOST ? 2 : kIfSmem;
+    return KIND == KIND_UNCUT       ? 64
+           : KIND == KIND_CUT       ? 32 * kPt + 64
+           : KIND == KIND_INTERFACE ? kIfSmem
+                                    : 2;
 }
 
 // ---------------------------------------------------------------------------
@@ -548,7 +615,7 @@ __global__ void __launch_bounds__(32 * warps_of<KIND>()) brick_linear(BrickArgs 
     const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
     if (w >= p.n) return;
     const int64_t e = p.list[w];
-    constexpr int SIDES = KIND <= KIND_CUT ? 1 : 2;
+    constexpr int SIDES = sides_of(KIND);
     // lane -> row node and the columns it takes: bulk (a, pair of b), double
     // (side, a, other side) with all eight b
     const int s = SIDES == 1 ? 0 : lane >> 4, s2 = SIDES == 1 ? 0 : lane & 1;
@@ -580,6 +647,13 @@ __global__ void __launch_bounds__(32 * warps_of<KIND>()) brick_linear(BrickArgs 
         gtab = p.tab + face * kGhostTab;
     }
     if (KIND == KIND_INTERFACE) ic = interface_coef(p, e, area, s, s2, 1.0);
+    SideCoef sd;
+    if (KIND == KIND_SIDE) {
+        const int ord = p.code[e] - kFastSide;
+        sd = side_coef(p, e, ord, lane);
+        gtab = p.tab + ord * kSideTab;
+        for (int f = 0; f < 3; ++f) ua[f] -= p.value[f];
+    }
     const double ld = (p.lam_c + p.mu_c) / p.mu_c, lo = p.lam_c / p.mu_c;
 #pragma unroll 2
     for (int t = 0; t < nb; ++t) {
@@ -589,6 +663,14 @@ __global__ void __launch_bounds__(32 * warps_of<KIND>()) brick_linear(BrickArgs 
         if (KIND == KIND_CUT) bulk_block(ws + 32 * kPt, gt, a, b, ld, lo, K);
         if (KIND == KIND_GHOST) ghost_block(gc, gtab, b, lane, p.normal_field, K);
         if (KIND == KIND_INTERFACE) interface_block(ic, ws, a, b, K);
+        if (KIND == KIND_SIDE) {
+            if (p.neumann) {
+                const double nn = sd.nn * __ldg(gtab + 192 + b * 8 + a);
+                for (int f = 0; f < 3; ++f) r[f] = fma(-nn, p.value[f], r[f]);
+                continue;
+            }
+            side_block(sd, gtab, p.beta, a, b, K);
+        }
         // the lane that holds column node b (of side s2)
         const int src = SIDES == 1 ? b * 4 : s2 * 16 + b * 2;
         const int cb = __shfl_sync(0xffffffffu, col, src);
@@ -625,7 +707,7 @@ __global__ void __launch_bounds__(32 * warps_of<KIND>()) brick_linear(BrickArgs 
 // additions) and P^T (K P) the same way along the rows, scattered as it is formed.
 template <int KIND>
 struct QuadLayout {
-    static constexpr int SIDES = KIND <= KIND_CUT ? 1 : 2, NP = 24 * SIDES, NA = 81 * SIDES;
+    static constexpr int SIDES = sides_of(KIND), NP = 24 * SIDES, NA = 81 * SIDES;
     static constexpr int K = 0, KT = K + NP * NP, R = KT + NP * NA, WS = R + NP, END = WS + warp_doubles<KIND>();
     static constexpr size_t bytes = (size_t)END * 8 + 576 + SIDES * (27 + 27 * 4 * 4) + 64 +
                                     (size_t)(27 * SIDES) * (27 * SIDES) * 2;
@@ -903,9 +985,15 @@ void brick_classify(const fem_gpu_ctx* c, SetData& s) {
     s.fast.clear();
     s.fmap.clear();
     const int sides = s.kind == 2 ? 2 : 1;
-    if (c->dim != 3 || c->shape != FEM_GPU_SHAPE_RECTANGULAR || s.kind == 1 || s.neq == 0) return;
+    if (c->dim != 3 || c->shape != FEM_GPU_SHAPE_RECTANGULAR || s.neq == 0) return;
     if (!s.node_rho.empty()) return;
     const int W = s.maxnb;
+    if (s.kind == 1) {
+        // boundary facets: linear splines, the whole projection
+        if (W != 8 || s.side.integration_rule != FEM_GPU_RULE_QUAD_2x2) return;
+        for (int k = 0; k < 9; ++k)
+            if (s.side_select[k] != (k % 4 ? 0.0 : 1.0)) return;
+    }
     if ((W != 8 && W != 27) || (s.kind == 0 && s.bulk.model_type != FEM_GPU_MODEL_3D)) return;
     if (s.kind == 0 && !s.ig_off.empty() && s.bulk.ig_cell_type != FEM_GPU_CELL_TET4) return;
     const bool iface = s.kind == 2 && !is_ghost_iwg(s.dside.iwg_type);
@@ -919,7 +1007,9 @@ void brick_classify(const fem_gpu_ctx* c, SetData& s) {
             ok = s.nb[r] == W && brick(&s.xe[r * 24]) && extraction_map(&s.T[r * 8 * W], W, W, &s.fmap[r * W]);
         }
         if (!ok) return;
-        if (s.kind == 0) {
+        if (s.kind == 1) {
+            s.fast[i] = (uint8_t)(kFastSide + s.ordinal[i]);
+        } else if (s.kind == 0) {
             s.fast[i] = kFastBulk;
         } else if (iface) {
             const int64_t a = s.fc_off[i] * 9, b = s.fc_off[i + 1] * 9;
@@ -976,6 +1066,25 @@ fem_gpu_status brick_upload(fem_gpu_ctx* c, SetData& s) {
                     tab[pair_off(i, j) + t] = sum;
                 }
             }
+    } else if (s.kind == 1) {
+        const Rule r = gauss_rule(s.side.integration_rule);
+        tab.assign((size_t)6 * kSideTab, 0.0);
+        for (int o = 0; o < 6; ++o) {
+            const int k = o == 1 || o == 3 ? 0 : o == 0 || o == 2 ? 1 : 2, t1 = k == 0 ? 1 : 0, t2 = k == 2 ? 1 : 2;
+            for (int q = 0; q < r.n; ++q) {
+                double xi[3], N[8], dN[24];
+                xi[k] = o == 1 || o == 2 || o == 5 ? 1.0 : -1.0;
+                xi[t1] = r.pts[q * 2];
+                xi[t2] = r.pts[q * 2 + 1];
+                lagrange(FEM_GPU_CELL_HEX8, xi, N, dN);
+                for (int b = 0; b < 8; ++b)
+                    for (int a = 0; a < 8; ++a) {
+                        double* t = &tab[(size_t)o * kSideTab + b * 8 + a];
+                        for (int i = 0; i < 3; ++i) t[i * 64] += r.w[q] * N[a] * dN[i * 8 + b];
+                        t[192] += r.w[q] * N[a] * N[b];
+                    }
+            }
+        }
     } else if (s.kind == 2 && is_ghost_iwg(s.dside.iwg_type)) {
         const Rule r = gauss_rule(s.dside.integration_rule);
         tab.assign((size_t)6 * kGhostTab, 0.0);
@@ -999,17 +1108,22 @@ fem_gpu_status brick_upload(fem_gpu_ctx* c, SetData& s) {
             }
         }
     }
-    cudaError_t e = upload(s.d_fast, s.fast, st);
-    if (e == cudaSuccess) e = upload(s.d_fmap, s.fmap, st);
-    if (e == cudaSuccess) e = upload(s.d_flist, s.flist, st);
-    if (e == cudaSuccess) e = upload(s.d_ftab, tab, st);
+    // tables, list, kinds and maps in one buffer
+    const size_t nt = tab.size() * sizeof(double), nl = s.flist.size() * sizeof(int32_t);
+    std::vector<uint8_t> all(nt + nl + s.fast.size() + s.fmap.size());
+    if (nt) std::memcpy(all.data(), tab.data(), nt);
+    std::memcpy(all.data() + nt, s.flist.data(), nl);
+    std::memcpy(all.data() + nt + nl, s.fast.data(), s.fast.size());
+    std::memcpy(all.data() + nt + nl + s.fast.size(), s.fmap.data(), s.fmap.size());
+    s.ftab_bytes = nt;
+    cudaError_t e = upload(s.d_fast, all, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? FEM_GPU_OK
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("brick data: ") + cudaGetErrorString(e));
 }
 
 void brick_release(SetData& s) {
-    for (DeviceBuf* b : {&s.d_fast, &s.d_fmap, &s.d_flist, &s.d_ftab}) dfree(*b);
+    dfree(s.d_fast);
 }
 
 int64_t brick_count(const SetData& s, int64_t first, int64_t count) {
@@ -1025,9 +1139,11 @@ fem_gpu_status brick_launch(fem_gpu_ctx* c, const SetData& s, int64_t first, int
     cudaStream_t st = (cudaStream_t)stream;
     BrickArgs a{};
     a.n = n;
-    a.list = (const int32_t*)s.d_flist.p + (std::lower_bound(s.flist.begin(), s.flist.end(), first) - s.flist.begin());
-    a.code = (const uint8_t*)s.d_fast.p;
-    a.map = (const uint8_t*)s.d_fmap.p;
+    const uint8_t* data = (const uint8_t*)s.d_fast.p;
+    a.list = (const int32_t*)(data + s.ftab_bytes) +
+             (std::lower_bound(s.flist.begin(), s.flist.end(), first) - s.flist.begin());
+    a.code = data + s.ftab_bytes + s.flist.size() * sizeof(int32_t);
+    a.map = a.code + s.fast.size();
     a.xe = (const double*)s.d_xe.p;
     a.E = (const double*)s.d_E.p;
     a.bases = (const int32_t*)s.d_bases.p;
@@ -1035,7 +1151,7 @@ fem_gpu_status brick_launch(fem_gpu_ctx* c, const SetData& s, int64_t first, int
     a.gp = (const double*)s.d_gp.p;
     a.gw = (const double*)s.d_gw.p;
     a.ngp = s.ngp;
-    a.tab = (const double*)s.d_ftab.p;
+    a.tab = (const double*)data;
     a.rowptr = (const int32_t*)c->d_rowptr.p;
     a.ulen = (const int32_t*)c->d_ulen.p;
     a.nu = c->num_used;
@@ -1043,7 +1159,9 @@ fem_gpu_status brick_launch(fem_gpu_ctx* c, const SetData& s, int64_t first, int
     a.vals = vals;
     a.rhs = rhs;
     a.status = (int*)c->d_status.p;
-    const double nu = s.kind == 0 ? s.bulk.poisson_ratio : s.dside.poisson_ratio;
+    const double nu = s.kind == 0   ? s.bulk.poisson_ratio
+                      : s.kind == 1 ? s.side.poisson_ratio
+                                    : s.dside.poisson_ratio;
     a.lam_c = nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
     a.mu_c = 1.0 / (2.0 * (1.0 + nu));
     int kind = KIND_UNCUT;
@@ -1052,6 +1170,14 @@ fem_gpu_status brick_launch(fem_gpu_ctx* c, const SetData& s, int64_t first, int
         a.off = (const int64_t*)s.d_igoff.p;
         a.x = (const double*)s.d_igx.p;
         a.xi = (const double*)s.d_igxi.p;
+    } else if (s.kind == 1) {
+        kind = KIND_SIDE;
+        a.neumann = s.side.iwg_type == FEM_GPU_IWG_STRUC_LINEAR_NEUMANN;
+        a.beta = s.side.iwg_type == FEM_GPU_IWG_STRUC_LINEAR_DIRICHLET_SYMMETRIC_NITSCHE ? -1.0 : 1.0;
+        a.alpha = s.side.nitsche_alpha;
+        a.thickness = s.side_thickness;
+        for (int d = 0; d < 3; ++d) a.value[d] = s.side.value[d];
+        if (a.neumann) a.vals = nullptr;  // K = 0
     } else {
         kind = is_ghost_iwg(s.dside.iwg_type) ? KIND_GHOST : KIND_INTERFACE;
         a.normal_field = s.dside.iwg_type == FEM_GPU_IWG_GHOST_NORMAL_FIELD;
@@ -1066,7 +1192,7 @@ fem_gpu_status brick_launch(fem_gpu_ctx* c, const SetData& s, int64_t first, int
     using Fn = void (*)(BrickArgs);
     cudaError_t e = cudaSuccess;
     if (s.maxnb == 8) {
-        static const Fn fn[4] = {brick_linear<0>, brick_linear<1>, brick_linear<2>, brick_linear<3>};
+        static const Fn fn[5] = {brick_linear<0>, brick_linear<1>, brick_linear<2>, brick_linear<3>, brick_linear<4>};
         const int w = kind == KIND_INTERFACE ? warps_of<KIND_INTERFACE>() : warps_of<KIND_UNCUT>();
         fn[kind]<<<(unsigned)((n + w - 1) / w), 32 * w, 0, st>>>(a);
     } else {

@@ -14,10 +14,13 @@ namespace fem {
 //   1        bulk cell or cluster
 //   2 + face ghost on a whole cell face; face = 2 axis + (leader side up)
 //   8        interface inside one cell (both sides the same brick)
-constexpr uint8_t kFastBulk = 1, kFastGhost = 2, kFastInterface = 8;
+//   10 + ord boundary facet of ordinal ord (Neumann, Nitsche Dirichlet)
+constexpr uint8_t kFastBulk = 1, kFastGhost = 2, kFastInterface = 8, kFastSide = 10;
 
 // ghost tables: per face 7 matrices over (b, lane), lane = (side, node, other side)
 constexpr int kGhostMats = 7, kGhostTab = kGhostMats * 256;
+// boundary tables: per ordinal the face integrals N_a dN_b (3) and N_a N_b over (b, a)
+constexpr int kSideTab = 4 * 64;
 
 void brick_classify(const fem_gpu_ctx* c, SetData& s);
 fem_gpu_status brick_upload(fem_gpu_ctx* c, SetData& s);

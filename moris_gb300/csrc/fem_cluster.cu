@@ -1279,7 +1279,8 @@ fem_gpu_status enqueue_batch(fem_gpu_ctx* c, Batch* b, const double* u, double* 
         r = launch(c, k, a, st);
     }
     for (size_t s = 0; s < c->sets.size() && r == FEM_GPU_OK; ++s)
-        r = brick_launch(c, c->sets[s], 0, c->sets[s].neq, u, vals, rhs, st);
+        if (c->sets[s].kind != 1)  // boundary facets follow below
+            r = brick_launch(c, c->sets[s], 0, c->sets[s].neq, u, vals, rhs, st);
     for (size_t s = 0; s < c->sets.size() && r == FEM_GPU_OK; ++s)
         if (c->sets[s].kind == 1 && c->sets[s].neq > 0) r = side(c, (int)s, u, vals, rhs, st);
     return r;

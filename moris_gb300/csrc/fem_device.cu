@@ -1155,6 +1155,8 @@ fem_gpu_status launch_side(fem_gpu_ctx* c, int si, int mode, int64_t first, int6
     if (count <= 0) return FEM_GPU_OK;
     SetData& s = c->sets[si];
     SetData& ds = s;
+    if (mode == MODE_ASSEMBLE && brick_count(s, first, count) == count)
+        return brick_launch(c, s, first, count, u, vals, rhs, c->stream);
     SideArgs a{};
     a.ns = count;
     a.iwg = s.side.iwg_type;
@@ -1543,7 +1545,7 @@ fem_gpu_status device_finalize(fem_gpu_ctx* c) {
     if ((st = lattice_finalize(c)) != FEM_GPU_OK) return st;
     for (size_t k = 0; k < c->sets.size(); ++k) {
         SetData& s = c->sets[k];
-        if (s.kind != 0 || !s.ig_off.empty() || s.lattice) continue;
+        if (s.kind == 2 || !s.ig_off.empty() || s.lattice) continue;
         brick_classify(c, s);
         if ((st = brick_upload(c, s)) != FEM_GPU_OK) return st;
     }

@@ -91,7 +91,8 @@ struct SetData {
     bool pinned = false;    // variant chosen by fem_gpu_set_variant: that kernel assembles the set
     std::vector<uint8_t> fast, fmap;  // brick kernels (fem_brick.cu): kind per equation object, column maps
     std::vector<int32_t> flist;       // their equation objects
-    DeviceBuf d_fast, d_fmap, d_flist, d_ftab;
+    DeviceBuf d_fast;                 // their tables (ftab_bytes), list, kinds and maps
+    size_t ftab_bytes = 0;
     bool lattice = false;   // the set covers a tensor lattice (fem_lattice.cu)
     DeviceBuf d_latE, d_latrho;  // lattice sets: modulus in cell order (if the set's order differs), nodal densities
     double tuned_ms = 0.0;  // time of the chosen variant on the tuning run

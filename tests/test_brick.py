@@ -130,3 +130,36 @@ def test_xfem_clusters_match_oracle(torch, order, n, rule, tri, ghost, mixed):
     check()
     vh, rh = prod.assemble_host(un)
     assert csr_row_rel_err(rp, vh, vo) <= RTOL and rel_err(rh, ro) <= RTOL
+
+
+@pytest.mark.parametrize("iwg", [mg.IWG_STRUC_LINEAR_NEUMANN, mg.IWG_STRUC_LINEAR_DIRICHLET_SYMMETRIC_NITSCHE,
+                                 mg.IWG_STRUC_LINEAR_DIRICHLET_UNSYMMETRIC_NITSCHE])
+@pytest.mark.parametrize("ordinal", range(6))
+def test_boundary_facets_match_oracle(torch, iwg, ordinal):
+    """Every facet of a brick, unequal edges, prescribed value and thickness."""
+    from oracle import OracleModel
+    mesh = mg.hmr_uniform_mesh(3, (3, 2, 4), (1.0, 0.7, 1.9), 1)
+    mesh["coords"][:, 2] *= 0.5 + mesh["coords"][:, 2]
+    nc = len(mesh["cells"])
+    cells = np.arange(nc, dtype=np.int32)
+    E = uniform01(6, nc) + 0.2
+    prod = mg.FemModel(3, mesh, mg.SHAPE_RECTANGULAR)
+    orc = OracleModel(3, mg.CELL_HEX8, mg.SHAPE_RECTANGULAR, mesh)
+    prod.add_bulk_set(cells, E, 0.3, mg.RULE_HEX_2x2x2, mg.MODEL_3D)
+    orc.add_bulk_set(mg.CELL_HEX8, mg.RULE_HEX_2x2x2, mg.MODEL_3D, cells, E, 0.3)
+    some, val = cells[::2], (0.02, -0.01, 0.03)
+    prod.add_side_set(iwg, some, np.full(len(some), ordinal), E[some], 0.25, mg.RULE_QUAD_2x2, mg.MODEL_3D, alpha=20.0,
+                      value=val, thickness=0.8)
+    orc.add_side_set(iwg, mg.RULE_QUAD_2x2, mg.MODEL_3D, some, np.full(len(some), ordinal), E[some], 0.25, 20.0, val)
+    orc.set_side_options(0, 0.8, None)
+    prod.finalize()
+    orc.finalize()
+    un = uniform01(8, prod.num_adofs) - 0.5
+    rp, _ = prod.graph()
+    vals = torch.empty(prod.nnz, dtype=torch.float64, device="cuda")
+    rhs = torch.empty(prod.num_adofs, dtype=torch.float64, device="cuda")
+    for u in (un, np.zeros_like(un)):
+        vo, ro = orc.assemble(u)
+        prod.assemble(torch.tensor(u, device="cuda") if u is un else None, vals, rhs)
+        assert csr_row_rel_err(rp, vals.cpu().numpy(), vo) <= RTOL
+        assert rel_err(rhs.cpu().numpy(), ro) <= RTOL
