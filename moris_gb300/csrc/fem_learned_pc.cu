@@ -32,6 +32,7 @@
 
 #include "fem_conv_umma.cuh"
 #include "fem_internal.hpp"
+#include "fem_reduce.cuh"
 #include "fem_spmv.cuh"
 
 namespace {
@@ -725,23 +726,7 @@ __global__ void density_channel_kernel(int nf, int nc, int F, const double* rho,
 }
 
 // ---- flexible CG building blocks -------------------------------------------
-__device__ __forceinline__ double warp_sum_d(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ void block_sum_add(double v, double* out) {
-    __shared__ double red[32];
-    v = warp_sum_d(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
-        v = warp_sum_d(v);
-        if (lane == 0) atomicAdd(out, v);
-    }
-}
+constexpr int kFcgThreads = 256;
 
 __global__ void fcg_spmv_dot(int64_t n, const int32_t* rp, const int32_t* ci, const double* v, const double* p,
                              double* q, double* dot) {
@@ -757,7 +742,8 @@ __global__ void fcg_spmv_dot(int64_t n, const int32_t* rp, const int32_t* ci, co
             acc = fma(s, p[row], acc);
         }
     }
-    block_sum_add(acc, dot);
+    const double sum[1] = {acc};
+    fem::block_sum_add<kFcgThreads, fem::kLanesPerRow, 1>(sum, {dot});
 }
 
 
@@ -814,13 +800,17 @@ __global__ void fcg_residual(int64_t n, const int32_t* rp, const int32_t* ci, co
             bb = fma(b[row], b[row], bb);
         }
     }
-    block_sum_add(rr, dots);
-    block_sum_add(bb, dots + 1);
+    const double sum[2] = {rr, bb};
+    fem::block_sum_add<kFcgThreads, fem::kLanesPerRow, 2>(sum, {dots, dots + 1});
 }
 
 constexpr int kMaxM = 16;
+constexpr int kFcgSums = kMaxM + 3;
 struct VecSet {
     const double* v[kMaxM];
+};
+struct Coef {
+    double c[kMaxM];
 };
 
 // dots[j] += z . q_j for j < m
@@ -831,27 +821,33 @@ __global__ void fcg_multi_dot(int64_t n, const double* z, VecSet q, int m, doubl
         const double zi = z[i];
         for (int j = 0; j < m; ++j) acc[j] = fma(zi, q.v[j][i], acc[j]);
     }
-    for (int j = 0; j < m; ++j) block_sum_add(acc[j], dots + j);
+    for (int j = 0; j < m; ++j) {
+        const double sum[1] = {acc[j]};
+        if (j) __syncthreads();
+        fem::block_sum_add<kFcgThreads, 1, 1>(sum, {dots + j});
+    }
 }
-
-// p = z - sum_j c_j p_j ; dots[0] += p . r (alpha numerator)
-struct Coef {
-    double c[kMaxM];
-};
-__global__ void fcg_orthogonalize(int64_t n, const double* z, VecSet pj, Coef c, int m, const double* r, double* p,
-                                  double* dots) {
+// p = z - sum_j (dots[j] / pq of direction j) p_j; pr += p.r
+__global__ void fcg_orthogonalize(int64_t n, const double* z, VecSet pj, Coef pq, int m, const double* dots,
+                                  const double* r, double* p, double* pr_out) {
     double pr = 0.0;
+    double c[kMaxM];
+    for (int j = 0; j < m; ++j) c[j] = dots[j] / pq.c[j];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double v = z[i];
-        for (int j = 0; j < m; ++j) v = fma(-c.c[j], pj.v[j][i], v);
+        for (int j = 0; j < m; ++j) v = fma(-c[j], pj.v[j][i], v);
         p[i] = v;
         pr = fma(v, r[i], pr);
     }
-    block_sum_add(pr, dots);
+    const double sum[1] = {pr};
+    fem::block_sum_add<kFcgThreads, 1, 1>(sum, {pr_out});
 }
-
-// x += a p; r -= a q; dots[0] += r.r
-__global__ void fcg_step(int64_t n, double a, double* x, const double* p, double* r, const double* q, double* dots) {
+// x += a p, r -= a q with a = pr / pAp, rr += r.r; nothing on a breakdown (the host
+// reads the three sums after this kernel, once per iteration)
+__global__ void fcg_step(int64_t n, const double* pr, const double* pAp, double* x, const double* p, double* r,
+                         const double* q, double* rr_out) {
+    if (!(*pAp > 0.0) || !isfinite(*pr)) return;
+    const double a = *pr / *pAp;
     double rr = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         x[i] = fma(a, p[i], x[i]);
@@ -859,7 +855,8 @@ __global__ void fcg_step(int64_t n, double a, double* x, const double* p, double
         r[i] = rn;
         rr = fma(rn, rn, rr);
     }
-    block_sum_add(rr, dots);
+    const double sum[1] = {rr};
+    fem::block_sum_add<kFcgThreads, 1, 1>(sum, {rr_out});
 }
 
 }  // namespace
@@ -986,12 +983,17 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
         if (e == cudaSuccess) bufs.push_back(*ptr);
         return e;
     };
-    cudaError_t e = alloc((void**)&r, n * 8);
-    if (e == cudaSuccess) e = alloc((void**)&z, n * 8);
-    if (e == cudaSuccess) e = alloc((void**)&dinv, n * 8);
-    if (e == cudaSuccess) e = alloc((void**)&dots, kMaxM * 8);
-    if (e == cudaSuccess) e = alloc((void**)&P, (size_t)(M + 1) * n * 8);
-    if (e == cudaSuccess) e = alloc((void**)&Q, (size_t)(M + 1) * n * 8);
+    // r, z, 1/diag, M + 1 directions p and products q, the sums: one allocation
+    double* work = nullptr;
+    cudaError_t e = alloc((void**)&work, ((size_t)(2 * M + 5) * n + kFcgSums) * 8);
+    if (e == cudaSuccess) {
+        r = work;
+        z = r + n;
+        dinv = z + n;
+        P = dinv + n;
+        Q = P + (size_t)(M + 1) * n;
+        dots = Q + (size_t)(M + 1) * n;
+    }
     if (cnn && e == cudaSuccess) {
         e = alloc((void**)&cin, cnn->V * 4 * sizeof(float));
         if (e == cudaSuccess) e = cudaMemset(cin, 0, cnn->V * 4 * sizeof(float));
@@ -1005,14 +1007,10 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
         cleanup();
         return fail(c, FEM_GPU_OUT_OF_MEMORY, "fcg workspace");
     }
-    const int tpb = 256;
+    const int tpb = kFcgThreads;
     const unsigned rb = (unsigned)std::min<int64_t>((n * fem::kLanesPerRow + tpb - 1) / tpb, (int64_t)sm_count() * 16);
-    const unsigned vb = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 16);
-    double hd[kMaxM];
-    auto readn = [&](int k) {
-        cudaMemcpy(hd, dots, k * sizeof(double), cudaMemcpyDeviceToHost);
-        cudaMemset(dots, 0, kMaxM * 8);
-    };
+    const unsigned vb = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 4);
+    double hd[3];
     const int nc = cnn ? cnn->n : 0;
     // with the V-cycle as base, a stalled learned correction is switched off
     // after kNetWindow iterations without a 10 % residual reduction and the
@@ -1039,10 +1037,10 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
     };
     if (cnn && node_density) density_channel_kernel<<<lpc_grid((int64_t)nc * nc * nc), 256>>>(nf, nc, factor,
                                                                                                 node_density, cin);
-    cudaMemset(dots, 0, kMaxM * 8);
+    cudaMemset(dots, 0, kFcgSums * 8);
     fcg_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb>>>(n, rowptr, colidx, vals, dinv);
     fcg_residual<<<rb, tpb>>>(n, rowptr, colidx, vals, b, x, r, dots);
-    readn(2);
+    cudaMemcpy(hd, dots, 2 * sizeof(double), cudaMemcpyDeviceToHost);
     const double bn = std::sqrt(hd[1] > 0 ? hd[1] : 1.0);
     double rn = std::sqrt(hd[0]);
     const double tol = opts->rel_tol * bn;
@@ -1063,40 +1061,33 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
             qs.v[j] = Q + (int64_t)slot * n;
             ps.v[j] = P + (int64_t)slot * n;
         }
-        if (m > 0) {
-            fcg_multi_dot<<<vb, tpb>>>(n, z, qs, m, dots);
-            readn(m);
-            for (int j = 0; j < m; ++j) {
-                const int slot = (it - 1 - j + (M + 1) * 4) % (M + 1);
-                cf.c[j] = hd[j] / pq[slot];
-            }
-        }
+        // dots: z.q_j of the m directions, then p.r, p.Ap and r.r
+        double* sums = dots + kMaxM;
+        cudaMemsetAsync(dots, 0, kFcgSums * 8, 0);
+        for (int j = 0; j < m; ++j) cf.c[j] = pq[(it - 1 - j + (M + 1) * 4) % (M + 1)];
+        if (m > 0) fcg_multi_dot<<<vb, tpb>>>(n, z, qs, m, dots);
         const int cur = it % (M + 1);
         double* p = P + (int64_t)cur * n;
         double* q = Q + (int64_t)cur * n;
-        fcg_orthogonalize<<<vb, tpb>>>(n, z, ps, cf, m, r, p, dots);
-        readn(1);
-        const double pr = hd[0];
+        fcg_orthogonalize<<<vb, tpb>>>(n, z, ps, cf, m, dots, r, p, sums);
         if (mg) {
             // the level-0 stencil of the hierarchy is the CSR's operator without indices
-            if (!mg_operator(mg, p, q, dots)) {
+            if (!mg_operator(mg, p, q, sums + 1)) {
                 ok = false;
                 break;
             }
         } else {
-            fcg_spmv_dot<<<rb, tpb>>>(n, rowptr, colidx, vals, p, q, dots);
+            fcg_spmv_dot<<<rb, tpb>>>(n, rowptr, colidx, vals, p, q, sums + 1);
         }
-        readn(1);
-        const double pAp = hd[0];
+        fcg_step<<<vb, tpb>>>(n, sums, sums + 1, x, p, r, q, sums + 2);
+        cudaMemcpy(hd, sums, 3 * sizeof(double), cudaMemcpyDeviceToHost);
+        const double pr = hd[0], pAp = hd[1];
         if (!(pAp > 0.0) || !std::isfinite(pr)) {
             fallback = 1;
             break;
         }
         pq[cur] = pAp;
-        const double alpha = pr / pAp;
-        fcg_step<<<vb, tpb>>>(n, alpha, x, p, r, q, dots);
-        readn(1);
-        rn = std::sqrt(hd[0]);
+        rn = std::sqrt(hd[2]);
         ++it;
         ++stored;
         if (rn < 0.9 * best) {
@@ -1129,9 +1120,9 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
         fb_iters = pr.iterations;
     }
     // convergence test: the true residual of the final iterate
-    cudaMemset(dots, 0, kMaxM * 8);
+    cudaMemset(dots, 0, kFcgSums * 8);
     fcg_residual<<<rb, tpb>>>(n, rowptr, colidx, vals, b, x, r, dots);
-    readn(2);
+    cudaMemcpy(hd, dots, 2 * sizeof(double), cudaMemcpyDeviceToHost);
     const double true_rel = std::sqrt(hd[0]) / bn;
     cleanup();
     if (rep) {

@@ -25,7 +25,7 @@
 //     symmetric positive definite operator;
 //   * the coarsest level (n_L <= coarse_max) is solved with its dense inverse,
 //     formed by Gauss-Jordan elimination on the device (the operator is SPD,
-//     so no pivoting; two launches per pivot, so a small coarsest grid);
+//     so no pivoting), 16 pivots per launch;
 //   * the finest fp32_levels levels smooth, restrict and prolong in FP32 (an
 //     FP32 copy of the stencil, FP32 vectors): the FP64 stencil sweep is bound
 //     by the FP64 pipe (243 FMAs per node), the FP32 one by HBM.  The V-cycle
@@ -43,6 +43,7 @@
 #include <vector>
 
 #include "fem_internal.hpp"
+#include "fem_reduce.cuh"
 
 using fem::fail;
 
@@ -52,23 +53,7 @@ __host__ __device__ __forceinline__ int64_t sidx(int k, int f, int g, int64_t N,
     return (int64_t)((k * 3 + f) * 3 + g) * N + i;
 }
 
-__device__ __forceinline__ double mg_warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ void mg_block_sum_add(double v, double* out) {
-    __shared__ double red[32];
-    v = mg_warp_sum(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
-        v = mg_warp_sum(v);
-        if (lane == 0) atomicAdd(out, v);
-    }
-}
+constexpr int kTpb = 256;  // threads per block of every kernel that sums
 
 // level-0 stencil from the CSR of the assembled operator (one thread per row);
 // err |= 1 for a column outside the 27-node neighbourhood
@@ -193,7 +178,8 @@ __global__ void mg_power(int n, const TS* __restrict__ S, const TV* __restrict__
             acc += (double)v * (double)v;
         }
     }
-    mg_block_sum_add(acc, dots);
+    const double sum[1] = {acc};
+    fem::block_sum_add<kTpb, 1, 1>(sum, {dots});
 }
 
 template <typename TV>
@@ -201,7 +187,8 @@ __global__ void mg_sumsq(int64_t m, const TV* __restrict__ x, double* dots) {
     double acc = 0.0;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x)
         acc += (double)x[t] * (double)x[t];
-    mg_block_sum_add(acc, dots);
+    const double sum[1] = {acc};
+    fem::block_sum_add<kTpb, 1, 1>(sum, {dots});
 }
 
 template <typename TV>
@@ -240,7 +227,8 @@ __global__ void mg_apply_dot(int n, const double* __restrict__ S, const double* 
             acc = fma(p[f * N + i], s[f], acc);
         }
     }
-    mg_block_sum_add(acc, dot);
+    const double sum[1] = {acc};
+    fem::block_sum_add<kTpb, 1, 1>(sum, {dot});
 }
 
 // Chebyshev start with x = 0: r = b, d = D^-1 b / theta, x = d
@@ -502,17 +490,64 @@ __global__ void mg_dense(int n, const double* __restrict__ S, double* __restrict
     }
 }
 
-// Gauss-Jordan inversion in place, pivot k: stash row k and column k, then
-// update every entry (a[k][k] > 0 for an SPD operator)
-// Gauss-Jordan step k of the in-place inverse, from A to B (two buffers, so the
-// pivot row and column are read from the previous step without a copy)
-__global__ void mg_gj_step(int64_t m, const double* __restrict__ A, double* __restrict__ B, int64_t k) {
-    const double inv = 1.0 / A[k * m + k];
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m * m; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / m, j = t - i * m;
-        const double rk = (j == k ? 1.0 : A[k * m + j]) * inv;
-        if (i == k) B[t] = rk;
-        else B[t] = (j == k ? 0.0 : A[t]) - A[i * m + k] * rk;
+// Gauss-Jordan inversion, kGj pivots at a time, from A to B (two buffers, so the
+// pivot rows and columns are read from the previous step without a copy): with K
+// the pivot rows, P = A_KK^-1 and Y = P A_K. (columns of K: P itself),
+//   B_K. = Y,   B_i. = A_i. - A_iK Y  (A_iK read as 0 in the first term).
+// One CTA per 32 x 32 tile; every CTA inverts the 16 x 16 pivot block itself (a
+// thread per entry, one barrier per pivot; > 0 pivots of an SPD operator, so no
+// pivoting).  One launch per pivot was latency-bound: 375 unknowns (the 5^3
+// coarsest grid) took 1.97 ms, here 24 launches take 0.42 ms.
+constexpr int kGj = 16, kGjTile = 32;
+__global__ void __launch_bounds__(kGj * kGj) mg_gj_block(int m, const double* __restrict__ A, double* __restrict__ B,
+                                                         int k0) {
+    __shared__ double P[2][kGj][kGj + 1], Y[kGj][kGjTile + 1], C[kGjTile][kGj + 1], inv[kGj];
+    const int tid = threadIdx.x, i = tid / kGj, j = tid % kGj;
+    const int nk = min(kGj, m - k0), i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
+    // a short last block is completed with the identity
+    const double d = i < nk && j < nk ? A[(int64_t)(k0 + i) * m + k0 + j] : (i == j ? 1.0 : 0.0);
+    P[0][i][j] = d;
+    if (tid == 0) inv[0] = 1.0 / d;
+    for (int t = tid; t < kGjTile * kGj; t += kGj * kGj) {
+        const int r = t / kGj, k = t % kGj;
+        C[r][k] = i0 + r < m && k < nk ? A[(int64_t)(i0 + r) * m + k0 + k] : 0.0;
+        const int kk = t / kGjTile, c = t % kGjTile;
+        Y[kk][c] = kk < nk && j0 + c < m ? A[(int64_t)(k0 + kk) * m + j0 + c] : 0.0;
+    }
+    __syncthreads();
+    for (int k = 0; k < kGj; ++k) {
+        const double(*a)[kGj + 1] = P[k & 1];
+        const double rk = (j == k ? 1.0 : a[k][j]) * inv[k];
+        const double v = i == k ? rk : (j == k ? 0.0 : a[i][j]) - a[i][k] * rk;
+        P[(k + 1) & 1][i][j] = v;
+        if (i == k + 1 && j == k + 1) inv[k + 1] = 1.0 / v;
+        __syncthreads();
+    }
+    static_assert(kGj % 2 == 0, "the inverse ends in the first buffer");
+    // Y = P A_K. (in place through registers)
+    double y[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int c = j + h * kGj, col = j0 + c - k0;
+        double s = 0.0;
+        for (int k = 0; k < kGj; ++k) s = fma(P[0][i][k], Y[k][c], s);
+        y[h] = col >= 0 && col < nk ? P[0][i][col] : s;
+    }
+    __syncthreads();
+    Y[i][j] = y[0];
+    Y[i][j + kGj] = y[1];
+    __syncthreads();
+    for (int t = tid; t < kGjTile * kGjTile; t += kGj * kGj) {
+        const int r = t / kGjTile, c = t % kGjTile, row = i0 + r, col = j0 + c;
+        if (row >= m || col >= m) continue;
+        double v;
+        if (row >= k0 && row < k0 + nk) {
+            v = Y[row - k0][c];
+        } else {
+            v = col >= k0 && col < k0 + nk ? 0.0 : A[(int64_t)row * m + col];
+            for (int k = 0; k < kGj; ++k) v = fma(-C[r][k], Y[k][c], v);
+        }
+        B[(int64_t)row * m + col] = v;
     }
 }
 
@@ -523,13 +558,17 @@ __global__ void mg_gemv(int64_t m, const double* __restrict__ A, const double* _
     for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < m; row += warps) {
         double s = 0.0;
         for (int64_t j = lane; j < m; j += 32) s = fma(A[row * m + j], b[j], s);
-        s = mg_warp_sum(s);
+        s = fem::warp_total(s);
         if (lane == 0) x[row] = s;
     }
 }
 
 unsigned blocks_for(int64_t work, int tpb) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + tpb - 1) / tpb, (int64_t)fem::sm_count() * 32));
+}
+// of a sum over short rows of work: fewer blocks, each ends with a block sum
+unsigned sum_blocks(int64_t work, int tpb) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + tpb - 1) / tpb, (int64_t)fem::sm_count() * 4));
 }
 
 }  // namespace
@@ -555,26 +594,33 @@ struct fem_mg {
     double* dots = nullptr;
     double* pdots = nullptr;  // power-iteration norms (power_iters + 1)
     int* err = nullptr;
-    std::vector<void*> bufs;
-    ~fem_mg() {
-        cudaDeviceSynchronize();
-        for (void* p : bufs) cudaFree(p);
-    }
-    template <typename T>
-    bool alloc(T** p, size_t count) {
-        if (cudaMalloc((void**)p, count * sizeof(T)) != cudaSuccess) return false;
-        bufs.push_back(*p);
-        return true;
-    }
-    bool alloc_vec(void** p, size_t count, bool f32) {
-        if (f32) return alloc((float**)p, count);
-        return alloc((double**)p, count);
-    }
+    // all arrays in one allocation (45 of their own cost a millisecond to make and
+    // another to free): reserved one by one, then placed by commit()
+    struct Arena {
+        char* base = nullptr;
+        size_t bytes = 0;
+        std::vector<std::pair<void**, size_t>> at;
+        template <typename T>
+        void reserve(T** p, size_t count) {
+            at.push_back({(void**)p, bytes});
+            bytes += (count * sizeof(T) + 255) / 256 * 256;
+        }
+        bool commit() {
+            if (cudaMalloc((void**)&base, bytes) != cudaSuccess) {
+                base = nullptr;
+                return false;
+            }
+            for (auto& [p, o] : at) *p = base + o;
+            return true;
+        }
+        ~Arena() {
+            if (base) cudaFree(base);
+        }
+    } arena;
+    ~fem_mg() { cudaDeviceSynchronize(); }
 };
 
 namespace {
-
-constexpr int kTpb = 256;
 
 template <typename TV>
 struct Cheb {
@@ -652,28 +698,26 @@ void vcycle(fem_mg* g, size_t l, const void* b, void* x) {
     else level_cycle<double>(g, l, (const double*)b, (double*)x);
 }
 
-// lambda_max(D^-1 A) of a level by power iteration from the seeded vector in
-// px (FP64; converted for an FP32 level); px / py are finest-size scratch
+// power iteration for lambda_max(D^-1 A) of a level from the seeded vector in px
+// (FP64; converted for an FP32 level); px / py are finest-size scratch.  Squared
+// norms on the device: pd[0] = |x0|^2, pd[it + 1] = |y_it|^2 with y_it = D^-1 A x_it
+// and x_(it+1) = y_it / |y_it|, the normalisation done by the next step as it reads
+// y_it.
 template <typename TS, typename TV>
-double power_lambda(fem_mg* g, const fem_mg::Level& L, const TS* S, const TV* dinv, double* px, double* py, int iters) {
-    const unsigned vb = blocks_for(3 * L.N, kTpb);
+void power_iterate(const fem_mg::Level& L, const TS* S, const TV* dinv, double* px, double* py, int iters, double* pd) {
+    const unsigned vb = blocks_for(3 * L.N, kTpb), sb = sum_blocks(3 * L.N, kTpb);
     TV *x = (TV*)px, *y = (TV*)py;
     if (!std::is_same<TV, double>::value) {
         mg_convert<double, TV><<<vb, kTpb>>>(3 * L.N, px, y);
         mg_scale<TV><<<vb, kTpb>>>(3 * L.N, 1.0, y, x);
     }
-    // squared norms on the device: pd[0] = |x0|^2, pd[it + 1] = |y_it|^2 with
-    // y_it = D^-1 A x_it and x_(it+1) = y_it / |y_it|, the normalisation done by
-    // the next step as it reads y_it; the host reads the norms once at the end
-    double* pd = g->pdots;
-    cudaMemset(pd, 0, (iters + 1) * sizeof(double));
-    mg_sumsq<TV><<<vb, kTpb>>>(3 * L.N, x, pd);
+    mg_sumsq<TV><<<sb, kTpb>>>(3 * L.N, x, pd);
     for (int it = 0; it < iters; ++it) {
         mg_power<TS, TV><<<blocks_for(L.N, kTpb), kTpb>>>(L.n, S, dinv, x, it ? pd + it : nullptr, y, pd + it + 1);
         std::swap(x, y);
     }
-    std::vector<double> h(iters + 1, 0.0);
-    cudaMemcpy(h.data(), pd, (iters + 1) * sizeof(double), cudaMemcpyDeviceToHost);
+}
+double power_lambda(const double* h, int iters) {
     double xn = std::sqrt(h[0]), lam = 0.0;
     for (int it = 0; it < iters; ++it) {
         const double yn = std::sqrt(h[it + 1]);
@@ -746,22 +790,43 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
     fem_mg* g = new fem_mg();
     g->o = o;
     g->lv.resize(ns.size());
-    bool ok = g->alloc(&g->dots, 4) && g->alloc(&g->pdots, (size_t)std::max(o.power_iters, 1) + 1) &&
-              g->alloc(&g->err, 1);
-    for (size_t l = 0; ok && l < ns.size(); ++l) {
+    const size_t iters = (size_t)o.power_iters + 1;
+    fem_mg::Arena& ar = g->arena;
+    ar.reserve(&g->dots, 4);
+    ar.reserve(&g->pdots, iters * ns.size());
+    ar.reserve(&g->err, 1);
+    for (size_t l = 0; l < ns.size(); ++l) {
         fem_mg::Level& L = g->lv[l];
         L.n = ns[l];
         L.N = (int64_t)L.n * L.n * L.n;
         L.fp32 = (int)l < o.fp32_levels && l + 1 < ns.size();
-        ok = g->alloc(&L.S, 243 * L.N) && g->alloc(&L.dinv, 3 * L.N) && g->alloc_vec(&L.r, 3 * L.N, L.fp32) &&
-             g->alloc_vec(&L.d0, 3 * L.N, L.fp32) && g->alloc_vec(&L.d1, 3 * L.N, L.fp32);
-        if (ok && (l > 0 || L.fp32)) ok = g->alloc_vec(&L.x, 3 * L.N, L.fp32) && g->alloc_vec(&L.b, 3 * L.N, L.fp32);
-        if (ok && L.fp32) ok = g->alloc(&L.S32, 243 * L.N) && g->alloc(&L.dinv32, 3 * L.N);
+        const size_t w = L.fp32 ? sizeof(float) : sizeof(double);
+        ar.reserve(&L.S, 243 * L.N);
+        ar.reserve(&L.dinv, 3 * L.N);
+        for (void** v : {&L.r, &L.d0, &L.d1}) ar.reserve((char**)v, 3 * L.N * w);
+        if (l > 0 || L.fp32)
+            for (void** v : {&L.x, &L.b}) ar.reserve((char**)v, 3 * L.N * w);
+        if (L.fp32) {
+            ar.reserve(&L.S32, 243 * L.N);
+            ar.reserve(&L.dinv32, 3 * L.N);
+        }
     }
     g->m = 3 * g->lv.back().N;
-    double* ainv2 = nullptr;
-    if (ok) ok = g->alloc(&g->ainv, g->m * g->m) && g->alloc(&ainv2, g->m * g->m);
-    if (!ok) {
+    ar.reserve(&g->ainv, g->m * g->m);
+    // scratch of the setup: the boxes of the Galerkin products, the vectors of the
+    // power iterations, the second buffer of the inversion
+    fem_mg::Arena scratch;
+    double *t1 = nullptr, *t2 = nullptr, *px = nullptr, *py = nullptr, *ainv2 = nullptr;
+    {
+        const int64_t n0 = ns[0], n1 = ns[1];
+        scratch.reserve(&t1, 243 * n0 * n0 * n1);
+        scratch.reserve(&t2, 243 * n0 * n1 * n1);
+        scratch.reserve(&px, 3 * n0 * n0 * n0);
+        scratch.reserve(&py, 3 * n0 * n0 * n0);
+        scratch.reserve(&ainv2, g->m * g->m);
+    }
+    if (!ar.commit() || !scratch.commit()) {
+        cudaGetLastError();
         delete g;
         return fail(c, FEM_GPU_OUT_OF_MEMORY, "multigrid hierarchy");
     }
@@ -773,26 +838,13 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
     mg_csr_to_stencil<<<blocks_for(3 * L0.N, kCsRows), kCsPart * kCsRows, kCsSmem>>>(L0.n, rowptr, colidx, vals,
                                                                                     L0.S, g->err);
     mg_check_symmetric<<<blocks_for(L0.N, kTpb), kTpb>>>(L0.n, L0.S, g->err);
-    {
-        // Galerkin products axis by axis through two scratch boxes (freed after setup)
-        const int64_t n0 = L0.n, n1 = (n0 - 1) / 2 + 1;
-        double *t1 = nullptr, *t2 = nullptr;
-        if (cudaMalloc(&t1, 243 * n0 * n0 * n1 * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&t2, 243 * n0 * n1 * n1 * sizeof(double)) != cudaSuccess) {
-            cudaFree(t1);
-            delete g;
-            return fail(c, FEM_GPU_OUT_OF_MEMORY, "multigrid Galerkin scratch");
-        }
-        for (size_t l = 0; l + 1 < g->lv.size(); ++l) {
-            const int nf = g->lv[l].n, ncs = g->lv[l + 1].n;
-            const int3 a{nf, nf, nf}, b{nf, nf, ncs}, cc{nf, ncs, ncs}, d{ncs, ncs, ncs};
-            mg_rap_axis<2><<<blocks_for(9 * (int64_t)b.x * b.y * b.z, 128), 128>>>(a, b, g->lv[l].S, t1);
-            mg_rap_axis<1><<<blocks_for(9 * (int64_t)cc.x * cc.y * cc.z, 128), 128>>>(b, cc, t1, t2);
-            mg_rap_axis<0><<<blocks_for(9 * (int64_t)d.x * d.y * d.z, 128), 128>>>(cc, d, t2, g->lv[l + 1].S);
-        }
-        cudaDeviceSynchronize();
-        cudaFree(t1);
-        cudaFree(t2);
+    // Galerkin products axis by axis through two scratch boxes
+    for (size_t l = 0; l + 1 < g->lv.size(); ++l) {
+        const int nf = g->lv[l].n, ncs = g->lv[l + 1].n;
+        const int3 a{nf, nf, nf}, b{nf, nf, ncs}, cc{nf, ncs, ncs}, d{ncs, ncs, ncs};
+        mg_rap_axis<2><<<blocks_for(9 * (int64_t)b.x * b.y * b.z, 128), 128>>>(a, b, g->lv[l].S, t1);
+        mg_rap_axis<1><<<blocks_for(9 * (int64_t)cc.x * cc.y * cc.z, 128), 128>>>(b, cc, t1, t2);
+        mg_rap_axis<0><<<blocks_for(9 * (int64_t)d.x * d.y * d.z, 128), 128>>>(cc, d, t2, g->lv[l + 1].S);
     }
     int herr = 0;
     cudaMemcpy(&herr, g->err, sizeof(int), cudaMemcpyDeviceToHost);
@@ -802,12 +854,8 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
                                                    : "multigrid: operator is not symmetric");
     }
     // smoother data: diagonal, FP32 copies, lambda_max(D^-1 A) by power iteration
-    // (FP64, in two scratch vectors of the finest size)
-    double *px = nullptr, *py = nullptr;
-    if (!g->alloc(&px, 3 * L0.N) || !g->alloc(&py, 3 * L0.N)) {
-        delete g;
-        return fail(c, FEM_GPU_OUT_OF_MEMORY, "multigrid hierarchy");
-    }
+    // (norms on the device, read once for all levels)
+    cudaMemset(g->pdots, 0, iters * ns.size() * sizeof(double));
     for (size_t l = 0; l + 1 < g->lv.size(); ++l) {
         fem_mg::Level& L = g->lv[l];
         const unsigned vb = blocks_for(3 * L.N, kTpb);
@@ -819,25 +867,33 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
         mg_random<<<vb, kTpb>>>(3 * L.N, 0x5EEDULL + l, px);
         // FP64 levels iterate on the FP64 stencil; FP32 levels on their FP32 copy
         // (the smoothing interval needs lambda_max to a few digits only)
-        double lam = L.fp32 ? power_lambda<float, float>(g, L, L.S32, L.dinv32, px, py, o.power_iters)
-                            : power_lambda<double, double>(g, L, L.S, L.dinv, px, py, o.power_iters);
-        L.lmax = lam;
-        if (!(lam > 0.0) || !std::isfinite(lam)) {
-            delete g;
-            return fail(c, FEM_GPU_NONFINITE, "multigrid: power iteration gave no positive lambda_max");
-        }
+        if (L.fp32) power_iterate<float, float>(L, L.S32, L.dinv32, px, py, o.power_iters, g->pdots + l * iters);
+        else power_iterate<double, double>(L, L.S, L.dinv, px, py, o.power_iters, g->pdots + l * iters);
     }
     // coarsest level: dense inverse
     fem_mg::Level& LC = g->lv.back();
     cudaMemset(g->ainv, 0, g->m * g->m * sizeof(double));
     mg_dense<<<blocks_for(g->m, kTpb), kTpb>>>(LC.n, LC.S, g->ainv);
-    for (int64_t k = 0; k < g->m; ++k) {
-        mg_gj_step<<<blocks_for(g->m * g->m, kTpb), kTpb>>>(g->m, g->ainv, ainv2, k);
-        std::swap(g->ainv, ainv2);
+    const unsigned tiles = (unsigned)((g->m + kGjTile - 1) / kGjTile);
+    double *from = g->ainv, *to = ainv2;
+    for (int64_t k = 0; k < g->m; k += kGj) {
+        mg_gj_block<<<dim3(tiles, tiles), kGj * kGj>>>((int)g->m, from, to, (int)k);
+        std::swap(from, to);
     }
-    if (cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess) {
+    if (from != g->ainv) cudaMemcpyAsync(g->ainv, from, g->m * g->m * sizeof(double), cudaMemcpyDeviceToDevice, 0);
+    std::vector<double> norms(iters * ns.size(), 0.0);
+    if (cudaMemcpy(norms.data(), g->pdots, norms.size() * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess) {
         delete g;
         return fail(c, FEM_GPU_CUDA_ERROR, "multigrid setup");
+    }
+    for (size_t l = 0; l + 1 < g->lv.size(); ++l) {
+        const double lam = power_lambda(norms.data() + l * iters, o.power_iters);
+        g->lv[l].lmax = lam;
+        if (!(lam > 0.0) || !std::isfinite(lam)) {
+            delete g;
+            return fail(c, FEM_GPU_NONFINITE, "multigrid: power iteration gave no positive lambda_max");
+        }
     }
     g->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     *out = g;

@@ -176,3 +176,18 @@ def test_unsymmetric_operator_is_rejected(torch):
         Multigrid(m, rp, ci, bad)
     assert e.value.status == 1
     Multigrid(m, rp, ci, vals).close()  # the symmetric one is accepted
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,coarse_max", [(8, 3), (12, 7)])
+def test_blocked_inverse_of_short_last_blocks(torch, n, coarse_max):
+    """The V-cycle with a dense inverse of 81 = 5 x 16 + 1 and 1,029 = 64 x 16 + 5
+    unknowns (16 pivots at a time), to the 1e-10 of cond(A_L) at contrast 1e3."""
+    from moris_gb300.multigrid import Multigrid
+    m, rp, ci, vals, b, A = device_system(n, 1.0)
+    h = Multigrid(m, rp, ci, vals, coarse_max=coarse_max, fp32_levels=0)
+    o = mo.Hierarchy(A, n + 1, coarse_max=coarse_max)
+    r = np.random.default_rng(12).standard_normal(m.num_adofs)
+    z = h.apply(torch.tensor(r, device="cuda"), torch.empty(m.num_adofs, dtype=torch.float64, device="cuda"))
+    zo = o.vcycle(r)
+    assert float(np.max(np.abs(z.cpu().numpy() - zo)) / np.max(np.abs(zo))) <= 1e-10
