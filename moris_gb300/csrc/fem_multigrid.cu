@@ -125,42 +125,84 @@ __global__ void mg_diag_inv(int64_t N, const double* __restrict__ S, double* __r
     }
 }
 
-// s[f] = sum_k sum_g S[k][f][g][i] x[g][i + off_k] for the three rows of node i,
-// accumulated in the vector type TV (FP32 levels: FP32 FMAs)
-template <typename TS, typename TV>
-__device__ __forceinline__ void stencil_rows(int n, int64_t N, const TS* __restrict__ S, const TV* __restrict__ x,
-                                             int64_t i, TV s[3]) {
-    const int ix = (int)(i % n), iy = (int)((i / n) % n), iz = (int)(i / ((int64_t)n * n));
-    s[0] = s[1] = s[2] = TV(0);
+// out(t, pre(t), (A x)_t) for every row t = f N + i of a stencil; pre loads what out
+// needs, ahead of the sum.  A warp takes 32 consecutive nodes and one of the nine
+// (dz, dy) rows of neighbours (FP32; one dz plane in FP64, whose pipe also pays for
+// the sums over the warps): its 27 coefficients and 9 values per lane are loads that
+// do not wait for one another, where a thread per node walked the nine rows one after
+// the other.  The rows meet in shared memory; warp f ends component f.
+// Measured, FP32 Chebyshev step, thread per node -> here: 9^3 nodes 23 -> 4.0 us,
+// 17^3 22.5 -> 4.3, 33^3 24 -> 9.4, 65^3 59 -> 46.7 (5.9 TB/s; with the coefficients
+// in 243 planes instead of tiles 57).  FP64 product at 65^3: 121 -> 124 us, 107 of
+// them FP64 instructions.
+template <typename TV>
+struct Sweep {
+    static constexpr int G = sizeof(TV) == 4 ? 9 : 3, threads = 32 * G, per_sm = sizeof(TV) == 4 ? 4 : 10;
+};
+template <typename TS, typename TV, typename L, typename F>
+__device__ __forceinline__ void stencil_sweep(int n, const TS* __restrict__ S, const TV* __restrict__ x, L&& pre,
+                                              F&& out) {
+    constexpr int G = Sweep<TV>::G;
+    __shared__ TV red[G][3][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int N = n * n * n;  // 243 N doubles are on the device: N < 2^28
+    for (int i0 = blockIdx.x * 32; i0 < N; i0 += gridDim.x * 32) {
+        const int i = i0 + lane, ic = min(i, N - 1);
+        const int ix = ic % n, iy = ic / n % n, iz = ic / (n * n);
+        const int64_t t = (int64_t)(w < 3 ? w : 0) * N + ic;
+        decltype(pre(t)) own{};
+        if (w < 3) own = pre(t);
+        // FP32: 243 x 32 coefficients of the tile in sequence (mg_stencil32)
+        const int64_t tap = sizeof(TS) == 4 ? 32 : N;
+        const TS* Si = S + (sizeof(TS) == 4 ? (int64_t)(i0 / 32) * (243 * 32) + lane : ic);
+        TV s[3] = {TV(0), TV(0), TV(0)};
 #pragma unroll
-    for (int dz = -1; dz <= 1; ++dz) {
-        if (iz + dz < 0 || iz + dz >= n) continue;
-#pragma unroll
-        for (int dy = -1; dy <= 1; ++dy) {
-            if (iy + dy < 0 || iy + dy >= n) continue;
+        for (int r = 0; r < 9 / G; ++r) {
+            const int row = w * (9 / G) + r, dz = row / 3 - 1, dy = row % 3 - 1;
+            const bool in = (unsigned)(iz + dz) < (unsigned)n && (unsigned)(iy + dy) < (unsigned)n;
+            const TS* Sr = Si + 27 * row * tap;
+            const TV* xr = x + ic + n * (dy + n * dz);
+            TV xg[3][3];
 #pragma unroll
             for (int dx = -1; dx <= 1; ++dx) {
-                if (ix + dx < 0 || ix + dx >= n) continue;
-                const int k = (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
-                const int64_t j = i + dx + (int64_t)n * (dy + (int64_t)n * dz);
+                const bool inx = in && (unsigned)(ix + dx) < (unsigned)n;
 #pragma unroll
-                for (int g = 0; g < 3; ++g) {
-                    const TV xg = __ldg(x + g * N + j);
-#pragma unroll
-                    for (int f = 0; f < 3; ++f) s[f] = fma((TV)__ldg(S + sidx(k, f, g, N, i)), xg, s[f]);
-                }
+                for (int g = 0; g < 3; ++g) xg[dx + 1][g] = inx ? __ldg(xr + (int64_t)g * N + dx) : TV(0);
             }
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int g = 0; g < 3; ++g)
+#pragma unroll
+                    for (int f = 0; f < 3; ++f)
+                        s[f] = fma((TV)__ldg(Sr + ((d * 3 + f) * 3 + g) * tap), xg[d][g], s[f]);
         }
+#pragma unroll
+        for (int f = 0; f < 3; ++f) red[w][f][lane] = s[f];
+        __syncthreads();
+        if (w < 3) {
+            TV v = red[0][w][lane];
+#pragma unroll
+            for (int k = 1; k < G; ++k) v += red[k][w][lane];
+            if (i < N) out(t, own, v);
+        }
+        __syncthreads();
     }
+}
+unsigned sweep_blocks(int64_t N) { return (unsigned)((N + 31) / 32); }
+// of a sweep that ends in a block sum: an atomic of every block to one address takes
+// 10 ns (8,583 blocks: 97 us for a sweep of 57)
+template <typename TV>
+unsigned sum_sweep_blocks(int64_t N) {
+    return std::min<unsigned>(sweep_blocks(N), (unsigned)fem::sm_count() * Sweep<TV>::per_sm * 2);
 }
 
 // power iteration step: y = D^-1 A (a x), a = 1 / sqrt(*xx) (1 without xx: x
 // is the previous step's y, normalised here instead of in a pass of its own);
 // dots[0] += y.y (in the level's precision)
 template <typename TS, typename TV>
-__global__ void mg_power(int n, const TS* __restrict__ S, const TV* __restrict__ dinv, const TV* __restrict__ x,
+__global__ void __launch_bounds__(Sweep<TV>::threads, Sweep<TV>::per_sm) mg_power(int n, const TS* __restrict__ S, const TV* __restrict__ dinv, const TV* __restrict__ x,
                          const double* __restrict__ xx, TV* __restrict__ y, double* dots) {
-    const int64_t N = (int64_t)n * n * n;
     double a = 1.0;
     if (xx) {
         const double d = *xx;
@@ -168,18 +210,13 @@ __global__ void mg_power(int n, const TS* __restrict__ S, const TV* __restrict__
     }
     const TV at = (TV)a;
     double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        TV s[3];
-        stencil_rows<TS, TV>(n, N, S, x, i, s);
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            const TV v = dinv[f * N + i] * s[f] * at;
-            y[f * N + i] = v;
-            acc += (double)v * (double)v;
-        }
-    }
+    stencil_sweep<TS, TV>(n, S, x, [&](int64_t t) { return dinv[t]; }, [&](int64_t t, TV d, TV s) {
+        const TV v = d * s * at;
+        y[t] = v;
+        acc += (double)v * (double)v;
+    });
     const double sum[1] = {acc};
-    fem::block_sum_add<kTpb, 1, 1>(sum, {dots});
+    fem::block_sum_add<Sweep<TV>::threads, 1, 1>(sum, {dots});
 }
 
 template <typename TV>
@@ -213,22 +250,28 @@ __global__ void mg_convert(int64_t m, const TA* __restrict__ a, TB* __restrict__
         b[t] = (TB)a[t];
 }
 
+// FP32 copy of a stencil in tiles of 32 nodes, S32[tile][tap][32]: a block of a sweep
+// reads 31 KB in sequence, where 243 planes of the node grid were as many DRAM streams
+// of one (for odd N misaligned) line each
+__global__ void mg_stencil32(int64_t N, const double* __restrict__ S, float* __restrict__ S32) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+    float* b = S32 + (int64_t)blockIdx.x * (243 * 32) + lane;
+#pragma unroll 8
+    for (int k = threadIdx.x >> 5; k < 243; k += kTpb / 32) b[k * 32] = i < N ? (float)S[k * N + i] : 0.0f;
+}
+
 // q = A p on an FP64 stencil and dot += p.q (the outer Krylov product)
-__global__ void mg_apply_dot(int n, const double* __restrict__ S, const double* __restrict__ p, double* __restrict__ q,
-                             double* dot) {
-    const int64_t N = (int64_t)n * n * n;
+__global__ void __launch_bounds__(Sweep<double>::threads, Sweep<double>::per_sm)
+    mg_apply_dot(int n, const double* __restrict__ S, const double* __restrict__ p, double* __restrict__ q,
+                 double* dot) {
     double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        double s[3];
-        stencil_rows<double, double>(n, N, S, p, i, s);
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            q[f * N + i] = s[f];
-            acc = fma(p[f * N + i], s[f], acc);
-        }
-    }
+    stencil_sweep<double, double>(n, S, p, [&](int64_t t) { return p[t]; }, [&](int64_t t, double pt, double s) {
+        q[t] = s;
+        acc = fma(pt, s, acc);
+    });
     const double sum[1] = {acc};
-    fem::block_sum_add<kTpb, 1, 1>(sum, {dot});
+    fem::block_sum_add<Sweep<double>::threads, 1, 1>(sum, {dot});
 }
 
 // Chebyshev start with x = 0: r = b, d = D^-1 b / theta, x = d
@@ -244,116 +287,96 @@ __global__ void mg_cheb_init(int64_t m, const TV* __restrict__ b, const TV* __re
     }
 }
 
+template <typename TV>
+struct Row {
+    TV r, d, dinv, x;
+};
+
 // Chebyshev step: r -= A din; dout = c1 din + c2 D^-1 r; x += dout
 template <typename TS, typename TV>
-__global__ void mg_cheb_step(int n, const TS* __restrict__ S, const TV* __restrict__ din, TV* __restrict__ r,
-                             const TV* __restrict__ dinv, TV c1, TV c2, TV* __restrict__ dout, TV* __restrict__ x) {
-    const int64_t N = (int64_t)n * n * n;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        TV s[3];
-        stencil_rows<TS, TV>(n, N, S, din, i, s);
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            const int64_t t = f * N + i;
-            const TV rt = r[t] - s[f];
-            const TV dt = fma(c1, din[t], c2 * dinv[t] * rt);
+__global__ void __launch_bounds__(Sweep<TV>::threads, Sweep<TV>::per_sm)
+    mg_cheb_step(int n, const TS* __restrict__ S, const TV* __restrict__ din, TV* __restrict__ r,
+                 const TV* __restrict__ dinv, TV c1, TV c2, TV* __restrict__ dout, TV* __restrict__ x) {
+    stencil_sweep<TS, TV>(
+        n, S, din, [&](int64_t t) { return Row<TV>{r[t], din[t], dinv[t], x[t]}; },
+        [&](int64_t t, const Row<TV>& o, TV s) {
+            const TV rt = o.r - s;
+            const TV dt = fma(c1, o.d, c2 * o.dinv * rt);
             r[t] = rt;
             dout[t] = dt;
-            x[t] += dt;
-        }
-    }
+            x[t] = o.x + dt;
+        });
 }
 
 // r -= A d
 template <typename TS, typename TV>
-__global__ void mg_residual_update(int n, const TS* __restrict__ S, const TV* __restrict__ d, TV* __restrict__ r) {
-    const int64_t N = (int64_t)n * n * n;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        TV s[3];
-        stencil_rows<TS, TV>(n, N, S, d, i, s);
-#pragma unroll
-        for (int f = 0; f < 3; ++f) r[f * N + i] -= s[f];
-    }
+__global__ void __launch_bounds__(Sweep<TV>::threads, Sweep<TV>::per_sm)
+    mg_residual_update(int n, const TS* __restrict__ S, const TV* __restrict__ d, TV* __restrict__ r) {
+    stencil_sweep<TS, TV>(n, S, d, [&](int64_t t) { return r[t]; },
+                          [&](int64_t t, TV rt, TV s) { r[t] = rt - s; });
 }
 
 // first post-smoothing step after the coarse correction e:
 // r -= A e; d = D^-1 r / theta; x += e + d
 template <typename TS, typename TV>
-__global__ void mg_post_first(int n, const TS* __restrict__ S, const TV* __restrict__ e, TV* __restrict__ r,
-                              const TV* __restrict__ dinv, TV inv_theta, TV* __restrict__ d, TV* __restrict__ x) {
-    const int64_t N = (int64_t)n * n * n;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        TV s[3];
-        stencil_rows<TS, TV>(n, N, S, e, i, s);
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            const int64_t t = f * N + i;
-            const TV rt = r[t] - s[f];
-            const TV dt = dinv[t] * rt * inv_theta;
+__global__ void __launch_bounds__(Sweep<TV>::threads, Sweep<TV>::per_sm)
+    mg_post_first(int n, const TS* __restrict__ S, const TV* __restrict__ e, TV* __restrict__ r,
+                  const TV* __restrict__ dinv, TV inv_theta, TV* __restrict__ d, TV* __restrict__ x) {
+    stencil_sweep<TS, TV>(
+        n, S, e, [&](int64_t t) { return Row<TV>{r[t], e[t], dinv[t], x[t]}; },
+        [&](int64_t t, const Row<TV>& o, TV s) {
+            const TV rt = o.r - s;
+            const TV dt = o.dinv * rt * inv_theta;
             r[t] = rt;
             d[t] = dt;
-            x[t] += e[t] + dt;
-        }
-    }
+            x[t] = o.x + (o.d + dt);
+        });
 }
 
-// full-weighting restriction bc = P^T r (fine grid nf = 2 (nc - 1) + 1)
+// full-weighting restriction bc = P^T r (fine grid nf = 2 (nc - 1) + 1), a thread per
+// coarse row, the 27 loads independent
 template <typename TF, typename TC>
 __global__ void mg_restrict(int nf, int nc, const TF* __restrict__ r, TC* __restrict__ bc) {
-    const int64_t Nc = (int64_t)nc * nc * nc, Nf = (int64_t)nf * nf * nf;
-    for (int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; I < Nc; I += (int64_t)gridDim.x * blockDim.x) {
-        const int X = (int)(I % nc), Y = (int)((I / nc) % nc), Z = (int)(I / ((int64_t)nc * nc));
-        TF s[3] = {TF(0), TF(0), TF(0)};
-        for (int az = -1; az <= 1; ++az) {
-            const int z = 2 * Z + az;
-            if (z < 0 || z >= nf) continue;
-            for (int ay = -1; ay <= 1; ++ay) {
-                const int y = 2 * Y + ay;
-                if (y < 0 || y >= nf) continue;
+    const int Nc = nc * nc * nc, Nf = nf * nf * nf;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * Nc; t += gridDim.x * blockDim.x) {
+        const int g = t / Nc, I = t - g * Nc;
+        const int X = I % nc, Y = I / nc % nc, Z = I / (nc * nc);
+        const TF* rg = r + (int64_t)g * Nf + 2 * (X + nf * (Y + nf * Z));
+        TF s = TF(0);
+#pragma unroll
+        for (int az = -1; az <= 1; ++az)
+#pragma unroll
+            for (int ay = -1; ay <= 1; ++ay)
+#pragma unroll
                 for (int ax = -1; ax <= 1; ++ax) {
-                    const int x = 2 * X + ax;
-                    if (x < 0 || x >= nf) continue;
+                    const bool in = (unsigned)(2 * X + ax) < (unsigned)nf && (unsigned)(2 * Y + ay) < (unsigned)nf &&
+                                    (unsigned)(2 * Z + az) < (unsigned)nf;
                     const TF w = TF((ax ? 0.5 : 1.0) * (ay ? 0.5 : 1.0) * (az ? 0.5 : 1.0));
-                    const int64_t i = x + (int64_t)nf * (y + (int64_t)nf * z);
-                    for (int g = 0; g < 3; ++g) s[g] = fma(w, r[g * Nf + i], s[g]);
+                    s = fma(w, in ? rg[ax + nf * (ay + nf * az)] : TF(0), s);
                 }
-            }
-        }
-        for (int g = 0; g < 3; ++g) bc[g * Nc + I] = (TC)s[g];
+        bc[t] = (TC)s;
     }
 }
 
 // trilinear prolongation e = P xc
 template <typename TC, typename TF>
 __global__ void mg_prolong(int nf, int nc, const TC* __restrict__ xc, TF* __restrict__ e) {
-    const int64_t Nc = (int64_t)nc * nc * nc, Nf = (int64_t)nf * nf * nf;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < Nf; i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nf), y = (int)((i / nf) % nf), z = (int)(i / ((int64_t)nf * nf));
-        const int x0 = x >> 1, y0 = y >> 1, z0 = z >> 1;
-        const int x1 = x0 + (x & 1), y1 = y0 + (y & 1), z1 = z0 + (z & 1);
+    const int Nc = nc * nc * nc, Nf = nf * nf * nf;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * Nf; t += gridDim.x * blockDim.x) {
+        const int g = t / Nf, i = t - g * Nf;
+        const int x = i % nf, y = i / nf % nf, z = i / (nf * nf);
         const TC wx = (x & 1) ? TC(0.5) : TC(1), wy = (y & 1) ? TC(0.5) : TC(1), wz = (z & 1) ? TC(0.5) : TC(1);
-        for (int g = 0; g < 3; ++g) {
-            const TC* c = xc + g * Nc;
-            auto at = [&](int a, int b, int cc) { return c[a + (int64_t)nc * (b + (int64_t)nc * cc)]; };
-            TC s = at(x0, y0, z0);
-            if (x & 1) s += at(x1, y0, z0);
-            if (y & 1) {
-                TC t = at(x0, y1, z0);
-                if (x & 1) t += at(x1, y1, z0);
-                s += t;
-            }
-            if (z & 1) {
-                TC t = at(x0, y0, z1);
-                if (x & 1) t += at(x1, y0, z1);
-                if (y & 1) {
-                    TC u = at(x0, y1, z1);
-                    if (x & 1) u += at(x1, y1, z1);
-                    t += u;
-                }
-                s += t;
-            }
-            e[g * Nf + i] = (TF)(s * wx * wy * wz);
+        const TC* c = xc + (int64_t)g * Nc + (x >> 1) + nc * ((y >> 1) + nc * (z >> 1));
+        TC v[2][2][2];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int a = k & 1, b = k >> 1 & 1, d = k >> 2;
+            const bool in = (!a || (x & 1)) && (!b || (y & 1)) && (!d || (z & 1));
+            v[d][b][a] = in ? c[a + nc * (b + nc * d)] : TC(0);
         }
+        const TC s = ((v[0][0][0] + v[0][0][1]) + (v[0][1][0] + v[0][1][1])) +
+                     ((v[1][0][0] + v[1][0][1]) + (v[1][1][0] + v[1][1][1]));
+        e[t] = (TF)(s * wx * wy * wz);
     }
 }
 
@@ -638,17 +661,17 @@ struct Cheb {
 template <typename TS, typename TV>
 void smooth_pre(const fem_mg::Level& L, const TS* S, const TV* dinv, const fem_mg_opts& o, const TV* b, TV* x) {
     const Cheb<double> c(L, o);
-    const unsigned vb = blocks_for(3 * L.N, kTpb), nb = blocks_for(L.N, kTpb);
+    const unsigned vb = blocks_for(3 * L.N, kTpb), nb = sweep_blocks(L.N);
     TV *r = (TV*)L.r, *din = (TV*)L.d0, *dout = (TV*)L.d1;
     mg_cheb_init<TV><<<vb, kTpb>>>(3 * L.N, b, dinv, (TV)c.inv_theta, r, din, x);
     double rho = 1.0 / c.sigma;
     for (int k = 1; k < o.degree; ++k) {
         const double rn = 1.0 / (2.0 * c.sigma - rho);
-        mg_cheb_step<TS, TV><<<nb, kTpb>>>(L.n, S, din, r, dinv, (TV)(rn * rho), (TV)(2.0 * rn / c.delta), dout, x);
+        mg_cheb_step<TS, TV><<<nb, Sweep<TV>::threads>>>(L.n, S, din, r, dinv, (TV)(rn * rho), (TV)(2.0 * rn / c.delta), dout, x);
         rho = rn;
         std::swap(din, dout);
     }
-    mg_residual_update<TS, TV><<<nb, kTpb>>>(L.n, S, din, r);
+    mg_residual_update<TS, TV><<<nb, Sweep<TV>::threads>>>(L.n, S, din, r);
 }
 
 // Chebyshev post-smoothing after the coarse correction e, which lives in d1:
@@ -656,13 +679,13 @@ void smooth_pre(const fem_mg::Level& L, const TS* S, const TV* dinv, const fem_m
 template <typename TS, typename TV>
 void smooth_post(const fem_mg::Level& L, const TS* S, const TV* dinv, const fem_mg_opts& o, const TV* e, TV* x) {
     const Cheb<double> c(L, o);
-    const unsigned nb = blocks_for(L.N, kTpb);
+    const unsigned nb = sweep_blocks(L.N);
     TV *r = (TV*)L.r, *din = (TV*)L.d0, *dout = (TV*)L.d1;
-    mg_post_first<TS, TV><<<nb, kTpb>>>(L.n, S, e, r, dinv, (TV)c.inv_theta, din, x);
+    mg_post_first<TS, TV><<<nb, Sweep<TV>::threads>>>(L.n, S, e, r, dinv, (TV)c.inv_theta, din, x);
     double rho = 1.0 / c.sigma;
     for (int k = 1; k < o.degree; ++k) {
         const double rn = 1.0 / (2.0 * c.sigma - rho);
-        mg_cheb_step<TS, TV><<<nb, kTpb>>>(L.n, S, din, r, dinv, (TV)(rn * rho), (TV)(2.0 * rn / c.delta), dout, x);
+        mg_cheb_step<TS, TV><<<nb, Sweep<TV>::threads>>>(L.n, S, din, r, dinv, (TV)(rn * rho), (TV)(2.0 * rn / c.delta), dout, x);
         rho = rn;
         std::swap(din, dout);
     }
@@ -678,12 +701,12 @@ void level_cycle(fem_mg* g, size_t l, const TV* b, TV* x) {
     const bool f32 = std::is_same<TV, float>::value;
     if (f32) smooth_pre(L, L.S32, L.dinv32, g->o, (const float*)b, (float*)x);
     else smooth_pre(L, L.S, L.dinv, g->o, (const double*)b, (double*)x);
-    if (C.fp32) mg_restrict<TV, float><<<blocks_for(C.N, kTpb), kTpb>>>(L.n, C.n, (const TV*)L.r, (float*)C.b);
-    else mg_restrict<TV, double><<<blocks_for(C.N, kTpb), kTpb>>>(L.n, C.n, (const TV*)L.r, (double*)C.b);
+    if (C.fp32) mg_restrict<TV, float><<<blocks_for(3 * C.N, kTpb), kTpb>>>(L.n, C.n, (const TV*)L.r, (float*)C.b);
+    else mg_restrict<TV, double><<<blocks_for(3 * C.N, kTpb), kTpb>>>(L.n, C.n, (const TV*)L.r, (double*)C.b);
     vcycle(g, l + 1, C.b, C.x);
     TV* e = (TV*)L.d1;
-    if (C.fp32) mg_prolong<float, TV><<<blocks_for(L.N, kTpb), kTpb>>>(L.n, C.n, (const float*)C.x, e);
-    else mg_prolong<double, TV><<<blocks_for(L.N, kTpb), kTpb>>>(L.n, C.n, (const double*)C.x, e);
+    if (C.fp32) mg_prolong<float, TV><<<blocks_for(3 * L.N, kTpb), kTpb>>>(L.n, C.n, (const float*)C.x, e);
+    else mg_prolong<double, TV><<<blocks_for(3 * L.N, kTpb), kTpb>>>(L.n, C.n, (const double*)C.x, e);
     if (f32) smooth_post(L, L.S32, L.dinv32, g->o, (const float*)e, (float*)x);
     else smooth_post(L, L.S, L.dinv, g->o, (const double*)e, (double*)x);
 }
@@ -713,7 +736,8 @@ void power_iterate(const fem_mg::Level& L, const TS* S, const TV* dinv, double* 
     }
     mg_sumsq<TV><<<sb, kTpb>>>(3 * L.N, x, pd);
     for (int it = 0; it < iters; ++it) {
-        mg_power<TS, TV><<<blocks_for(L.N, kTpb), kTpb>>>(L.n, S, dinv, x, it ? pd + it : nullptr, y, pd + it + 1);
+        mg_power<TS, TV><<<sum_sweep_blocks<TV>(L.N), Sweep<TV>::threads>>>(
+            L.n, S, dinv, x, it ? pd + it : nullptr, y, pd + it + 1);
         std::swap(x, y);
     }
 }
@@ -733,7 +757,7 @@ double power_lambda(const double* h, int iters) {
 bool mg_operator(fem_mg* g, const double* p, double* q, double* dot) {
     if (!g) return false;
     const fem_mg::Level& L = g->lv[0];
-    mg_apply_dot<<<blocks_for(L.N, kTpb), kTpb>>>(L.n, L.S, p, q, dot);
+    mg_apply_dot<<<sum_sweep_blocks<double>(L.N), Sweep<double>::threads>>>(L.n, L.S, p, q, dot);
     return cudaGetLastError() == cudaSuccess;
 }
 
@@ -807,7 +831,7 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
         if (l > 0 || L.fp32)
             for (void** v : {&L.x, &L.b}) ar.reserve((char**)v, 3 * L.N * w);
         if (L.fp32) {
-            ar.reserve(&L.S32, 243 * L.N);
+            ar.reserve(&L.S32, 243 * 32 * (size_t)sweep_blocks(L.N));
             ar.reserve(&L.dinv32, 3 * L.N);
         }
     }
@@ -861,7 +885,7 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
         const unsigned vb = blocks_for(3 * L.N, kTpb);
         mg_diag_inv<<<blocks_for(3 * L.N, kTpb), kTpb>>>(L.N, L.S, L.dinv);
         if (L.fp32) {
-            mg_convert<double, float><<<blocks_for(243 * L.N, kTpb), kTpb>>>(243 * L.N, L.S, L.S32);
+            mg_stencil32<<<sweep_blocks(L.N), kTpb>>>(L.N, L.S, L.S32);
             mg_convert<double, float><<<vb, kTpb>>>(3 * L.N, L.dinv, L.dinv32);
         }
         mg_random<<<vb, kTpb>>>(3 * L.N, 0x5EEDULL + l, px);
