@@ -9,8 +9,10 @@
 //   k4  (one thread) advance the iteration counter
 // Scalars live in a device ring indexed by the iteration counter, so the
 // launches carry no host-side values and a chunk of iterations is captured
-// once into a CUDA graph and replayed.  The host reads the done flag once
-// per chunk; iterations after convergence return immediately on the device.
+// once into a CUDA graph and replayed.  Small systems, whose iteration is
+// shorter than its launches, take two per iteration (k_pair_*).  The host reads
+// the done flag once per chunk; iterations after convergence return immediately
+// on the device.
 #include <cuda_runtime.h>
 
 #include <chrono>
@@ -20,6 +22,7 @@
 #include <vector>
 
 #include "fem_internal.hpp"
+#include "fem_reduce.cuh"
 #include "fem_spmv.cuh"
 
 namespace {
@@ -28,31 +31,15 @@ struct CgState {
     int it;          // current iteration
     int done;        // 1 converged, 2 breakdown
     int converged_at;
-    int pad;
+    int stopped_at;  // k_pair_*: iteration whose test ended the solve
     double thresh2;  // (rtol * ||b||)^2
     double bn2;
     // ring of per-iteration scalars: [slot][0]=pq, [1]=rz, [2]=rr
     double ring[4][4];
 };
 
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// block reduction of one double into *out (atomic)
-__device__ __forceinline__ void block_add(double v, double* out) {
-    __shared__ double red[32];
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
-        v = warp_sum(v);
-        if (lane == 0) atomicAdd(out, v);
-    }
-}
+// threads per block of every kernel that sums
+constexpr int kThreads = 256;
 
 __global__ void k_diag_inv(int64_t n, const int32_t* rp, const int32_t* ci, const double* v, double* dinv,
                            int jacobi) {
@@ -80,24 +67,18 @@ __global__ void k_init(int64_t n, const int32_t* rp, const int32_t* ci, const do
                        const double* x, double* r, double* z, double* p, const double* dinv, CgState* st) {
     const int sub = threadIdx.x % fem::kLanesPerRow;
     const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / fem::kLanesPerRow;
-    double rz = 0.0, rr = 0.0, bb = 0.0;
+    double sum[3] = {0.0, 0.0, 0.0};
     const double s = fem::csr_row_dot(n, rp, ci, v, x, row, sub);
-    if (row < n) {
-        if (sub == 0) {
-            const double ri = b[row] - s, zi = dinv[row] * ri;
-            r[row] = ri;
-            z[row] = zi;
-            p[row] = zi;
-            rz = ri * zi;
-            rr = ri * ri;
-            bb = b[row] * b[row];
-        }
+    if (row < n && sub == 0) {
+        const double ri = b[row] - s, zi = dinv[row] * ri;
+        r[row] = ri;
+        z[row] = zi;
+        p[row] = zi;
+        sum[0] = ri * zi;
+        sum[1] = ri * ri;
+        sum[2] = b[row] * b[row];
     }
-    block_add(rz, &st->ring[0][1]);
-    __syncthreads();
-    block_add(rr, &st->ring[0][2]);
-    __syncthreads();
-    block_add(bb, &st->bn2);
+    fem::block_sum_add<kThreads, fem::kLanesPerRow, 3>(sum, {&st->ring[0][1], &st->ring[0][2], &st->bn2});
 }
 
 // q = A p (warp per row, grid-stride over rows so that each block adds its
@@ -120,7 +101,8 @@ __global__ void k_spmv_pq(int64_t n, const int32_t* rp, const int32_t* ci, const
             pq = fma(s, p[row], pq);
         }
     }
-    block_add(pq, &st->ring[slot][0]);
+    const double sum[1] = {pq};
+    fem::block_sum_add<kThreads, fem::kLanesPerRow, 1>(sum, {&st->ring[slot][0]});
 }
 
 __global__ void k_update_xr(int64_t n, double* x, double* r, double* z, const double* p, const double* q,
@@ -138,9 +120,8 @@ __global__ void k_update_xr(int64_t n, double* x, double* r, double* z, const do
         rz = fma(ri, zi, rz);
         rr = fma(ri, ri, rr);
     }
-    block_add(rz, &st->ring[nxt][1]);
-    __syncthreads();
-    block_add(rr, &st->ring[nxt][2]);
+    const double sum[2] = {rz, rr};
+    fem::block_sum_add<kThreads, 1, 2>(sum, {&st->ring[nxt][1], &st->ring[nxt][2]});
 }
 
 __global__ void k_update_p(int64_t n, double* p, const double* z, CgState* st) {
@@ -166,6 +147,153 @@ __global__ void k_advance(CgState* st, int max_iter) {
     }
     for (int k = 0; k < 4; ++k) st->ring[nn][k] = 0.0;
     (void)slot;
+}
+
+// Two launches per iteration.  The direction p = z + beta p is formed where the
+// product gathers it (one FMA and one more load per nonzero, no pass of its
+// own), written for the next iteration to the other of two arrays; convergence
+// and breakdown of an iteration are tested by the next product, every block from
+// the same ring values.  k is the iteration within the chunk; chunks are multiples
+// of four, so k & 3 is the ring slot and no load waits for the iteration counter,
+// which is advanced at the chunk's end (k_pair_end).  An iteration of a small
+// system is a chain of L2 latencies: the launches overlap (programmatic
+// dependent launch), and the first entries of the thread's row, which no kernel
+// writes, are loaded before the previous one is waited for.
+constexpr int kPairCached = 5;  // entries per lane of a row loaded ahead
+
+struct PairScalars {
+    double rz, rr, pq_prev, rz_prev;
+    int base, done;
+    __device__ PairScalars(const CgState* st, int k)
+        : rz(st->ring[k & 3][1]), rr(st->ring[k & 3][2]), pq_prev(st->ring[(k + 3) & 3][0]),
+          rz_prev(st->ring[(k + 3) & 3][1]), base(st->it), done(st->done) {}
+    // of the iteration before k: 0 go on, 1 converged, 2 breakdown (NaN or p.Ap == 0), 3 limit
+    __device__ int test(double thresh2, int k, int max_iter) const {
+        if (base + k == 0) return 0;  // k_set_thresh has tested the start
+        if (rr <= thresh2) return 1;
+        if (!(rz == rz) || pq_prev == 0.0) return 2;
+        return base + k >= max_iter ? 3 : 0;
+    }
+};
+// by one thread; st->it stays until the chunk's end, other blocks still read it
+__device__ __forceinline__ void pair_record(CgState* st, int it, int state) {
+    if (state == 1) st->converged_at = it;
+    st->stopped_at = it;
+    st->done = state;
+}
+
+__global__ void __launch_bounds__(kThreads) k_pair_product(int n, const int32_t* __restrict__ rp,
+                                                           const int32_t* __restrict__ ci,
+                                                           const double* __restrict__ v, const double* z, double* pa,
+                                                           double* pb, double* q, CgState* st, int k, int max_iter) {
+    constexpr int L = fem::kLanesPerRow;
+    const int sub = threadIdx.x % L, row = (blockIdx.x * kThreads + threadIdx.x) / L;
+    int j = 0, e = 0;
+    if (row < n) {
+        j = rp[row] + sub;
+        e = rp[row + 1];
+    }
+    int32_t cc[kPairCached];
+    double cv[kPairCached];
+#pragma unroll
+    for (int m = 0; m < kPairCached; ++m) {
+        const bool in = j + m * L < e;
+        cc[m] = in ? ci[j + m * L] : -1;
+        cv[m] = in ? v[j + m * L] : 0.0;
+    }
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const PairScalars s(st, k);
+    const double* po = k & 1 ? pb : pa;
+    double* pn = k & 1 ? pa : pb;
+    if (s.done) return;
+    const int state = s.test(st->thresh2, k, max_iter);
+    if (state) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) pair_record(st, s.base + k, state);
+        return;
+    }
+    const double beta = s.base + k ? s.rz / s.rz_prev : 0.0;
+    double dot = 0.0, pq = 0.0, a[kPairCached];
+#pragma unroll
+    for (int m = 0; m < kPairCached; ++m) a[m] = cc[m] >= 0 ? fma(beta, po[cc[m]], z[cc[m]]) : 0.0;
+#pragma unroll
+    for (int m = 0; m < kPairCached; ++m) dot = fma(cv[m], a[m], dot);
+#pragma unroll 4
+    for (j += kPairCached * L; j < e; j += L) {
+        const int c = ci[j];
+        dot = fma(v[j], fma(beta, po[c], z[c]), dot);
+    }
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    if (sub == 0 && row < n) {
+        const double p = fma(beta, po[row], z[row]);
+        pn[row] = p;
+        q[row] = dot;
+        pq = dot * p;
+    }
+    const double sum[1] = {pq};
+    fem::block_sum_add<kThreads, L, 1>(sum, {&st->ring[k & 3][0]});
+    if (blockIdx.x == 0 && threadIdx.x < 4) st->ring[(k + 2) & 3][threadIdx.x] = 0.0;
+}
+
+constexpr int kPairThreads = 128;  // of the update: a small system spreads over more SMs
+__global__ void __launch_bounds__(kPairThreads) k_pair_update(int n, double* x, double* r, double* z,
+                                                              const double* pa, const double* pb, const double* q,
+                                                              const double* dinv, CgState* st, int k) {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (st->done) return;
+    const int nxt = (k + 1) & 3;
+    const double* p = k & 1 ? pa : pb;
+    const double alpha = st->ring[k & 3][1] / st->ring[k & 3][0];
+    double sum[2] = {0.0, 0.0};
+    const int i = blockIdx.x * kPairThreads + threadIdx.x;
+    if (i < n) {
+        x[i] = fma(alpha, p[i], x[i]);
+        const double ri = fma(-alpha, q[i], r[i]);
+        r[i] = ri;
+        const double zi = dinv[i] * ri;
+        z[i] = zi;
+        sum[0] = ri * zi;
+        sum[1] = ri * ri;
+    }
+    fem::block_sum_add<kPairThreads, 1, 2>(sum, {&st->ring[nxt][1], &st->ring[nxt][2]});
+}
+
+// end of a chunk: its last iteration's test, and the next chunk's base
+__global__ void k_pair_end(CgState* st, int chunk, int max_iter) {
+    const PairScalars s(st, chunk);
+    if (!s.done) {
+        const int state = s.test(st->thresh2, chunk, max_iter);
+        st->it = s.base + chunk;
+        if (state) pair_record(st, s.base + chunk, state);
+    } else {
+        st->it = st->stopped_at;
+    }
+}
+
+// Two launches where every lane group has one row and every SM at most one block
+// of the product (9,728 rows on GB300).  Microseconds per iteration, four launches ->
+// two: plane systems of 578 rows 18.3 -> 11.0, 2,178 rows 14.7 -> 9.2, 8,450 rows
+// 14.7 -> 9.7; solids of 1,029 rows 18.8 -> 13.7, 6,591 rows 17.5 -> 13.1.  Past the
+// line the second gather costs more than the launches: 13,122 rows 15.0 -> 14.1,
+// 18,818 rows 15.0 -> 15.1, 132,098 rows 33 -> 39, solid of 14,739 rows 18.5 -> 49.
+bool pair_system(int64_t n) { return n * fem::kLanesPerRow <= (int64_t)fem::sm_count() * kThreads; }
+
+// launch that may begin before the previous kernel of the stream has ended
+// (which it waits for itself)
+template <class... P, class... A>
+cudaError_t launch_overlapped(void (*f)(P...), unsigned blocks, unsigned threads, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, f, P(args)...);
 }
 
 __global__ void k_set_thresh(CgState* st, double rtol) {
@@ -210,18 +338,20 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     const auto t0 = std::chrono::steady_clock::now();
     double *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *dinv = nullptr;
     CgState* st = nullptr;
-    cudaError_t e = cudaMallocAsync(&r, 5 * n * sizeof(double), sm);
+    cudaError_t e = cudaMallocAsync(&r, 6 * n * sizeof(double), sm);
     if (e == cudaSuccess) e = cudaMallocAsync(&st, sizeof(CgState), sm);
     if (e != cudaSuccess) return fail(c, FEM_GPU_OUT_OF_MEMORY, "pcg workspace");
     z = r + n;
     p = z + n;
     q = p + n;
-    dinv = q + n;
+    dinv = q + n;  // then the second direction array of the two-launch iteration
+    const bool pair = pair_system(n);
+    const unsigned upd_blocks = (unsigned)((n + kPairThreads - 1) / kPairThreads);
     cudaMemsetAsync(st, 0, sizeof(CgState), sm);
-    const int tpb = 256;
+    const int tpb = kThreads;
     const unsigned row_blocks = (unsigned)((n * fem::kLanesPerRow + tpb - 1) / tpb);
     const unsigned spmv_blocks = (unsigned)std::min<int64_t>(row_blocks, (int64_t)sm_count() * 16);
-    const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 16);
+    const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 8);
     k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv,
                                                                 opts->preconditioner == 1);
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, st);
@@ -233,13 +363,23 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     cudaGraphExec_t exec = nullptr;
     e = cudaStreamBeginCapture(sm, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        for (int k = 0; k < chunk; ++k) {
+        for (int k = 0; k < chunk && pair; ++k) {
+            e = launch_overlapped(k_pair_product, row_blocks, tpb, sm, n, rowptr, colidx, vals, z, p, dinv + n, q, st,
+                                  k, opts->max_iter);
+            if (e == cudaSuccess)
+                e = launch_overlapped(k_pair_update, upd_blocks, kPairThreads, sm, n, x, r, z, p, dinv + n, q, dinv,
+                                      st, k);
+            if (e != cudaSuccess) break;
+        }
+        if (pair) k_pair_end<<<1, 1, 0, sm>>>(st, chunk, opts->max_iter);
+        for (int k = 0; k < chunk && !pair; ++k) {
             k_spmv_pq<<<spmv_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, p, q, st);
             k_update_xr<<<vec_blocks, tpb, 0, sm>>>(n, x, r, z, p, q, dinv, st);
             k_update_p<<<vec_blocks, tpb, 0, sm>>>(n, p, z, st);
             k_advance<<<1, 1, 0, sm>>>(st, opts->max_iter);
         }
-        e = cudaStreamEndCapture(sm, &graph);
+        const cudaError_t ended = cudaStreamEndCapture(sm, &graph);
+        if (e == cudaSuccess) e = ended;
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     CgState hs{};
@@ -248,7 +388,7 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
         for (int launched = 0; launched < opts->max_iter + chunk; launched += chunk) {
             e = cudaGraphLaunch(exec, sm);
             if (e != cudaSuccess) break;
-            c->launches += 4 * chunk;
+            c->launches += pair ? 2 * chunk + 1 : 4 * chunk;
             e = cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, sm);
             if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
             if (e != cudaSuccess || hs.done) break;
@@ -374,9 +514,9 @@ extern "C" fem_gpu_status fem_gpu_pcg_noalloc(fem_gpu_ctx* c, const int32_t* row
     // the array keeps the previous call's contents: the state must start at zero
     cudaError_t e = cudaMemsetAsync(cs, 0, sizeof(CgState), sm);
     if (e != cudaSuccess) return fail(c, FEM_GPU_CUDA_ERROR, std::string("pcg_noalloc: ") + cudaGetErrorString(e));
-    const int tpb = 256;
+    const int tpb = kThreads;
     const unsigned row_blocks = (unsigned)((n * fem::kLanesPerRow + tpb - 1) / tpb);
-    const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 16);
+    const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 8);
     k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv,
                                                                 opts->preconditioner == 1);
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, cs);
@@ -439,10 +579,10 @@ extern "C" fem_gpu_status fem_gpu_pcg_snapshots(fem_gpu_ctx* c, const int32_t* r
     }
     double *z = r + n, *p = z + n, *q = p + n, *dinv = q + n;
     cudaMemsetAsync(st, 0, sizeof(CgState), sm);
-    const int tpb = 256;
+    const int tpb = kThreads;
     const unsigned row_blocks = (unsigned)((n * fem::kLanesPerRow + tpb - 1) / tpb);
     const unsigned spmv_blocks = (unsigned)std::min<int64_t>(row_blocks, (int64_t)sm_count() * 16);
-    const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 16);
+    const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 8);
     k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv, opts->preconditioner == 1);
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, st);
     k_set_thresh<<<1, 1, 0, sm>>>(st, opts->rel_tol);
