@@ -1247,7 +1247,7 @@ fem_gpu_status assemble_set(fem_gpu_ctx* c, int set, const double* u, double* va
     SetData& s = c->sets[set];
     if (cluster_set(c, set))
         return cluster_launch_set(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0);
-    if (lattice_set(c, set)) return lattice_assemble(c, set, u, vals, rhs, true, true);
+    if (lattice_assembles(c, set)) return lattice_assemble(c, set, u, vals, rhs, true, true);
     if (brick_range(c, set, 0, s.neq)) return brick_launch(c, s, 0, s.neq, u, vals, rhs, c->stream);
     if (s.kind == 0)
         return launch_bulk(c, set, MODE_ASSEMBLE, 0, s.neq, u, vals, rhs, nullptr, nullptr, 0, nullptr, nullptr);
@@ -1694,7 +1694,7 @@ fem_gpu_status fem_gpu_assemble(fem_gpu_ctx* c, const double* u, double* vals, d
     // assembly are element ranges, which the lattice kernels do not have)
     int lead = -1;
     for (int k = 0; k < (int)c->sets.size() && lead < 0 && !hp; ++k)
-        if (lattice_set(c, k)) lead = k;
+        if (lattice_assembles(c, k)) lead = k;
     if (!acc && lead < 0) {
         if (sv.dev) cudaMemsetAsync(sv.dev, 0, c->nnz * sizeof(double), sm);
         if (sr.dev) cudaMemsetAsync(sr.dev, 0, nad * sizeof(double), sm);
@@ -1707,7 +1707,7 @@ fem_gpu_status fem_gpu_assemble(fem_gpu_ctx* c, const double* u, double* vals, d
         if (cluster_set(c, k))
             return cluster_launch_set(c, k, MODE_ASSEMBLE, first, count, (const double*)su.dev, (double*)sv.dev,
                                       (double*)sr.dev, nullptr, nullptr, 0);
-        if (lead >= 0 && lattice_set(c, k))
+        if (lead >= 0 && lattice_assembles(c, k))
             return lattice_assemble(c, k, (const double*)su.dev, (double*)sv.dev, (double*)sr.dev, true, true);
         if (brick_range(c, k, first, count))
             return brick_launch(c, s, first, count, (const double*)su.dev, (double*)sv.dev, (double*)sr.dev, c->stream);

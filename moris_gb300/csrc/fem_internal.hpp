@@ -183,6 +183,15 @@ fem_gpu_status assemble_set(fem_gpu_ctx* c, int set, const double* u, double* va
 fem_gpu_status lattice_finalize(fem_gpu_ctx* c);
 void lattice_release(fem_gpu_ctx* c);
 inline bool lattice_set(const fem_gpu_ctx* c, int set) { return c->sets[set].lattice && !c->sets[set].pinned; }
+// Quadratic splines take three kernels in sequence (stencil, projection, residual),
+// each a chain of 10 to 25 us however few the cells; below this many cells one launch
+// of the element loop is the faster assembly.  Measured, element loop / lattice:
+// distorted cells 5^3 58 / 88 us, 8^3 78 / 93, 12^3 168 / 138; bricks 6 x 12 x 6 50 /
+// 66, 15 x 13 x 11 120 / 88.
+constexpr int64_t kLatticeQuadCells = 1024;
+inline bool lattice_assembles(const fem_gpu_ctx* c, int set) {
+    return lattice_set(c, set) && (c->sets[set].maxnb != 27 || c->num_cells >= kLatticeQuadCells);
+}
 fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs, bool acc_v,
                                 bool acc_r);
 // device address of fem_gpu_pcg_noalloc's fixed array on the current device,

@@ -25,8 +25,14 @@
 // density set with linear splines 13.4 -> 3.56 ms, matrix-free product of 48 x
 // 47 x 45 quadratic cells 969 -> 206 us.  The stencil and projection kernels
 // keep the FP64 pipe 72-77 % busy, lattice_density 55 % (register-bound
-// occupancy).  Smaller models gain less but none was slower, so there is no
-// size limit.
+// occupancy).  Below 1,024 cells quadratic splines keep the element loop
+// (kLatticeQuadCells).
+//
+// Cells of any shape on the same lattice of nodes (FEM_GPU_SHAPE_GENERAL): the cells
+// add their matrices to the block stencil (fem_hex.cuh), or to the CSR for linear
+// splines, and the projection is the same.  26 x 23 x 21 quadratic 699 -> 545 us (hex
+// 371, projection 128); 26^3 linear 467 -> 294 us, matrix-free products 401 -> 206
+// (linear) and 622 -> 264 us.
 //
 // A model takes this path when lattice_finalize finds all of the above to hold
 // exactly (coordinates, numbering, weights, and a CSR whose rows are the full
@@ -39,6 +45,7 @@
 #include <vector>
 
 #include "fem_bits.cuh"
+#include "fem_hex.cuh"
 #include "fem_internal.hpp"
 
 namespace fem {
@@ -752,6 +759,7 @@ __global__ void __launch_bounds__(32 * (2 * P + 1)) lattice_plane(PlaneArgs p) {
 
 struct Lattice {
     int dim = 3, p = 0;
+    bool brick = true;  // axis-aligned cells (FEM_GPU_SHAPE_RECTANGULAR)
     int ne[3], nn[3], nb[3];
     int64_t pitch = 0;
     DeviceBuf jac;     // half edge lengths and their reciprocals
@@ -785,20 +793,17 @@ const double* axis_weights(int p) {
 // exactly (the extraction weights of order 3, which are not dyadic, up to 1e-15)
 bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
     const int D = c->dim;
-    if (c->shape != FEM_GPU_SHAPE_RECTANGULAR || c->num_used != c->num_bases) return false;
+    L.brick = c->shape == FEM_GPU_SHAPE_RECTANGULAR;
+    if ((D == 2 && !L.brick) || c->num_used != c->num_bases || c->num_cells < 1) return false;
     const double* X = c->coords.data();
     const int64_t N = c->num_nodes;
-    int64_t nn[3] = {1, 1, 1}, step[3] = {1, 1, 1};
-    // nodes with the coordinates of node 0 along all later axes
-    for (int d = 0; d + 1 < D; ++d) {
-        step[d + 1] = step[d];
-        const auto same = [&](int64_t n) {
-            for (int k = d + 1; k < D; ++k)
-                if (X[n * D + k] != X[k]) return false;
-            return true;
-        };
-        while (nn[d] * step[d] < N && same(nn[d] * step[d])) ++nn[d];
-        step[d + 1] = step[d] * nn[d];
+    // edges from the first cell's nodes: (0, 1) is nn0, (0, 0, 1) is nn0 nn1
+    int64_t nn[3] = {c->cells[3], 1, 1}, step[3] = {1, nn[0], 1};
+    if (nn[0] < 2) return false;
+    if (D == 3) {
+        step[2] = c->cells[4];
+        if (step[2] < nn[0] || step[2] % nn[0]) return false;
+        nn[1] = step[2] / nn[0];
     }
     if (N % step[D - 1]) return false;
     nn[D - 1] = N / step[D - 1];
@@ -817,7 +822,7 @@ bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
         if (nn[d] < 2 || nn[d] > 1 << 20) return false;
         cells *= L.ne[d];
         bases *= L.nb[d];
-        for (int e = 0; e < L.ne[d]; ++e) {
+        for (int e = 0; L.brick && e < L.ne[d]; ++e) {
             jac.push_back(0.5 * (X[(e + 1) * step[d] * D + d] - X[e * step[d] * D + d]));
             if (!(jac.back() > 0.0)) return false;
         }
@@ -827,7 +832,7 @@ bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
     const double tol = L.p == 3 ? 1e-15 : 0.0;
     for (int64_t n = 0, k = 0; n < N; ++n) {
         const int64_t i[3] = {n % nn[0], n / nn[0] % nn[1], n / (nn[0] * nn[1])};
-        for (int d = 0; d < D; ++d)
+        for (int d = 0; L.brick && d < D; ++d)
             if (X[n * D + d] != X[i[d] * step[d] * D + d]) return false;
         if (c->t_off[n + 1] - c->t_off[n] != width) return false;
         for (int q = 0; q < width; ++q, ++k) {
@@ -888,7 +893,8 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
             seen[s.ip_cell[i]] = 1;
             ordered &= s.ip_cell[i] == i;
         }
-        if (!once) continue;
+        // cells of any shape: the modulus and the coordinates in the set's order
+        if (!once || (!L.brick && (!ordered || !s.node_rho.empty()))) continue;
         if (!ordered && e == cudaSuccess) {
             std::vector<double> E(s.neq);
             for (int64_t i = 0; i < s.neq; ++i) E[s.ip_cell[i]] = s.E[i];
@@ -1047,7 +1053,7 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         }
         a.wq[at] = r.w[q] * mu * scale / 64.0;
     }
-    if (!a.rho) {
+    if (L.brick && !a.rho) {
         // coefficients of every offset: the reference sums for the element and
         // nodes that lattice_const counts with a plus sign
         for (int k = 0; k < 27; ++k) {
@@ -1086,6 +1092,37 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
             L.nn[0], L.nn[1], L.nn[2], u, un);
         c->launches++;
     }
+    if (!L.brick) {
+        HexArgs h{};
+        for (int d = 0; d < 3; ++d) {
+            h.ne[d] = L.ne[d];
+            h.nn[d] = L.nn[d];
+        }
+        h.pitch = L.pitch;
+        h.E = a.E;
+        h.xe = (const double*)s.d_xe.p;
+        for (int i = 0; i < N; ++i) h.xq[i] = a.xq[i];
+        for (int i = 0; i < r.n; ++i) h.wq[i] = 64.0 * a.wq[i];
+        h.ld = a.ld;
+        h.lo = a.lo;
+        h.u = a.u;
+        h.r = a.r;
+        h.S = a.S;
+        h.vals = vals;
+        h.rowptr = a.rowptr;
+        h.status = a.status;
+        // the cells add to what they find
+        if (quad && vals) e = cudaMemsetAsync(a.S, 0, L.S.bytes, st);
+        if (!quad && vals && !acc_v) e = cudaMemsetAsync(vals, 0, c->nnz * sizeof(double), st);
+        if (e == cudaSuccess && rhs && !a.acc_r) e = cudaMemsetAsync(a.r, 0, 3 * nodes * sizeof(double), st);
+        const unsigned g = (unsigned)((c->num_cells + kHexWarps - 1) / kHexWarps);
+        using Fn = void (*)(HexArgs);
+        static const Fn cells[2][2] = {{hex_cells<2, HEX_STENCIL>, hex_cells<2, HEX_CSR>},
+                                       {hex_cells<3, HEX_STENCIL>, hex_cells<3, HEX_CSR>}};
+        const Fn hex = vals ? cells[N == 3][quad ? HEX_STENCIL : HEX_CSR] : N == 2 ? hex_residual<2> : hex_residual<3>;
+        if (vals || want_u) hex<<<g, 32 * kHexWarps, 0, st>>>(h);
+        c->launches += vals || want_u;
+    }
     const unsigned ctas = (unsigned)((nodes + kStencilNodes - 1) / kStencilNodes);
     const int out = !vals ? OUT_NONE : quad ? OUT_STENCIL : OUT_CSR;
     using Fn = void (*)(LatArgs);
@@ -1097,8 +1134,15 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         else lattice_moments<3><<<g, 128, 0, st>>>(a);
         c->launches++;
     }
-    fn[a.rho != nullptr][out]<<<ctas, kStencilThreads, 0, st>>>(a);
-    c->launches++;
+    if (L.brick) {
+        fn[a.rho != nullptr][out]<<<ctas, kStencilThreads, 0, st>>>(a);
+        c->launches++;
+    }
+    if (quad && rhs && e == cudaSuccess) {
+        lattice_restrict<<<(unsigned)std::min<int64_t>((3 * (c->num_used) + 255) / 256, grid3), 256, 0, st>>>(
+            L.nn[0], L.nn[1], L.nn[2], rn, 8.0, acc_r, rhs);
+        c->launches++;
+    }
     if (quad && vals && e == cudaSuccess) {
         ProjArgs q{};
         for (int d = 0; d < 3; ++d) {
@@ -1127,11 +1171,6 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         e = cudaFuncSetAttribute(lattice_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmem);
         if (e == cudaSuccess)
             lattice_project<<<dim3((unsigned)tiles, (unsigned)q.chunks), kProjThreads, kProjSmem, st>>>(q);
-        c->launches++;
-    }
-    if (quad && rhs && e == cudaSuccess) {
-        lattice_restrict<<<(unsigned)std::min<int64_t>((3 * (c->num_used) + 255) / 256, grid3), 256, 0, st>>>(
-            L.nn[0], L.nn[1], L.nn[2], rn, 8.0, acc_r, rhs);
         c->launches++;
     }
     if (e == cudaSuccess) e = cudaGetLastError();

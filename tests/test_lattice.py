@@ -29,7 +29,8 @@ def _assemble(torch, m, u, flags=0, vals=None, rhs=None):
     return vals, rhs
 
 
-SIZES = [(1, 1, 1), (2, 1, 3), (7, 3, 3), (8, 4, 4), (6, 2, 3), (9, 5, 2), (17, 6, 5)]
+# quadratic splines below 1,024 cells are assembled by the element loop
+SIZES = [(1, 1, 1), (2, 1, 3), (7, 3, 3), (8, 4, 4), (6, 2, 3), (9, 5, 2), (17, 6, 5), (4, 16, 16), (17, 9, 7)]
 
 
 @pytest.mark.parametrize("density", [False, True], ids=["E", "rho"])
