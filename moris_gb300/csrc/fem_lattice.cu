@@ -765,6 +765,9 @@ struct Lattice {
     DeviceBuf jac;     // half edge lengths and their reciprocals
     DeviceBuf S, vec;  // quadratic splines: stencil, nodal vectors
     DeviceBuf Q;       // density sets: element sums
+    // the last use of S, vec and Q: a call on another stream waits for it
+    cudaEvent_t done = nullptr;
+    cudaStream_t last = nullptr;
 };
 
 void dfree(DeviceBuf& b) {
@@ -930,6 +933,9 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
         }
     }
     if (rho && e == cudaSuccess) e = cudaMemsetAsync(K->Q.p, 0, K->Q.bytes, st);
+    if ((rho || quad) && e == cudaSuccess) e = cudaEventCreateWithFlags(&K->done, cudaEventDisableTiming);
+    if (K->done && e == cudaSuccess) e = cudaEventRecord(K->done, st);
+    K->last = st;
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? FEM_GPU_OK
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice data: ") + cudaGetErrorString(e));
@@ -947,6 +953,7 @@ void lattice_release(fem_gpu_ctx* c) {
     dfree(L->S);
     dfree(L->vec);
     dfree(L->Q);
+    if (L->done) cudaEventDestroy(L->done);
     delete L;
     c->lattice = nullptr;
 }
@@ -1001,6 +1008,42 @@ fem_gpu_status plane_assemble(fem_gpu_ctx* c, const Lattice& L, const SetData& s
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice launch: ") + cudaGetErrorString(e));
 }
 
+// The workspaces of one call.  A matrix-free product returns before it has run, so a
+// call on another stream waits for the one before it; a captured call, which may be
+// replayed beside any other, takes memory of its own (nodes of the graph).
+struct LatticeWork {
+    Lattice& L;
+    cudaStream_t st;
+    bool shared = true;
+    void *S, *vec, *Q;
+    cudaError_t e = cudaSuccess;
+    LatticeWork(Lattice& l, cudaStream_t stream, bool stencil)
+        : L(l), st(stream), S(l.S.p), vec(l.vec.p), Q(l.Q.p) {
+        if (!L.done) return;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cudaGetLastError();
+        if (cs == cudaStreamCaptureStatusActive) {
+            shared = false;
+            S = vec = Q = nullptr;
+            if (L.S.p && stencil) e = cudaMallocAsync(&S, L.S.bytes, st);
+            if (L.vec.p && e == cudaSuccess) e = cudaMallocAsync(&vec, L.vec.bytes, st);
+            if (L.Q.p && e == cudaSuccess) e = cudaMallocAsync(&Q, L.Q.bytes, st);
+            if (Q && e == cudaSuccess) e = cudaMemsetAsync(Q, 0, L.Q.bytes, st);
+        } else if (L.last != st) {
+            e = cudaStreamWaitEvent(st, L.done, 0);
+        }
+    }
+    ~LatticeWork() {
+        if (!shared) {
+            for (void* p : {S, vec, Q})
+                if (p) cudaFreeAsync(p, st);
+        } else if (L.done) {
+            cudaEventRecord(L.done, st);
+            L.last = st;
+        }
+    }
+};
+
 }  // namespace
 
 // One lattice set: CSR values (nullable) and residual (nullable) of the adof
@@ -1013,7 +1056,10 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     cudaStream_t st = (cudaStream_t)c->stream;
     const int64_t nodes = (int64_t)L.nn[0] * L.nn[1] * L.nn[2];
     const bool quad = L.p == 2;
-    cudaError_t e = cudaSuccess;
+    LatticeWork work(L, st, vals != nullptr);
+    cudaError_t e = work.e;
+    if (e != cudaSuccess)
+        return fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice workspace: ") + cudaGetErrorString(e));
     LatArgs a{};
     for (int d = 0; d < 3; ++d) {
         a.ne[d] = L.ne[d];
@@ -1026,9 +1072,9 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     a.rowptr = (const int32_t*)c->d_rowptr.p;
     a.status = (int*)c->d_status.p;
     a.vals = vals;
-    a.S = (double*)L.S.p;
-    a.Q = (double*)L.Q.p;
-    double* un = (double*)L.vec.p;
+    a.S = (double*)work.S;
+    a.Q = (double*)work.Q;
+    double* un = (double*)work.vec;
     double* rn = un + 3 * nodes;
     const bool want_u = u && rhs;
     a.u = want_u ? (quad ? un : u) : nullptr;
