@@ -135,10 +135,6 @@ __global__ void __launch_bounds__(32 * kHexWarps) hex_cells(HexArgs p) {
     while (b >= 7 - a) b -= 7 - a++;
     b += a + 1;
     const int64_t na = cl.node(p, a), nb = cl.node(p, b);
-    double du[3] = {0.0, 0.0, 0.0};
-    if (p.u)
-#pragma unroll
-        for (int f = 0; f < 3; ++f) du[f] = __ldg(p.u + f * cl.nodes + nb) - __ldg(p.u + f * cl.nodes + na);
     __syncwarp();
     hex_gradients<N>(p, X, G, lane);
     __syncwarp();
@@ -201,6 +197,13 @@ __global__ void __launch_bounds__(32 * kHexWarps) hex_cells(HexArgs p) {
             for (int g = 0; g < 3; ++g)
                 K[f * 3 + g] = f == g ? fma(p.ld, A[f * 4], tr) : fma(p.lo, A[f * 3 + g], A[g * 3 + f]);
     }
+    // from here on with what an overlapped kernel writes: u, and the sums
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    double du[3] = {0.0, 0.0, 0.0};
+    if (p.u)
+#pragma unroll
+        for (int f = 0; f < 3; ++f) du[f] = p.u[f * cl.nodes + nb] - p.u[f * cl.nodes + na];
     __syncwarp();  // the gradients are read
     if (lane < 28) {
 #pragma unroll
@@ -284,13 +287,14 @@ __global__ void __launch_bounds__(32 * kHexWarps) hex_residual(HexArgs p) {
     double* T = GU;
     HexCell cl;
     if (!cl.init(p, (int64_t)blockIdx.x * kHexWarps + (threadIdx.x >> 5))) return;
-    if (lane < 24) {
-        X[lane] = __ldg(p.xe + cl.cell * 24 + lane);
-        U[lane] = __ldg(p.u + lane % 3 * cl.nodes + cl.node(p, lane / 3));
-    }
+    if (lane < 24) X[lane] = __ldg(p.xe + cl.cell * 24 + lane);
     const double E = __ldg(p.E + cl.cell);
     __syncwarp();
     hex_gradients<N>(p, X, GX, lane);
+    cudaGridDependencySynchronize();  // u
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (lane < 24) U[lane] = p.u[lane % 3 * cl.nodes + cl.node(p, lane / 3)];
+    __syncwarp();
     hex_gradients<N>(p, U, GU, lane);
     __syncwarp();
     if (lane < NQ) {

@@ -183,14 +183,19 @@ fem_gpu_status assemble_set(fem_gpu_ctx* c, int set, const double* u, double* va
 fem_gpu_status lattice_finalize(fem_gpu_ctx* c);
 void lattice_release(fem_gpu_ctx* c);
 inline bool lattice_set(const fem_gpu_ctx* c, int set) { return c->sets[set].lattice && !c->sets[set].pinned; }
-// Quadratic splines take three kernels in sequence (stencil, projection, residual),
-// each a chain of 10 to 25 us however few the cells; below this many cells one launch
-// of the element loop is the faster assembly.  Measured, element loop / lattice:
-// distorted cells 5^3 58 / 88 us, 8^3 78 / 93, 12^3 168 / 138; bricks 6 x 12 x 6 50 /
-// 66, 15 x 13 x 11 120 / 88.
-constexpr int64_t kLatticeQuadCells = 1024;
-inline bool lattice_assembles(const fem_gpu_ctx* c, int set) {
-    return lattice_set(c, set) && (c->sets[set].maxnb != 27 || c->num_cells >= kLatticeQuadCells);
+// The lattice path takes one to four kernels in sequence, each a chain of 5 to 25 us
+// however few the cells; on small models one launch of the element loop is faster.
+// Measured calls, element loop / lattice, in us.  Assembly of bricks: linear 7^3 42 /
+// 54, 10^3 54 / 51, 13^3 65 / 53; quadratic 7^3 55 / 73, 10^3 80 / 75, 13^3 129 / 100.
+// Products of bricks: linear 6^3 24 / 28, 10^3 28 / 28, 16^3 52 / 33; quadratic 6^3 24
+// / 37, 10^3 31 / 38, 16^3 64 / 44.  Cells of any shape: linear 5^3 54 / 43, products
+// 30 / 23; quadratic 7^3 68 / 77, 10^3 120 / 99, products 8^3 42 / 36.
+inline bool lattice_pays(const fem_gpu_ctx* c, int set, bool product) {
+    if (!lattice_set(c, set)) return false;
+    const bool quad = c->sets[set].maxnb == 27;
+    if (c->dim == 2) return true;
+    if (c->shape != FEM_GPU_SHAPE_RECTANGULAR) return !quad || c->num_cells >= (product ? 216 : 1000);
+    return c->num_cells >= (quad && product ? 1728 : 1000);
 }
 fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs, bool acc_v,
                                 bool acc_r);

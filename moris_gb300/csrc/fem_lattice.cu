@@ -25,8 +25,7 @@
 // density set with linear splines 13.4 -> 3.56 ms, matrix-free product of 48 x
 // 47 x 45 quadratic cells 969 -> 206 us.  The stencil and projection kernels
 // keep the FP64 pipe 72-77 % busy, lattice_density 55 % (register-bound
-// occupancy).  Below 1,024 cells quadratic splines keep the element loop
-// (kLatticeQuadCells).
+// occupancy).  Small models keep the element loop (lattice_pays).
 //
 // Cells of any shape on the same lattice of nodes (FEM_GPU_SHAPE_GENERAL): the cells
 // add their matrices to the block stencil (fem_hex.cuh), or to the CSR for linear
@@ -47,6 +46,7 @@
 #include "fem_bits.cuh"
 #include "fem_hex.cuh"
 #include "fem_internal.hpp"
+#include "fem_launch.cuh"
 
 namespace fem {
 namespace {
@@ -106,17 +106,28 @@ struct NodeOut {
             for (int f = 0; f < 3; ++f) row[f] = live ? __ldg(p.rowptr + f * nodes + node) : 0;
         }
     }
-    __device__ __forceinline__ void block(int dx, int dy, const double K[9]) {
-        const bool in = live && x + dx >= 0 && x + dx < p.nn[0] && y + dy >= 0 && y + dy < p.nn[1] && z + DZ >= 0 &&
-                        z + DZ < p.nn[2];
-        if (p.u && in) {
+    __device__ __forceinline__ bool inside(int dx, int dy) const {
+        return live && x + dx >= 0 && x + dx < p.nn[0] && y + dy >= 0 && y + dy < p.nn[1] && z + DZ >= 0 &&
+               z + DZ < p.nn[2];
+    }
+    // displacements of the row of neighbours dy, ahead of its blocks: plain loads (an
+    // earlier kernel that this one overlaps wrote them), which do not pass the stores
+    // of a block
+    __device__ __forceinline__ void neighbours(int dy, double un[3][3]) const {
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
             const int64_t j = node + dx + (int64_t)p.nn[0] * (dy + (int64_t)p.nn[1] * DZ);
 #pragma unroll
-            for (int g = 0; g < 3; ++g) {
-                const double ug = __ldg(p.u + g * nodes + j);
+            for (int g = 0; g < 3; ++g) un[dx + 1][g] = p.u && inside(dx, dy) ? p.u[g * nodes + j] : 0.0;
+        }
+    }
+    __device__ __forceinline__ void block(int dx, int dy, const double un[3][3], const double K[9]) {
+        const bool in = inside(dx, dy);
+        if (p.u && in) {
 #pragma unroll
-                for (int f = 0; f < 3; ++f) r[f] = fma(K[f * 3 + g], ug, r[f]);
-            }
+            for (int g = 0; g < 3; ++g)
+#pragma unroll
+                for (int f = 0; f < 3; ++f) r[f] = fma(K[f * 3 + g], un[dx + 1][g], r[f]);
         }
         if constexpr (OUT != OUT_NONE) {
 #pragma unroll
@@ -142,9 +153,9 @@ struct NodeOut {
                 }
         }
     }
-    __device__ void finish(double red[3][kStencilNodes][3]) {
+    __device__ void finish(double red[kStencilNodes][3]) {
         if (bad && live) atomicOr(p.status, 1);
-        for (int f = 0; f < 3; ++f) red[DZ + 1][threadIdx.x % kStencilNodes][f] = r[f];
+        for (int f = 0; f < 3; ++f) red[threadIdx.x % kStencilNodes][f] = r[f];
     }
 };
 
@@ -172,8 +183,9 @@ __device__ __forceinline__ void store_residual(const LatArgs& p, int64_t node, c
 // A thread forms the nine blocks of one z offset, so that 96 threads work on
 // 32 nodes: a small lattice still fills the SMs, and consecutive lanes are
 // consecutive nodes whatever the edge lengths (no partial tiles).
+// (A warp per (dy, dz) as well: 2 us less up to 13^3 cells, a quarter more from 16^3 on.)
 template <int OUT, int DZ>
-__device__ __forceinline__ void const_blocks(const LatArgs& p, int64_t node, double red[3][kStencilNodes][3]) {
+__device__ __forceinline__ void const_blocks(const LatArgs& p, int64_t node, double red[kStencilNodes][3]) {
     NodeOut<OUT, DZ> out(p, node);
     // columns after the z axis: weights 0-2 and the xy pair (v_2) sum, the xz
     // (v_1) and yz (v_0) pairs difference
@@ -208,9 +220,12 @@ __device__ __forceinline__ void const_blocks(const LatArgs& p, int64_t node, dou
                              : m == 3 || m == 4 ? w[0][m] - w[1][m]
                                                 : w[0][m] + w[1][m];
         }
+    cudaGridDependencySynchronize();  // the nodal displacements
+    cudaTriggerProgrammaticLaunchCompletion();
 #pragma unroll
     for (int dy = -1; dy <= 1; ++dy) {
-        double d[6][2];
+        double un[3][3], d[6][2];
+        out.neighbours(dy, un);
 #pragma unroll
         for (int m = 0; m < 6; ++m)
 #pragma unroll
@@ -230,7 +245,7 @@ __device__ __forceinline__ void const_blocks(const LatArgs& p, int64_t node, dou
             const double K[9] = {fma(p.ld, a0, tr), s[5] * q[3],       s[4] * q[4],
                                  s[5] * q[5],       fma(p.ld, a1, tr), s[3] * q[6],
                                  s[4] * q[7],       s[3] * q[8],       fma(p.ld, a2, tr)};
-            out.block(dx, dy, K);
+            out.block(dx, dy, un, K);
         }
     }
     out.finish(red);
@@ -241,9 +256,9 @@ __global__ void __launch_bounds__(kStencilThreads) lattice_const(LatArgs p) {
     __shared__ double red[3][kStencilNodes][3];
     const int64_t node = (int64_t)blockIdx.x * kStencilNodes + threadIdx.x % kStencilNodes;
     const int w = threadIdx.x / kStencilNodes;
-    if (w == 0) const_blocks<OUT, -1>(p, node, red);
-    else if (w == 1) const_blocks<OUT, 0>(p, node, red);
-    else const_blocks<OUT, 1>(p, node, red);
+    if (w == 0) const_blocks<OUT, -1>(p, node, red[0]);
+    else if (w == 1) const_blocks<OUT, 0>(p, node, red[1]);
+    else const_blocks<OUT, 1>(p, node, red[2]);
     __syncthreads();
     store_residual(p, node, red);
 }
@@ -422,12 +437,14 @@ __global__ void __launch_bounds__(128) lattice_moments(LatArgs p) {
 }
 
 template <int OUT, int DZ>
-__device__ __forceinline__ void density_blocks(const LatArgs& p, int64_t node, double red[3][kStencilNodes][3]) {
+__device__ __forceinline__ void density_blocks(const LatArgs& p, int64_t node, double red[kStencilNodes][3]) {
     NodeOut<OUT, DZ> out(p, node);
     const int64_t ey = p.ne[0] + 2, ez = ey * (p.ne[1] + 2), qs = ez * (p.ne[2] + 2);
     const double* q = p.Q + out.z * ez + out.y * ey + out.x;
 #pragma unroll
-    for (int dy = -1; dy <= 1; ++dy)
+    for (int dy = -1; dy <= 1; ++dy) {
+        double un[3][3];
+        out.neighbours(dy, un);
 #pragma unroll
         for (int dx = -1; dx <= 1; ++dx) {
             const double a0 = gather<0, 1, 1, DZ>(q, qs, ey, ez, kXX, dx, dy),
@@ -443,8 +460,9 @@ __device__ __forceinline__ void density_blocks(const LatArgs& p, int64_t node, d
             const double K[9] = {fma(p.ld, a0, tr), fma(p.lo, xy, yx), fma(p.lo, xz, zx),
                                  fma(p.lo, yx, xy), fma(p.ld, a1, tr), fma(p.lo, yz, zy),
                                  fma(p.lo, zx, xz), fma(p.lo, zy, yz), fma(p.ld, a2, tr)};
-            out.block(dx, dy, K);
+            out.block(dx, dy, un, K);
         }
+    }
     out.finish(red);
 }
 
@@ -453,9 +471,10 @@ __global__ void __launch_bounds__(kStencilThreads, 4) lattice_density(LatArgs p)
     __shared__ double red[3][kStencilNodes][3];
     const int64_t node = (int64_t)blockIdx.x * kStencilNodes + threadIdx.x % kStencilNodes;
     const int w = threadIdx.x / kStencilNodes;
-    if (w == 0) density_blocks<OUT, -1>(p, node, red);
-    else if (w == 1) density_blocks<OUT, 0>(p, node, red);
-    else density_blocks<OUT, 1>(p, node, red);
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (w == 0) density_blocks<OUT, -1>(p, node, red[0]);
+    else if (w == 1) density_blocks<OUT, 0>(p, node, red[1]);
+    else density_blocks<OUT, 1>(p, node, red[2]);
     __syncthreads();
     store_residual(p, node, red);
 }
@@ -531,6 +550,8 @@ __global__ void __launch_bounds__(kProjThreads, kProjCtas) lattice_project(ProjA
     }
     __syncthreads();
     bool bad = false;
+    cudaGridDependencySynchronize();  // the stencil
+    cudaTriggerProgrammaticLaunchCompletion();
     for (int z = z0 - 1; z < z1; ++z) {  // node plane z; basis layer z from z0 on
         const bool have = z >= 0 && z < p.nn[2];
         if (have) {
@@ -609,7 +630,8 @@ __global__ void __launch_bounds__(kProjThreads, kProjCtas) lattice_project(ProjA
 }
 
 // nodal values of a quadratic spline field: un[g][node] = 1/8 of the sum of its eight bases
-__global__ void lattice_nodal(int n0, int n1, int n2, const double* __restrict__ u, double* __restrict__ un) {
+__global__ void lattice_nodal(int n0, int n1, int n2, const double* __restrict__ u, double* un) {
+    cudaTriggerProgrammaticLaunchCompletion();
     const int64_t nodes = (int64_t)n0 * n1 * n2, nu = (int64_t)(n0 + 1) * (n1 + 1) * (n2 + 1);
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nodes;
          t += (int64_t)gridDim.x * blockDim.x) {
@@ -625,8 +647,9 @@ __global__ void lattice_nodal(int n0, int n1, int n2, const double* __restrict__
 }
 
 // r[f][basis] (+)= scale * the sum of rn over the basis' eight nodes
-__global__ void lattice_restrict(int n0, int n1, int n2, const double* __restrict__ rn, double scale, int acc,
-                                 double* __restrict__ r) {
+__global__ void lattice_restrict(int n0, int n1, int n2, const double* rn, double scale, int acc, double* r) {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     const int b0 = n0 + 1, b1 = n1 + 1, b2 = n2 + 1;
     const int64_t nodes = (int64_t)n0 * n1 * n2, nu = (int64_t)b0 * b1 * b2;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nu; t += (int64_t)gridDim.x * blockDim.x) {
@@ -669,6 +692,7 @@ struct PlaneArgs {
 
 template <int P>
 __global__ void __launch_bounds__(32 * (2 * P + 1)) lattice_plane(PlaneArgs p) {
+    cudaTriggerProgrammaticLaunchCompletion();
     constexpr int ND = 2 * P + 1;
     __shared__ double red[ND][32][2];
     const int lane = threadIdx.x & 31, Dy = (int)(threadIdx.x >> 5) - P;
@@ -1133,10 +1157,20 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         }
     }
     const unsigned grid3 = (unsigned)sm_count() * 16;
+    // the kernels of a call overlap their beginnings with the end of the one before
+    // (4 to 6 launches of 4 to 40 us on small lattices)
+    bool overlap = false;
+    // cells of any shape add to what they find
+    if (!L.brick) {
+        if (quad && vals) e = cudaMemsetAsync(a.S, 0, L.S.bytes, st);
+        if (!quad && vals && !acc_v) e = cudaMemsetAsync(vals, 0, c->nnz * sizeof(double), st);
+        if (e == cudaSuccess && rhs && !a.acc_r) e = cudaMemsetAsync(a.r, 0, 3 * nodes * sizeof(double), st);
+    }
     if (quad && want_u) {
         lattice_nodal<<<(unsigned)std::min<int64_t>((3 * nodes + 255) / 256, grid3), 256, 0, st>>>(
             L.nn[0], L.nn[1], L.nn[2], u, un);
         c->launches++;
+        overlap = true;
     }
     if (!L.brick) {
         HexArgs h{};
@@ -1157,36 +1191,37 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         h.vals = vals;
         h.rowptr = a.rowptr;
         h.status = a.status;
-        // the cells add to what they find
-        if (quad && vals) e = cudaMemsetAsync(a.S, 0, L.S.bytes, st);
-        if (!quad && vals && !acc_v) e = cudaMemsetAsync(vals, 0, c->nnz * sizeof(double), st);
-        if (e == cudaSuccess && rhs && !a.acc_r) e = cudaMemsetAsync(a.r, 0, 3 * nodes * sizeof(double), st);
         const unsigned g = (unsigned)((c->num_cells + kHexWarps - 1) / kHexWarps);
         using Fn = void (*)(HexArgs);
         static const Fn cells[2][2] = {{hex_cells<2, HEX_STENCIL>, hex_cells<2, HEX_CSR>},
                                        {hex_cells<3, HEX_STENCIL>, hex_cells<3, HEX_CSR>}};
         const Fn hex = vals ? cells[N == 3][quad ? HEX_STENCIL : HEX_CSR] : N == 2 ? hex_residual<2> : hex_residual<3>;
-        if (vals || want_u) hex<<<g, 32 * kHexWarps, 0, st>>>(h);
-        c->launches += vals || want_u;
+        if (e == cudaSuccess && (vals || want_u)) {
+            e = launch_kernel(hex, g, 32 * kHexWarps, 0, st, overlap, h);
+            c->launches++;
+            overlap = true;
+        }
     }
     const unsigned ctas = (unsigned)((nodes + kStencilNodes - 1) / kStencilNodes);
     const int out = !vals ? OUT_NONE : quad ? OUT_STENCIL : OUT_CSR;
     using Fn = void (*)(LatArgs);
-    const Fn fn[2][3] = {{lattice_const<0>, lattice_const<1>, lattice_const<2>},
-                         {lattice_density<0>, lattice_density<1>, lattice_density<2>}};
+    static const Fn density[3] = {lattice_density<0>, lattice_density<1>, lattice_density<2>};
+    static const Fn constant[3] = {lattice_const<0>, lattice_const<1>, lattice_const<2>};
     if (a.rho) {
         const unsigned g = (unsigned)std::min<int64_t>((c->num_cells + 127) / 128, (int64_t)sm_count() * 64);
         if (N == 2) lattice_moments<2><<<g, 128, 0, st>>>(a);
         else lattice_moments<3><<<g, 128, 0, st>>>(a);
+        density[out]<<<ctas, kStencilThreads, 0, st>>>(a);
+        c->launches += 2;
+        overlap = true;
+    } else if (L.brick && e == cudaSuccess) {
+        e = launch_kernel(constant[out], ctas, kStencilThreads, 0, st, overlap, a);
         c->launches++;
-    }
-    if (L.brick) {
-        fn[a.rho != nullptr][out]<<<ctas, kStencilThreads, 0, st>>>(a);
-        c->launches++;
+        overlap = true;
     }
     if (quad && rhs && e == cudaSuccess) {
-        lattice_restrict<<<(unsigned)std::min<int64_t>((3 * (c->num_used) + 255) / 256, grid3), 256, 0, st>>>(
-            L.nn[0], L.nn[1], L.nn[2], rn, 8.0, acc_r, rhs);
+        e = launch_kernel(lattice_restrict, (unsigned)std::min<int64_t>((3 * (c->num_used) + 255) / 256, grid3), 256, 0,
+                          st, overlap, L.nn[0], L.nn[1], L.nn[2], rn, 8.0, acc_r, rhs);
         c->launches++;
     }
     if (quad && vals && e == cudaSuccess) {
@@ -1216,7 +1251,8 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         }
         e = cudaFuncSetAttribute(lattice_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmem);
         if (e == cudaSuccess)
-            lattice_project<<<dim3((unsigned)tiles, (unsigned)q.chunks), kProjThreads, kProjSmem, st>>>(q);
+            e = launch_kernel(lattice_project, dim3((unsigned)tiles, (unsigned)q.chunks), kProjThreads, kProjSmem, st,
+                              overlap, q);
         c->launches++;
     }
     if (e == cudaSuccess) e = cudaGetLastError();

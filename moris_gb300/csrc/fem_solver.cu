@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "fem_internal.hpp"
+#include "fem_launch.cuh"
 #include "fem_reduce.cuh"
 #include "fem_spmv.cuh"
 
@@ -280,22 +281,6 @@ __global__ void k_pair_end(CgState* st, int chunk, int max_iter) {
 // 18,818 rows 15.0 -> 15.1, 132,098 rows 33 -> 39, solid of 14,739 rows 18.5 -> 49.
 bool pair_system(int64_t n) { return n * fem::kLanesPerRow <= (int64_t)fem::sm_count() * kThreads; }
 
-// launch that may begin before the previous kernel of the stream has ended
-// (which it waits for itself)
-template <class... P, class... A>
-cudaError_t launch_overlapped(void (*f)(P...), unsigned blocks, unsigned threads, cudaStream_t st, A... args) {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, f, P(args)...);
-}
-
 __global__ void k_set_thresh(CgState* st, double rtol) {
     const double bn2 = st->bn2 > 0.0 ? st->bn2 : 1.0;
     st->bn2 = bn2;
@@ -364,11 +349,11 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     e = cudaStreamBeginCapture(sm, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
         for (int k = 0; k < chunk && pair; ++k) {
-            e = launch_overlapped(k_pair_product, row_blocks, tpb, sm, n, rowptr, colidx, vals, z, p, dinv + n, q, st,
-                                  k, opts->max_iter);
+            e = launch_kernel(k_pair_product, row_blocks, tpb, 0, sm, true, n, rowptr, colidx, vals, z, p, dinv + n, q,
+                              st, k, opts->max_iter);
             if (e == cudaSuccess)
-                e = launch_overlapped(k_pair_update, upd_blocks, kPairThreads, sm, n, x, r, z, p, dinv + n, q, dinv,
-                                      st, k);
+                e = launch_kernel(k_pair_update, upd_blocks, kPairThreads, 0, sm, true, n, x, r, z, p, dinv + n, q,
+                                  dinv, st, k);
             if (e != cudaSuccess) break;
         }
         if (pair) k_pair_end<<<1, 1, 0, sm>>>(st, chunk, opts->max_iter);

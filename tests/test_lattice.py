@@ -64,7 +64,7 @@ def test_lattice_assembly_matches_oracle_and_element_loop(torch, ne, p, rule, de
 
 
 @pytest.mark.parametrize("p", [1, 2])
-@pytest.mark.parametrize("ne", [(1, 2, 1), (8, 3, 5)], ids=lambda n: "x".join(map(str, n)))
+@pytest.mark.parametrize("ne", [(1, 2, 1), (8, 3, 5), (13, 12, 12)], ids=lambda n: "x".join(map(str, n)))
 def test_lattice_apply_and_several_sets(torch, ne, p):
     """Two sets over the same cells in another order, graded cells, the
     matrix-free product and a non-finite modulus product's status."""
