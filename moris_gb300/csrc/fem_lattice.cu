@@ -672,10 +672,12 @@ __global__ void lattice_restrict(int n0, int n1, int n2, const double* rn, doubl
 //   A_xx(i, j) = sum_e E J_y / J_x D(i_x, j_x) M(i_y, j_y), ...
 // over the at most (p + 1)^2 elements that splines i and j share: summed along x,
 // then along y, four products per element and offset, no element matrix.  Lane =
-// basis, warp = y offset; a thread forms the 2 p + 1 blocks of its offsets and
-// their share of the residual.  The element loop spent a CTA on 8 x 8 to 32 x 32
-// matrices; measured (assembly with two side sets): 257 x 130, p = 2, 237 -> 107 us,
-// 24 x 17, p = 1, 61 -> 47 us.
+// basis, warp = y offset: p + 1 of the warps form the sums along x, which all share
+// (without that 864 instead of 560 FP64 instructions per basis, p = 2); a thread forms
+// the 2 p + 1 blocks of its offsets and their share of the residual.  The element loop spent a CTA on 8 x 8 to 32 x 32
+// matrices; measured (assembly with two side sets): 257 x 130, p = 2, 237 -> 68.5 us
+// (kernel 44, FP64 pipe 68 %), 256 x 256, p = 3, 544 -> 201 us, 24 x 17, p = 1, 61 ->
+// 33 us.
 struct PlaneArgs {
     int ne[2], nb[2];
     const double* E;
@@ -701,24 +703,21 @@ __global__ void __launch_bounds__(32 * (2 * P + 1)) lattice_plane(PlaneArgs p) {
     const int bx = live ? b % p.nb[0] : 0, by = live ? b / p.nb[0] : 0;
     const bool row = live && by + Dy >= 0 && by + Dy < p.nb[1];
     const int nj = p.ne[0] + p.ne[1];
-    double S[ND][4];  // xx, yy, xy, yx of offset Dx
-#pragma unroll
-    for (int d = 0; d < ND; ++d) S[d][0] = S[d][1] = S[d][2] = S[d][3] = 0.0;
-#pragma unroll 1
-    for (int iy = max(0, -Dy); iy <= min(P, P - Dy); ++iy) {
-        const int ey = by - iy, jy = iy + Dy;
-        if (!(row && ey >= 0 && ey < p.ne[1])) continue;
-        const double Jy = __ldg(p.jac + p.ne[0] + ey), Iy = __ldg(p.jac + nj + p.ne[0] + ey);
+    // sums along x over the elements of row by - iy, one warp per iy
+    __shared__ double xs[P + 1][ND][4][32];
+    if (Dy <= 0) {
+        const int iy = -Dy, ey = by - iy;
+        const bool have = live && ey >= 0 && ey < p.ne[1];
+        const double Jy = have ? __ldg(p.jac + p.ne[0] + ey) : 0.0, Iy = have ? __ldg(p.jac + nj + p.ne[0] + ey) : 0.0;
         double E[P + 1], wx[P + 1], wy[P + 1];
 #pragma unroll
         for (int i = 0; i <= P; ++i) {
             const int ex = bx - i;
-            const bool in = ex >= 0 && ex < p.ne[0];
+            const bool in = have && ex >= 0 && ex < p.ne[0];
             E[i] = in ? __ldg(p.E + (int64_t)ey * p.ne[0] + ex) * p.mu : 0.0;
             wx[i] = E[i] * Jy * (in ? __ldg(p.jac + nj + ex) : 0.0);
             wy[i] = E[i] * Iy * (in ? __ldg(p.jac + ex) : 0.0);
         }
-        const double My = p.M[iy][jy], Dyy = p.D[iy][jy], Gy = p.G[iy][jy], Hy = p.G[jy][iy];
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
             double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
@@ -731,10 +730,25 @@ __global__ void __launch_bounds__(32 * (2 * P + 1)) lattice_plane(PlaneArgs p) {
                 a2 = fma(E[i], p.G[i][j], a2);
                 a3 = fma(E[i], p.G[j][i], a3);
             }
-            S[d][0] = fma(a0, My, S[d][0]);
-            S[d][1] = fma(a1, Dyy, S[d][1]);
-            S[d][2] = fma(a2, Hy, S[d][2]);
-            S[d][3] = fma(a3, Gy, S[d][3]);
+            xs[iy][d][0][lane] = a0;
+            xs[iy][d][1][lane] = a1;
+            xs[iy][d][2][lane] = a2;
+            xs[iy][d][3][lane] = a3;
+        }
+    }
+    __syncthreads();
+    double S[ND][4];  // xx, yy, xy, yx of offset Dx
+#pragma unroll
+    for (int d = 0; d < ND; ++d) S[d][0] = S[d][1] = S[d][2] = S[d][3] = 0.0;
+    for (int iy = max(0, -Dy); iy <= min(P, P - Dy); ++iy) {
+        const int jy = iy + Dy;
+        const double My = p.M[iy][jy], Dyy = p.D[iy][jy], Gy = p.G[iy][jy], Hy = p.G[jy][iy];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            S[d][0] = fma(xs[iy][d][0][lane], My, S[d][0]);
+            S[d][1] = fma(xs[iy][d][1][lane], Dyy, S[d][1]);
+            S[d][2] = fma(xs[iy][d][2][lane], Hy, S[d][2]);
+            S[d][3] = fma(xs[iy][d][3][lane], Gy, S[d][3]);
         }
     }
     double r[2] = {0.0, 0.0};
