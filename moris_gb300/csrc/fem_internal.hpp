@@ -187,8 +187,8 @@ inline bool lattice_set(const fem_gpu_ctx* c, int set) { return c->sets[set].lat
 // however few the cells; on small models one launch of the element loop is faster.
 // Measured calls, element loop / lattice, in us.  Assembly of bricks: linear 7^3 42 /
 // 54, 10^3 54 / 51, 13^3 65 / 53; quadratic 7^3 55 / 73, 10^3 80 / 75, 13^3 129 / 100.
-// Products of bricks: linear 6^3 24 / 28, 10^3 28 / 28, 16^3 52 / 33; quadratic 6^3 24
-// / 37, 10^3 31 / 38, 16^3 64 / 44.  Cells of any shape: linear 5^3 54 / 43, products
+// Products of bricks: linear 6^3 24 / 28, 10^3 28 / 27, 16^3 53 / 27; quadratic 6^3 25
+// / 37, 10^3 31 / 38, 12^3 40 / 38, 16^3 63 / 38.  Cells of any shape: linear 5^3 54 / 43, products
 // 30 / 23; quadratic 7^3 68 / 77, 10^3 120 / 99, products 8^3 42 / 36.
 inline bool lattice_pays(const fem_gpu_ctx* c, int set, bool product) {
     if (!lattice_set(c, set)) return false;

@@ -23,7 +23,7 @@
 // Measured on GB300 against the element loop (whole calls, residual included):
 // 64^3 quadratic 7.75 -> 2.23 ms, 15 x 13 x 11 quadratic 120 -> 86 us, 96^3
 // density set with linear splines 13.4 -> 3.56 ms, matrix-free product of 48 x
-// 47 x 45 quadratic cells 969 -> 206 us.  The stencil and projection kernels
+// 47 x 45 quadratic cells 969 -> 80 us (lattice_product).  The stencil and projection kernels
 // keep the FP64 pipe 72-77 % busy, lattice_density 55 % (register-bound
 // occupancy).  Small models keep the element loop (lattice_pays).
 //
@@ -75,6 +75,7 @@ struct LatArgs {
     double coef[27][9];    // constant E: see lattice_const
     double xq[3], wq[27];  // density: 1-D points, weights (x fastest) times mu
     double beta, ld, lo;   // density exponent, (lam + mu) / mu, lam / mu
+    double wmu;            // lattice_product: mu times a scale over 8
 };
 
 // One warp's share of a node's row: the blocks of neighbour offsets
@@ -261,6 +262,108 @@ __global__ void __launch_bounds__(kStencilThreads) lattice_const(LatArgs p) {
     else const_blocks<OUT, 1>(p, node, red[2]);
     __syncthreads();
     store_residual(p, node, red);
+}
+
+// Residual alone, constant modulus per element: r += sum_e K_e u without a block.  On a
+// brick a trilinear field is a sum of the monomials x^m, m in {0, 1}^3, whose
+// gradients are orthogonal: with h_m = sum over the corners of s^m u (s = -+1) the
+// strains are single coefficients, the integral over the cell is V / 3^|n| for every
+// monomial x^n, and the corner forces come back by the transposed sums.  258 FP64
+// operations per cell and 24 coalesced atomics, where the stencil took 750 operations
+// per node: product of 48 x 47 x 45 quadratic cells 210 -> 80 us
+// (kernel 58, FP64 pipe 69 %).
+__global__ void __launch_bounds__(128) lattice_product(LatArgs p) {
+    const unsigned cells = (unsigned)p.ne[0] * p.ne[1] * p.ne[2], e = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = e < cells;
+    const unsigned ec = live ? e : 0, yz = ec / p.ne[0];
+    const int ex = (int)(ec - yz * p.ne[0]), ey = (int)(yz % p.ne[1]), ez = (int)(yz / p.ne[1]);
+    const int64_t nodes = (int64_t)p.nn[0] * p.nn[1] * p.nn[2];
+    const double J[3] = {__ldg(p.jac + ex), __ldg(p.jac + p.ne[0] + ey), __ldg(p.jac + p.ne[0] + p.ne[1] + ez)};
+    const double* ij = p.jac + p.ne[0] + p.ne[1] + p.ne[2];
+    const double k[3] = {__ldg(ij + ex), __ldg(ij + p.ne[0] + ey), __ldg(ij + p.ne[0] + p.ne[1] + ez)};
+    // V / 64 = detJ / 8 (the 1/8 of the field's and of the test function's monomials)
+    const double w = __ldg(p.E + ec) * p.wmu * (J[0] * J[1] * J[2]);
+    cudaGridDependencySynchronize();  // u, and the sums
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int64_t n0 = ((int64_t)ez * p.nn[1] + ey) * p.nn[0] + ex;
+    const int64_t sy = p.nn[0], sz = (int64_t)p.nn[0] * p.nn[1];
+    double h[3][8];  // component, monomial (bit d: x_d)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double* u = p.u + c * nodes + n0;
+#pragma unroll
+        for (int m = 0; m < 8; ++m) h[c][m] = u[(m & 1) + (m >> 1 & 1) * sy + (m >> 2) * sz];
+#pragma unroll
+        for (int b = 1; b < 8; b <<= 1)
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                if (!(m & b)) {
+                    const double lo = h[c][m], up = h[c][m | b];
+                    h[c][m] = lo + up;
+                    h[c][m | b] = up - lo;
+                }
+    }
+    // T[i][c][n]: stress i c over mu at the monomials n of the other two axes than i
+    // (index without bit i); gradients g(i, c, n) = k_i h[c][n + e_i]
+    double T[3][3][8];
+    {
+        double g[3][3][8];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int n = 0; n < 8; ++n)
+                    if (!(n & 1 << i)) g[i][c][n] = k[i] * h[c][n | 1 << i];
+        const double t0 = p.lo * (g[0][0][0] + g[1][1][0] + g[2][2][0]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int a = (i + 1) % 3, b = (i + 2) % 3, xi = 1 << i, xa = 1 << a, xb = 1 << b;
+            T[i][i][0] = fma(2.0, g[i][i][0], t0);
+            T[i][i][xa | xb] = (2.0 + p.lo) * g[i][i][xa | xb];
+            // monomial x_i: the strains along the other two axes
+            const double t = p.lo * (g[a][a][xi] + g[b][b][xi]);
+            T[a][a][xi] = fma(2.0, g[a][a][xi], t);
+            T[b][b][xi] = fma(2.0, g[b][b][xi], t);
+            // shear of the axes a and b
+            T[a][b][0] = T[b][a][0] = g[a][b][0] + g[b][a][0];
+            T[a][b][xi] = T[b][a][xi] = g[a][b][xi] + g[b][a][xi];
+            T[a][b][xb] = g[a][b][xb];
+            T[b][a][xa] = g[b][a][xa];
+            T[a][b][xb | xi] = g[a][b][xb | xi];
+            T[b][a][xa | xi] = g[b][a][xa | xi];
+        }
+    }
+    const double w3 = w * (1.0 / 3.0), w9 = w * (1.0 / 9.0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double r[8];
+        r[0] = 0.0;
+#pragma unroll
+        for (int m = 1; m < 8; ++m) {
+            double v = 0.0;
+#pragma unroll
+            for (int i = 2; i >= 0; --i)
+                if (m & 1 << i) v = fma(k[i], T[i][c][m & ~(1 << i)], v);
+            const int bits = (m & 1) + (m >> 1 & 1) + (m >> 2);
+            r[m] = (bits == 1 ? w : bits == 2 ? w3 : w9) * v;
+        }
+        // r(s) = sum_m s^m r_m
+#pragma unroll
+        for (int b = 1; b < 8; b <<= 1)
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                if (!(m & b)) {
+                    const double a = r[m], d = r[m | b];
+                    r[m] = a - d;
+                    r[m | b] = a + d;
+                }
+        if (live) {
+            double* q = p.r + c * nodes + n0;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) atomicAdd(q + (m & 1) + (m >> 1 & 1) * sy + (m >> 2) * sz, r[m]);
+        }
+    }
 }
 
 // 1-D factors of the density path.  Along an axis a pair of nodes (offset d)
@@ -1174,7 +1277,10 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     // the kernels of a call overlap their beginnings with the end of the one before
     // (4 to 6 launches of 4 to 40 us on small lattices)
     bool overlap = false;
-    // cells of any shape add to what they find
+    // a product of bricks with constant moduli, and cells of any shape, add to what they
+    // find
+    const bool product = L.brick && !a.rho && !vals;
+    if (product && !a.acc_r) e = cudaMemsetAsync(a.r, 0, 3 * nodes * sizeof(double), st);
     if (!L.brick) {
         if (quad && vals) e = cudaMemsetAsync(a.S, 0, L.S.bytes, st);
         if (!quad && vals && !acc_v) e = cudaMemsetAsync(vals, 0, c->nnz * sizeof(double), st);
@@ -1220,7 +1326,7 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     const int out = !vals ? OUT_NONE : quad ? OUT_STENCIL : OUT_CSR;
     using Fn = void (*)(LatArgs);
     static const Fn density[3] = {lattice_density<0>, lattice_density<1>, lattice_density<2>};
-    static const Fn constant[3] = {lattice_const<0>, lattice_const<1>, lattice_const<2>};
+    static const Fn constant[3] = {nullptr, lattice_const<1>, lattice_const<2>};
     if (a.rho) {
         const unsigned g = (unsigned)std::min<int64_t>((c->num_cells + 127) / 128, (int64_t)sm_count() * 64);
         if (N == 2) lattice_moments<2><<<g, 128, 0, st>>>(a);
@@ -1228,6 +1334,12 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         density[out]<<<ctas, kStencilThreads, 0, st>>>(a);
         c->launches += 2;
         overlap = true;
+    } else if (product && e == cudaSuccess) {
+        a.wmu = mu * scale / 8.0;
+        const unsigned g = (unsigned)((c->num_cells + 127) / 128);
+        if (want_u) e = launch_kernel(lattice_product, g, 128, 0, st, overlap, a);
+        c->launches += want_u;
+        overlap |= want_u;
     } else if (L.brick && e == cudaSuccess) {
         e = launch_kernel(constant[out], ctas, kStencilThreads, 0, st, overlap, a);
         c->launches++;
