@@ -8,28 +8,28 @@
 //
 //   lattice_const / lattice_density   the 27-point block stencil of sum_e K_e,
 //       one thread per node: every 3 x 3 block is a sum over the elements that
-//       share the node pair, gathered in a fixed order (no atomics, no zero
-//       fill, one store per value), and the nodal residual K u on the way;
+//       share the node pair, gathered in a fixed order (no atomics on values, no
+//       zero fill, one store per value), and the nodal residual K u on the way;
 //   lattice_project   T^T S T for quadratic splines, axis by axis: 3 -> 5 taps
 //       per axis with 5 additions (the weights are powers of two, folded into
-//       the modulus), written row by row into the CSR.
+//       the modulus), written row by row into the CSR;
+//   lattice_rows      the stencil as CSR rows for linear splines;
+//   lattice_product   the residual alone, without a stencil.
 //
 // The element loop (fem_bulk_cta.cuh) spends 6,561 atomic updates on each
 // quadratic element and is bound by shared-memory latency and the L2's atomic
 // rate; here a CSR value costs about 2.5 FP64 additions and one store.  The
-// FP64 pipe (2 lanes per SM and clock on GB300) binds: 2,340 additions per
-// basis for the projection, 750 operations per node for the stencil.
+// FP64 pipe (2 lanes per SM and clock on GB300) binds, 68-77 % busy: 2,340 additions
+// per basis for the projection, 750 operations per node for the stencil.
 //
 // Measured on GB300 against the element loop (whole calls, residual included):
-// 64^3 quadratic 7.75 -> 2.23 ms, 15 x 13 x 11 quadratic 120 -> 86 us, 96^3
-// density set with linear splines 13.4 -> 3.56 ms, matrix-free product of 48 x
-// 47 x 45 quadratic cells 969 -> 80 us (lattice_product).  The stencil and projection kernels
-// keep the FP64 pipe 72-77 % busy, lattice_density 55 % (register-bound
-// occupancy).  Small models keep the element loop (lattice_pays).
+// 64^3 quadratic 7.75 -> 2.25 ms, 15 x 13 x 11 quadratic 120 -> 82 us, 96^3 density set
+// with linear splines 13.4 -> 2.50 ms, matrix-free product of 48 x 47 x 45 quadratic
+// cells 969 -> 80 us.  Small models keep the element loop (lattice_pays).
 //
 // Cells of any shape on the same lattice of nodes (FEM_GPU_SHAPE_GENERAL): the cells
 // add their matrices to the block stencil (fem_hex.cuh), or to the CSR for linear
-// splines, and the projection is the same.  26 x 23 x 21 quadratic 699 -> 545 us (hex
+// splines, and the projection is the same.  26 x 23 x 21 quadratic 699 -> 534 us (hex
 // 371, projection 128); 26^3 linear 467 -> 294 us, matrix-free products 401 -> 206
 // (linear) and 622 -> 264 us.
 //
@@ -52,7 +52,7 @@ namespace fem {
 namespace {
 
 // a stencil CTA: 32 consecutive nodes, one warp per z offset
-constexpr int kStencilNodes = 32, kStencilThreads = 3 * kStencilNodes;
+constexpr int kStencilNodes = 32, kStencilThreads = 3 * kStencilNodes, kDensityThreads = 2 * kStencilNodes;
 // bases of a projection tile
 constexpr int kPX = 5, kPY = 3;
 
@@ -85,9 +85,9 @@ struct NodeOut {
     const LatArgs& p;
     int x, y, z;
     int64_t node, nodes;
+    double r[3] = {0.0, 0.0, 0.0};
     int32_t row[3];
     int cx, cy, cz, lx, ly, lz;  // CSR box of the node's row
-    double r[3] = {0.0, 0.0, 0.0};
     bool live, bad = false;
 
     __device__ NodeOut(const LatArgs& a, int64_t n) : p(a), node(n) {
@@ -153,6 +153,40 @@ struct NodeOut {
                     *v = p.acc_v ? *v + K[f * 3 + g] : K[f * 3 + g];
                 }
         }
+    }
+    // the block K of neighbour (dx, dy, DZ) at the neighbour's row: K^T, and its share of
+    // the neighbour's residual; ui: displacements of the node
+    __device__ __forceinline__ void transposed(int dx, int dy, const double ui[3], const double K[9]) {
+        const int k = 26 - ((dx + 1) + 3 * (dy + 1) + 9 * (DZ + 1));
+        const int64_t plane = (int64_t)p.nn[2] * p.nn[1] * p.pitch;
+        double* s = p.S + (int64_t)k * 9 * plane + ((int64_t)z * p.nn[1] + y) * p.pitch + x;
+        if constexpr (OUT == OUT_STENCIL) {
+            // no node writes the blocks that leave the lattice on the other side
+            const bool out = x - dx < 0 || x - dx >= p.nn[0] || y - dy < 0 || y - dy >= p.nn[1] || z - DZ < 0;
+            if (live && out) {
+#pragma unroll
+                for (int c = 0; c < 9; ++c) s[c * plane] = 0.0;
+            }
+        }
+        if (!inside(dx, dy)) return;
+        const int64_t j = node + dx + (int64_t)p.nn[0] * (dy + (int64_t)p.nn[1] * DZ);
+        if constexpr (OUT == OUT_STENCIL) {
+            s += ((int64_t)DZ * p.nn[1] + dy) * p.pitch + dx;
+#pragma unroll
+            for (int f = 0; f < 3; ++f)
+#pragma unroll
+                for (int g = 0; g < 3; ++g) s[(g * 3 + f) * plane] = K[f * 3 + g];
+        }
+        if (p.u) {
+#pragma unroll
+            for (int g = 0; g < 3; ++g)
+                atomicAdd(p.r + g * nodes + j, fma(K[6 + g], ui[2], fma(K[3 + g], ui[1], K[g] * ui[0])));
+        }
+    }
+    __device__ void finish_atomic() {
+        if (bad && live) atomicOr(p.status, 1);
+        if (p.u && live)
+            for (int f = 0; f < 3; ++f) atomicAdd(p.r + f * nodes + node, r[f]);
     }
     __device__ void finish(double red[kStencilNodes][3]) {
         if (bad && live) atomicOr(p.status, 1);
@@ -539,17 +573,28 @@ __global__ void __launch_bounds__(128) lattice_moments(LatArgs p) {
     }
 }
 
+// The operator is symmetric: a node forms the blocks of itself and of the 13
+// neighbours after it, and writes each to its own row and, transposed, to the
+// neighbour's.  The share of the residual that belongs to the neighbour is added with
+// coalesced atomics.  Two warps per 32 nodes, the plane of the node (5 blocks) and the
+// next one (9): 595 FP64 operations and 324 loads per node, where all 27 blocks took
+// 873 and 576.
 template <int OUT, int DZ>
-__device__ __forceinline__ void density_blocks(const LatArgs& p, int64_t node, double red[kStencilNodes][3]) {
+__device__ __forceinline__ void density_blocks(const LatArgs& p, int64_t node) {
     NodeOut<OUT, DZ> out(p, node);
     const int64_t ey = p.ne[0] + 2, ez = ey * (p.ne[1] + 2), qs = ez * (p.ne[2] + 2);
     const double* q = p.Q + out.z * ez + out.y * ey + out.x;
+    double ui[3] = {0.0, 0.0, 0.0};
+    if (p.u && out.live)
 #pragma unroll
-    for (int dy = -1; dy <= 1; ++dy) {
+        for (int g = 0; g < 3; ++g) ui[g] = p.u[g * out.nodes + node];
+#pragma unroll
+    for (int dy = DZ ? -1 : 0; dy <= 1; ++dy) {
         double un[3][3];
         out.neighbours(dy, un);
 #pragma unroll
         for (int dx = -1; dx <= 1; ++dx) {
+            if (DZ == 0 && dy == 0 && dx < 0) continue;
             const double a0 = gather<0, 1, 1, DZ>(q, qs, ey, ez, kXX, dx, dy),
                          a1 = gather<1, 0, 1, DZ>(q, qs, ey, ez, kYY, dx, dy),
                          a2 = gather<1, 1, 0, DZ>(q, qs, ey, ez, kZZ, dx, dy), tr = a0 + a1 + a2;
@@ -564,22 +609,61 @@ __device__ __forceinline__ void density_blocks(const LatArgs& p, int64_t node, d
                                  fma(p.lo, yx, xy), fma(p.ld, a1, tr), fma(p.lo, yz, zy),
                                  fma(p.lo, zx, xz), fma(p.lo, zy, yz), fma(p.ld, a2, tr)};
             out.block(dx, dy, un, K);
+            if (DZ || dy || dx) out.transposed(dx, dy, ui, K);
         }
     }
-    out.finish(red);
+    out.finish_atomic();
 }
 
 template <int OUT>
-__global__ void __launch_bounds__(kStencilThreads, 4) lattice_density(LatArgs p) {
-    __shared__ double red[3][kStencilNodes][3];
-    const int64_t node = (int64_t)blockIdx.x * kStencilNodes + threadIdx.x % kStencilNodes;
-    const int w = threadIdx.x / kStencilNodes;
+__global__ void __launch_bounds__(kDensityThreads, 6) lattice_density(LatArgs p) {
     cudaTriggerProgrammaticLaunchCompletion();
-    if (w == 0) density_blocks<OUT, -1>(p, node, red[0]);
-    else if (w == 1) density_blocks<OUT, 0>(p, node, red[1]);
-    else density_blocks<OUT, 1>(p, node, red[2]);
+    const int64_t node = (int64_t)blockIdx.x * kStencilNodes + threadIdx.x % kStencilNodes;
+    if (threadIdx.x < kStencilNodes) density_blocks<OUT, 0>(p, node);
+    else density_blocks<OUT, 1>(p, node);
+}
+
+// Linear splines: the stencil as CSR values, a CTA per 32 consecutive nodes and row
+// component, whose rows are one range of the CSR.  Bound by HBM (the stencil in, the
+// values out).  Written by the stencil kernels themselves, a lane per row, every value
+// is a sector of its own: a 96^3 density set took 3.39 ms so, and 2.50 with this kernel
+// (5.5 TB/s).
+// The constant-modulus kernel has less to hide the second pass behind and gains from
+// kRowsNodes on: 20^3 cells 52 us direct, 64 with rows, 32^3 114 and 128, 48^3 372 and
+// 337.
+constexpr int64_t kRowsNodes = 65536;
+__global__ void __launch_bounds__(256) lattice_rows(int n0, int n1, int n2, int64_t pitch, const double* S,
+                                                    const int32_t* __restrict__ rowptr, double* vals, int acc) {
+    __shared__ double rows[kStencilNodes * 81];
+    const int lane = threadIdx.x & 31, f = blockIdx.y;
+    const int nodes = n0 * n1 * n2, node0 = blockIdx.x * kStencilNodes, node = node0 + lane;
+    const bool live = node < nodes;
+    const int i = live ? node : 0, yz = i / n0, x = i - yz * n0, z = yz / n1, y = yz - z * n1;
+    const int lx = x > 0 ? -1 : 0, ly = y > 0 ? -1 : 0, lz = z > 0 ? -1 : 0;
+    const int cx = (x + 1 < n0 ? 2 : 1) - lx, cy = (y + 1 < n1 ? 2 : 1) - ly, ul = cx * cy * ((z + 1 < n2 ? 2 : 1) - lz);
+    const int64_t first = __ldg(rowptr + (int64_t)f * nodes + node0);
+    const int64_t last = __ldg(rowptr + (int64_t)f * nodes + min(node0 + kStencilNodes, nodes));
+    double* row = rows + (__ldg(rowptr + (int64_t)f * nodes + i) - first);
+    const int64_t plane = (int64_t)n2 * n1 * pitch;
+    const double* s = S + (int64_t)f * 3 * plane + (int64_t)yz * pitch + x;
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int w = threadIdx.x >> 5, at0 = -(lz * cy + ly) * cx - lx;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const int k = t * 8 + w, dx = k % 3 - 1, dy = k / 3 % 3 - 1, dz = k / 9 - 1;
+        if (k < 27 && live && (unsigned)(x + dx) < (unsigned)n0 && (unsigned)(y + dy) < (unsigned)n1 &&
+            (unsigned)(z + dz) < (unsigned)n2) {
+            const double* v = s + k * 9 * plane;
+            double* q = row + (dz * cy + dy) * cx + dx + at0;
+#pragma unroll
+            for (int g = 0; g < 3; ++g) q[g * ul] = v[g * plane];
+        }
+    }
     __syncthreads();
-    store_residual(p, node, red);
+    double* v = vals + first;
+    const int n = (int)(last - first);
+    for (int t = threadIdx.x; t < n; t += 256) v[t] = acc ? v[t] + rows[t] : rows[t];
 }
 
 // A = T^T S T for quadratic splines (basis b covers the nodes b-1 and b along
@@ -1052,13 +1136,13 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
     auto* K = new Lattice(L);
     c->lattice = K;
     if (e == cudaSuccess) e = upload(K->jac, jac, st);
-    // workspaces (quadratic splines: 243 doubles and six nodal values per node,
-    // 0.22 of the CSR values; density sets: 63 doubles per cell, 0.26 of them for
-    // linear splines); a device that cannot hold them keeps the element loop
+    // workspaces (243 doubles per node, 0.22 of the CSR values for quadratic and as
+    // much as them for linear splines; quadratic: six nodal values per node; density
+    // sets: 63 doubles per cell); a device that cannot hold them keeps the element loop
     bool rho = false;
     for (const SetData& s : c->sets) rho |= s.lattice && !s.node_rho.empty();
     const bool quad = c->dim == 3 && K->p == 2;
-    const size_t want[3] = {quad ? (size_t)243 * L.nn[2] * L.nn[1] * L.pitch : 0,
+    const size_t want[3] = {quad || (L.brick && c->dim == 3) ? (size_t)243 * L.nn[2] * L.nn[1] * L.pitch : 0,
                             quad ? (size_t)6 * c->num_nodes : 0,
                             rho ? (size_t)kQN * (L.ne[0] + 2) * (L.ne[1] + 2) * (L.ne[2] + 2) : 0};
     DeviceBuf* const buf[3] = {&K->S, &K->vec, &K->Q};
@@ -1074,7 +1158,7 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
         }
     }
     if (rho && e == cudaSuccess) e = cudaMemsetAsync(K->Q.p, 0, K->Q.bytes, st);
-    if ((rho || quad) && e == cudaSuccess) e = cudaEventCreateWithFlags(&K->done, cudaEventDisableTiming);
+    if (K->S.p && e == cudaSuccess) e = cudaEventCreateWithFlags(&K->done, cudaEventDisableTiming);
     if (K->done && e == cudaSuccess) e = cudaEventRecord(K->done, st);
     K->last = st;
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1209,10 +1293,12 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     a.pitch = L.pitch;
     a.E = (const double*)(s.d_latE.p ? s.d_latE.p : s.d_E.p);
     a.jac = (const double*)L.jac.p;
+    const int32_t* rowptr = (const int32_t*)c->d_rowptr.p;
     a.rho = s.node_rho.empty() ? nullptr : (const double*)s.d_latrho.p;
-    a.rowptr = (const int32_t*)c->d_rowptr.p;
     a.status = (int*)c->d_status.p;
     a.vals = vals;
+    a.rowptr = rowptr;
+    a.acc_v = acc_v;
     a.S = (double*)work.S;
     a.Q = (double*)work.Q;
     double* un = (double*)work.vec;
@@ -1220,7 +1306,6 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     const bool want_u = u && rhs;
     a.u = want_u ? (quad ? un : u) : nullptr;
     a.r = rhs ? (quad ? rn : rhs) : nullptr;
-    a.acc_v = acc_v;
     a.acc_r = quad ? 0 : acc_r;
     // material and rule: T^T S T with T = P / 8 is P^T (S / 64) P (exact powers of two)
     const double nu = s.bulk.poisson_ratio, scale = quad ? 1.0 / 64.0 : 1.0;
@@ -1280,7 +1365,7 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     // a product of bricks with constant moduli, and cells of any shape, add to what they
     // find
     const bool product = L.brick && !a.rho && !vals;
-    if (product && !a.acc_r) e = cudaMemsetAsync(a.r, 0, 3 * nodes * sizeof(double), st);
+    if ((product || (a.rho && a.r)) && !a.acc_r) e = cudaMemsetAsync(a.r, 0, 3 * nodes * sizeof(double), st);
     if (!L.brick) {
         if (quad && vals) e = cudaMemsetAsync(a.S, 0, L.S.bytes, st);
         if (!quad && vals && !acc_v) e = cudaMemsetAsync(vals, 0, c->nnz * sizeof(double), st);
@@ -1309,7 +1394,7 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         h.r = a.r;
         h.S = a.S;
         h.vals = vals;
-        h.rowptr = a.rowptr;
+        h.rowptr = rowptr;
         h.status = a.status;
         const unsigned g = (unsigned)((c->num_cells + kHexWarps - 1) / kHexWarps);
         using Fn = void (*)(HexArgs);
@@ -1323,15 +1408,15 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         }
     }
     const unsigned ctas = (unsigned)((nodes + kStencilNodes - 1) / kStencilNodes);
-    const int out = !vals ? OUT_NONE : quad ? OUT_STENCIL : OUT_CSR;
+    const int out = vals ? OUT_STENCIL : OUT_NONE;
+    const bool direct = !quad && !a.rho && nodes < kRowsNodes;
     using Fn = void (*)(LatArgs);
-    static const Fn density[3] = {lattice_density<0>, lattice_density<1>, lattice_density<2>};
-    static const Fn constant[3] = {nullptr, lattice_const<1>, lattice_const<2>};
+    static const Fn density[2] = {lattice_density<OUT_NONE>, lattice_density<OUT_STENCIL>};
     if (a.rho) {
         const unsigned g = (unsigned)std::min<int64_t>((c->num_cells + 127) / 128, (int64_t)sm_count() * 64);
         if (N == 2) lattice_moments<2><<<g, 128, 0, st>>>(a);
         else lattice_moments<3><<<g, 128, 0, st>>>(a);
-        density[out]<<<ctas, kStencilThreads, 0, st>>>(a);
+        density[out]<<<ctas, kDensityThreads, 0, st>>>(a);
         c->launches += 2;
         overlap = true;
     } else if (product && e == cudaSuccess) {
@@ -1341,13 +1426,18 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         c->launches += want_u;
         overlap |= want_u;
     } else if (L.brick && e == cudaSuccess) {
-        e = launch_kernel(constant[out], ctas, kStencilThreads, 0, st, overlap, a);
+        e = launch_kernel(direct ? lattice_const<OUT_CSR> : lattice_const<OUT_STENCIL>, ctas, kStencilThreads, 0, st, overlap, a);
         c->launches++;
         overlap = true;
     }
     if (quad && rhs && e == cudaSuccess) {
         e = launch_kernel(lattice_restrict, (unsigned)std::min<int64_t>((3 * (c->num_used) + 255) / 256, grid3), 256, 0,
                           st, overlap, L.nn[0], L.nn[1], L.nn[2], rn, 8.0, acc_r, rhs);
+        c->launches++;
+    }
+    if (!quad && L.brick && vals && !direct && e == cudaSuccess) {
+        e = launch_kernel(lattice_rows, dim3(ctas, 3), 256, 0, st, overlap, L.nn[0], L.nn[1], L.nn[2], L.pitch,
+                          (const double*)a.S, rowptr, vals, (int)acc_v);
         c->launches++;
     }
     if (quad && vals && e == cudaSuccess) {
@@ -1361,7 +1451,7 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
         q.pitch = L.pitch;
         q.S = a.S;
         q.vals = vals;
-        q.rowptr = a.rowptr;
+        q.rowptr = rowptr;
         q.acc = acc_v;
         q.status = a.status;
         // z ranges: every range repeats one node plane, and the CTAs should fill

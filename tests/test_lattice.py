@@ -98,6 +98,22 @@ def test_lattice_apply_and_several_sets(torch, ne, p):
     assert rel_err(out[0][2], out[0][1]) <= RTOL and rel_err(out[0][3], 2 * out[0][2]) <= RTOL
 
 
+def test_rows_of_a_large_linear_lattice(torch):
+    """From 65,536 nodes on, constant moduli go through the stencil as well (density
+    sets always do): against the element loop, and summed onto values that are there."""
+    prod, _, _ = problem(3, (41, 40, 38), 1, mg.SHAPE_RECTANGULAR, mg.RULE_HEX_2x2x2)
+    prod.finalize()
+    u = torch.tensor(uniform01(31, prod.num_adofs) - 0.5, device="cuda")
+    vals, rhs = _assemble(torch, prod, u)
+    v2, r2 = _assemble(torch, prod, u, mg.ACCUMULATE, vals.clone(), rhs.clone())
+    prod.set_variant(0, 2)
+    vg, rg = _assemble(torch, prod, u)
+    rp, _ = prod.graph()
+    assert csr_row_rel_err(rp, vals.cpu().numpy(), vg.cpu().numpy()) <= RTOL
+    assert csr_row_rel_err(rp, v2.cpu().numpy(), 2 * vg.cpu().numpy()) <= RTOL
+    assert rel_err(rhs.cpu().numpy(), rg.cpu().numpy()) <= RTOL and rel_err(r2.cpu().numpy(), 2 * rg.cpu().numpy()) <= RTOL
+
+
 def test_non_finite_blocks_are_reported(torch):
     """A modulus whose products overflow: both paths return the status."""
     for p in (1, 2):
