@@ -9,13 +9,16 @@
 //   k4  (one thread) advance the iteration counter
 // Scalars live in a device ring indexed by the iteration counter, so the
 // launches carry no host-side values and a chunk of iterations is captured
-// once into a CUDA graph and replayed.  Small systems, whose iteration is
-// shorter than its launches, take two per iteration (k_pair_*).  The host reads
-// the done flag once per chunk; iterations after convergence return immediately
-// on the device.
+// once into a CUDA graph and replayed.  The host reads the done flag once per
+// chunk; iterations after convergence return immediately on the device.  Small
+// systems, whose iteration is shorter than its launches, are solved by one cluster
+// of CTAs (k_cluster_cg) or take two launches per iteration (k_pair_*).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <mutex>
 #include <string>
@@ -33,6 +36,7 @@ struct CgState {
     int done;        // 1 converged, 2 breakdown
     int converged_at;
     int stopped_at;  // k_pair_*: iteration whose test ended the solve
+    int wide;        // a row longer than the limit given to k_diag_inv
     double thresh2;  // (rtol * ||b||)^2
     double bn2;
     // ring of per-iteration scalars: [slot][0]=pq, [1]=rz, [2]=rr
@@ -43,9 +47,10 @@ struct CgState {
 constexpr int kThreads = 256;
 
 __global__ void k_diag_inv(int64_t n, const int32_t* rp, const int32_t* ci, const double* v, double* dinv,
-                           int jacobi) {
+                           int jacobi, int limit, CgState* st) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (rp[i + 1] - rp[i] > limit) st->wide = 1;
     double d = 1.0;
     if (jacobi) {
         int lo = rp[i], hi = rp[i + 1] - 1;
@@ -273,6 +278,168 @@ __global__ void k_pair_end(CgState* st, int chunk, int max_iter) {
     }
 }
 
+// One cluster of 16 CTAs runs the iterations by itself: a thread per row with its
+// entries of x, r, p in registers, the rows of the matrix in shared memory (entry k of
+// all rows together, columns as 16 bits), sums over the cluster in the order of the
+// ranks.  z is exchanged through distributed shared memory with the second sum, and
+// every CTA forms p = z + beta p itself in the blocks of 32 entries that its columns
+// name.  An iteration is two cluster barriers, five of the CTA and W FMAs per row on 16
+// SMs: no launch and no trip to the L2.  Every CTA takes the same decisions from the
+// same sums, so all leave the loop together.
+// Microseconds per iteration, two launches -> here: plane systems of 578 rows 10.7 ->
+// 6.2, 2,178 rows 8.8 -> 6.0, 5,000 rows 8.4 -> 7.0, 8,450 rows 9.4 -> 9.3 to 9.9 (not
+// used); solids of 1,029 rows 13.7 -> 10.0, 3,000 rows 13.4 -> 10.3.
+constexpr int kClusterCtas = 16, kClusterRows = 320;  // rows per CTA at most
+constexpr int kClusterChunk = 2048;                   // iterations per launch
+struct ClusterShape {
+    int rows = 0, width = 0;  // rows per CTA (a multiple of 32), entries per row
+    size_t smem = 0;
+};
+ClusterShape cluster_shape(int64_t n, int width) {
+    ClusterShape c;
+    const int64_t rows = (n + kClusterCtas * 32 - 1) / (kClusterCtas * 32) * 32, blocks = (n + 31) / 32;
+    if (rows > kClusterRows) return c;
+    c.rows = (int)rows;
+    c.width = width;
+    c.smem = (blocks * 32 + 3 * rows + 3 * kClusterCtas + 4 + width * rows) * sizeof(double) +
+             width * rows * sizeof(uint16_t) + ((blocks + 31) / 32 + 1) * sizeof(unsigned) + blocks * sizeof(uint16_t);
+    return c;
+}
+
+__global__ void __launch_bounds__(kClusterRows) k_cluster_cg(int n, int W, const int32_t* __restrict__ rp,
+                                                     const int32_t* __restrict__ ci, const double* __restrict__ v,
+                                                     double* x, double* r, double* p, const double* dinv, CgState* st,
+                                                     int max_iter) {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char raw[];
+    const cg::cluster_group cluster = cg::this_cluster();
+    const int R = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = R >> 5;
+    const int rank = (int)cluster.block_rank(), row = rank * R + tid, NB = (n + 31) / 32;
+    const bool live = row < n;
+    double* P = (double*)raw;             // p, where this CTA reads it
+    double* zown = P + NB * 32;           // z of this CTA's rows
+    double* red = zown + R;               // [2][R]
+    double* slots = red + 2 * R;          // [3][rank]
+    double* bc = slots + 3 * kClusterCtas;
+    double* av = bc + 4;                  // [W][R]
+    uint16_t* ac = (uint16_t*)(av + (size_t)W * R);
+    unsigned* bits = (unsigned*)(ac + (size_t)W * R);
+    unsigned* count = bits + (NB + 31) / 32;
+    uint16_t* list = (uint16_t*)(count + 1);
+    if (st->done || st->wide) return;  // the same for all
+    for (int k = tid; k <= (NB + 31) / 32; k += R) bits[k] = 0;
+    __syncthreads();
+    const int j0 = live ? rp[row] : 0, len = live ? rp[row + 1] - j0 : 0;
+    for (int k = 0; k < W; ++k) {
+        const int c = k < len ? ci[j0 + k] : live ? row : 0;
+        av[k * R + tid] = k < len ? v[j0 + k] : 0.0;
+        ac[k * R + tid] = (uint16_t)c;
+        if (k < len && c / R != rank) atomicOr(bits + (c >> 10), 1u << (c >> 5 & 31));
+    }
+    __syncthreads();
+    for (int k = tid; k < NB; k += R)
+        if (bits[k >> 5] >> (k & 31) & 1) list[atomicAdd(count, 1u)] = (uint16_t)k;
+    __syncthreads();
+    const int blocks = (int)*count;
+    for (int b = warp; b < blocks; b += warps) {
+        const int at = list[b] * 32 + lane;
+        P[at] = at < n ? p[at] : 0.0;
+    }
+    double xi = 0.0, ri = 0.0, pi = 0.0, di = 0.0, zi = 0.0;
+    if (live) {
+        xi = x[row];
+        ri = r[row];
+        pi = p[row];
+        di = dinv[row];
+        P[row] = pi;
+    }
+    int it = st->it, state = 0;
+    double rz = st->ring[it & 3][1], rr = 0.0;
+    const double thresh2 = st->thresh2;
+    // sum of a[0..R) by one warp, to slot set k of every CTA
+    const auto share = [&](const double* a, int k) {
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        int m = lane;
+        for (; m + 96 < R; m += 128) {
+            s[0] += a[m];
+            s[1] += a[m + 32];
+            s[2] += a[m + 64];
+            s[3] += a[m + 96];
+        }
+        for (; m < R; m += 32) s[0] += a[m];
+        const double t = fem::warp_total((s[0] + s[1]) + (s[2] + s[3]));
+        if (lane < kClusterCtas) cluster.map_shared_rank(slots, lane)[k * kClusterCtas + rank] = t;
+    };
+    // all of p is read, and all CTAs run, before anything is written
+    cluster.sync();
+    for (int k = 0; k < kClusterChunk && !state; ++k) {
+        double q = 0.0;
+#pragma unroll 6
+        for (int m = 0; m < W; ++m) q = fma(av[m * R + tid], P[ac[m * R + tid]], q);
+        red[tid] = live ? q * pi : 0.0;
+        __syncthreads();
+        if (warp == 0) share(red, 0);
+        cluster.sync();
+        if (warp == 0) {
+            double t = slots[lane & 15];
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) {
+                bc[0] = t;
+                bc[1] = rz / t;
+            }
+        }
+        __syncthreads();
+        const double pq = bc[0], alpha = bc[1];
+        xi = fma(alpha, pi, xi);
+        ri = fma(-alpha, q, ri);
+        zi = di * ri;
+        zown[tid] = zi;
+        red[tid] = live ? ri * zi : 0.0;
+        red[R + tid] = live ? ri * ri : 0.0;
+        __syncthreads();
+        if (warp == 0) share(red, 1);
+        if (warp == warps - 1) share(red + R, 2);
+        cluster.sync();
+        if (warp == 0) {
+            double t = slots[kClusterCtas + lane];  // lanes 0 to 15 r.z, 16 to 31 r.r
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) {
+                bc[0] = t;
+                bc[1] = t / rz;
+            }
+            if (lane == 16) bc[2] = t;
+        }
+        __syncthreads();
+        rz = bc[0];
+        rr = bc[2];
+        ++it;
+        state = rr <= thresh2 ? 1 : !(rz == rz) || pq == 0.0 ? 2 : it >= max_iter ? 3 : 0;
+        const double beta = bc[1];
+        pi = fma(beta, pi, zi);
+        if (live) P[row] = pi;
+        for (int b = warp; b < blocks; b += warps) {
+            const int at = list[b] * 32, owner = at / R;
+            P[at + lane] = fma(beta, P[at + lane], cluster.map_shared_rank(zown, owner)[at - owner * R + lane]);
+        }
+        __syncthreads();
+    }
+    if (live) {
+        x[row] = xi;
+        r[row] = ri;
+        p[row] = pi;
+    }
+    cluster.sync();  // no CTA leaves while its memory is read, or the state before it is
+    if (rank == 0 && tid == 0) {
+        st->ring[it & 3][1] = rz;
+        st->ring[it & 3][2] = rr;
+        st->it = it;
+        if (state == 1) st->converged_at = it;
+        st->done = state;
+    }
+}
+
 // Two launches where every lane group has one row and every SM at most one block
 // of the product (9,728 rows on GB300).  Microseconds per iteration, four launches ->
 // two: plane systems of 578 rows 18.3 -> 11.0, 2,178 rows 14.7 -> 9.2, 8,450 rows
@@ -290,6 +457,36 @@ __global__ void k_set_thresh(CgState* st, double rtol) {
         st->converged_at = 0;
     }
 }
+
+// launch of k_cluster_cg for n rows of at most width entries
+struct ClusterLaunch {
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg{};
+    bool init(int64_t n, int width, cudaStream_t st) {
+        const ClusterShape s = cluster_shape(n, width);
+        int dev = 0, limit = 0, clusters = 0;
+        if (!s.rows || width < 1 || cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+            s.smem > (size_t)limit)
+            return false;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kClusterCtas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kClusterCtas);
+        cfg.blockDim = dim3((unsigned)s.rows);
+        cfg.dynamicSmemBytes = s.smem;
+        cfg.stream = st;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        const bool ok =
+            cudaFuncSetAttribute(k_cluster_cg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(k_cluster_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem) ==
+                cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, k_cluster_cg, &cfg) == cudaSuccess && clusters > 0;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }
+};
 
 }  // namespace
 
@@ -337,17 +534,35 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     const unsigned row_blocks = (unsigned)((n * fem::kLanesPerRow + tpb - 1) / tpb);
     const unsigned spmv_blocks = (unsigned)std::min<int64_t>(row_blocks, (int64_t)sm_count() * 16);
     const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 8);
-    k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv,
-                                                                opts->preconditioner == 1);
+    // one cluster where its shared memory holds the rows of the model's graph
+    const int width = c->dim * (c->ulen.empty() ? 0 : *std::max_element(c->ulen.begin(), c->ulen.end()));
+    ClusterLaunch cluster;
+    const bool clustered = cluster.init(n, width, sm);
+    k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv, opts->preconditioner == 1,
+                                                                clustered ? width : INT_MAX, st);
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, st);
     k_set_thresh<<<1, 1, 0, sm>>>(st, opts->rel_tol);
     c->launches += 3;
+    CgState hs{};
+    const auto read_state = [&] {
+        e = cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, sm);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
+        return e == cudaSuccess && !hs.done;
+    };
+    if (clustered)
+        do {
+            e = cudaLaunchKernelEx(&cluster.cfg, k_cluster_cg, (int)n, width, rowptr, colidx, vals, x, r, p,
+                                   (const double*)dinv, st, (int)opts->max_iter);
+            c->launches++;
+        } while (e == cudaSuccess && read_state() && !hs.wide);
+    // a matrix with longer rows than the model's graph takes the launches
+    const bool launches = !clustered || (hs.wide && !hs.done);
     // capture a chunk of iterations into a graph
     const int chunk = 32;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    e = cudaStreamBeginCapture(sm, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && launches) e = cudaStreamBeginCapture(sm, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess && launches) {
         for (int k = 0; k < chunk && pair; ++k) {
             e = launch_kernel(k_pair_product, row_blocks, tpb, 0, sm, true, n, rowptr, colidx, vals, z, p, dinv + n, q,
                               st, k, opts->max_iter);
@@ -366,17 +581,14 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
         const cudaError_t ended = cudaStreamEndCapture(sm, &graph);
         if (e == cudaSuccess) e = ended;
     }
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-    CgState hs{};
+    if (e == cudaSuccess && launches) e = cudaGraphInstantiate(&exec, graph, 0);
     fem_gpu_status result = FEM_GPU_OK;
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && launches) {
         for (int launched = 0; launched < opts->max_iter + chunk; launched += chunk) {
             e = cudaGraphLaunch(exec, sm);
             if (e != cudaSuccess) break;
             c->launches += pair ? 2 * chunk + 1 : 4 * chunk;
-            e = cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, sm);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
-            if (e != cudaSuccess || hs.done) break;
+            if (!read_state()) break;
         }
     }
     if (e != cudaSuccess) result = fail(c, FEM_GPU_CUDA_ERROR, std::string("pcg: ") + cudaGetErrorString(e));
@@ -503,7 +715,7 @@ extern "C" fem_gpu_status fem_gpu_pcg_noalloc(fem_gpu_ctx* c, const int32_t* row
     const unsigned row_blocks = (unsigned)((n * fem::kLanesPerRow + tpb - 1) / tpb);
     const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 8);
     k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv,
-                                                                opts->preconditioner == 1);
+                                                                opts->preconditioner == 1, INT_MAX, cs);
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, cs);
     k_set_thresh<<<1, 1, 0, sm>>>(cs, opts->rel_tol);
     c->launches += 3;
@@ -568,7 +780,8 @@ extern "C" fem_gpu_status fem_gpu_pcg_snapshots(fem_gpu_ctx* c, const int32_t* r
     const unsigned row_blocks = (unsigned)((n * fem::kLanesPerRow + tpb - 1) / tpb);
     const unsigned spmv_blocks = (unsigned)std::min<int64_t>(row_blocks, (int64_t)sm_count() * 16);
     const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 8);
-    k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv, opts->preconditioner == 1);
+    k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv, opts->preconditioner == 1,
+                                                                INT_MAX, st);
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, st);
     k_set_thresh<<<1, 1, 0, sm>>>(st, opts->rel_tol);
     CgState hs{};
