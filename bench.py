@@ -84,59 +84,22 @@ def c2_config(ne, adofs, nnz):
             "l2": "inputs exceed L2 (CSR values %.2f GB, element data > 1 GB)" % (8 * nnz / 1e9)}
 
 
-def flops_per_element(order=2, ngp=27, rect=True, density=False):
-    """FP64 flop count (FMA = 2, other ops 1) of the bulk kernel's formulation
-    for one interior hex8 element with B-spline extraction of `order` and
-    `ngp` Gauss points.
-
-    Column counts of the extraction T (8 nodes x (order+1)^3 bases): per
-    direction the two end nodes of a quadratic element see bases 0, 1, 2 with
-    (1, 2, 1) nonzeros, so column j has tc_j = product over directions (sum 64
-    = 8 nonzeros per node row); linear extraction at level 0 is the identity
-    (one nonzero per column and per node row).
-    rect=True is the constant-Jacobian (brick) path: the Gram matrix is a
-    scaled per-rule table; rect=False the per-Gauss-point path.  density=True
-    is the SIMP path: E(x_q) = E0 rho(x_q)^beta per Gauss point, so the Gram
-    matrix is summed per element over the points with those weights.
-    Quadratic extraction is the tensor product of (1/2, 1/2, 0) / (0, 1/2, 1/2):
-    K is formed as K/64, K T / 8 as (K/64) P summed axis by axis (19 additions
-    per row of K and column field, 8 node values -> 27 bases), and each entry
-    of T^T K T = P^T (K/64) P as a plain sum over the sparser column's nodes
-    (count - 1 additions)."""
-    tc1, nzrow = {1: ([1, 1], 1), 2: ([1, 2, 1], 8)}[order]
-    tc = [a * b * c for c in tc1 for b in tc1 for a in tc1]
-    NGP, NPD, NB, D = ngp, 24, len(tc), 3
-    nsym = NPD * (NPD + 1) // 2
-    if rect:
-        geo = D * 8 * 2 + 2 + D + 4                           # diagonal J, detJ, 3 divisions, products
-        gram = nsym * NGP * 2 + NGP * (8 * 2 + 3) if density else 0  # rho(x_q)^3, sum_q w_q E_q dN dN^T
-        kiso = nsym * 4 + 3 * 36 * 8                          # c_fg (lam G0 + mu G0') (+ trace on diagonal blocks)
-    else:
-        geo = NGP * (D * D * 8 * 2 + 40 + D * D * 8 * 2 + 1 + NPD)  # J, inverse, g = J^-1 dN, w*, w*g
-        gram = nsym * NGP * 2 + (NGP * (8 * 2 + 3) if density else 0)  # upper triangle of A
-        kiso = nsym * 3 + 3 * 36 * 4
-    upd = NPD * nzrow * 2                                     # u_pdof = T u_adof
-    resid = NPD * NPD * 2 + D * sum(tc) * 2                   # R_p = K u, R_a = T^T R_p
-    if order == 2:
-        kt = NPD * D * 19                                     # K T summed axis by axis (y, x, z stages)
-    else:
-        kt = (D * (D + 1) // 2) * 8 * sum(tc) * 2             # K T over the T column nonzeros
-    ka = 0                                                    # upper triangle of T^T (K T)
-    nad = D * NB
-    if order == 2:
-        # count-ordered adofs: the row holds the sparser column, count - 1 additions
-        srt = sorted(tc)
-        for x in range(nad):
-            ka += (srt[x // D] - 1) * (nad - x)
-    else:
-        for r in range(nad):
-            ka += tc[r % NB] * (nad - r) * 2
-    return geo + gram + kiso + upd + resid + kt + ka
+def lattice_ops(ne):
+    """(flops, FP64 instructions) of one assembly of an ne^3 brick lattice with
+    quadratic splines and constant moduli, residual included, counted from the
+    kernels (fem_lattice.cu); an FMA is two flops and one instruction.
+    Per node (ne + 1)^3: element weights 168, box sums 90, 27 blocks of 17 flops
+    (14 instructions), 243 FMAs of the residual, 24 of the nodal displacements.
+    Per basis (ne + 2)^3: 2,340 additions of the projection, 24 of the residual."""
+    nodes, bases = (ne + 1) ** 3, (ne + 2) ** 3
+    flops = nodes * (168 + 90 + 27 * 17 + 243 * 2 + 24) + bases * (2340 + 24)
+    return flops, nodes * (168 + 90 + 27 * 14 + 243 + 24) + bases * (2340 + 24)
 
 
-def flops_per_element_c2(rect=True):
-    """the headline workload: quadratic B-splines, HEX_3x3x3"""
-    return flops_per_element(2, 27, rect)
+def density_flops_per_element():
+    """flops of the density path for linear splines (HEX_2x2x2): 700 for a cell's 63
+    sums, 964 for a node's 14 blocks and the residual (one node per cell)"""
+    return 700 + 964
 
 
 def dense_gp_flops(ngp, npd=24, nv=6):
@@ -286,19 +249,16 @@ def c3_stats(x):
 
 
 def c3_flops(st):
-    """FP64 operations of the cluster kernel's formulation per step (counted
-    from the kernel code, FMA = 2):
-      uncut cell      5,050 (Gram from the rule table, isotropic K, R = K u, K T, T^T K T)
-      cut point         120 (IG->IP map, detJ, w*, monomials, 28 moment FMAs)
-      cut cluster    16,750 (Gram from the moments: 300 entries x 20 FMAs; epilogue
-                             as for an uncut cell)
-      interface facet 22,100 (7 points x 460 geometry, facet moments P and Q,
-                              normal-weighted cluster moments A1)
-      interface clus. 47,000 (K from A1 and Q, R = K u, K T, T^T K T on 48 x 48)
-      ghost cluster   86,000 (4 points geometry, n.D.B operators, 4 x 3 rank-1
-                              updates of the 48 x 48 block, epilogue)"""
-    return (5050 * st["uncut_cells"] + 120 * st["cut_points"] + 16750 * st["cut_clusters"] +
-            22100 * st["interface_facets"] + 47000 * st["interface_clusters"] + 86000 * st["ghost_faces"])
+    """FP64 operations of the brick kernels (fem_brick.cu) per step, counted from
+    the code (FMA = 2):
+      uncut cell       2,720 (63 scaled sums, 64 node pairs of 38 with the residual)
+      cut point          115 (IG->IP map, detJ, w*, monomials, 27 moment FMAs)
+      cut cluster      4,360 (the 63 sums from the moments, then as an uncut cell)
+      interface facet    785 (normal, 7 points, 4 x 27 moments)
+      interface clus. 27,400 (10 matrices from the moments, 256 node pairs of 46)
+      ghost face       9,500 (256 node pairs of 32, coefficients)"""
+    return (2720 * st["uncut_cells"] + 115 * st["cut_points"] + 4360 * st["cut_clusters"] +
+            785 * st["interface_facets"] + 27400 * st["interface_clusters"] + 9500 * st["ghost_faces"])
 
 
 def cpu_reference_c3(x, sets, seconds):
@@ -335,7 +295,7 @@ def cpu_reference_c3(x, sets, seconds):
 
 def run_c3(timed, stream, world, args):
     """Config 3: two-phase XFEM, 96^3 background cut by 40 spheres; every
-    cluster in one persistent graph-captured launch (fem_gpu_assemble_batched)."""
+    cluster in one captured graph (fem_gpu_assemble_batched)."""
     import torch
     import moris_gb300 as mg
     from moris_gb300 import workloads
@@ -514,7 +474,7 @@ def run_c5(timed, stream, args):
         moris_gb300/train_lpc.py on other density seeds), when a weight file exists.
     Each solve starts from x = 0 on device-resident CSR and right-hand side."""
     import torch
-    from moris_gb300 import ACCUMULATE, learned, workloads
+    from moris_gb300 import learned, workloads
     from moris_gb300.multigrid import Multigrid, fcg_config, fcg_mg
     m, mesh, rho = workloads.simp_3d(128, finalize=False)
     m.set_stream(stream.cuda_stream)
@@ -529,10 +489,10 @@ def run_c5(timed, stream, args):
     rhs_t = torch.empty_like(b)
     nel = len(mesh["cells"])
     ms_asm = timed(lambda: m.assemble(None, vals, rhs_t), 10, 3)
-    ms_asm_kernel = timed(lambda: m.assemble(None, vals, rhs_t, ACCUMULATE), 10, 2)
-    fpe = flops_per_element(1, 8, rect=True, density=True)
+    ms_asm_kernel = ms_asm  # no zero fill
+    fpe = density_flops_per_element()
     peak = fp64_peak()
-    asm = {"path": "per-Gauss-point E0 rho(x_q)^3 on HEX_2x2x2 (density-weighted Gram matrix per element), "
+    asm = {"path": "per-Gauss-point E0 rho(x_q)^3 on HEX_2x2x2 (63 density-weighted sums per element, block stencil), "
                    "linear B-splines", "elements": nel, "ms_per_assembly": ms_asm,
            "elements_per_s": nel / (ms_asm * 1e-3), "kernel_ms": ms_asm_kernel,
            "roofline": {"bound": "fp64", "achieved": fpe * nel / (ms_asm_kernel * 1e-3) / 1e12, "peak": peak,
@@ -791,8 +751,9 @@ def main():
     ms = timed(lambda: model.assemble(u, vals, rhs), args.steps, 0)
     clocks = sampler.stop()
     launches = model.launch_count() - l0
-    # kernel alone (accumulate: no zero fill) for the roofline
-    ms_kernel = timed(lambda: model.assemble(u, vals, rhs, mg.ACCUMULATE), max(5, args.steps // 4), 2)
+    # kernels for the roofline: a lattice assembly stores every value, without a zero
+    # fill, so that it is the kernels and the status read
+    ms_kernel = timed(lambda: model.assemble(u, vals, rhs), max(5, args.steps // 4), 2)
     # matrix-free Jv
     x = torch.tensor(rng.uniform(-1.0, 1.0, nad), device="cuda")
     y = torch.empty_like(x)
@@ -839,21 +800,13 @@ def main():
         if world > 1:
             dist.destroy_process_group()
         return
-    # roofline of the dominant kernel against the FP64 pipe, on the formulation's
-    # flop count (the tensor-product path leaves so few FP64 operations that the
-    # kernel is bound by shared-memory latency instead, as the limiter says)
+    # roofline against the FP64 pipe, on the flop count of the lattice kernels (mostly
+    # additions, one flop per instruction slot: pipe_frac is the share of the slots)
     peak = fp64_peak()
     dmma_alone = mg.probe_dmma_tflops()
     dmma_mixed = mg.probe_dmma_tflops(mixed=True)
-    fpe = flops_per_element_c2()
-    achieved = fpe * nc / (ms_kernel * 1e-3) / 1e12
-    traffic = None
-    prof = os.path.join(ROOT, "profiles", "bulk_kernel_hex8_q2_traffic.json")
-    if os.path.exists(prof) and args.ne == NE:
-        try:
-            traffic = json.load(open(prof)).get("dram_bytes_per_launch")
-        except Exception:
-            traffic = None
+    flops, instructions = lattice_ops(args.ne)
+    achieved = flops / (ms_kernel * 1e-3) / 1e12
     line = {
         "metric": "elements/s assembled (FP64 full Jacobian + residual into CSR)",
         "value": value, "unit": "elements/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -862,12 +815,14 @@ def main():
         "config": c2_config(args.ne, nad, nnz), "parallelism": "replicas" if world > 1 else "1 GPU",
         "gpu_launches": int(launches),
         "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                     "frac": achieved / peak, "traffic": traffic,
+                     "frac": achieved / peak,
+                     "pipe_frac": 2.0 * instructions / (ms_kernel * 1e-3) / 1e12 / peak,
+                     "csr_write_gbs": 8 * nnz / (ms_kernel * 1e-3) / 1e9,
                      "peak_source": "measured in-run (FP64 FMA-chain probe, fem_gpu_probe_fp64_tflops)",
-                     "limiter": "latency of the shared-memory load chains of T^T K T; ncu at 32^3: FP64 pipe 52 %, "
-                                "L1 72 %, L2 68 %, issue 36 %",
-                     "flops_per_element": fpe, "kernel_ms": ms_kernel,
+                     "limiter": "FP64 pipe (ncu at 36^3: lattice_const 73 %, lattice_project 68 % busy)",
+                     "flops_per_element": flops / nc, "kernel_ms": ms_kernel,
                      "fp64_tensor_probe_tflops": {"dmma": dmma_alone, "dmma_plus_dfma": dmma_mixed}},
+        "assembly_path": "tensor lattice (block stencil, axis-wise projection); host buffers: element loop",
         "kernel_variant": {"index": variant[0], "name": variant[2], "tuned_ms": variant[1]},
         "jv": {"ms_per_apply": ms_jv, "elements_per_s": nc / (ms_jv * 1e-3), "rel_err_vs_csr": jv_err},
         "setup_seconds": setup_s,
