@@ -1249,9 +1249,16 @@ fem_gpu_status launch_sides(fem_gpu_ctx* c, const double* u, double* vals, doubl
     SideBatch b{};
     int n = 0;
     fem_gpu_status st = FEM_GPU_OK;
+    std::vector<int> plane;
+    for (size_t k = 0; k < c->sets.size(); ++k)
+        if (c->sets[k].kind == 1 && c->sets[k].neq > 0 && c->sets[k].d_ptab.p) plane.push_back((int)k);
+    if (!plane.empty()) {
+        st = lattice_sides(c, plane, u, vals, rhs, overlap);
+        overlap = true;
+    }
     for (const SetData& s : c->sets) {
         if (st != FEM_GPU_OK) return st;
-        if (s.kind != 1 || s.neq == 0) continue;
+        if (s.kind != 1 || s.neq == 0 || s.d_ptab.p) continue;
         if (brick_count(s, 0, s.neq) == s.neq) {
             st = brick_launch(c, s, 0, s.neq, u, vals, rhs, c->stream);
             overlap = true;

@@ -94,6 +94,8 @@ struct SetData {
     DeviceBuf d_fast;                 // their tables (ftab_bytes), list, kinds and maps
     size_t ftab_bytes = 0;
     bool lattice = false;   // the set covers a tensor lattice (fem_lattice.cu)
+    DeviceBuf d_ptab, d_pfacet;  // side sets of plane lattices: products of the splines, facets
+    double side_wsum = 0.0;      // their sum of the rule's weights
     DeviceBuf d_latE, d_latrho;  // lattice sets: modulus in cell order (if the set's order differs), nodal densities
     double tuned_ms = 0.0;  // time of the chosen variant on the tuning run
 };
@@ -197,6 +199,8 @@ inline bool lattice_pays(const fem_gpu_ctx* c, int set, bool product) {
     if (c->shape != FEM_GPU_SHAPE_RECTANGULAR) return !quad || c->num_cells >= (product ? 216 : 1000);
     return c->num_cells >= (quad && product ? 1728 : 1000);
 }
+fem_gpu_status lattice_sides(fem_gpu_ctx* c, const std::vector<int>& sets, const double* u, double* vals, double* rhs,
+                             bool overlap);
 fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double* vals, double* rhs, bool acc_v,
                                 bool acc_r);
 // device address of fem_gpu_pcg_noalloc's fixed array on the current device,

@@ -982,6 +982,115 @@ __global__ void __launch_bounds__(32 * (2 * P + 1)) lattice_plane(PlaneArgs p) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// Boundary facets of plane lattices: as the boundary facets of bricks (fem_brick.cu),
+// with tables of the products between splines, because the extraction is the same for
+// every cell:  I_i(a, b) = integral N_a dN_b / dxi_i, NN(a, b) = integral N_a N_b per
+// facet ordinal.  K(a, b) = -T(a, b) + beta T(b, a)^T + gamma NN with T(k, k) = (lam +
+// 2 mu) n I_k, T(t, t) = mu n I_k, T(k, t) = lam n I_t, T(t, k) = mu n I_t for the normal
+// axis k; a constant displacement has no traction, so the residual is K (u - g).  A
+// warp per facet, a lane per pair (or three, or eight) of splines; the pairs' shares of
+// the residual meet in shared memory.  One short phase, where the general kernel
+// (side_cta_kernel) is a chain of twelve: 24 x 17 cells with clamp and load 32 -> 0 us.
+struct PlaneSide {
+    int64_t n;
+    const int32_t* facet;  // cell * 4 + ordinal
+    const double* E;
+    const double* tab;     // [ordinal][I_0, I_1, NN][b][a]
+    int neumann;
+    double lam, mu, alpha, beta, thickness, wsum, value[2];
+};
+constexpr int kPlaneSides = 4, kPlaneSideWarps = 4;
+struct PlaneSides {
+    PlaneSide set[kPlaneSides];
+    int ne[2], nb[2];
+    const double* jac;
+    const double* u;
+    double* vals;
+    double* rhs;
+    const int32_t* rowptr;
+    int* status;
+};
+
+template <int P>
+__global__ void __launch_bounds__(32 * kPlaneSideWarps) lattice_plane_sides(const __grid_constant__ PlaneSides p) {
+    constexpr int NB = (P + 1) * (P + 1), PAIRS = NB * NB, PER = (PAIRS + 31) / 32;
+    __shared__ double sm[kPlaneSideWarps][PAIRS][2];
+    const PlaneSide& s = p.set[blockIdx.y];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t e = (int64_t)blockIdx.x * kPlaneSideWarps + warp;
+    if (e >= s.n) return;
+    const int fc = __ldg(s.facet + e), ord = fc & 3, cell = fc >> 2, ci = cell % p.ne[0], cj = cell / p.ne[0];
+    const int nu = p.nb[0] * p.nb[1];
+    const bool x = ord & 1;  // the normal is along x
+    const double n = ord == 1 || ord == 2 ? 1.0 : -1.0;
+    const double J0 = __ldg(p.jac + ci), J1 = __ldg(p.jac + p.ne[0] + cj), E = __ldg(s.E + e);
+    const double Jk = x ? J0 : J1, Jt = x ? J1 : J0;
+    const double w = Jt * s.thickness, sc = n * w * E;
+    const double ck = sc / Jk, ct = sc / Jt;
+    const double kk = (s.lam + 2.0 * s.mu) * ck, tt = s.mu * ck, lt = s.lam * ct, mt = s.mu * ct;
+    const double nn = s.neumann ? w : s.alpha * E * w / (Jt * s.wsum);
+    const double* tab = s.tab + ord * 3 * PAIRS;
+    double K[PER][4];  // row component, column component
+    bool bad = false;
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+        const int t = lane + 32 * m, b = t / NB, a = t - b * NB;
+        if (t >= PAIRS) continue;
+        const double N = nn * __ldg(tab + 2 * PAIRS + t);
+        double r0, r1;
+        if (s.neumann) {
+            r0 = -N * s.value[0];
+            r1 = -N * s.value[1];
+        } else {
+            const int o = a * NB + b;
+            const double ik = __ldg(tab + (x ? 0 : PAIRS) + t), jk = s.beta * __ldg(tab + (x ? 0 : PAIRS) + o);
+            const double it = __ldg(tab + (x ? PAIRS : 0) + t), jt = s.beta * __ldg(tab + (x ? PAIRS : 0) + o);
+            const double k0 = fma(kk, jk - ik, N), k1 = fma(tt, jk - ik, N);
+            const double kt = fma(mt, jt, -lt * it), tk = fma(lt, jt, -mt * it);
+            K[m][0] = x ? k0 : k1;
+            K[m][1] = x ? kt : tk;
+            K[m][2] = x ? tk : kt;
+            K[m][3] = x ? k1 : k0;
+            const int j = (cj + b / (P + 1)) * p.nb[0] + ci + b % (P + 1);
+            const double u0 = (p.u ? __ldg(p.u + j) : 0.0) - s.value[0], u1 = (p.u ? __ldg(p.u + nu + j) : 0.0) - s.value[1];
+            r0 = fma(K[m][0], u0, K[m][1] * u1);
+            r1 = fma(K[m][2], u0, K[m][3] * u1);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) bad |= !fem_finite(K[m][k]);
+        }
+        sm[warp][t][0] = r0;
+        sm[warp][t][1] = r1;
+    }
+    __syncwarp();
+    double r = 0.0;
+    const int ra = lane % NB, rf = lane / NB;
+    if (rf < 2)
+#pragma unroll
+        for (int b = 0; b < NB; ++b) r += sm[warp][b * NB + ra][rf];
+    cudaGridDependencySynchronize();  // the sums of the kernel before
+    if (rf < 2 && p.rhs)
+        atomicAdd(p.rhs + rf * nu + (cj + ra / (P + 1)) * p.nb[0] + ci + ra % (P + 1), r);
+    if (p.vals && !s.neumann) {
+#pragma unroll
+        for (int m = 0; m < PER; ++m) {
+            const int t = lane + 32 * m, b = t / NB, a = t - b * NB;
+            if (t >= PAIRS) continue;
+            const int rx = ci + a % (P + 1), ry = cj + a / (P + 1), row = ry * p.nb[0] + rx;
+            const int lx = max(rx - P, 0), cx = min(rx + P, p.nb[0] - 1) - lx + 1;
+            const int ly = max(ry - P, 0), cy = min(ry + P, p.nb[1] - 1) - ly + 1;
+            const int at = (cj + b / (P + 1) - ly) * cx + ci + b % (P + 1) - lx, ul = cx * cy;
+            double* v0 = p.vals + __ldg(p.rowptr + row) + at;
+            double* v1 = p.vals + __ldg(p.rowptr + nu + row) + at;
+            atomicAdd(v0, K[m][0]);
+            atomicAdd(v0 + ul, K[m][1]);
+            atomicAdd(v1, K[m][2]);
+            atomicAdd(v1 + ul, K[m][3]);
+        }
+        if (bad) atomicOr(p.status, 1);
+    }
+}
+
 struct Lattice {
     int dim = 3, p = 0;
     bool brick = true;  // axis-aligned cells (FEM_GPU_SHAPE_RECTANGULAR)
@@ -1097,6 +1206,48 @@ bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
 
 void lattice_release(fem_gpu_ctx* c);
 
+// tables and facets of a side set of a plane lattice (identity projection)
+static cudaError_t plane_side_upload(const fem_gpu_ctx* c, const Lattice& L, SetData& s, cudaStream_t st) {
+    for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2; ++j)
+            if (s.side_select[i * 3 + j] != (i == j ? 1.0 : 0.0)) return cudaSuccess;
+    if (c->num_cells >= (int64_t)1 << 29) return cudaSuccess;
+    const Rule r = gauss_rule(s.side.integration_rule);
+    const int p1 = L.p + 1, NB = p1 * p1, PAIRS = NB * NB;
+    std::vector<double> tab((size_t)4 * 3 * PAIRS, 0.0);
+    static const int corner[4][2] = {{0, 0}, {1, 0}, {1, 1}, {0, 1}};
+    for (int o = 0; o < 4; ++o)
+        for (int q = 0; q < r.n; ++q) {
+            const int k = o & 1 ? 0 : 1;
+            double xi[2], N[4], dN[8], B[16] = {}, dB[2][16] = {};
+            xi[k] = o == 1 || o == 2 ? 1.0 : -1.0;
+            xi[1 - k] = r.pts[q * r.dim];
+            lagrange(FEM_GPU_CELL_QUAD4, xi, N, dN);
+            for (int n = 0; n < 4; ++n)
+                for (int b = 0; b < L.p; ++b)
+                    for (int a = 0; a < L.p; ++a) {
+                        const double w = axis_weights(L.p)[a] * axis_weights(L.p)[b];
+                        const int f = (corner[n][1] + b) * p1 + corner[n][0] + a;
+                        B[f] += w * N[n];
+                        for (int i = 0; i < 2; ++i) dB[i][f] += w * dN[i * 4 + n];
+                    }
+            for (int b = 0; b < NB; ++b)
+                for (int a = 0; a < NB; ++a) {
+                    double* t = &tab[(size_t)o * 3 * PAIRS + b * NB + a];
+                    for (int i = 0; i < 2; ++i) t[i * PAIRS] += r.w[q] * B[a] * dB[i][b];
+                    t[2 * PAIRS] += r.w[q] * B[a] * B[b];
+                }
+        }
+    std::vector<int32_t> facet(s.neq);
+    for (int64_t i = 0; i < s.neq; ++i) facet[i] = s.ip_cell[i] * 4 + s.ordinal[i];
+    s.side_wsum = 0.0;
+    for (double w : r.w) s.side_wsum += w;
+    cudaError_t e = upload(s.d_ptab, tab, st);
+    if (e == cudaSuccess) e = upload(s.d_pfacet, facet, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    return e;
+}
+
 // Finds out whether the model is a lattice and which of its bulk sets cover
 // every cell exactly once; those are assembled here (SetData::lattice).
 fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
@@ -1133,6 +1284,9 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
         s.lattice = any = true;
     }
     if (!any) return FEM_GPU_OK;
+    if (c->dim == 2)
+        for (SetData& s : c->sets)
+            if (s.kind == 1 && s.neq > 0 && e == cudaSuccess) e = plane_side_upload(c, L, s, st);
     auto* K = new Lattice(L);
     c->lattice = K;
     if (e == cudaSuccess) e = upload(K->jac, jac, st);
@@ -1170,6 +1324,8 @@ void lattice_release(fem_gpu_ctx* c) {
     for (SetData& s : c->sets) {
         dfree(s.d_latE);
         dfree(s.d_latrho);
+        dfree(s.d_ptab);
+        dfree(s.d_pfacet);
         s.lattice = false;
     }
     Lattice* L = (Lattice*)c->lattice;
@@ -1474,6 +1630,58 @@ fem_gpu_status lattice_assemble(fem_gpu_ctx* c, int set, const double* u, double
     if (e == cudaSuccess) e = cudaGetLastError();
     return e == cudaSuccess ? FEM_GPU_OK
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice launch: ") + cudaGetErrorString(e));
+}
+
+// The side sets among `sets` (at most kPlaneSides of a launch) of a plane lattice,
+// added to vals and rhs; see fem_launch.cuh for overlap (u is read ahead of the wait).
+fem_gpu_status lattice_sides(fem_gpu_ctx* c, const std::vector<int>& sets, const double* u, double* vals, double* rhs,
+                             bool overlap) {
+    const Lattice& L = *(const Lattice*)c->lattice;
+    PlaneSides a{};
+    for (int d = 0; d < 2; ++d) {
+        a.ne[d] = L.ne[d];
+        a.nb[d] = L.nb[d];
+    }
+    a.jac = (const double*)L.jac.p;
+    a.u = u;
+    a.vals = vals;
+    a.rhs = rhs;
+    a.rowptr = (const int32_t*)c->d_rowptr.p;
+    a.status = (int*)c->d_status.p;
+    cudaError_t e = cudaSuccess;
+    for (size_t k = 0; k < sets.size() && e == cudaSuccess; k += kPlaneSides) {
+        int64_t most = 0;
+        const int n = (int)std::min<size_t>(kPlaneSides, sets.size() - k);
+        for (int m = 0; m < n; ++m) {
+            const SetData& s = c->sets[sets[k + m]];
+            PlaneSide& q = a.set[m];
+            q.n = s.neq;
+            q.facet = (const int32_t*)s.d_pfacet.p;
+            q.E = (const double*)s.d_E.p;
+            q.tab = (const double*)s.d_ptab.p;
+            q.neumann = s.side.iwg_type == FEM_GPU_IWG_STRUC_LINEAR_NEUMANN;
+            const double nu = s.side.poisson_ratio;
+            q.lam = s.side.model_type == FEM_GPU_MODEL_PLANE_STRESS ? nu / (1.0 - nu * nu)
+                                                                    : nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
+            q.mu = 1.0 / (2.0 * (1.0 + nu));
+            q.alpha = s.side.nitsche_alpha;
+            q.beta = s.side.iwg_type == FEM_GPU_IWG_STRUC_LINEAR_DIRICHLET_SYMMETRIC_NITSCHE ? -1.0 : 1.0;
+            q.thickness = s.side_thickness;
+            q.wsum = s.side_wsum;
+            for (int d = 0; d < 2; ++d) q.value[d] = s.side.value[d];
+            most = std::max(most, q.n);
+        }
+        const dim3 grid((unsigned)((most + kPlaneSideWarps - 1) / kPlaneSideWarps), (unsigned)n);
+        void (*const fn)(PlaneSides) = L.p == 1   ? lattice_plane_sides<1>
+                                       : L.p == 2 ? lattice_plane_sides<2>
+                                                  : lattice_plane_sides<3>;
+        e = launch_kernel(fn, grid, 32 * kPlaneSideWarps, 0, (cudaStream_t)c->stream, overlap, a);
+        c->launches++;
+        overlap = true;
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return e == cudaSuccess ? FEM_GPU_OK
+                            : fail(c, FEM_GPU_CUDA_ERROR, std::string("side launch: ") + cudaGetErrorString(e));
 }
 
 }  // namespace fem

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import moris_gb300 as mg
+from oracle import OracleModel
 from tests.common import RTOL, csr_row_rel_err, problem, rel_err, uniform01
 
 pytestmark = pytest.mark.gpu
@@ -50,3 +51,45 @@ def test_six_side_sets(torch, dim, ne, p, shape):
     vo, ro = orc.assemble(un, nthreads=4)
     assert csr_row_rel_err(prod.graph()[0], vals.cpu().numpy(), vo) <= RTOL
     assert rel_err(rhs.cpu().numpy(), ro) <= RTOL
+
+
+@pytest.mark.parametrize("p", [1, 2, 3])
+@pytest.mark.parametrize("ne", [(1, 1), (1, 6), (13, 2)], ids=lambda n: "x".join(map(str, n)))
+def test_plane_lattice_facets(torch, ne, p):
+    """All four sides of a plane lattice: both Nitsche signs with a prescribed value,
+    plane stress, thickness, the one-point rule, and a set with a Select matrix, which
+    keeps the general kernel; against the oracle, with and without u."""
+    mesh = mg.hmr_uniform_mesh(2, ne, [1.3, 0.6], p)
+    nc = len(mesh["cells"])
+    prod = mg.FemModel(2, mesh, mg.SHAPE_RECTANGULAR)
+    orc = OracleModel(2, mg.CELL_QUAD4, mg.SHAPE_RECTANGULAR, mesh)
+    cells, E = np.arange(nc, dtype=np.int32), 0.1 + uniform01(3, nc)
+    prod.add_bulk_set(cells, E, 0.3, mg.RULE_QUAD_2x2, mg.MODEL_PLANE_STRESS)
+    orc.add_bulk_set(mg.CELL_QUAD4, mg.RULE_QUAD_2x2, mg.MODEL_PLANE_STRESS, cells, E, 0.3)
+    c = np.arange(nc)
+    x, y = c % ne[0], c // ne[0]
+    sym, uns, neu = (mg.IWG_STRUC_LINEAR_DIRICHLET_SYMMETRIC_NITSCHE, mg.IWG_STRUC_LINEAR_DIRICHLET_UNSYMMETRIC_NITSCHE,
+                     mg.IWG_STRUC_LINEAR_NEUMANN)
+    select = np.diag([1.0, 0.0])
+    sides = [(c[x == 0], 3, sym, mg.RULE_BAR_3, (0.3, -0.2), 1.0, None),
+             (c[x == ne[0] - 1], 1, uns, mg.RULE_BAR_3, (0.1, 0.4), 0.7, None),
+             (c[y == 0], 0, neu, mg.RULE_BAR_3, (0.5, -1.5), 1.0, None),
+             (c[y == ne[1] - 1], 2, sym, mg.RULE_BAR_1, (0.0, 0.25), 1.6, None),
+             (c[y == ne[1] - 1], 2, sym, mg.RULE_BAR_3, (0.2, 0.1), 1.0, select)]
+    for k, (cl, o, iwg, rule, value, thick, sel) in enumerate(sides):
+        cl = cl.astype(np.int32)
+        Es = 0.1 + uniform01(50 + k, len(cl))
+        prod.add_side_set(iwg, cl, np.full(len(cl), o), Es, 0.25, rule, mg.MODEL_PLANE_STRESS, alpha=20.0, value=value,
+                          thickness=thick, select=sel)
+        orc.add_side_set(iwg, rule, mg.MODEL_PLANE_STRESS, cl, np.full(len(cl), o), Es, 0.25, 20.0, value)
+        orc.set_side_options(k, thick, sel)
+    prod.finalize()
+    orc.finalize()
+    for un in (uniform01(31, prod.num_adofs) - 0.5, None):
+        vals = torch.full((prod.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+        rhs = torch.full((prod.num_adofs,), float("nan"), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        prod.assemble(None if un is None else torch.tensor(un, device="cuda"), vals, rhs)
+        vo, ro = orc.assemble(np.zeros(prod.num_adofs) if un is None else un)
+        assert csr_row_rel_err(prod.graph()[0], vals.cpu().numpy(), vo) <= RTOL
+        assert rel_err(rhs.cpu().numpy(), ro) <= RTOL
