@@ -864,7 +864,7 @@ __global__ void lattice_restrict(int n0, int n1, int n2, const double* rn, doubl
 // the 2 p + 1 blocks of its offsets and their share of the residual.  The element loop spent a CTA on 8 x 8 to 32 x 32
 // matrices; measured (assembly with two side sets): 257 x 130, p = 2, 237 -> 68.5 us
 // (kernel 44, FP64 pipe 68 %), 256 x 256, p = 3, 544 -> 201 us, 24 x 17, p = 1, 61 ->
-// 33 us.
+// 29 us.
 struct PlaneArgs {
     int ne[2], nb[2];
     const double* E;
@@ -991,7 +991,8 @@ __global__ void __launch_bounds__(32 * (2 * P + 1)) lattice_plane(PlaneArgs p) {
 // axis k; a constant displacement has no traction, so the residual is K (u - g).  A
 // warp per facet, a lane per pair (or three, or eight) of splines; the pairs' shares of
 // the residual meet in shared memory.  One short phase, where the general kernel
-// (side_cta_kernel) is a chain of twelve: 24 x 17 cells with clamp and load 32 -> 0 us.
+// (side_cta_kernel) is a chain of twelve: calls with clamp and load, 24 x 17 linear 32.5
+// -> 28.8 us, 24 x 24 cubic 53 -> 42 us.
 struct PlaneSide {
     int64_t n;
     const int32_t* facet;  // cell * 4 + ordinal
