@@ -192,12 +192,13 @@ inline bool lattice_set(const fem_gpu_ctx* c, int set) { return c->sets[set].lat
 // Products of bricks: linear 6^3 24 / 28, 10^3 28 / 27, 16^3 53 / 27; quadratic 6^3 25
 // / 37, 10^3 31 / 38, 12^3 40 / 38, 16^3 63 / 38.  Cells of any shape: linear 5^3 54 / 43, products
 // 30 / 23; quadratic 7^3 68 / 77, 10^3 120 / 99, products 8^3 42 / 36.
+constexpr int64_t kLatticeCells = 1000;
 inline bool lattice_pays(const fem_gpu_ctx* c, int set, bool product) {
     if (!lattice_set(c, set)) return false;
     const bool quad = c->sets[set].maxnb == 27;
     if (c->dim == 2) return true;
-    if (c->shape != FEM_GPU_SHAPE_RECTANGULAR) return !quad || c->num_cells >= (product ? 216 : 1000);
-    return c->num_cells >= (quad && product ? 1728 : 1000);
+    if (c->shape != FEM_GPU_SHAPE_RECTANGULAR) return !quad || c->num_cells >= (product ? 216 : kLatticeCells);
+    return c->num_cells >= (quad && product ? 1728 : kLatticeCells);
 }
 fem_gpu_status lattice_sides(fem_gpu_ctx* c, const std::vector<int>& sets, const double* u, double* vals, double* rhs,
                              bool overlap);

@@ -39,8 +39,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "fem_bits.cuh"
@@ -1097,8 +1100,9 @@ struct Lattice {
     bool brick = true;  // axis-aligned cells (FEM_GPU_SHAPE_RECTANGULAR)
     int ne[3], nn[3], nb[3];
     int64_t pitch = 0;
+    DeviceBuf mem;     // all of the following
     DeviceBuf jac;     // half edge lengths and their reciprocals
-    DeviceBuf S, vec;  // quadratic splines: stencil, nodal vectors
+    DeviceBuf S, vec;  // block stencil; quadratic splines: nodal vectors
     DeviceBuf Q;       // density sets: element sums
     // the last use of S, vec and Q: a call on another stream waits for it
     cudaEvent_t done = nullptr;
@@ -1166,38 +1170,72 @@ bool find_lattice(const fem_gpu_ctx* c, Lattice& L, std::vector<double>& jac) {
         }
     }
     if (c->num_cells != cells || c->num_bases != bases) return false;
+    // layers of nodes, cells and bases (rows of them in a plane), shared among threads
     const double* w1 = axis_weights(L.p);
     const double tol = L.p == 3 ? 1e-15 : 0.0;
-    for (int64_t n = 0, k = 0; n < N; ++n) {
-        const int64_t i[3] = {n % nn[0], n / nn[0] % nn[1], n / (nn[0] * nn[1])};
-        for (int d = 0; L.brick && d < D; ++d)
-            if (X[n * D + d] != X[i[d] * step[d] * D + d]) return false;
-        if (c->t_off[n + 1] - c->t_off[n] != width) return false;
-        for (int q = 0; q < width; ++q, ++k) {
-            const int a = q % L.p, b = q / L.p % L.p, z = q / (L.p * L.p);
-            const int64_t basis = ((i[2] + z) * L.nb[1] + i[1] + b) * L.nb[0] + i[0] + a;
-            const double w = w1[a] * w1[b] * (D == 3 ? w1[z] : 1.0);
-            if (c->t_bases[k] != basis || !(std::abs(c->t_w[k] - w) <= tol)) return false;
-        }
-    }
+    const int last = D - 1, npe = D == 2 ? 4 : 8;
     static const int corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
                                      {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
-    const int npe = D == 2 ? 4 : 8;
-    for (int64_t e = 0; e < cells; ++e) {
-        const int64_t i = e % L.ne[0], j = e / L.ne[0] % L.ne[1], k = e / ((int64_t)L.ne[0] * L.ne[1]);
-        for (int a = 0; a < npe; ++a)
-            if (c->cells[e * npe + a] != ((k + corner[a][2]) * nn[1] + j + corner[a][1]) * nn[0] + i + corner[a][0])
-                return false;
-    }
-    // CSR rows: the full box of bases within p along every axis (the bulk set
-    // puts the box into every row, so equal lengths are equal rows)
-    for (int64_t b = 0; b < bases; ++b) {
-        const int64_t i[3] = {b % L.nb[0], b / L.nb[0] % L.nb[1], b / ((int64_t)L.nb[0] * L.nb[1])};
-        int64_t len = 1;
-        for (int d = 0; d < D; ++d)
-            len *= std::min<int64_t>(i[d] + L.p, L.nb[d] - 1) - std::max<int64_t>(i[d] - L.p, 0) + 1;
-        if (c->ulen[b] != len) return false;
-    }
+    const auto layer = [&](int l) {
+        int64_t lo[3] = {0, 0, 0}, n[3] = {nn[0], nn[1], nn[2]};
+        lo[last] = l;
+        n[last] = l + 1;
+        // nodes: coordinates and extraction rows
+        for (int64_t z = lo[2]; z < n[2] && l < nn[last]; ++z)
+            for (int64_t y = lo[1]; y < n[1]; ++y)
+                for (int64_t x = 0; x < nn[0]; ++x) {
+                    const int64_t at = (z * nn[1] + y) * nn[0] + x;
+                    if (L.brick && (X[at * D] != X[x * D] || X[at * D + 1] != X[y * step[1] * D + 1] ||
+                                    (D == 3 && X[at * D + 2] != X[z * step[2] * D + 2])))
+                        return false;
+                    int64_t k = c->t_off[at];
+                    if (k != at * width || c->t_off[at + 1] != k + width) return false;
+                    for (int c2 = 0; c2 < (D == 3 ? L.p : 1); ++c2)
+                        for (int b = 0; b < L.p; ++b)
+                            for (int a = 0; a < L.p; ++a, ++k) {
+                                const int64_t basis = ((z + c2) * L.nb[1] + y + b) * L.nb[0] + x + a;
+                                const double w = w1[a] * w1[b] * (D == 3 ? w1[c2] : 1.0);
+                                if (c->t_bases[k] != basis || !(std::abs(c->t_w[k] - w) <= tol)) return false;
+                            }
+                }
+        // cells: node numbering
+        for (int d = 0; d < 3; ++d) n[d] = L.ne[d];
+        n[last] = l + 1;
+        for (int64_t z = lo[2]; z < n[2] && l < L.ne[last]; ++z)
+            for (int64_t y = lo[1]; y < n[1]; ++y)
+                for (int64_t x = 0; x < L.ne[0]; ++x) {
+                    const int64_t e = (z * L.ne[1] + y) * L.ne[0] + x;
+                    for (int a = 0; a < npe; ++a)
+                        if (c->cells[e * npe + a] !=
+                            ((z + corner[a][2]) * nn[1] + y + corner[a][1]) * nn[0] + x + corner[a][0])
+                            return false;
+                }
+        // CSR rows: the full box of bases within p along every axis (the bulk set
+        // puts the box into every row, so equal lengths are equal rows)
+        for (int d = 0; d < 3; ++d) n[d] = L.nb[d];
+        n[last] = l + 1;
+        const auto box = [&](int d, int64_t i) {
+            return std::min<int64_t>(i + L.p, L.nb[d] - 1) - std::max<int64_t>(i - L.p, 0) + 1;
+        };
+        for (int64_t z = lo[2]; z < n[2] && l < L.nb[last]; ++z)
+            for (int64_t y = lo[1]; y < n[1]; ++y) {
+                const int64_t yz = box(1, y) * (D == 3 ? box(2, z) : 1);
+                for (int64_t x = 0; x < L.nb[0]; ++x)
+                    if (c->ulen[(z * L.nb[1] + y) * L.nb[0] + x] != yz * box(0, x)) return false;
+            }
+        return true;
+    };
+    const int layers = L.nb[last];
+    const int nt = (int)std::min<int64_t>({16, std::max(1u, std::thread::hardware_concurrency()), 1 + N / 16384});
+    std::atomic<bool> ok{true};
+    std::vector<std::thread> th;
+    for (int t = 0; t < nt; ++t)
+        th.emplace_back([&, t] {
+            for (int l = t; l < layers && ok.load(std::memory_order_relaxed); l += nt)
+                if (!layer(l)) ok.store(false, std::memory_order_relaxed);
+        });
+    for (auto& t : th) t.join();
+    if (!ok) return false;
     L.pitch = (L.nn[0] + 3) / 4 * 4;
     for (size_t k = 0, n = jac.size(); k < n; ++k) jac.push_back(1.0 / jac[k]);
     return true;
@@ -1256,6 +1294,8 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
     std::vector<double> jac;
     cudaStream_t st = (cudaStream_t)c->stream;
     bool any = false;
+    // bricks that neither assembly nor product would take this way (lattice_pays)
+    if (c->dim == 3 && c->shape == FEM_GPU_SHAPE_RECTANGULAR && c->num_cells < kLatticeCells) return FEM_GPU_OK;
     for (const SetData& s : c->sets) any |= s.kind == 0 && s.ig_off.empty() && s.neq == c->num_cells;
     if (!any || !find_lattice(c, L, jac)) return FEM_GPU_OK;
     cudaError_t e = cudaSuccess;
@@ -1290,28 +1330,34 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
             if (s.kind == 1 && s.neq > 0 && e == cudaSuccess) e = plane_side_upload(c, L, s, st);
     auto* K = new Lattice(L);
     c->lattice = K;
-    if (e == cudaSuccess) e = upload(K->jac, jac, st);
     // workspaces (243 doubles per node, 0.22 of the CSR values for quadratic and as
     // much as them for linear splines; quadratic: six nodal values per node; density
-    // sets: 63 doubles per cell); a device that cannot hold them keeps the element loop
+    // sets: 63 doubles per cell), one allocation; a device that cannot hold them keeps
+    // the element loop
     bool rho = false;
     for (const SetData& s : c->sets) rho |= s.lattice && !s.node_rho.empty();
     const bool quad = c->dim == 3 && K->p == 2;
-    const size_t want[3] = {quad || (L.brick && c->dim == 3) ? (size_t)243 * L.nn[2] * L.nn[1] * L.pitch : 0,
+    const bool stencil = quad || (c->dim == 3 && L.brick && (rho || c->num_nodes >= kRowsNodes));
+    const size_t want[4] = {jac.size(), stencil ? (size_t)243 * L.nn[2] * L.nn[1] * L.pitch : 0,
                             quad ? (size_t)6 * c->num_nodes : 0,
                             rho ? (size_t)kQN * (L.ne[0] + 2) * (L.ne[1] + 2) * (L.ne[2] + 2) : 0};
-    DeviceBuf* const buf[3] = {&K->S, &K->vec, &K->Q};
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
-        if (!want[k]) continue;
+    DeviceBuf* const buf[4] = {&K->jac, &K->S, &K->vec, &K->Q};
+    size_t at[4], bytes = 0;
+    for (int k = 0; k < 4; ++k) {
+        at[k] = bytes;
         buf[k]->bytes = want[k] * sizeof(double);
-        if (cudaMalloc(&buf[k]->p, buf[k]->bytes) != cudaSuccess) {
-            cudaGetLastError();
-            buf[k]->p = nullptr;
-            cudaStreamSynchronize(st);
-            lattice_release(c);
-            return FEM_GPU_OK;
-        }
+        bytes += (buf[k]->bytes + 255) / 256 * 256;
     }
+    if (e == cudaSuccess && cudaMalloc(&K->mem.p, std::max<size_t>(bytes, 256)) != cudaSuccess) {
+        cudaGetLastError();
+        K->mem.p = nullptr;
+        cudaStreamSynchronize(st);
+        lattice_release(c);
+        return FEM_GPU_OK;
+    }
+    for (int k = 0; k < 4; ++k) buf[k]->p = want[k] ? (char*)K->mem.p + at[k] : nullptr;
+    if (e == cudaSuccess && !jac.empty())
+        e = cudaMemcpyAsync(K->jac.p, jac.data(), K->jac.bytes, cudaMemcpyHostToDevice, st);
     if (rho && e == cudaSuccess) e = cudaMemsetAsync(K->Q.p, 0, K->Q.bytes, st);
     if (K->S.p && e == cudaSuccess) e = cudaEventCreateWithFlags(&K->done, cudaEventDisableTiming);
     if (K->done && e == cudaSuccess) e = cudaEventRecord(K->done, st);
@@ -1331,10 +1377,7 @@ void lattice_release(fem_gpu_ctx* c) {
     }
     Lattice* L = (Lattice*)c->lattice;
     if (!L) return;
-    dfree(L->jac);
-    dfree(L->S);
-    dfree(L->vec);
-    dfree(L->Q);
+    dfree(L->mem);
     if (L->done) cudaEventDestroy(L->done);
     delete L;
     c->lattice = nullptr;
