@@ -409,13 +409,13 @@ fem_gpu_status fem_gpu_element_matrices(fem_gpu_ctx* ctx, int32_t set, int64_t f
 fem_gpu_status fem_gpu_assemble(fem_gpu_ctx* ctx, const double* u_adof, double* csr_vals, double* rhs,
                                 uint32_t flags);
 /* fill_matrix_and_RHS for every equation object of every bulk and
-   double-sided set in ONE persistent launch (uneven clusters: uncut cells,
-   cut clusters of 4 to hundreds of integration points, interface and ghost
-   clusters), work items taken from a device queue in decreasing cost order,
-   clusters above the split size cut into integration-point ranges.  The
-   zero-fill, the queue reset, the persistent kernel and the boundary side
-   sets are one CUDA graph, captured on the first call for a (u, vals, rhs)
-   triple and replayed afterwards.  Device buffers only. */
+   double-sided set in one CUDA graph, captured on the first call for a (u,
+   vals, rhs) triple and the accumulate flag and replayed afterwards: the
+   zero-fill, a kernel per set for its brick cells, clusters and faces, one
+   persistent launch for all others (work items taken from a device queue in
+   decreasing cost order, clusters above the split size cut into
+   integration-point ranges) and the boundary side sets.  Device buffers
+   only. */
 fem_gpu_status fem_gpu_assemble_batched(fem_gpu_ctx* ctx, const double* u_adof, double* csr_vals, double* rhs,
                                         uint32_t flags);
 /* waits for the context's stream and reports a non-finite element operator
