@@ -23,9 +23,9 @@
 // per basis for the projection, 750 operations per node for the stencil.
 //
 // Measured on GB300 against the element loop (whole calls, residual included):
-// 64^3 quadratic 7.75 -> 2.25 ms, 15 x 13 x 11 quadratic 120 -> 82 us, 96^3 density set
+// 64^3 quadratic 7.75 -> 2.25 ms, 15 x 13 x 11 quadratic 120 -> 79 us, 96^3 density set
 // with linear splines 13.4 -> 2.50 ms, matrix-free product of 48 x 47 x 45 quadratic
-// cells 969 -> 80 us.  Small models keep the element loop (lattice_pays).
+// cells 969 -> 76 us.  Small models keep the element loop (lattice_pays).
 //
 // Cells of any shape on the same lattice of nodes (FEM_GPU_SHAPE_GENERAL): the cells
 // add their matrices to the block stencil (fem_hex.cuh), or to the CSR for linear
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kStencilThreads) lattice_const(LatArgs p) {
 // strains are single coefficients, the integral over the cell is V / 3^|n| for every
 // monomial x^n, and the corner forces come back by the transposed sums.  258 FP64
 // operations per cell and 24 coalesced atomics, where the stencil took 750 operations
-// per node: product of 48 x 47 x 45 quadratic cells 210 -> 80 us
+// per node: product of 48 x 47 x 45 quadratic cells 210 -> 76 us
 // (kernel 58, FP64 pipe 69 %).
 __global__ void __launch_bounds__(128) lattice_product(LatArgs p) {
     const unsigned cells = (unsigned)p.ne[0] * p.ne[1] * p.ne[2], e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -822,14 +822,11 @@ __global__ void __launch_bounds__(kProjThreads, kProjCtas) lattice_project(ProjA
 // nodal values of a quadratic spline field: un[g][node] = 1/8 of the sum of its eight bases
 __global__ void lattice_nodal(int n0, int n1, int n2, const double* __restrict__ u, double* un) {
     cudaTriggerProgrammaticLaunchCompletion();
-    const int64_t nodes = (int64_t)n0 * n1 * n2, nu = (int64_t)(n0 + 1) * (n1 + 1) * (n2 + 1);
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nodes;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int g = (int)(t / nodes);
-        const int64_t i = t - g * nodes;
-        const int x = (int)(i % n0), y = (int)(i / n0 % n1), z = (int)(i / ((int64_t)n0 * n1));
-        const double* b = u + g * nu + ((int64_t)z * (n1 + 1) + y) * (n0 + 1) + x;
-        const int64_t sy = n0 + 1, sz = sy * (n1 + 1);
+    const unsigned nodes = (unsigned)n0 * n1 * n2, nu = (unsigned)(n0 + 1) * (n1 + 1) * (n2 + 1);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nodes; t += gridDim.x * blockDim.x) {
+        const unsigned g = (t >= nodes) + (t >= 2 * nodes), i = t - g * nodes, yz = i / n0, z = yz / n1;
+        const unsigned x = i - yz * n0, y = yz - z * n1, sy = n0 + 1, sz = sy * (n1 + 1);
+        const double* b = u + g * nu + (z * (n1 + 1) + y) * sy + x;
         const double lo = (b[0] + b[1]) + (b[sy] + b[sy + 1]);
         const double up = (b[sz] + b[sz + 1]) + (b[sz + sy] + b[sz + sy + 1]);
         un[t] = 0.125 * (lo + up);
@@ -840,17 +837,19 @@ __global__ void lattice_nodal(int n0, int n1, int n2, const double* __restrict__
 __global__ void lattice_restrict(int n0, int n1, int n2, const double* rn, double scale, int acc, double* r) {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
-    const int b0 = n0 + 1, b1 = n1 + 1, b2 = n2 + 1;
-    const int64_t nodes = (int64_t)n0 * n1 * n2, nu = (int64_t)b0 * b1 * b2;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nu; t += (int64_t)gridDim.x * blockDim.x) {
-        const int f = (int)(t / nu);
-        const int64_t i = t - f * nu;
-        const int x = (int)(i % b0), y = (int)(i / b0 % b1), z = (int)(i / ((int64_t)b0 * b1));
+    const unsigned b0 = n0 + 1, b1 = n1 + 1, nodes = (unsigned)n0 * n1 * n2, nu = b0 * b1 * (n2 + 1);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * nu; t += gridDim.x * blockDim.x) {
+        const unsigned f = (t >= nu) + (t >= 2 * nu), i = t - f * nu, yz = i / b0;
+        const int z = (int)(yz / b1), x = (int)(i - yz * b0), y = (int)(yz - z * b1);
+        const double* v = rn + (int64_t)f * nodes + ((int64_t)z * n1 + y) * n0 + x;
         double s = 0.0;
-        for (int k = max(z - 1, 0); k <= min(z, n2 - 1); ++k)
-            for (int j = max(y - 1, 0); j <= min(y, n1 - 1); ++j)
-                for (int l = max(x - 1, 0); l <= min(x, n0 - 1); ++l)
-                    s += rn[f * nodes + ((int64_t)k * n1 + j) * n0 + l];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {  // nodes z - 1, z; y - 1, y; x - 1, x
+            const int dz = (k >> 2) - 1, dy = (k >> 1 & 1) - 1, dx = (k & 1) - 1;
+            const bool in = (unsigned)(z + dz) < (unsigned)n2 && (unsigned)(y + dy) < (unsigned)n1 &&
+                            (unsigned)(x + dx) < (unsigned)n0;
+            s += in ? v[((int64_t)dz * n1 + dy) * n0 + dx] : 0.0;
+        }
         r[t] = acc ? fma(scale, s, r[t]) : scale * s;
     }
 }
