@@ -167,40 +167,60 @@ __global__ void k_advance(CgState* st, int max_iter) {
 // writes, are loaded before the previous one is waited for.
 constexpr int kPairCached = 5;  // entries per lane of a row loaded ahead
 
-struct PairScalars {
-    double rz, rr, pq_prev, rz_prev;
-    int base, done;
-    __device__ PairScalars(const CgState* st, int k)
-        : rz(st->ring[k & 3][1]), rr(st->ring[k & 3][2]), pq_prev(st->ring[(k + 3) & 3][0]),
-          rz_prev(st->ring[(k + 3) & 3][1]), base(st->it), done(st->done) {}
-    // of the iteration before k: 0 go on, 1 converged, 2 breakdown (NaN or p.Ap == 0), 3 limit
-    __device__ int test(double thresh2, int k, int max_iter) const {
-        if (base + k == 0) return 0;  // k_set_thresh has tested the start
-        if (rr <= thresh2) return 1;
-        if (!(rz == rz) || pq_prev == 0.0) return 2;
-        return base + k >= max_iter ? 3 : 0;
-    }
+// Sums p.Ap, r.z and r.r of four iterations, in eight parts each: an FP64 atomic of
+// every block to one address takes 10 ns, 1.3 us for a product.  One warp adds the
+// parts and divides, for the block (in every warp the division alone was 2,000 cycles
+// of the FP64 pipe), while the others load what the vectors' updates need.
+constexpr int kParts = 8;
+struct PairSums {
+    double v[4][3][kParts];
 };
+__device__ __forceinline__ double* pair_part(PairSums* s, int slot, int kind) {
+    return &s->v[slot][kind][blockIdx.x % kParts];
+}
+// of the iteration before k: 0 go on, 1 converged, 2 breakdown (NaN or p.Ap == 0), 3 limit
+__device__ __forceinline__ int pair_test(const CgState* st, double rz, double rr, double pq, int it, int max_iter) {
+    if (it == 0) return 0;  // k_set_thresh has tested the start
+    if (rr <= st->thresh2) return 1;
+    if (!(rz == rz) || pq == 0.0) return 2;
+    return it >= max_iter ? 3 : 0;
+}
 // by one thread; st->it stays until the chunk's end, other blocks still read it
-__device__ __forceinline__ void pair_record(CgState* st, int it, int state) {
+__device__ __forceinline__ void pair_record(CgState* st, int it, int state, double rr) {
     if (state == 1) st->converged_at = it;
+    st->ring[it & 3][2] = rr;
     st->stopped_at = it;
     st->done = state;
+}
+// totals of four sums by one warp: eight lanes each
+__device__ __forceinline__ double pair_total(const double* part) {
+    double t = *part;
+#pragma unroll
+    for (int o = kParts / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+__global__ void k_pair_begin(const CgState* st, PairSums* s) {
+    s->v[0][1][0] = st->ring[0][1];
+    s->v[0][2][0] = st->ring[0][2];
 }
 
 __global__ void __launch_bounds__(kThreads) k_pair_product(int n, const int32_t* __restrict__ rp,
                                                            const int32_t* __restrict__ ci,
                                                            const double* __restrict__ v, const double* z, double* pa,
-                                                           double* pb, double* q, CgState* st, int k, int max_iter) {
+                                                           double* pb, double* q, CgState* st, PairSums* sums, int k,
+                                                           int max_iter) {
     constexpr int L = fem::kLanesPerRow;
-    const int sub = threadIdx.x % L, row = (blockIdx.x * kThreads + threadIdx.x) / L;
+    __shared__ double sbeta;
+    __shared__ int stop;
+    const int sub = threadIdx.x % L, row = (blockIdx.x * kThreads + threadIdx.x) / L, lane = threadIdx.x & 31;
     int j = 0, e = 0;
     if (row < n) {
         j = rp[row] + sub;
         e = rp[row + 1];
     }
     int32_t cc[kPairCached];
-    double cv[kPairCached];
+    double cv[kPairCached], zc[kPairCached], pc[kPairCached];
 #pragma unroll
     for (int m = 0; m < kPairCached; ++m) {
         const bool in = j + m * L < e;
@@ -209,21 +229,35 @@ __global__ void __launch_bounds__(kThreads) k_pair_product(int n, const int32_t*
     }
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
-    const PairScalars s(st, k);
     const double* po = k & 1 ? pb : pa;
     double* pn = k & 1 ? pa : pb;
-    if (s.done) return;
-    const int state = s.test(st->thresh2, k, max_iter);
-    if (state) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) pair_record(st, s.base + k, state);
-        return;
+#pragma unroll
+    for (int m = 0; m < kPairCached; ++m) {
+        zc[m] = cc[m] >= 0 ? z[cc[m]] : 0.0;
+        pc[m] = cc[m] >= 0 ? po[cc[m]] : 0.0;
     }
-    const double beta = s.base + k ? s.rz / s.rz_prev : 0.0;
-    double dot = 0.0, pq = 0.0, a[kPairCached];
+    const bool own = sub == 0 && row < n;
+    const double zr = own ? z[row] : 0.0, pr = own ? po[row] : 0.0;
+    if (threadIdx.x < 32) {
+        // r.z, r.r, and p.Ap, r.z of the iteration before
+        const int what = lane / kParts, slot = what < 2 ? k & 3 : (k + 3) & 3;
+        const double t = pair_total(&sums->v[slot][what == 1 ? 2 : what == 2 ? 0 : 1][lane % kParts]);
+        const double rz = __shfl_sync(0xffffffffu, t, 0), rr = __shfl_sync(0xffffffffu, t, kParts),
+                     pq = __shfl_sync(0xffffffffu, t, 2 * kParts), old = __shfl_sync(0xffffffffu, t, 3 * kParts);
+        if (lane == 0) {
+            const int it = st->it + k, done = st->done;
+            const int state = done ? done : pair_test(st, rz, rr, pq, it, max_iter);
+            if (blockIdx.x == 0 && !done && state) pair_record(st, it, state, rr);
+            stop = state;
+            sbeta = it ? rz / old : 0.0;
+        }
+    }
+    __syncthreads();
+    if (stop) return;
+    const double beta = sbeta;
+    double dot = 0.0, pq = 0.0;
 #pragma unroll
-    for (int m = 0; m < kPairCached; ++m) a[m] = cc[m] >= 0 ? fma(beta, po[cc[m]], z[cc[m]]) : 0.0;
-#pragma unroll
-    for (int m = 0; m < kPairCached; ++m) dot = fma(cv[m], a[m], dot);
+    for (int m = 0; m < kPairCached; ++m) dot = fma(cv[m], fma(beta, pc[m], zc[m]), dot);
 #pragma unroll 4
     for (j += kPairCached * L; j < e; j += L) {
         const int c = ci[j];
@@ -231,48 +265,67 @@ __global__ void __launch_bounds__(kThreads) k_pair_product(int n, const int32_t*
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    if (sub == 0 && row < n) {
-        const double p = fma(beta, po[row], z[row]);
+    if (own) {
+        const double p = fma(beta, pr, zr);
         pn[row] = p;
         q[row] = dot;
         pq = dot * p;
     }
     const double sum[1] = {pq};
-    fem::block_sum_add<kThreads, L, 1>(sum, {&st->ring[k & 3][0]});
-    if (blockIdx.x == 0 && threadIdx.x < 4) st->ring[(k + 2) & 3][threadIdx.x] = 0.0;
+    fem::block_sum_add<kThreads, L, 1>(sum, {pair_part(sums, k & 3, 0)});
+    if (blockIdx.x == 0 && threadIdx.x < 3 * kParts) (&sums->v[(k + 2) & 3][0][0])[threadIdx.x] = 0.0;
 }
 
 constexpr int kPairThreads = 128;  // of the update: a small system spreads over more SMs
 __global__ void __launch_bounds__(kPairThreads) k_pair_update(int n, double* x, double* r, double* z,
                                                               const double* pa, const double* pb, const double* q,
-                                                              const double* dinv, CgState* st, int k) {
+                                                              const double* dinv, CgState* st, PairSums* sums, int k) {
+    __shared__ double salpha;
+    __shared__ int stop;
+    const int i = blockIdx.x * kPairThreads + threadIdx.x, lane = threadIdx.x & 31, at = i < n ? i : 0;
+    const double di = dinv[at];
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
-    if (st->done) return;
-    const int nxt = (k + 1) & 3;
     const double* p = k & 1 ? pa : pb;
-    const double alpha = st->ring[k & 3][1] / st->ring[k & 3][0];
+    const double xi = x[at], pi = p[at], qi = q[at];
+    double ri = r[at];
+    if (threadIdx.x < 32) {
+        const double t = pair_total(&sums->v[k & 3][lane < kParts ? 1 : 0][lane % kParts]);
+        const double rz = __shfl_sync(0xffffffffu, t, 0), pq = __shfl_sync(0xffffffffu, t, kParts);
+        if (lane == 0) {
+            stop = st->done;
+            salpha = rz / pq;
+        }
+    }
+    __syncthreads();
+    if (stop) return;
+    const double alpha = salpha;
     double sum[2] = {0.0, 0.0};
-    const int i = blockIdx.x * kPairThreads + threadIdx.x;
     if (i < n) {
-        x[i] = fma(alpha, p[i], x[i]);
-        const double ri = fma(-alpha, q[i], r[i]);
+        x[i] = fma(alpha, pi, xi);
+        ri = fma(-alpha, qi, ri);
         r[i] = ri;
-        const double zi = dinv[i] * ri;
+        const double zi = di * ri;
         z[i] = zi;
         sum[0] = ri * zi;
         sum[1] = ri * ri;
     }
-    fem::block_sum_add<kPairThreads, 1, 2>(sum, {&st->ring[nxt][1], &st->ring[nxt][2]});
+    const int nxt = (k + 1) & 3;
+    fem::block_sum_add<kPairThreads, 1, 2>(sum, {pair_part(sums, nxt, 1), pair_part(sums, nxt, 2)});
 }
 
 // end of a chunk: its last iteration's test, and the next chunk's base
-__global__ void k_pair_end(CgState* st, int chunk, int max_iter) {
-    const PairScalars s(st, chunk);
-    if (!s.done) {
-        const int state = s.test(st->thresh2, chunk, max_iter);
-        st->it = s.base + chunk;
-        if (state) pair_record(st, s.base + chunk, state);
+__global__ void k_pair_end(CgState* st, const PairSums* sums, int chunk, int max_iter) {
+    if (!st->done) {
+        double rz = 0.0, rr = 0.0, pq = 0.0;
+        for (int m = 0; m < kParts; ++m) {
+            rz += sums->v[chunk & 3][1][m];
+            rr += sums->v[chunk & 3][2][m];
+            pq += sums->v[(chunk + 3) & 3][0][m];
+        }
+        const int it = st->it + chunk, state = pair_test(st, rz, rr, pq, it, max_iter);
+        st->it = it;
+        if (state) pair_record(st, it, state, rr);
     } else {
         st->it = st->stopped_at;
     }
@@ -287,8 +340,8 @@ __global__ void k_pair_end(CgState* st, int chunk, int max_iter) {
 // SMs: no launch and no trip to the L2.  Every CTA takes the same decisions from the
 // same sums, so all leave the loop together.
 // Microseconds per iteration, two launches -> here: plane systems of 578 rows 10.7 ->
-// 6.2, 2,178 rows 8.8 -> 6.0, 5,000 rows 8.4 -> 7.0, 8,450 rows 9.4 -> 9.3 to 9.9 (not
-// used); solids of 1,029 rows 13.7 -> 10.0, 3,000 rows 13.4 -> 10.3.
+// 6.2, 2,178 rows 8.8 -> 6.0, 5,000 rows 7.6 -> 7.0, 8,450 rows 8.1 -> 9.3 to 9.9 (not
+// used); solids of 1,029 rows 13.7 -> 10.0, 3,000 rows 12.0 -> 10.3.
 constexpr int kClusterCtas = 16, kClusterRows = 320;  // rows per CTA at most
 constexpr int kClusterChunk = 2048;                   // iterations per launch
 struct ClusterShape {
@@ -442,10 +495,10 @@ __global__ void __launch_bounds__(kClusterRows) k_cluster_cg(int n, int W, const
 
 // Two launches where every lane group has one row and every SM at most one block
 // of the product (9,728 rows on GB300).  Microseconds per iteration, four launches ->
-// two: plane systems of 578 rows 18.3 -> 11.0, 2,178 rows 14.7 -> 9.2, 8,450 rows
-// 14.7 -> 9.7; solids of 1,029 rows 18.8 -> 13.7, 6,591 rows 17.5 -> 13.1.  Past the
-// line the second gather costs more than the launches: 13,122 rows 15.0 -> 14.1,
-// 18,818 rows 15.0 -> 15.1, 132,098 rows 33 -> 39, solid of 14,739 rows 18.5 -> 49.
+// two: plane systems of 5,618 rows 14.7 -> 7.6, 8,450 rows 14.7 -> 8.1; solids of 6,591
+// rows 17.5 -> 11.7.  Past the line the second gather costs more than the launches:
+// without the line 18,818 rows 15.0 -> 15.1, 132,098 rows 33 -> 39, solid of 14,739
+// rows 18.5 -> 49.
 bool pair_system(int64_t n) { return n * fem::kLanesPerRow <= (int64_t)fem::sm_count() * kThreads; }
 
 __global__ void k_set_thresh(CgState* st, double rtol) {
@@ -520,7 +573,7 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     const auto t0 = std::chrono::steady_clock::now();
     double *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *dinv = nullptr;
     CgState* st = nullptr;
-    cudaError_t e = cudaMallocAsync(&r, 6 * n * sizeof(double), sm);
+    cudaError_t e = cudaMallocAsync(&r, 6 * n * sizeof(double) + sizeof(PairSums), sm);
     if (e == cudaSuccess) e = cudaMallocAsync(&st, sizeof(CgState), sm);
     if (e != cudaSuccess) return fail(c, FEM_GPU_OUT_OF_MEMORY, "pcg workspace");
     z = r + n;
@@ -543,6 +596,7 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, st);
     k_set_thresh<<<1, 1, 0, sm>>>(st, opts->rel_tol);
     c->launches += 3;
+    PairSums* sums = (PairSums*)(dinv + 2 * n);
     CgState hs{};
     const auto read_state = [&] {
         e = cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, sm);
@@ -557,6 +611,11 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
         } while (e == cudaSuccess && read_state() && !hs.wide);
     // a matrix with longer rows than the model's graph takes the launches
     const bool launches = !clustered || (hs.wide && !hs.done);
+    if (pair && launches && e == cudaSuccess) {
+        e = cudaMemsetAsync(sums, 0, sizeof(PairSums), sm);
+        k_pair_begin<<<1, 1, 0, sm>>>(st, sums);
+        c->launches++;
+    }
     // capture a chunk of iterations into a graph
     const int chunk = 32;
     cudaGraph_t graph = nullptr;
@@ -565,13 +624,13 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     if (e == cudaSuccess && launches) {
         for (int k = 0; k < chunk && pair; ++k) {
             e = launch_kernel(k_pair_product, row_blocks, tpb, 0, sm, true, n, rowptr, colidx, vals, z, p, dinv + n, q,
-                              st, k, opts->max_iter);
+                              st, sums, k, opts->max_iter);
             if (e == cudaSuccess)
                 e = launch_kernel(k_pair_update, upd_blocks, kPairThreads, 0, sm, true, n, x, r, z, p, dinv + n, q,
-                                  dinv, st, k);
+                                  dinv, st, sums, k);
             if (e != cudaSuccess) break;
         }
-        if (pair) k_pair_end<<<1, 1, 0, sm>>>(st, chunk, opts->max_iter);
+        if (pair) k_pair_end<<<1, 1, 0, sm>>>(st, sums, chunk, opts->max_iter);
         for (int k = 0; k < chunk && !pair; ++k) {
             k_spmv_pq<<<spmv_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, p, q, st);
             k_update_xr<<<vec_blocks, tpb, 0, sm>>>(n, x, r, z, p, q, dinv, st);
