@@ -31,6 +31,7 @@
 
 namespace {
 
+constexpr int kParts = 8;
 struct CgState {
     int it;          // current iteration
     int done;        // 1 converged, 2 breakdown
@@ -41,10 +42,39 @@ struct CgState {
     double bn2;
     // ring of per-iteration scalars: [slot][0]=pq, [1]=rz, [2]=rr
     double ring[4][4];
+    // the sums p.Ap, r.z and r.r of four iterations, each in parts: an FP64 atomic of
+    // every block to one address takes 10 ns, 24 us for the blocks of a large product.
+    // Per iteration, one address -> parts: plane systems of 132,098 rows 27.0 -> 23.0 us,
+    // 526,338 rows 67 -> 59; solids of 107,811 rows 40.1 -> 37.4, 823,875 rows 210 -> 197.
+    double part[4][3][kParts];
 };
 
 // threads per block of every kernel that sums
 constexpr int kThreads = 256;
+
+__device__ __forceinline__ double* part_of(CgState* st, int slot, int kind) {
+    return &st->part[slot][kind][blockIdx.x % kParts];
+}
+// Totals of up to four sums by one warp, eight lanes each.  It also divides, for the
+// block: in every warp the division alone was 2,000 cycles of the FP64 pipe.
+__device__ __forceinline__ double sum_parts(const double* part) {
+    double t = *part;
+#pragma unroll
+    for (int o = kParts / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+// to all threads of the block: num / den of two sums (slot, kind), by its first warp
+__device__ __forceinline__ double block_quotient(const CgState* st, int ns, int nk, int ds, int dk) {
+    __shared__ double ratio;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        const double t = sum_parts(lane < kParts ? &st->part[ns][nk][lane] : &st->part[ds][dk][lane % kParts]);
+        const double den = __shfl_sync(0xffffffffu, t, kParts);
+        if (lane == 0) ratio = t / den;
+    }
+    __syncthreads();
+    return ratio;
+}
 
 __global__ void k_diag_inv(int64_t n, const int32_t* rp, const int32_t* ci, const double* v, double* dinv,
                            int jacobi, int limit, CgState* st) {
@@ -68,7 +98,7 @@ __global__ void k_diag_inv(int64_t n, const int32_t* rp, const int32_t* ci, cons
     dinv[i] = d;
 }
 
-// r = b - A x ; z = M^-1 r ; p = z ; accumulate r.z, r.r, b.b into slot 0
+// r = b - A x ; z = M^-1 r ; p = z ; accumulate r.z, r.r into slot 0, b.b into slot 3
 __global__ void k_init(int64_t n, const int32_t* rp, const int32_t* ci, const double* v, const double* b,
                        const double* x, double* r, double* z, double* p, const double* dinv, CgState* st) {
     const int sub = threadIdx.x % fem::kLanesPerRow;
@@ -84,7 +114,7 @@ __global__ void k_init(int64_t n, const int32_t* rp, const int32_t* ci, const do
         sum[1] = ri * ri;
         sum[2] = b[row] * b[row];
     }
-    fem::block_sum_add<kThreads, fem::kLanesPerRow, 3>(sum, {&st->ring[0][1], &st->ring[0][2], &st->bn2});
+    fem::block_sum_add<kThreads, fem::kLanesPerRow, 3>(sum, {part_of(st, 0, 1), part_of(st, 0, 2), part_of(st, 3, 2)});
 }
 
 // q = A p (warp per row, grid-stride over rows so that each block adds its
@@ -108,14 +138,14 @@ __global__ void k_spmv_pq(int64_t n, const int32_t* rp, const int32_t* ci, const
         }
     }
     const double sum[1] = {pq};
-    fem::block_sum_add<kThreads, fem::kLanesPerRow, 1>(sum, {&st->ring[slot][0]});
+    fem::block_sum_add<kThreads, fem::kLanesPerRow, 1>(sum, {part_of(st, slot, 0)});
 }
 
 __global__ void k_update_xr(int64_t n, double* x, double* r, double* z, const double* p, const double* q,
                             const double* dinv, CgState* st) {
     if (st->done) return;
     const int slot = st->it & 3, nxt = (st->it + 1) & 3;
-    const double alpha = st->ring[slot][1] / st->ring[slot][0];
+    const double alpha = block_quotient(st, slot, 1, slot, 0);
     double rz = 0.0, rr = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         x[i] = fma(alpha, p[i], x[i]);
@@ -127,32 +157,39 @@ __global__ void k_update_xr(int64_t n, double* x, double* r, double* z, const do
         rr = fma(ri, ri, rr);
     }
     const double sum[2] = {rz, rr};
-    fem::block_sum_add<kThreads, 1, 2>(sum, {&st->ring[nxt][1], &st->ring[nxt][2]});
+    fem::block_sum_add<kThreads, 1, 2>(sum, {part_of(st, nxt, 1), part_of(st, nxt, 2)});
 }
 
 __global__ void k_update_p(int64_t n, double* p, const double* z, CgState* st) {
     if (st->done) return;
     const int slot = st->it & 3, nxt = (st->it + 1) & 3;
-    if (st->ring[nxt][2] <= st->thresh2) return;  // k4 records convergence
-    const double beta = st->ring[nxt][1] / st->ring[slot][1];
+    const double beta = block_quotient(st, nxt, 1, slot, 1);  // (of no use once k4 records convergence)
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         p[i] = fma(beta, p[i], z[i]);
 }
 
+// (one warp)
 __global__ void k_advance(CgState* st, int max_iter) {
     if (st->done) return;
-    const int slot = st->it & 3, nxt = (st->it + 1) & 3, nn = (st->it + 2) & 3;
-    st->it += 1;
-    if (st->ring[nxt][2] <= st->thresh2) {
-        st->done = 1;
-        st->converged_at = st->it;
-    } else if (!(st->ring[nxt][1] == st->ring[nxt][1]) || st->ring[slot][0] == 0.0) {
-        st->done = 2;  // breakdown (NaN or p.Ap == 0)
-    } else if (st->it >= max_iter) {
-        st->done = 3;
+    const int it = st->it, slot = it & 3, nxt = (it + 1) & 3, nn = (it + 2) & 3, lane = threadIdx.x;
+    const int what = lane / kParts;  // r.z, r.r of the next iteration, p.Ap
+    const double t = sum_parts(&st->part[what == 2 ? slot : nxt][what == 0 ? 1 : what == 1 ? 2 : 0][lane % kParts]);
+    const double rz = __shfl_sync(0xffffffffu, t, 0), rr = __shfl_sync(0xffffffffu, t, kParts),
+                 pq = __shfl_sync(0xffffffffu, t, 2 * kParts);
+    if (lane < 3 * kParts) (&st->part[nn][0][0])[lane] = 0.0;
+    if (lane == 0) {
+        st->it = it + 1;
+        st->ring[nxt][1] = rz;
+        st->ring[nxt][2] = rr;
+        if (rr <= st->thresh2) {
+            st->done = 1;
+            st->converged_at = it + 1;
+        } else if (!(rz == rz) || pq == 0.0) {
+            st->done = 2;  // breakdown (NaN or p.Ap == 0)
+        } else if (it + 1 >= max_iter) {
+            st->done = 3;
+        }
     }
-    for (int k = 0; k < 4; ++k) st->ring[nn][k] = 0.0;
-    (void)slot;
 }
 
 // Two launches per iteration.  The direction p = z + beta p is formed where the
@@ -167,17 +204,6 @@ __global__ void k_advance(CgState* st, int max_iter) {
 // writes, are loaded before the previous one is waited for.
 constexpr int kPairCached = 5;  // entries per lane of a row loaded ahead
 
-// Sums p.Ap, r.z and r.r of four iterations, in eight parts each: an FP64 atomic of
-// every block to one address takes 10 ns, 1.3 us for a product.  One warp adds the
-// parts and divides, for the block (in every warp the division alone was 2,000 cycles
-// of the FP64 pipe), while the others load what the vectors' updates need.
-constexpr int kParts = 8;
-struct PairSums {
-    double v[4][3][kParts];
-};
-__device__ __forceinline__ double* pair_part(PairSums* s, int slot, int kind) {
-    return &s->v[slot][kind][blockIdx.x % kParts];
-}
 // of the iteration before k: 0 go on, 1 converged, 2 breakdown (NaN or p.Ap == 0), 3 limit
 __device__ __forceinline__ int pair_test(const CgState* st, double rz, double rr, double pq, int it, int max_iter) {
     if (it == 0) return 0;  // k_set_thresh has tested the start
@@ -192,23 +218,10 @@ __device__ __forceinline__ void pair_record(CgState* st, int it, int state, doub
     st->stopped_at = it;
     st->done = state;
 }
-// totals of four sums by one warp: eight lanes each
-__device__ __forceinline__ double pair_total(const double* part) {
-    double t = *part;
-#pragma unroll
-    for (int o = kParts / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    return t;
-}
-
-__global__ void k_pair_begin(const CgState* st, PairSums* s) {
-    s->v[0][1][0] = st->ring[0][1];
-    s->v[0][2][0] = st->ring[0][2];
-}
-
 __global__ void __launch_bounds__(kThreads) k_pair_product(int n, const int32_t* __restrict__ rp,
                                                            const int32_t* __restrict__ ci,
                                                            const double* __restrict__ v, const double* z, double* pa,
-                                                           double* pb, double* q, CgState* st, PairSums* sums, int k,
+                                                           double* pb, double* q, CgState* st, int k,
                                                            int max_iter) {
     constexpr int L = fem::kLanesPerRow;
     __shared__ double sbeta;
@@ -241,7 +254,7 @@ __global__ void __launch_bounds__(kThreads) k_pair_product(int n, const int32_t*
     if (threadIdx.x < 32) {
         // r.z, r.r, and p.Ap, r.z of the iteration before
         const int what = lane / kParts, slot = what < 2 ? k & 3 : (k + 3) & 3;
-        const double t = pair_total(&sums->v[slot][what == 1 ? 2 : what == 2 ? 0 : 1][lane % kParts]);
+        const double t = sum_parts(&st->part[slot][what == 1 ? 2 : what == 2 ? 0 : 1][lane % kParts]);
         const double rz = __shfl_sync(0xffffffffu, t, 0), rr = __shfl_sync(0xffffffffu, t, kParts),
                      pq = __shfl_sync(0xffffffffu, t, 2 * kParts), old = __shfl_sync(0xffffffffu, t, 3 * kParts);
         if (lane == 0) {
@@ -272,14 +285,14 @@ __global__ void __launch_bounds__(kThreads) k_pair_product(int n, const int32_t*
         pq = dot * p;
     }
     const double sum[1] = {pq};
-    fem::block_sum_add<kThreads, L, 1>(sum, {pair_part(sums, k & 3, 0)});
-    if (blockIdx.x == 0 && threadIdx.x < 3 * kParts) (&sums->v[(k + 2) & 3][0][0])[threadIdx.x] = 0.0;
+    fem::block_sum_add<kThreads, L, 1>(sum, {part_of(st, k & 3, 0)});
+    if (blockIdx.x == 0 && threadIdx.x < 3 * kParts) (&st->part[(k + 2) & 3][0][0])[threadIdx.x] = 0.0;
 }
 
 constexpr int kPairThreads = 128;  // of the update: a small system spreads over more SMs
 __global__ void __launch_bounds__(kPairThreads) k_pair_update(int n, double* x, double* r, double* z,
                                                               const double* pa, const double* pb, const double* q,
-                                                              const double* dinv, CgState* st, PairSums* sums, int k) {
+                                                              const double* dinv, CgState* st, int k) {
     __shared__ double salpha;
     __shared__ int stop;
     const int i = blockIdx.x * kPairThreads + threadIdx.x, lane = threadIdx.x & 31, at = i < n ? i : 0;
@@ -290,7 +303,7 @@ __global__ void __launch_bounds__(kPairThreads) k_pair_update(int n, double* x, 
     const double xi = x[at], pi = p[at], qi = q[at];
     double ri = r[at];
     if (threadIdx.x < 32) {
-        const double t = pair_total(&sums->v[k & 3][lane < kParts ? 1 : 0][lane % kParts]);
+        const double t = sum_parts(&st->part[k & 3][lane < kParts ? 1 : 0][lane % kParts]);
         const double rz = __shfl_sync(0xffffffffu, t, 0), pq = __shfl_sync(0xffffffffu, t, kParts);
         if (lane == 0) {
             stop = st->done;
@@ -311,17 +324,17 @@ __global__ void __launch_bounds__(kPairThreads) k_pair_update(int n, double* x, 
         sum[1] = ri * ri;
     }
     const int nxt = (k + 1) & 3;
-    fem::block_sum_add<kPairThreads, 1, 2>(sum, {pair_part(sums, nxt, 1), pair_part(sums, nxt, 2)});
+    fem::block_sum_add<kPairThreads, 1, 2>(sum, {part_of(st, nxt, 1), part_of(st, nxt, 2)});
 }
 
 // end of a chunk: its last iteration's test, and the next chunk's base
-__global__ void k_pair_end(CgState* st, const PairSums* sums, int chunk, int max_iter) {
+__global__ void k_pair_end(CgState* st, int chunk, int max_iter) {
     if (!st->done) {
         double rz = 0.0, rr = 0.0, pq = 0.0;
         for (int m = 0; m < kParts; ++m) {
-            rz += sums->v[chunk & 3][1][m];
-            rr += sums->v[chunk & 3][2][m];
-            pq += sums->v[(chunk + 3) & 3][0][m];
+            rz += st->part[chunk & 3][1][m];
+            rr += st->part[chunk & 3][2][m];
+            pq += st->part[(chunk + 3) & 3][0][m];
         }
         const int it = st->it + chunk, state = pair_test(st, rz, rr, pq, it, max_iter);
         st->it = it;
@@ -502,10 +515,18 @@ __global__ void __launch_bounds__(kClusterRows) k_cluster_cg(int n, int W, const
 bool pair_system(int64_t n) { return n * fem::kLanesPerRow <= (int64_t)fem::sm_count() * kThreads; }
 
 __global__ void k_set_thresh(CgState* st, double rtol) {
-    const double bn2 = st->bn2 > 0.0 ? st->bn2 : 1.0;
+    double rz = 0.0, rr = 0.0, bb = 0.0;
+    for (int k = 0; k < kParts; ++k) {
+        rz += st->part[0][1][k];
+        rr += st->part[0][2][k];
+        bb += st->part[3][2][k];  // b.b of k_init; iteration 1 clears the slot
+    }
+    const double bn2 = bb > 0.0 ? bb : 1.0;
     st->bn2 = bn2;
     st->thresh2 = rtol * rtol * bn2;
-    if (st->ring[0][2] <= st->thresh2) {
+    st->ring[0][1] = rz;
+    st->ring[0][2] = rr;
+    if (rr <= st->thresh2) {
         st->done = 1;
         st->converged_at = 0;
     }
@@ -573,7 +594,7 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     const auto t0 = std::chrono::steady_clock::now();
     double *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *dinv = nullptr;
     CgState* st = nullptr;
-    cudaError_t e = cudaMallocAsync(&r, 6 * n * sizeof(double) + sizeof(PairSums), sm);
+    cudaError_t e = cudaMallocAsync(&r, 6 * n * sizeof(double), sm);
     if (e == cudaSuccess) e = cudaMallocAsync(&st, sizeof(CgState), sm);
     if (e != cudaSuccess) return fail(c, FEM_GPU_OUT_OF_MEMORY, "pcg workspace");
     z = r + n;
@@ -596,7 +617,6 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     k_init<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, b, x, r, z, p, dinv, st);
     k_set_thresh<<<1, 1, 0, sm>>>(st, opts->rel_tol);
     c->launches += 3;
-    PairSums* sums = (PairSums*)(dinv + 2 * n);
     CgState hs{};
     const auto read_state = [&] {
         e = cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, sm);
@@ -611,11 +631,6 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
         } while (e == cudaSuccess && read_state() && !hs.wide);
     // a matrix with longer rows than the model's graph takes the launches
     const bool launches = !clustered || (hs.wide && !hs.done);
-    if (pair && launches && e == cudaSuccess) {
-        e = cudaMemsetAsync(sums, 0, sizeof(PairSums), sm);
-        k_pair_begin<<<1, 1, 0, sm>>>(st, sums);
-        c->launches++;
-    }
     // capture a chunk of iterations into a graph
     const int chunk = 32;
     cudaGraph_t graph = nullptr;
@@ -624,18 +639,18 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     if (e == cudaSuccess && launches) {
         for (int k = 0; k < chunk && pair; ++k) {
             e = launch_kernel(k_pair_product, row_blocks, tpb, 0, sm, true, n, rowptr, colidx, vals, z, p, dinv + n, q,
-                              st, sums, k, opts->max_iter);
+                              st, k, opts->max_iter);
             if (e == cudaSuccess)
                 e = launch_kernel(k_pair_update, upd_blocks, kPairThreads, 0, sm, true, n, x, r, z, p, dinv + n, q,
-                                  dinv, st, sums, k);
+                                  dinv, st, k);
             if (e != cudaSuccess) break;
         }
-        if (pair) k_pair_end<<<1, 1, 0, sm>>>(st, sums, chunk, opts->max_iter);
+        if (pair) k_pair_end<<<1, 1, 0, sm>>>(st, chunk, opts->max_iter);
         for (int k = 0; k < chunk && !pair; ++k) {
             k_spmv_pq<<<spmv_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, p, q, st);
             k_update_xr<<<vec_blocks, tpb, 0, sm>>>(n, x, r, z, p, q, dinv, st);
             k_update_p<<<vec_blocks, tpb, 0, sm>>>(n, p, z, st);
-            k_advance<<<1, 1, 0, sm>>>(st, opts->max_iter);
+            k_advance<<<1, 32, 0, sm>>>(st, opts->max_iter);
         }
         const cudaError_t ended = cudaStreamEndCapture(sm, &graph);
         if (e == cudaSuccess) e = ended;
@@ -680,7 +695,7 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
 // any allocating library call) after start-up.  For them the Jacobi-PCG work
 // vectors live in one file-scope device array of fixed size instead of
 // stream-ordered allocations, and the iterations are launched directly (no
-// graph instantiation).  The array holds the solver state (first 256 bytes)
+// graph instantiation).  The array holds the solver state (first 1,024 bytes)
 // and the five work vectors r, z, p, q and 1/diag(A), so systems up to
 // kNoAllocMaxRows rows are accepted; larger ones are rejected with
 // FEM_GPU_BAD_ARG.  Every GPU that loads the library keeps this array
@@ -692,7 +707,7 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
 namespace {
 
 constexpr int64_t kNoAllocMaxRows = 131072;
-constexpr int64_t kNoAllocStateDoubles = 32;  // 256 bytes for CgState
+constexpr int64_t kNoAllocStateDoubles = 128;  // 1,024 bytes for CgState
 static_assert(sizeof(CgState) <= kNoAllocStateDoubles * sizeof(double), "CgState fits the state slot");
 
 static __device__ __align__(256) double g_pcg_noalloc_scratch[kNoAllocStateDoubles + 5 * kNoAllocMaxRows];
@@ -785,7 +800,7 @@ extern "C" fem_gpu_status fem_gpu_pcg_noalloc(fem_gpu_ctx* c, const int32_t* row
             k_spmv_pq<<<row_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, p, q, cs);
             k_update_xr<<<vec_blocks, tpb, 0, sm>>>(n, x, r, z, p, q, dinv, cs);
             k_update_p<<<vec_blocks, tpb, 0, sm>>>(n, p, z, cs);
-            k_advance<<<1, 1, 0, sm>>>(cs, opts->max_iter);
+            k_advance<<<1, 32, 0, sm>>>(cs, opts->max_iter);
         }
         c->launches += 4 * chunk;
         e = cudaGetLastError();
@@ -850,7 +865,7 @@ extern "C" fem_gpu_status fem_gpu_pcg_snapshots(fem_gpu_ctx* c, const int32_t* r
             k_spmv_pq<<<spmv_blocks, tpb, 0, sm>>>(n, rowptr, colidx, vals, p, q, st);
             k_update_xr<<<vec_blocks, tpb, 0, sm>>>(n, x, r, z, p, q, dinv, st);
             k_update_p<<<vec_blocks, tpb, 0, sm>>>(n, p, z, st);
-            k_advance<<<1, 1, 0, sm>>>(st, opts->max_iter);
+            k_advance<<<1, 32, 0, sm>>>(st, opts->max_iter);
         }
         c->launches += 4 * every;
         e = cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, sm);
