@@ -743,7 +743,7 @@ __global__ void fcg_spmv_dot(int64_t n, const int32_t* rp, const int32_t* ci, co
         }
     }
     const double sum[1] = {acc};
-    fem::block_sum_add<kFcgThreads, fem::kLanesPerRow, 1>(sum, {dot});
+    fem::block_sum_add<kFcgThreads, fem::kLanesPerRow, 1>(sum, {fem::part_of(dot)});
 }
 
 
@@ -801,11 +801,11 @@ __global__ void fcg_residual(int64_t n, const int32_t* rp, const int32_t* ci, co
         }
     }
     const double sum[2] = {rr, bb};
-    fem::block_sum_add<kFcgThreads, fem::kLanesPerRow, 2>(sum, {dots, dots + 1});
+    fem::block_sum_add<kFcgThreads, fem::kLanesPerRow, 2>(sum, {fem::part_of(dots), fem::part_of(dots + fem::kSumParts)});
 }
 
 constexpr int kMaxM = 16;
-constexpr int kFcgSums = kMaxM + 3;
+constexpr int kFcgSums = kMaxM + 3, kP = fem::kSumParts;  // sums, each in parts
 struct VecSet {
     const double* v[kMaxM];
 };
@@ -813,7 +813,7 @@ struct Coef {
     double c[kMaxM];
 };
 
-// dots[j] += z . q_j for j < m
+// dots[j] += z . q_j for j < m (in parts)
 __global__ void fcg_multi_dot(int64_t n, const double* z, VecSet q, int m, double* dots) {
     double acc[kMaxM];
     for (int j = 0; j < kMaxM; ++j) acc[j] = 0.0;
@@ -824,15 +824,21 @@ __global__ void fcg_multi_dot(int64_t n, const double* z, VecSet q, int m, doubl
     for (int j = 0; j < m; ++j) {
         const double sum[1] = {acc[j]};
         if (j) __syncthreads();
-        fem::block_sum_add<kFcgThreads, 1, 1>(sum, {dots + j});
+        fem::block_sum_add<kFcgThreads, 1, 1>(sum, {fem::part_of(dots + j * kP)});
     }
 }
 // p = z - sum_j (dots[j] / pq of direction j) p_j; pr += p.r
 __global__ void fcg_orthogonalize(int64_t n, const double* z, VecSet pj, Coef pq, int m, const double* dots,
                                   const double* r, double* p, double* pr_out) {
     double pr = 0.0;
-    double c[kMaxM];
-    for (int j = 0; j < m; ++j) c[j] = dots[j] / pq.c[j];
+    // one warp divides for the block
+    __shared__ double c[kMaxM];
+    if (threadIdx.x < 32)
+        for (int j = 0; j < m; ++j) {
+            const double t = fem::parts_total(dots + j * kP);
+            if (threadIdx.x == 0) c[j] = t / pq.c[j];
+        }
+    __syncthreads();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double v = z[i];
         for (int j = 0; j < m; ++j) v = fma(-c[j], pj.v[j][i], v);
@@ -840,14 +846,24 @@ __global__ void fcg_orthogonalize(int64_t n, const double* z, VecSet pj, Coef pq
         pr = fma(v, r[i], pr);
     }
     const double sum[1] = {pr};
-    fem::block_sum_add<kFcgThreads, 1, 1>(sum, {pr_out});
+    fem::block_sum_add<kFcgThreads, 1, 1>(sum, {fem::part_of(pr_out)});
 }
 // x += a p, r -= a q with a = pr / pAp, rr += r.r; nothing on a breakdown (the host
 // reads the three sums after this kernel, once per iteration)
 __global__ void fcg_step(int64_t n, const double* pr, const double* pAp, double* x, const double* p, double* r,
                          const double* q, double* rr_out) {
-    if (!(*pAp > 0.0) || !isfinite(*pr)) return;
-    const double a = *pr / *pAp;
+    __shared__ double alpha;
+    __shared__ int stop;
+    if (threadIdx.x < 32) {
+        const double num = fem::parts_total(pr), den = fem::parts_total(pAp);
+        if (threadIdx.x == 0) {
+            stop = !(den > 0.0) || !isfinite(num);
+            alpha = num / den;
+        }
+    }
+    __syncthreads();
+    if (stop) return;
+    const double a = alpha;
     double rr = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         x[i] = fma(a, p[i], x[i]);
@@ -856,7 +872,7 @@ __global__ void fcg_step(int64_t n, const double* pr, const double* pAp, double*
         rr = fma(rn, rn, rr);
     }
     const double sum[1] = {rr};
-    fem::block_sum_add<kFcgThreads, 1, 1>(sum, {rr_out});
+    fem::block_sum_add<kFcgThreads, 1, 1>(sum, {fem::part_of(rr_out)});
 }
 
 }  // namespace
@@ -985,7 +1001,7 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
     };
     // r, z, 1/diag, M + 1 directions p and products q, the sums: one allocation
     double* work = nullptr;
-    cudaError_t e = alloc((void**)&work, ((size_t)(2 * M + 5) * n + kFcgSums) * 8);
+    cudaError_t e = alloc((void**)&work, ((size_t)(2 * M + 5) * n + kFcgSums * kP) * 8);
     if (e == cudaSuccess) {
         r = work;
         z = r + n;
@@ -1011,6 +1027,14 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
     const unsigned rb = (unsigned)std::min<int64_t>((n * fem::kLanesPerRow + tpb - 1) / tpb, (int64_t)sm_count() * 16);
     const unsigned vb = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 4);
     double hd[3];
+    const auto read_sums = [&](const double* from, int count) {  // totals of sums on the device
+        double h[3 * kP];
+        cudaMemcpy(h, from, (size_t)count * kP * sizeof(double), cudaMemcpyDeviceToHost);
+        for (int k = 0; k < count; ++k) {
+            hd[k] = 0.0;
+            for (int m = 0; m < kP; ++m) hd[k] += h[k * kP + m];
+        }
+    };
     const int nc = cnn ? cnn->n : 0;
     // with the V-cycle as base, a stalled learned correction is switched off
     // after kNetWindow iterations without a 10 % residual reduction and the
@@ -1037,10 +1061,10 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
     };
     if (cnn && node_density) density_channel_kernel<<<lpc_grid((int64_t)nc * nc * nc), 256>>>(nf, nc, factor,
                                                                                                 node_density, cin);
-    cudaMemset(dots, 0, kFcgSums * 8);
+    cudaMemset(dots, 0, kFcgSums * kP * 8);
     fcg_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb>>>(n, rowptr, colidx, vals, dinv);
     fcg_residual<<<rb, tpb>>>(n, rowptr, colidx, vals, b, x, r, dots);
-    cudaMemcpy(hd, dots, 2 * sizeof(double), cudaMemcpyDeviceToHost);
+    read_sums(dots, 2);
     const double bn = std::sqrt(hd[1] > 0 ? hd[1] : 1.0);
     double rn = std::sqrt(hd[0]);
     const double tol = opts->rel_tol * bn;
@@ -1062,8 +1086,8 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
             ps.v[j] = P + (int64_t)slot * n;
         }
         // dots: z.q_j of the m directions, then p.r, p.Ap and r.r
-        double* sums = dots + kMaxM;
-        cudaMemsetAsync(dots, 0, kFcgSums * 8, 0);
+        double* sums = dots + kMaxM * kP;
+        cudaMemsetAsync(dots, 0, kFcgSums * kP * 8, 0);
         for (int j = 0; j < m; ++j) cf.c[j] = pq[(it - 1 - j + (M + 1) * 4) % (M + 1)];
         if (m > 0) fcg_multi_dot<<<vb, tpb>>>(n, z, qs, m, dots);
         const int cur = it % (M + 1);
@@ -1072,15 +1096,15 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
         fcg_orthogonalize<<<vb, tpb>>>(n, z, ps, cf, m, dots, r, p, sums);
         if (mg) {
             // the level-0 stencil of the hierarchy is the CSR's operator without indices
-            if (!mg_operator(mg, p, q, sums + 1)) {
+            if (!mg_operator(mg, p, q, sums + kP)) {
                 ok = false;
                 break;
             }
         } else {
-            fcg_spmv_dot<<<rb, tpb>>>(n, rowptr, colidx, vals, p, q, sums + 1);
+            fcg_spmv_dot<<<rb, tpb>>>(n, rowptr, colidx, vals, p, q, sums + kP);
         }
-        fcg_step<<<vb, tpb>>>(n, sums, sums + 1, x, p, r, q, sums + 2);
-        cudaMemcpy(hd, sums, 3 * sizeof(double), cudaMemcpyDeviceToHost);
+        fcg_step<<<vb, tpb>>>(n, sums, sums + kP, x, p, r, q, sums + 2 * kP);
+        read_sums(sums, 3);
         const double pr = hd[0], pAp = hd[1];
         if (!(pAp > 0.0) || !std::isfinite(pr)) {
             fallback = 1;
@@ -1120,9 +1144,9 @@ static fem_gpu_status fcg_run(fem_gpu_ctx* c, const int32_t* rowptr, const int32
         fb_iters = pr.iterations;
     }
     // convergence test: the true residual of the final iterate
-    cudaMemset(dots, 0, kFcgSums * 8);
+    cudaMemset(dots, 0, kFcgSums * kP * 8);
     fcg_residual<<<rb, tpb>>>(n, rowptr, colidx, vals, b, x, r, dots);
-    cudaMemcpy(hd, dots, 2 * sizeof(double), cudaMemcpyDeviceToHost);
+    read_sums(dots, 2);
     const double true_rel = std::sqrt(hd[0]) / bn;
     cleanup();
     if (rep) {

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kCsPart * kCsRows) mg_csr_to_stencil(int n, co
     double* sv = reinterpret_cast<double*>(cs_smem);
     int32_t* sc = reinterpret_cast<int32_t*>(sv + kCsCap);
     // 32-bit throughout (3 N rows and their nonzeros are int32 in the CSR): the kernel is
-    // bound by its index operations; setup at 65^3 nodes 3.86 -> 3.72 ms
+    // bound by its index operations: 438 -> 286 us at 65^3 nodes
     const int N = n * n * n, rows = 3 * N, n2 = n * n;
     for (int r0 = blockIdx.x * kCsRows; r0 < rows; r0 += gridDim.x * kCsRows) {
         const int r1 = r0 + kCsRows < rows ? r0 + kCsRows : rows;
@@ -206,8 +206,7 @@ __device__ __forceinline__ void stencil_sweep(int n, const TS* __restrict__ S, c
     }
 }
 unsigned sweep_blocks(int64_t N) { return (unsigned)((N + 31) / 32); }
-// of a sweep that ends in a block sum: an atomic of every block to one address takes
-// 10 ns (8,583 blocks: 97 us for a sweep of 57)
+// of a sweep that ends in a block sum: two rounds of resident blocks (an atomic each)
 template <typename TV>
 unsigned sum_sweep_blocks(int64_t N) {
     return std::min<unsigned>(sweep_blocks(N), (unsigned)fem::sm_count() * Sweep<TV>::per_sm * 2);
@@ -215,24 +214,26 @@ unsigned sum_sweep_blocks(int64_t N) {
 
 // power iteration step: y = D^-1 A (a x), a = 1 / sqrt(*xx) (1 without xx: x
 // is the previous step's y, normalised here instead of in a pass of its own);
-// dots[0] += y.y (in the level's precision)
+// dots += y.y (in the level's precision; xx and dots in parts)
 template <typename TS, typename TV>
 __global__ void __launch_bounds__(Sweep<TV>::threads, Sweep<TV>::per_sm) mg_power(int n, const TS* __restrict__ S, const TV* dinv, const TV* x,
                          const double* __restrict__ xx, TV* y, double* dots) {
-    double a = 1.0;
-    if (xx) {
-        const double d = *xx;
-        a = d > 0.0 ? 1.0 / sqrt(d) : 0.0;
+    // the scale by one warp: FP64 roots and divisions in every warp took the pipe longer
+    // than the sums of the sweep (65^3 nodes 56 -> 48 us with it and the sums in parts, 33^3
+    // 17 -> 11); read behind the first barrier of the sweep
+    __shared__ TV scale;
+    if (threadIdx.x < 32) {
+        const double d = xx ? fem::parts_total(xx) : 1.0;
+        if (threadIdx.x == 0) scale = (TV)(d > 0.0 ? 1.0 / sqrt(d) : 0.0);
     }
-    const TV at = (TV)a;
     double acc = 0.0;
     stencil_sweep<TS, TV>(n, S, x, [&](int64_t t) { return dinv[t]; }, [&](int64_t t, TV d, TV s) {
-        const TV v = d * s * at;
+        const TV v = d * s * scale;
         y[t] = v;
         acc += (double)v * (double)v;
     });
     const double sum[1] = {acc};
-    fem::block_sum_add<Sweep<TV>::threads, 1, 1>(sum, {dots});
+    fem::block_sum_add<Sweep<TV>::threads, 1, 1>(sum, {fem::part_of(dots)});
 }
 
 template <typename TV>
@@ -241,7 +242,7 @@ __global__ void mg_sumsq(int64_t m, const TV* __restrict__ x, double* dots) {
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x)
         acc += (double)x[t] * (double)x[t];
     const double sum[1] = {acc};
-    fem::block_sum_add<kTpb, 1, 1>(sum, {dots});
+    fem::block_sum_add<kTpb, 1, 1>(sum, {fem::part_of(dots)});
 }
 
 template <typename TV>
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(Sweep<double>::threads, Sweep<double>::per_sm)
         acc = fma(pt, s, acc);
     });
     const double sum[1] = {acc};
-    fem::block_sum_add<Sweep<double>::threads, 1, 1>(sum, {dot});
+    fem::block_sum_add<Sweep<double>::threads, 1, 1>(sum, {fem::part_of(dot)});
 }
 
 // Chebyshev start with x = 0: r = b, d = D^-1 b / theta, x = d
@@ -772,14 +773,20 @@ void power_iterate(const fem_mg::Level& L, const TS* S, const TV* dinv, double* 
     mg_sumsq<TV><<<sb, kTpb>>>(3 * L.N, x, pd);
     for (int it = 0; it < iters; ++it) {
         mg_power<TS, TV><<<sum_sweep_blocks<TV>(L.N), Sweep<TV>::threads>>>(
-            L.n, S, dinv, x, it ? pd + it : nullptr, y, pd + it + 1);
+            L.n, S, dinv, x, it ? pd + it * fem::kSumParts : nullptr, y,
+            pd + (it + 1) * fem::kSumParts);
         std::swap(x, y);
     }
 }
-double power_lambda(const double* h, int iters) {
-    double xn = std::sqrt(h[0]), lam = 0.0;
+double power_lambda(const double* parts, int iters) {
+    const auto norm = [&](int k) {
+        double v = 0.0;
+        for (int m = 0; m < fem::kSumParts; ++m) v += parts[k * fem::kSumParts + m];
+        return std::sqrt(v);
+    };
+    double xn = norm(0), lam = 0.0;
     for (int it = 0; it < iters; ++it) {
-        const double yn = std::sqrt(h[it + 1]);
+        const double yn = norm(it + 1);
         lam = yn / xn;
         if (!(yn > 0.0)) break;
         xn = 1.0;
@@ -851,7 +858,7 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
     const size_t iters = (size_t)o.power_iters + 1;
     fem_mg::Arena& ar = g->arena;
     ar.reserve(&g->dots, 4);
-    ar.reserve(&g->pdots, iters * ns.size());
+    ar.reserve(&g->pdots, iters * ns.size() * fem::kSumParts);
     ar.reserve(&g->err, 1);
     for (size_t l = 0; l < ns.size(); ++l) {
         fem_mg::Level& L = g->lv[l];
@@ -913,7 +920,7 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
     }
     // smoother data: diagonal, FP32 copies, lambda_max(D^-1 A) by power iteration
     // (norms on the device, read once for all levels)
-    cudaMemset(g->pdots, 0, iters * ns.size() * sizeof(double));
+    cudaMemset(g->pdots, 0, iters * ns.size() * fem::kSumParts * sizeof(double));
     for (size_t l = 0; l + 1 < g->lv.size(); ++l) {
         fem_mg::Level& L = g->lv[l];
         const unsigned vb = blocks_for(3 * L.N, kTpb);
@@ -925,8 +932,8 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
         mg_random<<<vb, kTpb>>>(3 * L.N, 0x5EEDULL + l, px);
         // FP64 levels iterate on the FP64 stencil; FP32 levels on their FP32 copy
         // (the smoothing interval needs lambda_max to a few digits only)
-        if (L.fp32) power_iterate<float, float>(L, L.S32, L.dinv32, px, py, o.power_iters, g->pdots + l * iters);
-        else power_iterate<double, double>(L, L.S, L.dinv, px, py, o.power_iters, g->pdots + l * iters);
+        if (L.fp32) power_iterate<float, float>(L, L.S32, L.dinv32, px, py, o.power_iters, g->pdots + l * iters * fem::kSumParts);
+        else power_iterate<double, double>(L, L.S, L.dinv, px, py, o.power_iters, g->pdots + l * iters * fem::kSumParts);
     }
     // coarsest level: dense inverse
     fem_mg::Level& LC = g->lv.back();
@@ -939,14 +946,14 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
         std::swap(from, to);
     }
     if (from != g->ainv) cudaMemcpyAsync(g->ainv, from, g->m * g->m * sizeof(double), cudaMemcpyDeviceToDevice, 0);
-    std::vector<double> norms(iters * ns.size(), 0.0);
+    std::vector<double> norms(iters * ns.size() * fem::kSumParts, 0.0);
     if (cudaMemcpy(norms.data(), g->pdots, norms.size() * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess ||
         cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess) {
         delete g;
         return fail(c, FEM_GPU_CUDA_ERROR, "multigrid setup");
     }
     for (size_t l = 0; l + 1 < g->lv.size(); ++l) {
-        const double lam = power_lambda(norms.data() + l * iters, o.power_iters);
+        const double lam = power_lambda(norms.data() + l * iters * fem::kSumParts, o.power_iters);
         g->lv[l].lmax = lam;
         if (!(lam > 0.0) || !std::isfinite(lam)) {
             delete g;

@@ -41,4 +41,15 @@ __device__ __forceinline__ void block_sum_add(const double (&v)[NV], double* con
     if (lane == 0) atomicAdd(o, s);
 }
 
+// A sum over the grid is kept in parts: an FP64 atomic of every block to one address
+// takes 10 ns.  part_of: where the block adds; parts_total: the total, by a whole warp.
+constexpr int kSumParts = 8;
+__device__ __forceinline__ double* part_of(double* sum) { return sum + blockIdx.x % kSumParts; }
+__device__ __forceinline__ double parts_total(const double* sum) {
+    double t = sum[threadIdx.x % kSumParts];
+#pragma unroll
+    for (int o = kSumParts / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
 }  // namespace fem
