@@ -2,8 +2,10 @@
 // stream has ended (programmatic dependent launch).
 //
 // The kernel must call cudaGridDependencySynchronize() before it touches what earlier
-// kernels write, and, if it triggers a dependent launch itself, only after that: a
-// later kernel may then take everything before its predecessor as complete.  overlap
+// kernels write, and, if it triggers a dependent launch itself, only after that (or it is
+// never launched with overlap): a later kernel may then take everything before its
+// predecessor as complete.  Data that the predecessor writes is read with plain loads,
+// not __ldg or const __restrict__, which may move ahead of the wait.  overlap
 // is set only where the previous operation of the stream is a kernel of this library,
 // one of another library may trigger before its inputs are complete.
 #pragma once
