@@ -26,9 +26,9 @@
 // weights, facet corners); the rest stays with the general kernel.
 //
 // Measured on GB300, batched assembly with residual, general kernel -> here:
-// 64^3 cells cut by 40 spheres, linear splines 32.5 -> 4.60 ms (ghost 27, cut
+// 64^3 cells cut by 40 spheres, linear splines 32.5 -> 4.34 ms (ghost 27, cut
 // 24, uncut 22, interface 19 % of it); 22^3, 12 spheres, quadratic splines 7.93
-// -> 0.885 ms.  The general kernel spent 27 k FP64 products on a ghost face (now
+// -> 0.870 ms.  The general kernel spent 27 k FP64 products on a ghost face (now
 // 4 k) and 180 k on an interface cluster (now 19 k).  Bound: the L2's FP64
 // atomics (576 per cell, 1,408 per ghost face, 2,304 per interface) and the FP64
 // pipe about equally.
@@ -65,6 +65,7 @@ struct BrickArgs {
     double lam_c, mu_c, alpha, beta;
     double value[3], thickness;  // boundary facets
     const double* tab;     // uncut: 63 reference sums; ghost: kGhostTab per face
+    const double* geo;     // reciprocals and roots of the cells (kGeoUncut, kGeoGhost per object)
     const int64_t* off;    // integration cells / facets of an object
     const double* x;       // their vertex coordinates
     const double* xi;      // their parametric coordinates
@@ -152,11 +153,17 @@ struct Scatter {
 
 // ---------------------------------------------------------------------------
 // the 63 sums of a bulk object, times mu, into q (warp-wide); index tables in tab
+// Per object, computed once when the set is classified, because a division or a root
+// takes a warp 12 to 20 instructions of the FP64 pipe, a sixth of an uncut cell (64^3
+// cells, 40 spheres 4.60 -> 4.34 ms for the batch): the
+// reciprocal half lengths of an uncut cell; of both cells of a ghost face, then
+// sqrt(16 J_t1 J_t2 / pi) and J_t1 J_t2.
+constexpr int kGeoUncut = 3, kGeoGhost = 8;
 __device__ void uncut_sums(const BrickArgs& p, int64_t e, double* q, int lane) {
     const double* X = p.xe + e * 24;
     // lane d = 0..2: half length along axis d and its reciprocal
     const int d = lane % 3;
-    const double j = 0.5 * (__ldg(X + 18 + d) - __ldg(X + d)), r = 1.0 / j;
+    const double j = 0.5 * (__ldg(X + 18 + d) - __ldg(X + d)), r = __ldg(p.geo + e * kGeoUncut + d);
     const double j0 = shfl(j, 0), j1 = shfl(j, 1), j2 = shfl(j, 2);
     // scale of the component pair t = 0..5 (xx, yy, zz, xy, xz, yz) on lane t:
     // E mu detJ / (J_i J_j)
@@ -311,14 +318,13 @@ __device__ GhostCoef ghost_coef(const BrickArgs& p, int64_t e, int face, int s, 
     c.k = face >> 1;
     c.t1 = c.k == 0 ? 1 : 0;
     c.t2 = c.k == 2 ? 1 : 2;
-    // reciprocal half lengths: lane 3 side + axis (one division for the warp)
+    // reciprocal half lengths: lane 3 side + axis
     const int lane = threadIdx.x & 31, q = lane % 6;
-    const double* XL = p.xe + e * 48;
-    const double rr = 2.0 / (XL[(q / 3) * 24 + 18 + q % 3] - XL[(q / 3) * 24 + q % 3]);
+    const double* geo = p.geo + e * kGeoGhost;
+    const double rr = __ldg(geo + q);
     const double rk = shfl(rr, s * 3 + c.k), r1 = shfl(rr, s * 3 + c.t1), r2 = shfl(rr, s * 3 + c.t2);
     const double ok = shfl(rr, s2 * 3 + c.k), o1 = shfl(rr, s2 * 3 + c.t1), o2 = shfl(rr, s2 * 3 + c.t2);
-    const double area4 = 0.25 * (XL[18 + c.t1] - XL[c.t1]) * (XL[18 + c.t2] - XL[c.t2]);  // J_t1 J_t2
-    const double gam = p.alpha * sqrt(16.0 * area4 / 3.14159265358979323846) * area4 * (s == s2 ? scale : -scale);
+    const double gam = p.alpha * __ldg(geo + 6) * __ldg(geo + 7) * (s == s2 ? scale : -scale);
     if (p.normal_field) {
         c.kk = c.kk_t = gam * p.E[e] * rk * ok;
         c.c11 = c.c22 = c.lam1 = c.lam2 = c.mu1 = c.mu2 = c.tk1 = c.tk2 = 0.0;
@@ -984,6 +990,7 @@ int ghost_face(const SetData& s, int64_t i) {
 void brick_classify(const fem_gpu_ctx* c, SetData& s) {
     s.fast.clear();
     s.fmap.clear();
+    s.fgeo.clear();
     const int sides = s.kind == 2 ? 2 : 1;
     if (c->dim != 3 || c->shape != FEM_GPU_SHAPE_RECTANGULAR || s.neq == 0) return;
     if (!s.node_rho.empty()) return;
@@ -1000,6 +1007,8 @@ void brick_classify(const fem_gpu_ctx* c, SetData& s) {
     if (iface && (s.nfv != 3 || gauss_rule(s.dside.integration_rule).n > 7)) return;
     s.fast.assign(s.neq, 0);
     s.fmap.assign((size_t)s.neq * sides * W, 0);
+    const int geo = s.kind == 0 && s.ig_off.empty() ? kGeoUncut : s.kind == 2 && !iface ? kGeoGhost : 0;
+    s.fgeo.assign((size_t)s.neq * geo, 0.0);
     const auto classify = [&](int64_t i) {
         bool ok = true;
         for (int k = 0; k < sides && ok; ++k) {
@@ -1011,6 +1020,8 @@ void brick_classify(const fem_gpu_ctx* c, SetData& s) {
             s.fast[i] = (uint8_t)(kFastSide + s.ordinal[i]);
         } else if (s.kind == 0) {
             s.fast[i] = kFastBulk;
+            for (int d = 0; !s.fgeo.empty() && d < 3; ++d)
+                s.fgeo[i * kGeoUncut + d] = 1.0 / (0.5 * (s.xe[i * 24 + 18 + d] - s.xe[i * 24 + d]));
         } else if (iface) {
             const int64_t a = s.fc_off[i] * 9, b = s.fc_off[i + 1] * 9;
             if (std::equal(&s.xe[i * 48], &s.xe[i * 48] + 24, &s.xe[i * 48] + 24) &&
@@ -1018,7 +1029,14 @@ void brick_classify(const fem_gpu_ctx* c, SetData& s) {
                 s.fast[i] = kFastInterface;
         } else {
             const int face = ghost_face(s, i);
-            if (face >= 0) s.fast[i] = (uint8_t)(kFastGhost + face);
+            if (face < 0) return;
+            s.fast[i] = (uint8_t)(kFastGhost + face);
+            const double* X = &s.xe[i * 48];
+            double* g = &s.fgeo[i * kGeoGhost];
+            for (int q = 0; q < 6; ++q) g[q] = 2.0 / (X[(q / 3) * 24 + 18 + q % 3] - X[(q / 3) * 24 + q % 3]);
+            const int k = face >> 1, t1 = k == 0 ? 1 : 0, t2 = k == 2 ? 1 : 2;
+            g[7] = 0.25 * (X[18 + t1] - X[t1]) * (X[18 + t2] - X[t2]);
+            g[6] = std::sqrt(16.0 * g[7] / 3.14159265358979323846);
         }
     };
     const int nt = (int)std::min<int64_t>(std::max(1u, std::thread::hardware_concurrency()), 1 + s.neq / 4096);
@@ -1031,6 +1049,7 @@ void brick_classify(const fem_gpu_ctx* c, SetData& s) {
     if (std::none_of(s.fast.begin(), s.fast.end(), [](uint8_t f) { return f != 0; })) {
         s.fast.clear();
         s.fmap.clear();
+        s.fgeo.clear();
     }
 }
 
@@ -1108,7 +1127,11 @@ fem_gpu_status brick_upload(fem_gpu_ctx* c, SetData& s) {
             }
         }
     }
-    // tables, list, kinds and maps in one buffer
+    // tables, reciprocals, list, kinds and maps in one buffer
+    s.ftab_count = tab.size();
+    tab.insert(tab.end(), s.fgeo.begin(), s.fgeo.end());
+    s.fgeo.clear();
+    s.fgeo.shrink_to_fit();
     const size_t nt = tab.size() * sizeof(double), nl = s.flist.size() * sizeof(int32_t);
     std::vector<uint8_t> all(nt + nl + s.fast.size() + s.fmap.size());
     if (nt) std::memcpy(all.data(), tab.data(), nt);
@@ -1152,6 +1175,7 @@ fem_gpu_status brick_launch(fem_gpu_ctx* c, const SetData& s, int64_t first, int
     a.gw = (const double*)s.d_gw.p;
     a.ngp = s.ngp;
     a.tab = (const double*)data;
+    a.geo = a.tab + s.ftab_count;
     a.rowptr = (const int32_t*)c->d_rowptr.p;
     a.ulen = (const int32_t*)c->d_ulen.p;
     a.nu = c->num_used;

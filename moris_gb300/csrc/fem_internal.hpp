@@ -92,7 +92,8 @@ struct SetData {
     std::vector<uint8_t> fast, fmap;  // brick kernels (fem_brick.cu): kind per equation object, column maps
     std::vector<int32_t> flist;       // their equation objects
     DeviceBuf d_fast;                 // their tables (ftab_bytes), list, kinds and maps
-    size_t ftab_bytes = 0;
+    size_t ftab_bytes = 0, ftab_count = 0;  // doubles in front of the list; of them tables
+    std::vector<double> fgeo;               // reciprocals and roots, until they are uploaded
     bool lattice = false;   // the set covers a tensor lattice (fem_lattice.cu)
     DeviceBuf d_ptab, d_pfacet;  // side sets of plane lattices: products of the splines, facets
     double side_wsum = 0.0;      // their sum of the rule's weights
