@@ -746,12 +746,14 @@ __global__ void __launch_bounds__(kProjThreads, kProjCtas) lattice_project(ProjA
         const bool have = z >= 0 && z < p.nn[2];
         if (have) {
             if (xiy <= wy) {
+                // (plain loads: the kernel that writes the stencil may still run when this
+                // one starts, see fem_launch.cuh)
                 double v[kPX + 1][3];
                 const double* s0 = xs + z * layer;
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
 #pragma unroll
-                    for (int i = 0; i <= kPX; ++i) v[i][k] = xin >> i & 1 ? __ldg(s0 + i) : 0.0;
+                    for (int i = 0; i <= kPX; ++i) v[i][k] = xin >> i & 1 ? s0[i] : 0.0;
                     s0 += 9 * plane;
                 }
                 double* o = X + xiy * kPX * 135 + xl;
