@@ -552,10 +552,11 @@ struct ClusterLaunch {
         cfg.stream = st;
         cfg.attrs = at;
         cfg.numAttrs = 1;
+        // the attributes belong to the function: the same values whatever the system, because
+        // other threads launch theirs between these lines and this one's launch
         const bool ok =
             cudaFuncSetAttribute(k_cluster_cg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaFuncSetAttribute(k_cluster_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem) ==
-                cudaSuccess &&
+            cudaFuncSetAttribute(k_cluster_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) == cudaSuccess &&
             cudaOccupancyMaxActiveClusters(&clusters, k_cluster_cg, &cfg) == cudaSuccess && clusters > 0;
         if (!ok) cudaGetLastError();
         return ok;
