@@ -1105,9 +1105,7 @@ struct Lattice {
     DeviceBuf jac;     // half edge lengths and their reciprocals
     DeviceBuf S, vec;  // block stencil; quadratic splines: nodal vectors
     DeviceBuf Q;       // density sets: element sums
-    // the last use of S, vec and Q: a call on another stream waits for it
-    cudaEvent_t done = nullptr;
-    cudaStream_t last = nullptr;
+    cudaEvent_t done = nullptr;  // the last use of S, vec and Q
 };
 
 void dfree(DeviceBuf& b) {
@@ -1362,7 +1360,6 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
     if (rho && e == cudaSuccess) e = cudaMemsetAsync(K->Q.p, 0, K->Q.bytes, st);
     if (K->S.p && e == cudaSuccess) e = cudaEventCreateWithFlags(&K->done, cudaEventDisableTiming);
     if (K->done && e == cudaSuccess) e = cudaEventRecord(K->done, st);
-    K->last = st;
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? FEM_GPU_OK
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice data: ") + cudaGetErrorString(e));
@@ -1434,9 +1431,12 @@ fem_gpu_status plane_assemble(fem_gpu_ctx* c, const Lattice& L, const SetData& s
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice launch: ") + cudaGetErrorString(e));
 }
 
-// The workspaces of one call.  A matrix-free product returns before it has run, so a
-// call on another stream waits for the one before it; a captured call, which may be
-// replayed beside any other, takes memory of its own (nodes of the graph).
+// The workspaces of one call.  A matrix-free product returns before it has run, so every
+// call waits for the one before it: the same handle need not be the same stream (the
+// per-thread default stream is one handle for all threads, and that of a destroyed stream
+// is given out again), and on the stream of the call before the wait is empty.  A captured
+// call, which may be replayed beside any other, takes memory of its own (nodes of the
+// graph).
 struct LatticeWork {
     Lattice& L;
     cudaStream_t st;
@@ -1455,7 +1455,7 @@ struct LatticeWork {
             if (L.vec.p && e == cudaSuccess) e = cudaMallocAsync(&vec, L.vec.bytes, st);
             if (L.Q.p && e == cudaSuccess) e = cudaMallocAsync(&Q, L.Q.bytes, st);
             if (Q && e == cudaSuccess) e = cudaMemsetAsync(Q, 0, L.Q.bytes, st);
-        } else if (L.last != st) {
+        } else {
             e = cudaStreamWaitEvent(st, L.done, 0);
         }
     }
@@ -1465,7 +1465,6 @@ struct LatticeWork {
                 if (p) cudaFreeAsync(p, st);
         } else if (L.done) {
             cudaEventRecord(L.done, st);
-            L.last = st;
         }
     }
 };
