@@ -609,8 +609,11 @@ extern "C" fem_gpu_status fem_gpu_pcg(fem_gpu_ctx* c, const int32_t* rowptr, con
     const unsigned row_blocks = (unsigned)((n * fem::kLanesPerRow + tpb - 1) / tpb);
     const unsigned spmv_blocks = (unsigned)std::min<int64_t>(row_blocks, (int64_t)sm_count() * 16);
     const unsigned vec_blocks = (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, (int64_t)sm_count() * 8);
-    // one cluster where its shared memory holds the rows of the model's graph
-    const int width = c->dim * (c->ulen.empty() ? 0 : *std::max_element(c->ulen.begin(), c->ulen.end()));
+    // one cluster where its shared memory holds the rows of the model's graph (their
+    // longest is sought only where the rows are few enough)
+    int width = 0;
+    if (n <= kClusterCtas * kClusterRows && !c->ulen.empty())
+        width = c->dim * *std::max_element(c->ulen.begin(), c->ulen.end());
     ClusterLaunch cluster;
     const bool clustered = cluster.init(n, width, sm);
     k_diag_inv<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, sm>>>(n, rowptr, colidx, vals, dinv, opts->preconditioner == 1,
