@@ -640,7 +640,6 @@ struct fem_mg {
     int64_t m = 0;
     fem_mg_opts o{};
     double setup_seconds = 0.0;
-    double* dots = nullptr;
     double* pdots = nullptr;  // power-iteration norms (power_iters + 1)
     int* err = nullptr;
     // all arrays in one allocation (45 of their own cost a millisecond to make and
@@ -857,7 +856,6 @@ fem_gpu_status fem_mg_create(fem_gpu_ctx* c, const int32_t* rowptr, const int32_
     g->lv.resize(ns.size());
     const size_t iters = (size_t)o.power_iters + 1;
     fem_mg::Arena& ar = g->arena;
-    ar.reserve(&g->dots, 4);
     ar.reserve(&g->pdots, iters * ns.size() * fem::kSumParts);
     ar.reserve(&g->err, 1);
     for (size_t l = 0; l < ns.size(); ++l) {
