@@ -1140,6 +1140,13 @@ fem_gpu_status brick_upload(fem_gpu_ctx* c, SetData& s) {
     std::memcpy(all.data() + nt + nl + s.fast.size(), s.fmap.data(), s.fmap.size());
     s.ftab_bytes = nt;
     cudaError_t e = upload(s.d_fast, all, st);
+    if (e == cudaErrorMemoryAllocation) {  // the general kernels need none of it
+        cudaGetLastError();
+        s.fast.clear();
+        s.fmap.clear();
+        s.flist.clear();
+        return FEM_GPU_OK;
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? FEM_GPU_OK
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("brick data: ") + cudaGetErrorString(e));

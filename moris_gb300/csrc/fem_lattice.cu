@@ -1347,9 +1347,9 @@ fem_gpu_status lattice_finalize(fem_gpu_ctx* c) {
         buf[k]->bytes = want[k] * sizeof(double);
         bytes += (buf[k]->bytes + 255) / 256 * 256;
     }
-    if (e == cudaSuccess && cudaMalloc(&K->mem.p, std::max<size_t>(bytes, 256)) != cudaSuccess) {
+    if (e == cudaSuccess) e = cudaMalloc(&K->mem.p, std::max<size_t>(bytes, 256));
+    if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        K->mem.p = nullptr;
         cudaStreamSynchronize(st);
         lattice_release(c);
         return FEM_GPU_OK;
