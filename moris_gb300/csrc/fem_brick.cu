@@ -184,13 +184,16 @@ __device__ void uncut_sums(const BrickArgs& p, int64_t e, double* q, int lane) {
 
 // cut cluster: the moments of its points, then the sums.  A lane forms one
 // point (w*, xi), lane l < 27 owns moment l = (p, q, r) and adds the 32 points of
-// the round from shared memory, one FMA each.
+// the round from shared memory, one FMA each, in eight sums: one sum over the 96 to 240
+// points of a cluster carried a rounding error of 7e-16, eight 1e-16.
 constexpr int kPt = 13;  // doubles per staged point: x^p y^q (9), w z^r (3), padding
 __device__ void cut_sums(const BrickArgs& p, int64_t e, double* st, double* q, int lane) {
     const int64_t c0 = p.off[e];
     const int np = (int)(p.off[e + 1] - c0) * p.ngp;
     const int l = lane < 27 ? lane : 0;
-    double acc = 0.0;
+    double acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.0;
     for (int q0 = 0; q0 < np; q0 += 32) {
         const int t = q0 + lane;
         if (t < np) {
@@ -237,12 +240,15 @@ __device__ void cut_sums(const BrickArgs& p, int64_t e, double* st, double* q, i
         const int n = min(32, np - q0);
         const double* o = st + l % 9;
         const double* z = st + 9 + l / 9;
-#pragma unroll 4
-        for (int k = 0; k < n; ++k) acc = fma(o[k * kPt], z[k * kPt], acc);
+        int k = 0;
+        for (; k + 8 <= n; k += 8)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] = fma(o[(k + j) * kPt], z[(k + j) * kPt], acc[j]);
+        for (; k < n; ++k) acc[0] = fma(o[k * kPt], z[k * kPt], acc[0]);
         __syncwarp();
     }
     double* M = st;  // the moments
-    if (lane < 27) M[lane] = acc;
+    if (lane < 27) M[lane] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
     __syncwarp();
     const double* X = p.xe + e * 24;
     const int d = lane % 3;
