@@ -402,7 +402,9 @@ __device__ void interface_matrices(const BrickArgs& p, int64_t e, double* sm, do
     const int l = lane < 27 ? lane : 0;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     double meas = 0.0, wsum = 0.0;
-    for (int k = 0; k < ngp; ++k) wsum += __ldg(p.gw + k);
+    // from the last point to the first, whose weight is the largest: the other way round
+    // the seven weights' sum is an ulp low in every facet and with it the penalty
+    for (int k = ngp - 1; k >= 0; --k) wsum += __ldg(p.gw + k);
     for (int b0 = 0; b0 < nf; b0 += 32) {
         // facet normals and measures: detJ = |t1 x t2| / 2 of a TRI3
         if (b0 + lane < nf) {
@@ -453,8 +455,9 @@ __device__ void interface_matrices(const BrickArgs& p, int64_t e, double* sm, do
             for (int k = 0; k < m; ++k) {
                 const double* o = st + k * ngp * kPt + l % 9;
                 const double* z = st + k * ngp * kPt + 9 + l / 9;
-                double s = o[0] * z[0];
-                for (int g2 = 1; g2 < ngp; ++g2) s = fma(o[g2 * kPt], z[g2 * kPt], s);
+                int g2 = ngp - 1;
+                double s = o[g2 * kPt] * z[g2 * kPt];
+                while (--g2 >= 0) s = fma(o[g2 * kPt], z[g2 * kPt], s);
                 const double* n = nrm + (r0 + k) * 4;
                 acc[0] = fma(n[0], s, acc[0]);
                 acc[1] = fma(n[1], s, acc[1]);

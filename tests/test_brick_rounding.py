@@ -166,7 +166,8 @@ def _part(sets, part):
         [(k, a) for k, a in sets if a.get("iwg") == mg.IWG_STRUC_LINEAR_INTERFACE_SYMMETRIC_NITSCHE]
 
 
-@pytest.mark.parametrize("order,n,spheres,geometry,part,units", [(1, 9, 4, 3, "cut", 2.5), (2, 5, 2, 5, "cut", 2.5)])
+@pytest.mark.parametrize("order,n,spheres,geometry,part,units", [(1, 9, 4, 3, "cut", 2.5), (2, 5, 2, 5, "cut", 2.5),
+                                                               (1, 9, 4, 3, "interface", 2.1)])
 def test_values_against_extended_precision(order, n, spheres, geometry, part, units):
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
