@@ -167,7 +167,7 @@ def _part(sets, part):
 
 
 @pytest.mark.parametrize("order,n,spheres,geometry,part,units", [(1, 9, 4, 3, "cut", 2.5), (2, 5, 2, 5, "cut", 2.5),
-                                                               (1, 9, 4, 3, "interface", 2.1)])
+                                                               (1, 9, 4, 3, "interface", 2.1), (1, 9, 4, 3, "all", 2.5)])
 def test_values_against_extended_precision(order, n, spheres, geometry, part, units):
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
