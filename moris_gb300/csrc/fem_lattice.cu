@@ -1431,12 +1431,14 @@ fem_gpu_status plane_assemble(fem_gpu_ctx* c, const Lattice& L, const SetData& s
                             : fail(c, FEM_GPU_CUDA_ERROR, std::string("lattice launch: ") + cudaGetErrorString(e));
 }
 
-// The workspaces of one call.  A matrix-free product returns before it has run, so every
-// call waits for the one before it: the same handle need not be the same stream (the
-// per-thread default stream is one handle for all threads, and that of a destroyed stream
-// is given out again), and on the stream of the call before the wait is empty.  A captured
-// call, which may be replayed beside any other, takes memory of its own (nodes of the
-// graph).
+// The workspaces of one call.  A matrix-free product returns before it has run, so a call
+// waits for the one before it, whatever its stream: a handle does not name a stream (that
+// of a destroyed stream is given out again), and on the stream of the call before the wait
+// is empty.  Memory of its own, instead, has a captured call, which may be replayed beside
+// any other (nodes of the graph), and a product on the per-thread default stream, one handle
+// for a stream of every thread that goes with its thread: ordered by events, products of two
+// threads that ended while they were pending left cudaDeviceSynchronize waiting.  (An
+// assembly has run when it returns.)
 struct LatticeWork {
     Lattice& L;
     cudaStream_t st;
@@ -1448,7 +1450,7 @@ struct LatticeWork {
         if (!L.done) return;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cudaGetLastError();
-        if (cs == cudaStreamCaptureStatusActive) {
+        if (cs == cudaStreamCaptureStatusActive || (st == cudaStreamPerThread && !stencil)) {
             shared = false;
             S = vec = Q = nullptr;
             if (L.S.p && stencil) e = cudaMallocAsync(&S, L.S.bytes, st);

@@ -1,6 +1,6 @@
 """Matrix-free products of one lattice model from two threads in turn, each on its
 per-thread default stream.  Both streams have the same handle, so the model's workspaces
-cannot be ordered by comparing handles."""
+cannot be ordered by comparing handles.  A thread ends only when its stream has run."""
 import threading
 
 import pytest
@@ -40,6 +40,7 @@ def test_products_on_the_per_thread_streams_of_two_threads(shape, density):
                 errors.append(e)
             finally:
                 turn[1 - k].release()
+        torch.cuda.ExternalStream(PER_THREAD_STREAM).synchronize()
 
     threads = [threading.Thread(target=products, args=(k,)) for k in (0, 1)]
     for t in threads:
