@@ -823,7 +823,8 @@ def main():
                      "flops_per_element": flops / nc, "kernel_ms": ms_kernel,
                      "fp64_tensor_probe_tflops": {"dmma": dmma_alone, "dmma_plus_dfma": dmma_mixed}},
         "assembly_path": "tensor lattice (block stencil, axis-wise projection); host buffers: element loop",
-        "kernel_variant": {"index": variant[0], "name": variant[2], "tuned_ms": variant[1]},
+        "element_loop_variant": {"index": variant[0], "name": variant[2], "tuned_ms": variant[1],
+                                 "use": "host-buffer assembly (e2e)"},
         "jv": {"ms_per_apply": ms_jv, "elements_per_s": nc / (ms_jv * 1e-3), "rel_err_vs_csr": jv_err},
         "setup_seconds": setup_s,
     }

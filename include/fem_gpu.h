@@ -386,7 +386,9 @@ fem_gpu_status fem_gpu_add_side_set(fem_gpu_ctx* ctx, const fem_gpu_side_set_des
 fem_gpu_status fem_gpu_add_double_side_set(fem_gpu_ctx* ctx, const fem_gpu_double_side_set_desc* desc,
                                            int32_t* set_index);
 /* host-side MSI work (adof numbering, element T, sparsity, scatter maps)
-   plus the upload of everything the kernels read */
+   plus the upload of everything the kernels read and the workspaces of the
+   model (tensor lattices: up to 306 doubles per node, for products alone as
+   well; a device without room for them keeps the element loop) */
 fem_gpu_status fem_gpu_finalize(fem_gpu_ctx* ctx);
 /* like fem_gpu_finalize but host side only (no device allocation) */
 fem_gpu_status fem_gpu_finalize_host(fem_gpu_ctx* ctx);
@@ -622,9 +624,16 @@ fem_gpu_status fem_gpu_fcg_mg(fem_gpu_ctx* ctx, const int32_t* rowptr, const int
    fallback, default 200) of fem_gpu_fcg / fem_gpu_fcg_mg; process-wide */
 fem_gpu_status fem_gpu_fcg_config(int32_t depth, int32_t window);
 
-/* autotuner: times every kernel variant of each bulk set on (up to
-   max_elements, <= 0 = all) of its elements, assembling into scratch
-   buffers, and keeps the fastest per set.  Setup-time call; optional. */
+/* autotuner of the element loop: times every variant of it for each bulk set
+   on (up to max_elements, <= 0 = all) of its elements, assembling into
+   scratch buffers, and keeps the fastest per set.  Setup-time call; optional.
+   The loop assembles what has no kernels of its own: refined or truncated
+   meshes, small models, element outputs, quadratic splines into host buffers.
+   fem_gpu_assemble takes tensor lattices and linear brick cells through other
+   kernels, which have no variants: for those sets the variant and the time
+   that fem_gpu_get_variant gives are not those of the assembly.
+   fem_gpu_set_variant pins a set to the element loop with that variant, on
+   every path that the loop can take. */
 fem_gpu_status fem_gpu_autotune(fem_gpu_ctx* ctx, int64_t max_elements);
 fem_gpu_status fem_gpu_get_variant(const fem_gpu_ctx* ctx, int32_t set, int32_t* variant, double* tuned_ms,
                                    const char** name);
