@@ -26,9 +26,9 @@
 // weights, facet corners); the rest stays with the general kernel.
 //
 // Measured on GB300, batched assembly with residual, general kernel -> here:
-// 64^3 cells cut by 40 spheres, linear splines 32.5 -> 4.34 ms (ghost 27, cut
+// 64^3 cells cut by 40 spheres, linear splines 32.5 -> 4.36 ms (ghost 27, cut
 // 24, uncut 22, interface 19 % of it); 22^3, 12 spheres, quadratic splines 7.93
-// -> 0.870 ms.  The general kernel spent 27 k FP64 products on a ghost face (now
+// -> 0.869 ms.  The general kernel spent 27 k FP64 products on a ghost face (now
 // 4 k) and 180 k on an interface cluster (now 19 k).  Bound: the L2's FP64
 // atomics (576 per cell, 1,408 per ghost face, 2,304 per interface) and the FP64
 // pipe about equally.

@@ -23,13 +23,13 @@
 // per basis for the projection, 750 operations per node for the stencil.
 //
 // Measured on GB300 against the element loop (whole calls, residual included):
-// 64^3 quadratic 7.75 -> 2.25 ms, 15 x 13 x 11 quadratic 120 -> 79 us, 96^3 density set
+// 64^3 quadratic 7.75 -> 2.21 ms, 15 x 13 x 11 quadratic 120 -> 78 us, 96^3 density set
 // with linear splines 13.4 -> 2.50 ms, matrix-free product of 48 x 47 x 45 quadratic
 // cells 969 -> 76 us.  Small models keep the element loop (lattice_pays).
 //
 // Cells of any shape on the same lattice of nodes (FEM_GPU_SHAPE_GENERAL): the cells
 // add their matrices to the block stencil (fem_hex.cuh), or to the CSR for linear
-// splines, and the projection is the same.  26 x 23 x 21 quadratic 699 -> 534 us (hex
+// splines, and the projection is the same.  26 x 23 x 21 quadratic 699 -> 531 us (hex
 // 371, projection 128); 26^3 linear 467 -> 294 us, matrix-free products 401 -> 206
 // (linear) and 622 -> 264 us.
 //
